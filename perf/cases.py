@@ -336,11 +336,13 @@ def work(case):
 
 
 def tolerance(case):
-    # bf16 operands, 32-bit sums.  Measured against 64 bits: 0.0002 to 0.0023 (train base, score); the same speech step twice, with
-    # atomic sums in another order: 0.0026, single values 0.35 of the root mean square; a search with 2^-9 of noise on every weight:
-    # scores 0.0016 apart, the same words.
-    if case["kind"] in ("train_text", "train_audio"):
-        return {"rel": 0.01, "max": 0.9}
+    # bf16 operands, 32-bit sums.  Measured: text models against 64 bits 0.0002 to 0.0024; the speech models' gradients 0.011 apart
+    # (single values 0.77 of the root mean square) between two orders of the 32-bit sums in a few of the forward products, for their 36
+    # layers pass the last bit of bf16 on; a search with 2^-9 of noise on every weight: scores 0.0016 apart, the same words.
+    if case["kind"] == "train_audio":
+        return {"rel": 0.03, "max": 0.99}
+    if case["kind"] == "train_text":
+        return {"rel": 0.015, "max": 0.9}
     return {"rel": 0.01, "differ": 0.005}
 
 
