@@ -176,8 +176,12 @@ class _GraphedStep:
 
     def _body(self, ban_eos: bool):
         from .. import ops
-        hidden = self.model.decoder.step_static(self.tok, self.pos_t, self.state)
-        logits = self.model.generator(hidden)
+        ops.ext().set_step_overlap(True)        # this thread's launches, until the step's last GEMM
+        try:
+            hidden = self.model.decoder.step_static(self.tok, self.pos_t, self.state)
+            logits = self.model.generator(hidden)
+        finally:
+            ops.ext().set_step_overlap(False)
         if logits.dtype not in (torch.float32, torch.bfloat16):
             logits = logits.float()
         ts, ti, _ = ops.ext().beam_topk(logits, self.scores, self.force, self.K, self.cfg.pad, self.cfg.eos, ban_eos)

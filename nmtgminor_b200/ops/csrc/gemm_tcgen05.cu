@@ -373,6 +373,8 @@ namespace b200 {
 const char* launch_gemm_pair(const GemmDesc* d, const GemmArgs& a, int bn, cudaStream_t stream);
 const char* launch_gather_copy(const GemmDesc* d, cudaStream_t stream);
 bool plan_pair_gather(const GemmDesc* d, int bn, GatherArgs* g);
+bool skinny_takes(const GemmDesc* d, int sms);
+const char* launch_gemm_skinny(const GemmDesc* d, int sms, cudaStream_t stream);
 }
 using namespace b200;
 
@@ -445,6 +447,7 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   // only lever is the number of CTAs pulling it in; take the widest tile that still gives every SM a tile,
   // down to 64 columns
   const bool skinny = g_gemm_variant == 0 && d->M <= 512 && !d->out_fp32 && d->force_bn == 0 && d->split_k <= 1 && !d->colsum;
+  if (skinny && skinny_takes(d, sms)) return launch_gemm_skinny(d, sms, stream);
   if (skinny) {
     if (d->gather) { const char* e = gather_first(); if (e) return e; }
     const int num_m = (d->M + BM - 1) / BM;

@@ -233,3 +233,29 @@ def test_sm_reserve_only_changes_the_grid():
     assert torch.equal(got, want)
     if y is not None:
         assert torch.isfinite(y.float()).all()
+
+
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (4, 1024, 1024), (16, 132, 72), (17, 512, 2048), (33, 3072, 1000), (64, 32000, 512),
+                                   (65, 1000, 4096), (200, 1024, 1024), (257, 2048, 512), (512, 256, 256)])
+def test_few_row_gemm(M, N, K, overlap):
+    """Few-row products: 128-feature tiles, K cut over a cluster, every tile edge; strided activations, in-place residual."""
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w, bias = rnd(M, K + 8)[:, :K], rnd(N, K) * K ** -0.5, rnd(N)
+    out = ops.empty_rows(M, N, "cuda")
+    res = rnd(M, N)
+    acc = x.double() @ w.double().t() + bias.double()
+    ops.ext().set_step_overlap(overlap)
+    try:
+        for act, fn in ((0, lambda t: t), (1, torch.relu), (2, torch.nn.functional.gelu), (3, torch.nn.functional.silu)):
+            ops.gemm(x, w, out, bias=bias, act=act)
+            # one rounding to bf16 (2^-9) and 32-bit sums of K products of order K^-0.5
+            assert torch.allclose(out.double(), fn(acc), rtol=2 ** -8, atol=2 ** -10), (act, (out.double() - fn(acc)).abs().max())
+        y = ops.empty_rows(M, N, "cuda")
+        y.copy_(res)
+        ops.gemm(x, w, y, residual=y)
+        assert torch.allclose(y.double(), acc - bias.double() + res.double(), rtol=2 ** -8, atol=2 ** -10)
+    finally:
+        ops.ext().set_step_overlap(False)
+    assert ops.check_status() == 0
