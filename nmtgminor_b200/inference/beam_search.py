@@ -7,9 +7,9 @@ continuations ending in EOS are moved into a per-sentence table of finished hypo
 are re-indexed accordingly.  A sentence stops when it has ``beam`` finished hypotheses and its best active
 score can no longer enter the table; the loop ends when all sentences stopped or ``max_len`` is reached.
 The batch is not shrunk when sentences finish (static shapes keep the step graph-capturable); finished
-sentences simply stop contributing.  On a GPU the loop reads from the device only every fourth step (the "all sentences done" flag), finished sentences
-are masked in between, and the decoder step is replayed as a CUDA graph (``BeamConfig.cuda_graph``); on the CPU one
-``any()`` per step skips the merge of finished hypotheses when no EOS was produced.
+sentences simply stop contributing.  On a GPU a search without constraints runs as one captured CUDA graph per step
+(``_DeviceSearch``); the others read from the device only every fourth step (the "all sentences done" flag), with finished
+sentences masked in between.  On the CPU one ``any()`` per step skips the merge of finished hypotheses when no EOS was produced.
 
 Constraints supported: minimum length, maximum length (absolute or ``a * src_len + b``), length-normalised
 scores (``score / len^alpha``), n-gram blocking, forced target prefixes, banned first tokens, vocabulary
@@ -46,7 +46,7 @@ class BeamConfig:
     diversity_rate: float = 0.0  # > 0: sibling-rank penalty (the k-th best continuation of a hypothesis loses k * rate)
     vocab_mask: Optional[torch.Tensor] = None   # bool [V], True = allowed
     fused_step: bool = True     # CUDA: fused log-softmax + top-k kernel when no constraint needs full log-probabilities
-    cuda_graph: bool = True     # CUDA + fused_step: replay the decoder step (embedding ... top-k) as a captured graph
+    cuda_graph: bool = True     # CUDA + fused_step: replay whole search steps as a captured graph
 
 
 @dataclass
@@ -118,102 +118,150 @@ def _masked_topk(lprobs, cfg, step, max_rows, prefix_tokens, banned_first, token
     return top_scores, top_idx, V
 
 
-class _GraphedStep:
-    """One decoding step (embedding, decoder layers over the preallocated caches, output projection, fused
-    log-softmax + top-k) as CUDA graphs.  The cache write position and the token positions live on the device and are
-    advanced inside the graph; hypothesis reordering swaps every layer's cache with its spare buffer, so there is one
-    graph per swap parity.  The first steps (cache allocation, warm-up, steps that must not emit EOS) run eagerly
-    through the same code."""
+def _replayable(model, state) -> bool:
+    """Whether every step of ``model`` is its decoder's static step over fused key/value caches, so that a captured step sees
+    everything it needs at fixed addresses."""
+    from ..models.layers import SelfAttention
+    from ..models.transformer import Seq2SeqBase
+    dec = getattr(model, "decoder", None)
+    if dec is None or not hasattr(dec, "step_static") or getattr(type(model), "step", None) is not Seq2SeqBase.step:
+        return False
+    if getattr(dec, "language_embedding", None) is not None or getattr(dec, "adapters", None) is not None:
+        return False
+    attn = [m for m in dec.modules() if isinstance(m, SelfAttention)]
+    return (len(attn) == len(state.buffers) and all(type(m).step is SelfAttention.step and not m.rotary and m.dim // m.heads == 64 for m in attn)
+            and state.context.is_cuda and state.context.dtype == torch.bfloat16)
 
-    def __init__(self, model, state, cfg, K: int, R: int):
+
+class _DeviceSearch:
+    """A search whose steps never leave the device: embedding, decoder layers over preallocated caches, output projection, best
+    continuations and all bookkeeping (finished hypotheses, next active set, ancestors of every cached position) read and
+    write tables at fixed addresses, so one captured CUDA graph is replayed per step.  Hypotheses are not moved when they
+    are re-ranked: every step leaves a (word, parent, score) record, the words of the finished ones are traced back at the end,
+    and attention finds a hypothesis's past through a table of cache rows.
+
+    Tables, caches and the graph are kept on the model for later batches of the same geometry; a search takes its set out of the pool
+    and puts it back when its results are on the host, so concurrent searches have sets of their own."""
+
+    MAX_KEPT = 4
+
+    def __init__(self, model, state, cfg, K: int, B: int, T: int, max_len_per):
         dev = state.context.device
-        self.model, self.state, self.cfg, self.K = model, state, cfg, K
-        cap = state.buffers[0].get("cap", 0)
+        R = B * K
+        self.model, self.state, self.cfg, self.K, self.B, self.T = model, state, cfg, K, B, T
+        cap = (T + 2 + 63) // 64 * 64                    # the geometry of a batch, rounded so that batches share it
         emb = getattr(model.decoder, "embed", None)
         if emb is not None and hasattr(emb, "renew"):
             before = id(getattr(emb, "pos", None))
-            emb.renew(cap + 2)
+            emb.renew(cap)
             if id(getattr(emb, "pos", None)) != before:
                 model.__dict__.pop("_decode_pools", None)      # graphs captured against the old position table are stale
-        # Buffers and captured graphs are pooled on the model and reused by later batches of the same geometry
-        # (rows, cache capacity, padded source length): the projected encoder states of a new batch are copied into
-        # the pooled encoder-decoder caches, so the pointers recorded in the graphs stay valid.
-        cross = [b for b in state.buffers if "c_k" in b and "c_len" in b]
-        src_cap = (max(b["c_k"].shape[1] for b in cross) + 15) // 16 * 16 if cross else 0
-        n_sent = cross[0]["c_k"].shape[0] if cross else 0
-        key = (R, cap, n_sent, src_cap, len(state.buffers), str(dev), cfg.pad, cfg.eos)
-        pools = model.__dict__.setdefault("_decode_pools", {})
-        pool = pools.get(key)
+        from ..models.layers import SelfAttention
+        widths = [m.dim for m in model.decoder.modules() if isinstance(m, SelfAttention)]
+        cross = [b for b in state.buffers if "c_k" in b]
+        src_cap = (max(b["c_k"].shape[1] for b in cross) + 63) // 64 * 64 if cross else 0
+        self.key = (B, K, cap, src_cap, len(state.buffers), str(dev), cfg.pad, cfg.eos)
+        self.pools = model.__dict__.setdefault("_decode_pools", {})
+        pool = self.pools.pop(self.key, None)
         if pool is None:
-            if len(pools) >= 4:
-                pools.pop(next(iter(pools)))
-            pool = pools[key] = {"graphs": {}, "layers": [dict() for _ in state.buffers], "eager_steps": 0,
-                                 "tok": torch.zeros(R, dtype=torch.long, device=dev), "pos_t": torch.zeros(R, dtype=torch.long, device=dev),
-                                 "scores": torch.zeros(R, dtype=torch.float32, device=dev),
-                                 "force": torch.zeros(R, dtype=torch.uint8, device=dev),
-                                 "pos_dev": torch.zeros(1, dtype=torch.int32, device=dev)}
+            mk = lambda shape, dt: torch.zeros(shape, dtype=dt, device=dev)
+            i32, f32, i64 = torch.int32, torch.float32, torch.int64
+            pool = {"graph": None, "warm": 0, "tables": [
+                mk(3, i32), mk(cap + 1, f32), mk(B, i32), mk(R, f32), mk(R, torch.uint8), mk(B, torch.uint8), mk(R, i64), mk(R, i64),
+                mk((R, cap), i32), mk(B, i32), mk((B, K), f32), mk((B, K), i32), mk((B, K), i32), mk((B, K), f32),
+                mk((cap, R), i32), mk((cap, R), i32), mk((cap, R), f32)], "layers": []}
+            for buf, H in zip(state.buffers, widths):
+                keep = {"k": torch.empty(R, cap, H, dtype=torch.bfloat16, device=dev), "v": torch.empty(R, cap, H, dtype=torch.bfloat16, device=dev)}
+                if "c_k" in buf:
+                    shape = (B, src_cap, buf["c_k"].shape[2])
+                    keep.update(c_k=mk(shape, torch.bfloat16), c_v=mk(shape, torch.bfloat16), c_len=mk(B, i32))
+                pool["layers"].append(keep)
+            pool["done_host"] = [torch.zeros(B, dtype=torch.uint8, pin_memory=True) for _ in range(2)]
         self.pool = pool
-        self.tok, self.pos_t, self.scores, self.force = pool["tok"], pool["pos_t"], pool["scores"], pool["force"]
-        self.graphs = pool["graphs"]
-        self.pos_t.zero_()
-        pool["pos_dev"].zero_()
-        state.pos_dev = pool["pos_dev"]
+        (ctl, inv_norm, max_rows, scores, force, done, tok, pos_rows, anc, fin_count, fin_score) = pool["tables"][:11]
+        self.tok, self.pos_rows, self.done = tok, pos_rows, done
+        normalize = bool(cfg.normalize and cfg.alpha > 0)
+        ctl.copy_(torch.tensor([T, cfg.min_len, int(normalize)], dtype=torch.int32))
+        # reciprocal of the length penalty in the precision of a division by a host scalar
+        inv_norm[1:T + 2].copy_(1.0 / torch.tensor([float(n) ** cfg.alpha if normalize else 1.0 for n in range(1, T + 2)], dtype=torch.float32))
+        max_rows.copy_(max_len_per)
+        scores.fill_(float("-inf"))
+        scores.view(B, K)[:, 0] = 0.0                       # only the first hypothesis is alive at step 0
+        force.copy_(torch.where(max_len_per <= 0, 1, 2 if cfg.min_len > 0 else 0).repeat_interleave(K))
+        tok.fill_(cfg.bos)
+        fin_score.fill_(float("-inf"))
+        for t in (done, pos_rows, fin_count):
+            t.zero_()
         for buf, keep in zip(state.buffers, pool["layers"]):
-            buf["pos_dev"] = pool["pos_dev"]
-            if "c_k" in buf and "c_len" in buf:
-                if "c_k" not in keep:
-                    H = buf["c_k"].shape[2]
-                    keep["c_k"] = torch.zeros(n_sent, src_cap, H, dtype=buf["c_k"].dtype, device=dev)
-                    keep["c_v"] = torch.zeros_like(keep["c_k"])
-                    keep["c_len"] = torch.zeros(n_sent, dtype=torch.int32, device=dev)
+            if "c_k" in buf:
                 ts = buf["c_k"].shape[1]
                 keep["c_k"][:, :ts].copy_(buf["c_k"])
                 keep["c_v"][:, :ts].copy_(buf["c_v"])
                 keep["c_len"].copy_(buf["c_len"])
-                buf["c_k"], buf["c_v"], buf["c_len"] = keep["c_k"], keep["c_v"], keep["c_len"]
-            if "k" in keep:       # self-attention caches of an earlier batch: same pointers, contents are overwritten
-                buf["k"], buf["v"], buf["k_spare"], buf["v_spare"] = keep["k"], keep["v"], keep["k_spare"], keep["v_spare"]
+            buf.update(keep)
+            buf.update(anc=anc, pos_rows=pos_rows, beam=K, cap=cap)
 
-    def _body(self, ban_eos: bool):
+    def _body(self):
         from .. import ops
-        ops.ext().set_step_overlap(True)        # this thread's launches, until the step's last GEMM
+        ops.ext().set_step_overlap(True)        # this thread's launches
         try:
-            hidden = self.model.decoder.step_static(self.tok, self.pos_t, self.state)
+            hidden = self.model.decoder.step_static(self.tok, self.pos_rows, self.state)
             logits = self.model.generator(hidden)
+            if logits.dtype not in (torch.float32, torch.bfloat16):
+                logits = logits.float()
+            ops.ext().beam_step(logits, self.pool["tables"], self.K, self.cfg.pad, self.cfg.eos)
         finally:
             ops.ext().set_step_overlap(False)
-        if logits.dtype not in (torch.float32, torch.bfloat16):
-            logits = logits.float()
-        ts, ti, _ = ops.ext().beam_topk(logits, self.scores, self.force, self.K, self.cfg.pad, self.cfg.eos, ban_eos)
-        self.state.pos_dev.add_(1)
-        self.pos_t.add_(1)
-        return ts, ti, logits.shape[1]
 
-    def run(self, last_tokens, scores, force_eos, ban_eos: bool, step: int):
-        self.tok.copy_(last_tokens)
-        self.scores.copy_(scores)
-        # control byte per row: 1 = only EOS may follow (length limit), 2 = EOS banned (minimum length), 0 = free
-        self.force.copy_(force_eos)
-        if ban_eos:
-            self.force.add_(2).clamp_(max=2).sub_(force_eos.to(torch.uint8))      # 0 -> 2, 1 -> 1
-        key = self.state.buffers[0]["k"].data_ptr() if "k" in self.state.buffers[0] else None
-        if key is None or self.pool["eager_steps"] < 2:
-            self.pool["eager_steps"] += 1
-            out = self._body(False)
-            for buf, keep in zip(self.state.buffers, self.pool["layers"]):
-                if "k" in buf and "k" not in keep:        # caches allocated by the first step: keep them for later batches
-                    keep.update(k=buf["k"], v=buf["v"], k_spare=buf["k_spare"], v_spare=buf["v_spare"])
-            return out
-        entry = self.graphs.get(key)
-        if entry is None:
+    def _step(self):
+        pool = self.pool
+        if pool["warm"] < 2:                    # lazy initialisation happens outside the capture
+            pool["warm"] += 1
+            return self._body()
+        if pool["graph"] is None:
             g = torch.cuda.CUDAGraph()
             torch.cuda.synchronize()
-            with torch.cuda.graph(g):
-                out = self._body(False)
-            # capture records the launches without running them: replay once for this step's result
-            self.graphs[key] = entry = (g, out)
-        entry[0].replay()
-        return entry[1]
+            with torch.cuda.graph(g, capture_error_mode="thread_local"):
+                self._body()
+            pool["graph"] = g                   # captured, not run
+        pool["graph"].replay()
+
+    def run(self):
+        """All steps, then per sentence the ``n_best`` finished hypotheses, best first."""
+        from .. import ops
+        cfg, K = self.cfg, self.K
+        seen = None
+        for step in range(self.T + 1):
+            self._step()
+            if step % 4 == 3 and step < self.T:
+                # "all sentences done", read four steps late so that the device never waits for the host
+                if seen is not None:
+                    seen[0].synchronize()
+                    if bool(seen[1].all()):
+                        break
+                host = self.pool["done_host"][(step // 4) & 1]
+                host.copy_(self.done, non_blocking=True)
+                event = torch.cuda.Event()
+                event.record()
+                seen = (event, host)
+        tables = self.pool["tables"]
+        n = min(cfg.n_best, K)
+        words, word_scores = ops.ext().beam_trace(tables, K, cfg.pad, cfg.eos, n)
+        scores, last = tables[10][:, :n].cpu(), tables[11][:, :n].cpu()
+        longest = int(last.masked_fill(scores == float("-inf"), 0).max()) + 1
+        words, word_scores = words[:, :, :longest].cpu(), word_scores[:, :, :longest].cpu()
+        if len(self.pools) >= self.MAX_KEPT:
+            self.pools.pop(next(iter(self.pools)), None)
+        self.pools[self.key] = self.pool
+        results = []
+        for b in range(self.B):
+            hyps = []
+            for k in range(n):
+                if torch.isfinite(scores[b, k]):
+                    m = int(last[b, k]) + 1
+                    hyps.append(Hypothesis(words[b, k, :m].tolist(), float(scores[b, k]), word_scores[b, k, :m].tolist()))
+            results.append(hyps or [Hypothesis([cfg.eos], float("-inf"))])
+        return results
 
 
 @torch.no_grad()
@@ -231,6 +279,12 @@ def beam_search(model, batch, cfg: BeamConfig, prefix_tokens: Optional[torch.Ten
     else:
         max_len_per = torch.full((B,), cfg.max_len, device=device, dtype=torch.long)
     T = int(max_len_per.max().item())
+    # fused step: log-softmax, masks and the per-sentence top-2K in two kernels, no [R, V] log-probabilities
+    fused = (device.type == "cuda" and cfg.fused_step and getattr(model, "supports_logits_step", False)
+             and not cfg.sampling and cfg.no_repeat_ngram_size <= 0 and cfg.vocab_mask is None and 2 * K <= 64
+             and cfg.diversity_rate <= 0)
+    if fused and cfg.cuda_graph and prefix_tokens is None and banned_first is None and _replayable(model, state):
+        return _DeviceSearch(model, state, cfg, K, B, T, max_len_per).run()
     R = B * K
     tokens = torch.full((R, T + 2), cfg.pad, dtype=torch.long, device=device)
     tokens[:, 0] = cfg.bos
@@ -248,23 +302,10 @@ def beam_search(model, batch, cfg: BeamConfig, prefix_tokens: Optional[torch.Ten
 
     if hasattr(state, "set_cache_capacity") and device.type == "cuda":
         state.set_cache_capacity(T + 2)
-    # fused step: log-softmax, masks and the per-sentence top-2K in two kernels, no [R, V] log-probabilities
-    fused = (device.type == "cuda" and cfg.fused_step and getattr(model, "supports_logits_step", False)
-             and not cfg.sampling and cfg.no_repeat_ngram_size <= 0 and cfg.vocab_mask is None and 2 * K <= 64
-             and cfg.diversity_rate <= 0)
-
-    graphed = None
-    if (fused and cfg.cuda_graph and prefix_tokens is None and banned_first is None and hasattr(state, "enable_device_positions")
-            and hasattr(getattr(model, "decoder", None), "step_static")):
-        graphed = _GraphedStep(model, state, cfg, K, R)
-
     for step in range(T + 1):
         use_fused = (fused and not (prefix_tokens is not None and step < prefix_tokens.shape[1])
                      and not (banned_first is not None and step == 0))
-        if graphed is not None:
-            top_scores, top_idx, V = graphed.run(tokens[:, step], scores.reshape(-1), step >= max_rows, step < cfg.min_len, step)
-            lprobs = None
-        elif use_fused:
+        if use_fused:
             from .. import ops
             logits = model.step(tokens[:, :step + 1], state, logits_only=True)["logits"]
             V = logits.shape[1]

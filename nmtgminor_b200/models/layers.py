@@ -268,20 +268,18 @@ class SelfAttention(nn.Module):
         q, k, v = qkv[:, :H], qkv[:, H:2 * H], qkv[:, 2 * H:]
         B = x.shape[0]
         if _fused_decode(qkv, H, h) and cache.get("cap"):
+            if "anc" in cache:
+                # a replayed search step: positions and the rows that hold every hypothesis's past live on the device
+                ctx = ops.ext().decode_self(qkv, cache["k"], cache["v"], cache["anc"], cache["pos_rows"], cache["beam"], h, (H // h) ** -0.5)
+                return self.out(ctx, residual=residual)
             # preallocated [rows, cap, H] caches: append in place, attend with the single-query kernel
             pos = cache.get("pos", 0)
             if "k" not in cache:
                 for name in ("k", "v", "k_spare", "v_spare"):
                     cache[name] = torch.empty(B, cache["cap"], H, dtype=qkv.dtype, device=qkv.device)
-            pos_dev = cache.get("pos_dev")
-            if pos_dev is not None:
-                # the write position lives on the device (advanced once per step by the caller): graph-replayable
-                ops.ext().cache_append(k, v, cache["k"], cache["v"], 0, pos_dev)
-                ctx = ops.ext().decode_attn(q, cache["k"], cache["v"], None, cache["cap"], h, (H // h) ** -0.5, pos_dev, 1)
-            else:
-                ops.ext().cache_append(k, v, cache["k"], cache["v"], pos)
-                ctx = ops.ext().decode_attn(q, cache["k"], cache["v"], None, pos + 1, h, (H // h) ** -0.5)
-                cache["pos"] = pos + 1
+            ops.ext().cache_append(k, v, cache["k"], cache["v"], pos)
+            ctx = ops.ext().decode_attn(q, cache["k"], cache["v"], None, pos + 1, h, (H // h) ** -0.5)
+            cache["pos"] = pos + 1
             return self.out(ctx, residual=residual)
         if "k" not in cache:
             cache["k"], cache["v"] = k.view(B, 1, H), v.view(B, 1, H)
@@ -322,7 +320,7 @@ class CrossAttention(nn.Module):
         ck, cv = cache["c_k"], cache["c_v"]
         if "c_len" in cache and _fused_decode(q, self.dim, self.heads):
             # one cache row per sentence, shared by its hypotheses
-            ctx = ops.ext().decode_attn(q, ck, cv, cache["c_len"], ck.shape[1], self.heads, (self.dim // self.heads) ** -0.5)
+            ctx = ops.ext().decode_cross(q, ck, cv, cache["c_len"], self.heads, (self.dim // self.heads) ** -0.5)
             return self.out(ctx, residual=residual)
         if ck.shape[0] != q.shape[0]:
             rep = q.shape[0] // ck.shape[0]

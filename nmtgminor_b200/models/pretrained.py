@@ -104,9 +104,15 @@ class PretrainedStyleDecoder(nn.Module):
         return self.final_norm(x) if self.final_norm is not None else x
 
     def step(self, tokens, position: int, state: DecodingState):
+        return self.step_static(tokens, torch.full_like(tokens, position), state)
+
+    def step_static(self, tokens, positions, state: DecodingState):
+        """One new position per hypothesis, the positions given on the device (``TransformerDecoder.step_static``)."""
         B = tokens.shape[0]
-        seqs = PackedSeqs(tokens, torch.full_like(tokens, position), torch.arange(B + 1, dtype=torch.int32, device=tokens.device), 1)
-        x = self.embed(seqs, 0.0)
+        cu = getattr(self, "_step_cu", None)
+        if cu is None or cu.numel() != B + 1 or cu.device != tokens.device:
+            cu = self._step_cu = torch.arange(B + 1, dtype=torch.int32, device=tokens.device)
+        x = self.embed(PackedSeqs(tokens, positions, cu, 1), 0.0)
         if self.emb_norm is not None:
             x = self.emb_norm(x)
         for i, layer in enumerate(self.layers):

@@ -193,7 +193,7 @@ class TransformerDecoder(nn.Module):
 
     def step_static(self, tokens, positions, state: "DecodingState"):
         """``step`` with the positions given as a device tensor and no host-side bookkeeping, so that the whole call
-        can be captured in a CUDA graph (``state.enable_device_positions()`` must have been called)."""
+        can be captured in a CUDA graph (``inference.beam_search`` keeps its tables in ``state.buffers``)."""
         B = tokens.shape[0]
         cu = getattr(self, "_step_cu", None)
         if cu is None or cu.numel() != B + 1 or cu.device != tokens.device:
@@ -240,13 +240,6 @@ class DecodingState:
         for buf in self.buffers:
             buf["cap"] = int(cap)
 
-    def enable_device_positions(self):
-        """Keep the write position of the self-attention caches in a device integer (``pos_dev``) that the caller
-        advances once per step, so that a decoding step can be captured in a CUDA graph and replayed."""
-        self.pos_dev = torch.zeros(1, dtype=torch.int32, device=self.context.device)
-        for buf in self.buffers:
-            buf["pos_dev"] = self.pos_dev
-
     def reorder(self, index, reorder_context: bool = True):
         rows = index.numel()
         if reorder_context:
@@ -255,13 +248,7 @@ class DecodingState:
             if getattr(self, "src_tokens", None) is not None:
                 self.src_tokens = self.src_tokens.index_select(0, index)
         for buf in self.buffers:
-            if "k_spare" in buf and buf.get("pos_dev") is not None:
-                H = buf["k"].shape[2]
-                ops.ext().gather_rows(buf["k"], buf["k_spare"], index, -1, buf["pos_dev"], H)
-                ops.ext().gather_rows(buf["v"], buf["v_spare"], index, -1, buf["pos_dev"], H)
-                buf["k"], buf["k_spare"] = buf["k_spare"], buf["k"]
-                buf["v"], buf["v_spare"] = buf["v_spare"], buf["v"]
-            elif "k_spare" in buf:
+            if "k_spare" in buf:
                 # preallocated caches: copy only the filled prefix of every row into the spare buffers and swap
                 filled = buf.get("pos", 0) * buf["k"].shape[2]
                 ops.ext().gather_rows(buf["k"], buf["k_spare"], index, filled)
@@ -270,7 +257,7 @@ class DecodingState:
                 buf["v"], buf["v_spare"] = buf["v_spare"], buf["v"]
             for k in list(buf.keys()):
                 val = buf[k]
-                if k == "pos_dev" or (k in ("k", "v", "k_spare", "v_spare") and "k_spare" in buf):
+                if k in ("k", "v", "k_spare", "v_spare") and "k_spare" in buf:
                     continue
                 # per-sentence entries (encoder-decoder caches shared by the hypotheses) keep their order
                 if torch.is_tensor(val) and val.dim() > 0 and val.shape[0] == rows:

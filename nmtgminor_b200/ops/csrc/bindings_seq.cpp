@@ -233,6 +233,87 @@ void cache_append(const Tensor& k_new, const Tensor& v_new, Tensor& k_cache, Ten
                        static_cast<int>(pos), dev_int(pos_dev, "pos_dev"), cur_stream()));
 }
 
+Tensor decode_self(const Tensor& qkv, Tensor& k_cache, Tensor& v_cache, const Tensor& anc, const Tensor& pos_rows, int64_t K, int64_t heads,
+                   double scale) {
+  TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == at::kBFloat16 && qkv.dim() == 2 && qkv.stride(1) == 1 && qkv.size(1) == 3 * heads * 64 &&
+              (reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 15) == 0);
+  need(k_cache, at::kBFloat16, "k_cache"); need(v_cache, at::kBFloat16, "v_cache"); need(anc, at::kInt, "anc"); need(pos_rows, at::kLong, "pos_rows");
+  const int R = qkv.size(0);
+  TORCH_CHECK(k_cache.dim() == 3 && k_cache.sizes() == v_cache.sizes() && k_cache.size(0) == R && k_cache.size(2) == heads * 64);
+  TORCH_CHECK(K > 0 && R % K == 0 && anc.dim() == 2 && anc.size(0) == R && anc.size(1) == k_cache.size(1) && pos_rows.numel() == R);
+  c10::cuda::CUDAGuard guard(qkv.device());
+  Tensor out = torch::empty({R, heads * 64}, qkv.options());
+  ck(nmtg_decode_self(qkv.data_ptr(), qkv.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), anc.data_ptr<int>(),
+                      reinterpret_cast<const long*>(pos_rows.data_ptr<int64_t>()), out.data_ptr(), R / static_cast<int>(K), static_cast<int>(K),
+                      static_cast<int>(heads), static_cast<int>(k_cache.size(1)), static_cast<float>(scale), cur_stream()));
+  return out;
+}
+
+Tensor decode_cross(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& lengths, int64_t heads, double scale) {
+  TORCH_CHECK(q.is_cuda() && q.scalar_type() == at::kBFloat16 && q.dim() == 2 && q.stride(1) == 1 && q.size(1) == heads * 64);
+  need(k_cache, at::kBFloat16, "k_cache"); need(v_cache, at::kBFloat16, "v_cache"); need(lengths, at::kInt, "lengths");
+  TORCH_CHECK(k_cache.dim() == 3 && k_cache.sizes() == v_cache.sizes() && k_cache.size(2) == heads * 64);
+  const int R = q.size(0), B = k_cache.size(0);
+  TORCH_CHECK(B > 0 && R % B == 0 && lengths.numel() == B, "query rows must be a multiple of cache rows");
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor out = torch::empty({R, heads * 64}, q.options());
+  ck(nmtg_decode_cross(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), lengths.data_ptr<int>(), out.data_ptr(), B, R / B,
+                       static_cast<int>(heads), static_cast<int>(k_cache.size(1)), static_cast<float>(scale), cur_stream()));
+  return out;
+}
+
+// Tables of a search in the order of NmtgBeam (ctl, inv_norm, max_rows, scores, force, done, tok, pos_rows, anc, fin_count, fin_score,
+// fin_step, fin_row, fin_last, hist_tok, hist_par, hist_score).
+NmtgBeam beam_tables(const std::vector<Tensor>& t, int64_t K, int64_t pad, int64_t eos, int* B, int* steps) {
+  TORCH_CHECK(t.size() == 17, "beam tables: 17 tensors are expected");
+  const at::ScalarType types[17] = {at::kInt, at::kFloat, at::kInt, at::kFloat, at::kByte, at::kByte, at::kLong, at::kLong, at::kInt,
+                                    at::kInt, at::kFloat, at::kInt, at::kInt, at::kFloat, at::kInt, at::kInt, at::kFloat};
+  for (int i = 0; i < 17; ++i) need(t[i], types[i], "beam tables");
+  const int64_t R = t[3].numel();
+  TORCH_CHECK(K >= 1 && K <= 32 && R > 0 && R % K == 0);
+  const int64_t b = R / K;
+  TORCH_CHECK(t[0].numel() == 3 && t[2].numel() == b && t[4].numel() == R && t[5].numel() == b && t[6].numel() == R && t[7].numel() == R);
+  TORCH_CHECK(t[8].dim() == 2 && t[8].size(0) == R && t[9].numel() == b);
+  for (int i = 10; i <= 13; ++i) TORCH_CHECK(t[i].numel() == R);
+  TORCH_CHECK(t[14].dim() == 2 && t[14].size(1) == R && t[15].sizes() == t[14].sizes() && t[16].sizes() == t[14].sizes());
+  TORCH_CHECK(t[1].numel() >= t[14].size(0) + 1 && t[8].size(1) >= t[14].size(0), "beam tables: too few lengths or positions for the steps");
+  NmtgBeam s;
+  s.K = K; s.R = R; s.cap = t[8].size(1); s.pad = pad; s.eos = eos;
+  s.ctl = t[0].data_ptr<int>(); s.inv_norm = t[1].data_ptr<float>(); s.max_rows = t[2].data_ptr<int>(); s.scores = t[3].data_ptr<float>();
+  s.force = t[4].data_ptr<uint8_t>(); s.done = t[5].data_ptr<uint8_t>();
+  s.tok = reinterpret_cast<long*>(t[6].data_ptr<int64_t>()); s.pos_rows = reinterpret_cast<long*>(t[7].data_ptr<int64_t>());
+  s.anc = t[8].data_ptr<int>(); s.fin_count = t[9].data_ptr<int>(); s.fin_score = t[10].data_ptr<float>(); s.fin_step = t[11].data_ptr<int>();
+  s.fin_row = t[12].data_ptr<int>(); s.fin_last = t[13].data_ptr<float>(); s.hist_tok = t[14].data_ptr<int>(); s.hist_par = t[15].data_ptr<int>();
+  s.hist_score = t[16].data_ptr<float>();
+  *B = b;
+  *steps = t[14].size(0);
+  return s;
+}
+
+void beam_step(const Tensor& logits, const std::vector<Tensor>& tables, int64_t K, int64_t pad, int64_t eos) {
+  int B, steps;
+  const NmtgBeam s = beam_tables(tables, K, pad, eos, &B, &steps);
+  TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1 && logits.size(0) == s.R);
+  TORCH_CHECK(eos >= 0 && eos < logits.size(1), "beam_step: EOS outside the vocabulary");
+  c10::cuda::CUDAGuard guard(logits.device());
+  const int64_t V = logits.size(1), pieces = (V + 4095) / 4096;
+  auto fo = torch::dtype(torch::kFloat).device(logits.device());
+  Tensor lse = torch::empty({s.R, pieces, 2}, fo), part = torch::empty({s.R, pieces, 2 * K}, fo.dtype(torch::kLong));
+  ck(nmtg_beam_step(&s, logits.data_ptr(), logits.stride(0), dtype_code(logits), lse.data_ptr(), part.data_ptr(), B, static_cast<int>(V),
+                    cur_stream()));
+}
+
+std::vector<Tensor> beam_trace(const std::vector<Tensor>& tables, int64_t K, int64_t pad, int64_t eos, int64_t n_best) {
+  int B, steps;
+  const NmtgBeam s = beam_tables(tables, K, pad, eos, &B, &steps);
+  c10::cuda::CUDAGuard guard(tables[3].device());
+  Tensor words = torch::full({B, n_best, steps}, pad, tables[6].options());
+  Tensor scores = torch::zeros({B, n_best, steps}, tables[3].options());
+  ck(nmtg_beam_trace(&s, B, static_cast<int>(n_best), reinterpret_cast<long*>(words.data_ptr<int64_t>()), scores.data_ptr<float>(), steps,
+                     cur_stream()));
+  return {words, scores};
+}
+
 std::vector<Tensor> rel_attn_fwd(const Tensor& qkv, const Tensor& r, const Tensor& u, const Tensor& w, const Tensor& cu, int64_t heads,
                                  int64_t max_len, int64_t r_center, bool causal, double scale, double p, int64_t seed, int64_t stream_id) {
   need(qkv, at::kBFloat16, "qkv"); need(r, at::kBFloat16, "r"); need(u, at::kFloat, "u"); need(w, at::kFloat, "w"); need(cu, at::kInt, "cu");
@@ -286,6 +367,10 @@ void bind_sequence_ops(pybind11::module& m) {
         py::arg("filled_dev") = py::none(), py::arg("unit_elems") = 0);
   m.def("decode_attn", &decode_attn, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("lengths"), py::arg("len"),
         py::arg("heads"), py::arg("scale"), py::arg("len_dev") = py::none(), py::arg("len_add") = 0);
+  m.def("decode_self", &decode_self);
+  m.def("decode_cross", &decode_cross);
+  m.def("beam_step", &beam_step);
+  m.def("beam_trace", &beam_trace);
   m.def("cache_append", &cache_append, py::arg("k_new"), py::arg("v_new"), py::arg("k_cache"), py::arg("v_cache"), py::arg("pos"),
         py::arg("pos_dev") = py::none());
 }

@@ -15,6 +15,8 @@
 
 namespace b200 {
 
+bool step_overlap();
+
 constexpr int kLnWarps = 4;
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -32,6 +34,8 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int nvec = hidden >> 3;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // decoding steps: see nmtg_set_step_overlap
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int row = blockIdx.x * kLnWarps + warp; row < rows; row += gridDim.x * kLnWarps) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * hidden);
     float v[VPL][8];
@@ -415,11 +419,18 @@ const char* nmtg_layernorm_fwd(const void* x, const void* gamma, const void* bet
   const int cap = num_sms() * 16;
   if (grid > cap) grid = cap;
   return dispatch_vpl(hidden, [&](auto vpl) -> const char* {
-    ln_fwd_kernel<decltype(vpl)::value><<<grid, kLnWarps * 32, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(gamma),
-        reinterpret_cast<const __nv_bfloat16*>(beta), reinterpret_cast<__nv_bfloat16*>(y), mean, rstd, rows, hidden,
-        eps);
-    cudaError_t e = cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kLnWarps * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = step_overlap() ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, ln_fwd_kernel<decltype(vpl)::value>, reinterpret_cast<const __nv_bfloat16*>(x),
+                                       reinterpret_cast<const __nv_bfloat16*>(gamma), reinterpret_cast<const __nv_bfloat16*>(beta),
+                                       reinterpret_cast<__nv_bfloat16*>(y), mean, rstd, rows, hidden, eps);
     return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
   });
 }

@@ -87,6 +87,41 @@ const char* nmtg_decode_attn(const void* q, long q_ld, const void* k_cache, cons
 const char* nmtg_cache_append(const void* k_new, const void* v_new, long ld, void* k_cache, void* v_cache, int R, int heads,
                               int cap, int pos, const int* pos_dev, cudaStream_t stream);
 
+// ---- one replayable beam-search step (decode_step.cu) -------------------------------------------------------------
+// Tables of a search over B sentences x K hypotheses (R = B K rows), all on the device.
+struct NmtgBeam {
+  int K, R, cap, pad, eos;
+  const int* ctl;          // {T, min_len, normalize}
+  const float* inv_norm;   // [n] = 1 / n^alpha for lengths up to T + 1
+  const int* max_rows;     // [B] step at which only EOS may follow
+  float* scores;           // [R] sums of log-probabilities
+  uint8_t* force;          // [R] 1 = only EOS may follow, 2 = EOS is banned, 0 = free
+  uint8_t* done;           // [B]
+  long* tok;               // [R] last word of every hypothesis
+  long* pos_rows;          // [R] its position = the current step
+  int* anc;                // [R, cap] cache row that holds position j of hypothesis r
+  int* fin_count;          // [B]
+  float* fin_score;        // [B, K] finished hypotheses, best first; -inf = none
+  int* fin_step;           // [B, K] step of the EOS
+  int* fin_row;            // [B, K] hypothesis (0 .. K-1) that it ended
+  float* fin_last;         // [B, K] log-probability of the EOS
+  int* hist_tok;           // [steps, R] word chosen at a step, its parent (0 .. K-1) and its log-probability
+  int* hist_par;
+  float* hist_score;
+};
+// qkv: bf16 [R, 3 * heads * 64]; the new keys / values go to row r, position pos_rows[r] of the caches [R, cap, heads * 64]
+const char* nmtg_decode_self(const void* qkv, long ld, void* k_cache, void* v_cache, const int* anc, const long* pos_rows, void* out,
+                             int B, int K, int heads, int cap, float scale, cudaStream_t stream);
+// q: bf16 [B K, heads * 64]; ck / cv: bf16 [B, cap, heads * 64], lengths int32 [B]
+const char* nmtg_decode_cross(const void* q, long ld, const void* ck, const void* cv, const int* lengths, void* out, int B, int K,
+                              int heads, int cap, float scale, cudaStream_t stream);
+// logits [R, V] (dtype 0 = fp32, 1 = bf16); workspaces: part_lse 8 bytes x [R, pieces], part 8 bytes x [R, pieces, 2K] with
+// pieces = ceil(V / 4096).  Advances every table by one step.
+const char* nmtg_beam_step(const NmtgBeam* s, const void* logits, long ld, int dtype, void* part_lse, void* part, int B, int V,
+                           cudaStream_t stream);
+// words / word_scores [B, n_best, width]: the finished hypotheses, fin_step + 1 entries each
+const char* nmtg_beam_trace(const NmtgBeam* s, int B, int n_best, long* words, float* word_scores, int width, cudaStream_t stream);
+
 // ---- relative-position (Transformer-XL) self-attention on packed sequences of at most 128 tokens ---------------
 // qkv: bf16 [N, 3 * heads * 64]; r: bf16 [L, heads * 64], row r_center - d = projected embedding of distance d;
 // u / w: fp32 [heads, 64] content / position biases; cu: int32 [B + 1]; out: bf16 [N, heads * 64]; lse: fp32 [heads, N].

@@ -131,3 +131,121 @@ def test_fused_beam_search_matches_unfused_and_cpu():
     cpu = beam_search(model, batch, BeamConfig(beam_size=4, n_best=2, max_len=20, min_len=2))
     agree = sum(a[0].tokens == c[0].tokens for a, c in zip(res["fused"], cpu))
     assert agree >= 4, "best hypotheses differ between the bf16 GPU path and the fp32 CPU path"
+
+
+@pytest.mark.parametrize("B,K,heads,cap,pos", [(1, 1, 1, 64, 0), (3, 2, 2, 64, 1), (2, 4, 3, 64, 33), (5, 3, 2, 192, 130), (2, 6, 1, 320, 319), (1, 12, 2, 64, 40)])
+def test_step_self_attention(B, K, heads, cap, pos):
+    """Append + attention through a table of ancestor rows: first position, block edges, several CTAs per sentence."""
+    g = torch.Generator(device="cuda").manual_seed(pos + K)
+    R, hid = B * K, heads * 64
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    qkv, kc, vc = rnd(R, 3 * hid + 8)[:, :3 * hid], rnd(R, cap, hid), rnd(R, cap, hid)
+    anc = (torch.randint(0, K, (B, K, cap), device="cuda", generator=g) + torch.arange(B, device="cuda")[:, None, None] * K).int().view(R, cap).contiguous()
+    before = kc.clone(), vc.clone()
+    out = ops.ext().decode_self(qkv, kc, vc, anc, torch.full((R,), pos, dtype=torch.long, device="cuda"), K, heads, 0.125)
+    q, k, v = (t.double().view(R, heads, 64) for t in qkv.split(hid, 1))
+    take = lambda c: torch.stack([c[anc[:, j].long(), j] for j in range(pos)], 1).double().view(R, pos, heads, 64) if pos else k.new_zeros(R, 0, heads, 64)
+    keys, vals = torch.cat([take(before[0]), k[:, None]], 1), torch.cat([take(before[1]), v[:, None]], 1)
+    p = torch.softmax(torch.einsum("rhd,rjhd->rhj", q, keys) * 0.125, -1)
+    want = torch.einsum("rhj,rjhd->rhd", p, vals).reshape(R, hid)
+    assert (out.double() - want).abs().max() < 2 ** -8 * want.abs().max()          # one rounding to bf16 of a 32-bit result
+    before[0][:, pos], before[1][:, pos] = qkv[:, hid:2 * hid], qkv[:, 2 * hid:]
+    assert torch.equal(kc, before[0]) and torch.equal(vc, before[1])
+
+
+@pytest.mark.parametrize("B,K,heads,cap", [(1, 1, 1, 31), (2, 4, 2, 100), (1, 5, 2, 513), (3, 2, 4, 1500), (2, 9, 1, 1536), (1, 4, 16, 4096)])
+def test_step_cross_attention(B, K, heads, cap):
+    """One sentence's hypotheses over its shared keys, the long ones cut over a cluster; lengths 0, 1 and full among them."""
+    g = torch.Generator(device="cuda").manual_seed(cap)
+    hid = heads * 64
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    q, k, v = rnd(B * K, hid), rnd(B, cap, hid), rnd(B, cap, hid)
+    for lens in ([cap] * B, [1] * B, [0] * B, [(cap * (i + 2)) // (B + 3) for i in range(B)]):
+        out = ops.ext().decode_cross(q, k, v, torch.tensor(lens, dtype=torch.int32, device="cuda"), heads, 0.125)
+        for b, n in enumerate(lens):
+            qb, kb, vb = q[b * K:(b + 1) * K].double().view(K, heads, 64), k[b, :n].double().view(n, heads, 64), v[b, :n].double().view(n, heads, 64)
+            want = torch.einsum("khj,jhd->khd", torch.softmax(torch.einsum("khd,jhd->khj", qb, kb) * 0.125, -1), vb).reshape(K, hid)
+            assert (out[b * K:(b + 1) * K].double() - want).abs().max() <= 2 ** -8 * want.abs().max() + 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,K,V,T,min_len,normalize", [(1, 1, 40, 6, 0, False), (3, 4, 50, 12, 1, False), (5, 4, 4097, 9, 3, True),
+                                                       (2, 6, 8200, 7, 0, True), (2, 32, 5000, 5, 1, False), (4, 3, 1000, 10, 10, True)])
+def test_device_search_matches_host_bookkeeping(dtype, B, K, V, T, min_len, normalize):
+    """The step kernels against the tensor statements of the same search, on logits that depend on the last word and the step."""
+    from types import SimpleNamespace
+
+    from nmtgminor_b200.inference import beam_search as bs
+    g = torch.Generator(device="cuda").manual_seed(V + T)
+    ld = (V + 7) // 8 * 8
+    by_word = torch.randn(V, ld, device="cuda", generator=g)
+    by_word[:, 3] += 1.5                                   # EOS is likely enough to end hypotheses early
+    by_step = torch.randn(T + 2, ld, device="cuda", generator=g)
+    logits_of = lambda tok, step: (by_word[tok] + by_step[step]).to(dtype)[:, :V]
+    lens = torch.randint(2, 9, (B,), device="cuda", generator=g)
+
+    class State:
+        buffers = []
+
+        def __init__(self):
+            self.context = torch.zeros(B * K, 8, 4, device="cuda")
+            self.src_pad_mask = (torch.arange(8, device="cuda")[None] >= lens[:, None]).repeat_interleave(K, 0)
+
+        def reorder(self, index):
+            pass
+
+    model = SimpleNamespace(supports_logits_step=True, decoder=torch.nn.Module(), create_decoder_state=lambda batch, k: State())
+    model.step = lambda tokens, state, logits_only=False: {"logits": logits_of(tokens[:, -1], tokens.shape[1] - 1)}
+    cfg = bs.BeamConfig(beam_size=K, n_best=K, max_len=T, min_len=min_len, dynamic_max_len=True, len_a=1.0, len_b=T - 8, normalize=normalize,
+                        alpha=0.6 if normalize else 0.0)
+    want = bs.beam_search(model, None, cfg)
+    limit = (lens.float() + T - 8).clamp(max=T).long()
+
+    class Search(bs._DeviceSearch):
+        def _body(self):
+            step = int(self.pos_rows[0])
+            ops.ext().beam_step(logits_of(self.tok, min(step, T + 1)), self.pool["tables"], K, cfg.pad, cfg.eos)
+
+        _step = _body
+
+    for _ in range(2):                                      # the second search takes the first one's tables
+        got = Search(model, State(), cfg, K, B, int(limit.max()), limit).run()
+        for a, b in zip(want, got):
+            assert [h.tokens for h in a] == [h.tokens for h in b]
+            for x, y in zip(a, b):
+                assert abs(x.score - y.score) <= 2e-5 * max(1.0, abs(x.score)) or x.score == y.score
+                assert torch.allclose(torch.tensor(x.positional_scores), torch.tensor(y.positional_scores), atol=2e-4)
+
+
+@pytest.mark.parametrize("beam", [1, 2, 5])
+def test_replayed_search_matches_the_stepwise_one(beam):
+    """Captured steps against the same search launched kernel by kernel, over enough steps and batches that the replays matter; with
+    one hypothesis per sentence the encoder's keys have as many rows as there are hypotheses."""
+    from nmtgminor_b200.data.dataset import collate
+    from nmtgminor_b200.data.synthetic import synthetic_dict
+    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
+    from nmtgminor_b200.models.transformer import Transformer
+    from nmtgminor_b200.options import default_options
+    from nmtgminor_b200.parallel.flat import FlatParameterStore
+    torch.manual_seed(beam)
+    d = synthetic_dict(300)
+    opt = default_options(["-model_size", "256", "-layers", "3", "-n_heads", "4", "-inner_size", "512", "-ffn_activation", "relu"])
+    model = Transformer(opt, {"src": d, "tgt": d}).eval()
+    with torch.no_grad():
+        # every word prefers its successor by a wide margin, so that rounding does not change the best hypothesis
+        order = torch.randperm(296) + 4
+        model.generator.weight[order] = 1.5 * model.decoder.embed.weight[order.roll(1)]
+        model.generator.weight[order[0]] += 1.5 * model.decoder.embed.weight[2]
+    FlatParameterStore(model, "cuda")
+    for b in model.buffers():
+        b.data = b.data.cuda()
+    g = torch.Generator().manual_seed(3)
+    for _ in range(3):
+        src = [torch.randint(4, 300, (int(n),), generator=g) for n in torch.randint(3, 40, (7,), generator=g)]
+        batch = collate(src, None, padded=True, packed=True, round_to=1).cuda("cuda")
+        res = [beam_search(model, batch, BeamConfig(beam_size=beam, max_len=40, min_len=30, cuda_graph=c)) for c in (False, True)]
+        for a, b in zip(*res):
+            assert a[0].tokens == b[0].tokens
+            # the logits are bf16 of up to 32: one rounding that falls the other way moves a score by 2^-3; two of them
+            assert abs(a[0].score - b[0].score) <= 0.25
+    assert ops.check_status() == 0
