@@ -447,9 +447,9 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   // only lever is the number of CTAs pulling it in; take the widest tile that still gives every SM a tile,
   // down to 64 columns
   const bool skinny = g_gemm_variant == 0 && d->M <= 512 && !d->out_fp32 && d->force_bn == 0 && d->split_k <= 1 && !d->colsum;
-  if (skinny && skinny_takes(d, sms)) return launch_gemm_skinny(d, sms, stream);
   if (skinny) {
     if (d->gather) { const char* e = gather_first(); if (e) return e; }
+    if (skinny_takes(d, sms)) return launch_gemm_skinny(d, sms, stream);
     const int num_m = (d->M + BM - 1) / BM;
     int bn = 64;
     if (static_cast<long>(num_m) * ((d->N + 255) / 256) >= sms) bn = 256;
