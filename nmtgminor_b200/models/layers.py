@@ -67,9 +67,20 @@ class PackedSeqs:
 
     def pad(self, x: torch.Tensor, time_first: bool = True):
         """Packed ``[tokens, ...]`` -> padded ``[T, B, ...]`` (or ``[B, T, ...]``)."""
+        if _one_kernel_pad(x, self.cu):
+            bounds = self.cu.tolist()
+            if bounds[-1] <= x.shape[0] and all(0 <= a <= b <= a + self.max_len for a, b in zip(bounds, bounds[1:])):
+                return ops.ext().pad_rows(x, self.cu, self.max_len, time_first)
         from ..ops.reference import pad_packed
         out, _ = pad_packed(x, self.cu, self.max_len)
         return out.transpose(0, 1).contiguous() if time_first else out
+
+
+def _one_kernel_pad(x, cu) -> bool:
+    """Plain GPU tensors that nothing differentiates through or transforms; the others are padded with tensor operations."""
+    return (x.is_cuda and cu.device == x.device and cu.dtype == torch.int32 and cu.is_contiguous() and x.is_contiguous() and type(x) is torch.Tensor
+            and not (torch.is_grad_enabled() and x.requires_grad) and not torch._C._functorch.is_functorch_wrapped_tensor(x)
+            and torch.autograd.forward_ad._current_level < 0 and not torch.jit.is_tracing() and ops.extension_available())
 
 
 def sinusoidal_table(n_pos: int, dim: int) -> torch.Tensor:

@@ -194,6 +194,23 @@ Tensor dropout_add(const Tensor& x, const OptTensor& residual, double p, int64_t
   return y;
 }
 
+Tensor pad_rows(const Tensor& x, const Tensor& cu, int64_t T, bool time_first) {
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.dim() >= 1, "pad_rows: x must be contiguous rows on a GPU");
+  TORCH_CHECK(cu.is_cuda() && cu.is_contiguous() && cu.scalar_type() == at::kInt && cu.numel() >= 1 && cu.device() == x.device(),
+              "pad_rows: cu must be int32 on the same GPU");
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t B = cu.numel() - 1;
+  std::vector<int64_t> shape = x.sizes().vec();
+  const int64_t rows = shape[0], per = rows > 0 ? x.numel() / rows : 0;
+  shape[0] = time_first ? B : T;
+  shape.insert(shape.begin(), time_first ? T : B);
+  if (rows == 0 || B * T * per == 0) return torch::zeros(shape, x.options());
+  Tensor out = torch::empty(shape, x.options());
+  ck(nmtg_pad_rows(x.data_ptr(), out.data_ptr(), cu.data_ptr<int>(), static_cast<int>(B), static_cast<int>(T), per * x.element_size(),
+                   static_cast<int>(rows), time_first, cur_stream()));
+  return out;
+}
+
 Tensor act_backward(const Tensor& dy, const Tensor& z, int64_t act, double p, int64_t seed, int64_t stream_id) {
   need_bf16(dy, "dy"); need_bf16(z, "z");
   TORCH_CHECK(dy.is_contiguous() && z.is_contiguous() && dy.numel() == z.numel());
@@ -566,6 +583,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dropout_colsum", &dropout_colsum);
   m.def("embed_fwd", &embed_fwd);
   m.def("embed_bwd", &embed_bwd);
+  m.def("pad_rows", &pad_rows);
   m.def("colsum", &colsum);
   m.def("sq_norm", &sq_norm);
   m.def("adamw_flat", &adamw_flat);

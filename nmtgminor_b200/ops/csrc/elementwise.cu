@@ -288,6 +288,23 @@ __global__ void colsum_wide_kernel(const __nv_bfloat16* __restrict__ x, float* _
   }
 }
 
+// Packed rows -> padded layout, zeros behind every sequence: one pass in units of sizeof(U) bytes, neighbouring threads on neighbouring
+// units.  It is bound by the bytes (one read, one write); one copy and one mask fill per sentence cost 2.5 ms of launches for the 128
+// sentences of a scoring batch whose kernels take 4.9 ms.
+template <typename U>
+__global__ void pad_rows_kernel(const U* __restrict__ x, U* __restrict__ out, const int* __restrict__ cu, int B, int T, long per, int rows,
+                                int time_first) {
+  const long total = static_cast<long>(B) * T * per;
+  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total; i += static_cast<long>(gridDim.x) * blockDim.x) {
+    const long slot = i / per, c = i - slot * per;
+    const int b = static_cast<int>(time_first ? slot % B : slot / T), t = static_cast<int>(time_first ? slot / B : slot % T);
+    const long row = static_cast<long>(cu[b]) + t;
+    U v{};
+    if (row >= 0 && row < cu[b + 1] && row < rows) v = x[row * per + c];
+    out[i] = v;
+  }
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -375,6 +392,26 @@ const char* nmtg_embed_bwd(const int64_t* tokens, const int64_t* positions, cons
   embed_bwd_kernel<<<grid, 64, 0, stream>>>(tokens, positions, reinterpret_cast<const __nv_bfloat16*>(dy), dtable, dpos,
                                             rows, hidden, vocab, max_pos, scale, p, seed, stream_id, seed_dev, pad_idx);
   return last_err();
+}
+
+const char* nmtg_pad_rows(const void* x, void* out, const int* cu, int B, int T, long row_bytes, int rows, int time_first, cudaStream_t stream) {
+  if (B <= 0 || T <= 0 || row_bytes <= 0) return nullptr;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | static_cast<uintptr_t>(row_bytes);
+  auto go = [&](auto unit) -> const char* {
+    using U = decltype(unit);
+    const long per = row_bytes / static_cast<long>(sizeof(U)), total = static_cast<long>(B) * T * per;
+    long blocks = (total + 255) / 256;
+    if (blocks > static_cast<long>(num_sms()) * 16) blocks = static_cast<long>(num_sms()) * 16;
+    pad_rows_kernel<U><<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<const U*>(x), static_cast<U*>(out), cu, B, T, per, rows,
+                                                                     time_first);
+    return last_err();
+  };
+  // the widest unit that the row length and both addresses allow
+  if (at % 16 == 0) return go(uint4{});
+  if (at % 8 == 0) return go(uint2{});
+  if (at % 4 == 0) return go(uint32_t{});
+  if (at % 2 == 0) return go(uint16_t{});
+  return go(uint8_t{});
 }
 
 const char* nmtg_colsum(const void* x, float* out, int rows, int cols, long ld, cudaStream_t stream) {

@@ -111,6 +111,8 @@ const char* nmtg_embed_bwd(const int64_t* tokens, const int64_t* positions, cons
                            int rows, int hidden, int vocab, int max_pos, float scale, float p, unsigned long long seed,
                            unsigned long long stream_id, const unsigned long long* seed_dev, int pad_idx,
                            cudaStream_t stream);
+// Packed rows of row_bytes each (sequence b: rows cu[b] .. cu[b + 1] - 1) -> out [B, T] or, with time_first, [T, B] rows, zeros elsewhere.
+const char* nmtg_pad_rows(const void* x, void* out, const int* cu, int B, int T, long row_bytes, int rows, int time_first, cudaStream_t stream);
 // out[c] += sum over rows of bf16 x[r, c]
 const char* nmtg_colsum(const void* x, float* out, int rows, int cols, long ld, cudaStream_t stream);
 

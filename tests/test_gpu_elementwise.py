@@ -245,3 +245,25 @@ def test_act_backward_one_pass(act, p):
     yr = {1: torch.relu, 2: torch.nn.functional.gelu, 3: torch.nn.functional.silu}[act](zr)
     yr.square().sum().backward()
     _close(x.grad, xr.grad, 0.15 * xr.grad.abs().max().item(), 5e-2, "linear+act input gradient")
+
+
+@pytest.mark.parametrize("dtype,width", [(torch.bfloat16, 64), (torch.bfloat16, 12), (torch.float32, 1), (torch.float32, 3), (torch.int64, 1),
+                                         (torch.bool, 5), (torch.bfloat16, 1)])
+def test_pad_rows_matches_tensor_operations(dtype, width):
+    """One pass over packed rows against one copy per sequence: empty, full and single sequences, rows behind the last one, every unit
+    width, and a view that starts off a 16-byte boundary."""
+    from nmtgminor_b200.models.layers import PackedSeqs
+    from nmtgminor_b200.ops.reference import pad_packed
+    g = torch.Generator(device="cuda").manual_seed(width)
+    for lengths, extra, max_len in (([3, 0, 7, 1], 5, 7), ([4], 0, 9), ([0, 0], 2, 3), ([130] * 9, 1, 130)):
+        n = sum(lengths) + extra
+        full = torch.randint(0, 2, (n + 1, width), device="cuda", generator=g) * 3 + 1
+        x = (full.to(dtype) if dtype != torch.bool else full > 1)[1:]
+        cu = torch.tensor([0] + lengths, device="cuda").cumsum(0).int()
+        seqs = PackedSeqs(torch.zeros(n, dtype=torch.long, device="cuda"), torch.zeros(n, dtype=torch.long, device="cuda"), cu, max_len)
+        want = pad_packed(x, cu, max_len)[0]
+        assert torch.equal(seqs.pad(x, time_first=False), want)
+        assert torch.equal(seqs.pad(x), want.transpose(0, 1)) and seqs.pad(x).is_contiguous()
+    too_long = PackedSeqs(seqs.tokens, seqs.positions, cu, 129)
+    with pytest.raises(RuntimeError):
+        too_long.pad(x)
