@@ -50,7 +50,7 @@ struct GemmDesc {
   float dropout_p; unsigned long long seed, stream_id;
   const unsigned long long* seed_dev;  // optional device word added to seed (lets graph replays draw new masks)
   int split_k;            // 0 = automatic (only when allow_split_k), else forced
-  int allow_split_k;
+  int allow_split_k;      // the sum over K may be split: fp32 outputs (atomic adds), and bf16 outputs with few rows (CTA clusters)
   int force_bn;           // 0 = automatic, 128 or 256
   int* status;            // device int, 0 = ok
   const NmtgGather* gather;  // optional: B is gathered from its owners by this call (see NmtgGather)

@@ -249,12 +249,12 @@ def test_few_row_gemm(M, N, K, overlap):
     ops.ext().set_step_overlap(overlap)
     try:
         for act, fn in ((0, lambda t: t), (1, torch.relu), (2, torch.nn.functional.gelu), (3, torch.nn.functional.silu)):
-            ops.gemm(x, w, out, bias=bias, act=act)
+            ops.gemm(x, w, out, bias=bias, act=act, allow_split_k=True)
             # one rounding to bf16 (2^-9) and 32-bit sums of K products of order K^-0.5
             assert torch.allclose(out.double(), fn(acc), rtol=2 ** -8, atol=2 ** -10), (act, (out.double() - fn(acc)).abs().max())
         y = ops.empty_rows(M, N, "cuda")
         y.copy_(res)
-        ops.gemm(x, w, y, residual=y)
+        ops.gemm(x, w, y, residual=y, allow_split_k=True)
         assert torch.allclose(y.double(), acc - bias.double() + res.double(), rtol=2 ** -8, atol=2 ** -10)
     finally:
         ops.ext().set_step_overlap(False)
