@@ -122,7 +122,10 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
     uint32_t r[32];
     tmem_ld32(taddr, r);
     tmem_ld_wait();
-    if (!row_ok || p.ablate == 1) return;
+    const bool live = row_ok && p.ablate != 1;
+    // column sums straight from registers need every lane of the warp (single-CTA kernel; the host pairs them with the mask epilogue only)
+    const bool sum_here = (kFeat & kEpiColsum) && p.colsum != nullptr && stage_row == nullptr;
+    if (!live && !sum_here) return;
     float v[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
@@ -278,6 +281,26 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
         *reinterpret_cast<uint4*>(stage_row + (((stage_half * 4 + g) ^ (stage_r & 7)) << 4)) = o;
       }
     } else {
+      if (sum_here) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = live ? __bfloat162float(__float2bfloat16(v[j])) : 0.f;
+        float t[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) t[j] = v[j];
+        // 32 rows x 32 columns: the lanes halve their lists while they add, lane l ends with column l
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const bool hi = (threadIdx.x & o) != 0;
+#pragma unroll
+          for (int j = 0; j < o; ++j) {
+            const float keep = hi ? t[j + o] : t[j], give = hi ? t[j] : t[j + o];
+            t[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+        const int c = col0 + static_cast<int>(threadIdx.x & 31);
+        if (c < p.N) atomicAdd(p.colsum + c, t[0]);
+        if (!live) return;
+      }
       __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<size_t>(row) * p.ld_out + col0;
       if (full_cols) {
 #pragma unroll

@@ -367,6 +367,28 @@ static const char* launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, con
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
 
+// The epilogues of the shapes a training step is made of (as in the CTA-pair kernel); anything else takes the general one.
+template <int BN>
+static const char* launch_gemm_special(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& a, int grid, bool generic,
+                                       cudaStream_t stream) {
+  constexpr uint32_t kPlain = kEpiBf16;
+  constexpr uint32_t kFc1 = kEpiBf16 | kEpiBias | kEpiActFwd | kEpiDrop | kEpiMaskOut;
+  constexpr uint32_t kOutRes = kEpiBf16 | kEpiBias | kEpiDrop | kEpiRes;
+  constexpr uint32_t kDgradMask = kEpiBf16 | kEpiMaskBwd | kEpiColsum;
+  constexpr uint32_t kAccum = kEpiF32;
+  constexpr uint32_t kFc1Preact = kEpiBf16 | kEpiBias | kEpiActFwd | kEpiDrop | kEpiPreact;
+  constexpr uint32_t kDgradAct = kEpiBf16 | kEpiActBwd | kEpiDrop;
+  const uint32_t need = generic ? kEpiAll : gemm_epilogue_features(a);
+  if ((need & ~kPlain) == 0) return launch_gemm<BN, kPlain>(ta, tb, a, grid, stream);
+  if ((need & ~kAccum) == 0) return launch_gemm<BN, kAccum>(ta, tb, a, grid, stream);
+  if ((need & ~kDgradMask) == 0) return launch_gemm<BN, kDgradMask>(ta, tb, a, grid, stream);
+  if ((need & ~kOutRes) == 0) return launch_gemm<BN, kOutRes>(ta, tb, a, grid, stream);
+  if ((need & ~kFc1) == 0) return launch_gemm<BN, kFc1>(ta, tb, a, grid, stream);
+  if ((need & ~kFc1Preact) == 0) return launch_gemm<BN, kFc1Preact>(ta, tb, a, grid, stream);
+  if ((need & ~kDgradAct) == 0) return launch_gemm<BN, kDgradAct>(ta, tb, a, grid, stream);
+  return launch_gemm<BN>(ta, tb, a, grid, stream);
+}
+
 }  // namespace b200
 
 namespace b200 {
@@ -398,6 +420,41 @@ void nmtg_set_gemm_variant(int v) {
   else if (v == 20 || v == 21) b200::g_pair_tma_store = v - 20;   // 20: per-thread stores, 21: TMA-store epilogue (default)
   else if (v >= 10) g_gemm_ablate = v - 10;
   else g_gemm_variant = v;
+}
+
+// Tile width (64 or 128 columns, one CTA each) for a problem that is smaller than a wave of such tiles, or 0 for the CTA-pair kernel.
+// A 64-deep step of the main loop takes much the same time in all three kernels when a CTA has one tile to work on (0.31 us,
+// 0.36 us for a pair: latency, not bandwidth), so what counts is the fixed cost - set-up, and an epilogue that nothing hides,
+// over 64, 128 or 256 columns - and how many SMs take part.  Measured (us, pair / 64 / 128 columns): 1920 x 512 x 512 with
+// dropout and residual 12.5 / 7.3 / 8.8, 704 x 1024 x 256 with ReLU, dropout and mask 11.5 / 6.2 / 7.5, 3840 x 512 x 2048 22.7 / 25.3 (two
+// waves) / 17.7, weight gradient 512 x 512 x 1920 14.1 / 8.7 / 10.0; beyond one wave the pair wins: 3840 x 1024 x 1024 16.2 / 26.4 /
+// 17.6.  The estimates below are fitted to such measurements for widths 256 to 1024 and 704 to 5632 rows.
+static int one_wave_tile(const GemmDesc* d, int sms, int num_kb, int* split) {
+  const bool sums = d->out_fp32 && d->allow_split_k && d->accumulate;
+  if (d->out_fp32 && !sums) return 0;
+  const int clusters = sms / 2, bn_pair = d->N > 128 ? 256 : 128;
+  const long pairs = static_cast<long>((d->M + 2 * BM - 1) / (2 * BM)) * ((d->N + bn_pair - 1) / bn_pair);
+  long pair_split = 1;
+  while (sums && pairs * pair_split * 2 <= clusters && num_kb / (pair_split * 2) >= 8) pair_split *= 2;
+  const long waves = (pairs * pair_split + clusters - 1) / clusters;
+  double best = (sums ? 9.5 : 8.0) + 0.36 * static_cast<double>((num_kb + pair_split - 1) / pair_split) * waves - 0.5;
+  int bn = 0;
+  for (int w = 64; w <= 128; w += 64) {
+    const long tiles = static_cast<long>((d->M + BM - 1) / BM) * ((d->N + w - 1) / w);
+    if (tiles > sms) continue;
+    long s = 1;
+    if (sums) {                          // at least six steps for a CTA: the partial tiles meet in atomic adds
+      s = sms / tiles < num_kb / 6 ? sms / tiles : num_kb / 6;
+      if (s < 1) s = 1;
+    }
+    const double t = (w == 64 ? 5.2 : 6.0) + (sums ? 0.4 : 0.0) + 0.31 * static_cast<double>((num_kb + s - 1) / s);
+    if (t < best) {
+      best = t;
+      bn = w;
+      *split = static_cast<int>(s);
+    }
+  }
+  return bn;
 }
 
 // Returns nullptr on success, else a static error string.
@@ -480,12 +537,17 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
       return launch_gemm<64, kActivated>(ta, tb, a, grid, stream);
     }
     if (bn == 256) return launch_gemm<256>(ta, tb, a, grid, stream);
-    if (bn == 128) return launch_gemm<128>(ta, tb, a, grid, stream);
-    return launch_gemm<64>(ta, tb, a, grid, stream);
+    if (bn == 128) return launch_gemm_special<128>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
+    return launch_gemm_special<64>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
   }
+  // ---- problems whose 128 x 64 or 128 x 128 tiles are one wave: see one_wave_tile
+  int narrow_bn = 0, narrow_split = 1;
+  if (g_gemm_variant == 0 && d->M > BM && !d->gather && d->force_bn == 0 && d->split_k <= 0 && a.trace == nullptr && g_gemm_ablate == 0 &&
+      (!d->colsum || (gemm_epilogue_features(a) & ~(kEpiBf16 | kEpiMaskBwd | kEpiColsum)) == 0))
+    narrow_bn = one_wave_tile(d, sms, num_kb, &narrow_split);
   // ---- CTA-pair kernel (256-row tiles): the default for everything but very small M ----------------
   if (d->colsum && d->M <= BM) return "gemm: the column-sum output needs more than 128 rows (CTA-pair kernel)";
-  if ((g_gemm_variant != 1 || d->colsum) && d->M > BM) {
+  if (g_gemm_variant != 1 && d->M > BM && narrow_bn == 0) {
     int bn = (d->N > 128) ? 256 : 128;
     if (d->force_bn == 128 || d->force_bn == 256) bn = d->force_bn;
     if (d->gather) {
@@ -525,10 +587,12 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
     auto waves_eff = [&](long t) { long w = (t + sms - 1) / sms; return static_cast<double>(t) / (w * sms); };
     if (bn == 256 && waves_eff(t128) > waves_eff(t256) + 0.15) bn = 128;
   }
-  if (d->force_bn == 128 || d->force_bn == 256) bn = d->force_bn;
+  if (d->force_bn == 64 || d->force_bn == 128 || d->force_bn == 256) bn = d->force_bn;
+  if (narrow_bn) bn = narrow_bn;
   const int num_n = (d->N + bn - 1) / bn;
   int split = 1;
   if (d->split_k > 0) split = d->split_k;
+  else if (narrow_bn) split = narrow_split;
   else if (d->out_fp32 && d->allow_split_k) {
     long tiles = static_cast<long>(num_m) * num_n;
     while (tiles * split * 2 <= sms && num_kb / (split * 2) >= 8) split *= 2;
@@ -548,5 +612,6 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   long tiles = static_cast<long>(num_m) * num_n * split;
   int grid = static_cast<int>(tiles < sms ? tiles : sms);
   if (bn == 256) return launch_gemm<256>(ta, tb, a, grid, stream);
-  return launch_gemm<128>(ta, tb, a, grid, stream);
+  if (bn == 64) return launch_gemm_special<64>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
+  return launch_gemm_special<128>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
 }

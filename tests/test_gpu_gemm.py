@@ -259,3 +259,40 @@ def test_few_row_gemm(M, N, K, overlap):
     finally:
         ops.ext().set_step_overlap(False)
     assert ops.check_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 64, 64), (200, 72, 128), (704, 256, 1024), (1000, 1032, 264), (1920, 512, 512), (2300, 520, 200), (3840, 512, 1000)])
+def test_one_wave_tiles(M, N, K):
+    """Products that fit a wave of narrow tiles, next to the same ones on the CTA-pair kernel: every epilogue of a training step, with the
+    column sums from registers, ragged rows and columns, and weight gradients split over K."""
+    e = ops.ext()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w, bias, res, dy = rnd(M, K), rnd(N, K) * K ** -0.5, rnd(N), rnd(M, N), rnd(M, N) * K ** -0.5
+    got = {}
+    for name, forced in (("auto", 0), ("pair", 256)):
+        e.set_gemm_variant(0)
+        out = {}
+        n = lambda: torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+        ops.gemm(x, w, out.setdefault("plain", n()), force_bn=forced)
+        out["bits"] = torch.zeros(M, (N + 31) // 32, device="cuda", dtype=torch.int32)
+        ops.gemm(x, w, out.setdefault("fc1", n()), bias=bias, act=1, dropout_p=0.25, seed=3, stream_id=9, mask=out["bits"], force_bn=forced)
+        ops.gemm(x, w, out.setdefault("pre_out", n()), bias=bias, act=2, preact=out.setdefault("pre", n()), force_bn=forced)
+        ops.gemm(x, w, out.setdefault("res", n()), bias=bias, residual=res, dropout_p=0.25, seed=3, stream_id=10, force_bn=forced)
+        ops.gemm(x, w, out.setdefault("act_bwd", n()), aux=res, act=6, force_bn=forced)
+        cs = out["colsum"] = torch.ones(N, device="cuda")
+        ops.gemm(x, w, out.setdefault("masked", n()), act=8, mask=out["bits"], alpha=1.25, colsum=cs, force_bn=forced)
+        dw = out["dw"] = torch.ones(N, K, device="cuda")
+        ops.gemm(dy, x, dw, a_mn_major=True, b_mn_major=True, accumulate=True, allow_split_k=True, force_bn=forced)
+        got[name] = out
+    assert ops.check_status() == 0
+    for k in got["auto"]:
+        a, b = got["auto"][k], got["pair"][k]
+        if k == "colsum":       # 32-bit sums of M values of order 1 in another order
+            want = 1 + got["auto"]["masked"].double().sum(0)
+            assert (a.double() - want).abs().max() < 2 ** -20 * M + 1e-4 and (b.double() - want).abs().max() < 2 ** -20 * M + 1e-4
+        elif k == "dw":
+            want = 1 + dy.double().t() @ x.double()
+            assert (a.double() - want).abs().max() < 2 ** -20 * M
+        else:                   # one accumulator per element, its products in the same order
+            assert torch.equal(a, b), k
