@@ -35,6 +35,7 @@ struct GemmArgs {
   const unsigned long long* seed_dev;
   int* status;
   int tma_store;           // bf16 output leaves through shared memory and TMA stores (CTA-pair kernel)
+  int tma_second;          // so does the pre-activation, and the aux operand comes in that way (see two_stagings)
   int ablate;              // profiling aid: 1 = read the accumulator but skip arithmetic and stores, 2 = skip the epilogue body,
                            // 3 (traced kernel only) = also skip the MMAs: operand streaming alone
   long long* trace;        // profiling aid: when set, the CTA-pair kernel writes up to 16 cycle counters per cluster (see gemm2cta_tcgen05.cu)
@@ -57,17 +58,39 @@ struct GatherArgs {
   int* counters;            // [0]: CTAs that have left the kernel, [1]: next unclaimed block, [2 + s]: finished blocks of segment s
 };
 
-__device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
+// erfc(|x| / sqrt 2) / 2, the upper tail of the normal distribution, by the Chebyshev fit of Press et al., Numerical Recipes, section 6.2
+// (erfcc; relative error below 1.2e-7 everywhere): one reciprocal, one exponential, ten multiply-adds and no branch.  1 + erff(x)
+// is no closer in the middle, loses the lower tail to cancellation, and its two ranges cost an epilogue of 32 unrolled elements 16 us of
+// 44 (6144 x 2048 x 512 with the GELU gradient).
+__device__ __forceinline__ float normal_tail(float x) {
+  const float z = fabsf(x) * 0.70710678118654752f;
+  const float t = __fdividef(1.f, fmaf(0.5f, z, 1.f));
+  float q = fmaf(t, 0.17087277f, -0.82215223f);
+  q = fmaf(t, q, 1.48851587f);
+  q = fmaf(t, q, -1.13520398f);
+  q = fmaf(t, q, 0.27886807f);
+  q = fmaf(t, q, -0.18628806f);
+  q = fmaf(t, q, 0.09678418f);
+  q = fmaf(t, q, 0.37409196f);
+  q = fmaf(t, q, 1.00002368f);
+  q = fmaf(t, q, -1.26551223f);
+  return 0.5f * t * __expf(fmaf(-z, z, q));
+}
+__device__ __forceinline__ float normal_cdf(float x) {
+  const float tail = normal_tail(x);
+  return x < 0.f ? tail : 1.f - tail;
+}
+__device__ __forceinline__ float gelu_f(float x) { return x * normal_cdf(x); }
 __device__ __forceinline__ float gelu_grad(float x) {
-  float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
-  float pdf = 0.3989422804014327f * __expf(-0.5f * x * x);
-  return cdf + x * pdf;
+  const float pdf = 0.3989422804014327f * __expf(-0.5f * x * x);
+  return normal_cdf(x) + x * pdf;
 }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 
 // One thread = one accumulator row; processes columns [col0, col0 + 32) read from TMEM address `taddr`:
 // alpha, bias, optional pre-activation store, activation or activation gradient, dropout, residual, store
 // (bf16, fp32, fp32 accumulate, or fp32 red.add for split-K).  Warp-collective (contains a tcgen05.ld).
+// `pre_row`: the same for the pre-activation; `aux_staged`: the aux operand has been copied into the staging row.
 // `stage_row` (optional): instead of writing bf16 results to global memory, place the 64-byte row fragment in a
 // shared-memory staging row laid out for a 128-byte-swizzled TMA store (logical 16-byte chunk j of row r sits at
 // chunk j ^ (r & 7)); `stage_half` selects the left / right 32 columns of the 64-column staging tile.
@@ -101,11 +124,12 @@ template <uint32_t kFeat = kEpiAll>
 __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const DropRng& rng, const bool do_drop, const int row,
                                                     const bool row_ok, const int col0, const uint32_t taddr,
                                                     uint8_t* stage_row = nullptr, const int stage_half = 0,
-                                                    const int stage_r = 0) {
+                                                    const int stage_r = 0, uint8_t* pre_row = nullptr,
+                                                    const bool aux_staged = false) {
     const bool full_cols = !(kFeat & kEpiRagged) || (col0 + 32 <= p.N);
     // global operands of the epilogue are requested BEFORE the TMEM load so their latency overlaps it
     uint4 aux_v[4], res_v[4];
-    const bool aux_vec = (kFeat & kEpiActBwd) && row_ok && full_cols && p.act >= kActReluBwd && p.act != kActMaskBwd && (p.ld_aux & 7) == 0;
+    const bool aux_vec = (kFeat & kEpiActBwd) && !aux_staged && row_ok && full_cols && p.act >= kActReluBwd && p.act != kActMaskBwd && (p.ld_aux & 7) == 0;
     uint32_t mask_word = 0;
     if ((kFeat & kEpiMaskBwd) && p.act == kActMaskBwd && row_ok) mask_word = p.mask[static_cast<size_t>(row) * p.ld_mask + (col0 >> 5)];
     const bool res_vec = (kFeat & kEpiRes) && row_ok && full_cols && p.residual != nullptr && (p.ld_res & 7) == 0;
@@ -150,7 +174,16 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
     }
     if ((kFeat & kEpiPreact) && p.preact) {
       __nv_bfloat16* pp = p.preact + static_cast<size_t>(row) * p.ld_out + col0;
-      if (full_cols) {
+      if (pre_row != nullptr) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint4 o;
+          __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(v[g * 8 + 2 * j], v[g * 8 + 2 * j + 1]);
+          *reinterpret_cast<uint4*>(pre_row + (((stage_half * 4 + g) ^ (stage_r & 7)) << 4)) = o;
+        }
+      } else if (full_cols) {
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           uint4 o;
@@ -171,7 +204,11 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
     } else if ((kFeat & kEpiActBwd) && p.act >= kActReluBwd) {
       const __nv_bfloat16* ap = p.aux + static_cast<size_t>(row) * p.ld_aux + col0;
       float av[32];
-      if (aux_vec) {
+      if (aux_staged) {       // the operand's row fragment lies where the result will be put
+#pragma unroll
+        for (int g4 = 0; g4 < 4; ++g4) aux_v[g4] = *reinterpret_cast<const uint4*>(stage_row + (((stage_half * 4 + g4) ^ (stage_r & 7)) << 4));
+      }
+      if (aux_vec || aux_staged) {
 #pragma unroll
         for (int g4 = 0; g4 < 4; ++g4) {
           uint4 u = aux_v[g4];
@@ -187,14 +224,20 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
 #pragma unroll
         for (int j = 0; j < 32; ++j) av[j] = (col0 + j < p.N) ? __bfloat162float(ap[j]) : 0.f;
       }
+      // one loop per activation: decided per element, the 32 copies of every branch overran the instruction cache (6144 x 2048 x 512
+      // with the ReLU gradient 45.8 us, 23.3 so)
+      if (p.act == kActReluBwd) {          // aux = relu output (after dropout)
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float a = av[j];
-        float g;
-        if (p.act == kActReluBwd) g = a > 0.f ? 1.f : 0.f;  // aux = relu output (after dropout)
-        else if (p.act == kActGeluBwd) g = gelu_grad(a);
-        else { float s = sigmoid_f(a); g = s * (1.f + a * (1.f - s)); }
-        v[j] *= g;
+        for (int j = 0; j < 32; ++j) v[j] *= av[j] > 0.f ? 1.f : 0.f;
+      } else if (p.act == kActGeluBwd) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] *= gelu_grad(av[j]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float s = sigmoid_f(av[j]);
+          v[j] *= s * (1.f + av[j] * (1.f - s));
+        }
       }
     } else if ((kFeat & kEpiActFwd) && p.act == kActRelu) {
 #pragma unroll

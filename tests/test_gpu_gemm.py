@@ -296,3 +296,47 @@ def test_one_wave_tiles(M, N, K):
             assert (a.double() - want).abs().max() < 2 ** -20 * M
         else:                   # one accumulator per element, its products in the same order
             assert torch.equal(a, b), k
+
+
+def test_gelu_epilogues_over_the_whole_range():
+    """GELU and its gradient against 64 bits for inputs from the lower tail to far above: every result within one bf16 rounding, plus
+    the 1.2e-7 of the tail's fit where the result cancels (the gradient's zero near -0.75)."""
+    n = 512
+    x = torch.linspace(-12, 12, 256 * n, device="cuda").view(256, n).bfloat16()
+    eye = torch.eye(n, device="cuda").bfloat16()
+    out, ones = torch.empty(256, n, device="cuda", dtype=torch.bfloat16), torch.ones(256, n, device="cuda").bfloat16()
+    xd = x.double()
+    cdf, pdf = 0.5 * torch.erfc(-xd / 2 ** 0.5), torch.exp(-0.5 * xd * xd) / (2 * torch.pi) ** 0.5
+    ops.gemm(x, eye, out, act=2)
+    assert ((out.double() - xd * cdf).abs() <= 2 ** -8 * (xd * cdf).abs() + 1e-37).all()
+    ops.gemm(ones, eye, out, aux=x, act=6)
+    want = cdf + xd * pdf
+    assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 3e-7 * (cdf + (xd * pdf).abs())).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(5000, 2048, 512), (6100, 1600, 192), (9000, 1344, 64)])
+def test_second_matrix_epilogues(M, N, K):
+    """Activation gradients and stored pre-activations of many-wave products, whose second matrix goes through shared memory: ragged rows,
+    a last column tile with work for half of the warps only; equal to the general epilogue, which reads and writes from the lanes."""
+    e = ops.ext()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w, bias, aux = rnd(M, K), rnd(N, K) * K ** -0.5, rnd(N), rnd(M, N)
+    got = []
+    try:
+        for variant in (30, 31):
+            e.set_gemm_variant(variant)
+            out = []
+            for act in (5, 6, 7):
+                for p in (0.0, 0.25):
+                    out.append(torch.zeros(M, N, device="cuda", dtype=torch.bfloat16))
+                    ops.gemm(x, w, out[-1], aux=aux, act=act, dropout_p=p, seed=3, stream_id=act)
+            for act in (1, 2, 3):
+                out += [torch.zeros(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+                ops.gemm(x, w, out[-2], bias=bias, act=act, preact=out[-1], dropout_p=0.25, seed=3, stream_id=act)
+            got.append(out)
+    finally:
+        e.set_gemm_variant(30)
+    assert ops.check_status() == 0
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
