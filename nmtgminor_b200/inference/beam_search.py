@@ -180,10 +180,11 @@ class _DeviceSearch:
         self.pool = pool
         (ctl, inv_norm, max_rows, scores, force, done, tok, pos_rows, anc, fin_count, fin_score) = pool["tables"][:11]
         self.tok, self.pos_rows, self.done = tok, pos_rows, done
-        normalize = bool(cfg.normalize and cfg.alpha > 0)
-        ctl.copy_(torch.tensor([T, cfg.min_len, int(normalize)], dtype=torch.int32))
+        # `normalize` alone decides the stop rule; scores are divided only if there is a length penalty as well
+        ctl.copy_(torch.tensor([T, cfg.min_len, int(bool(cfg.normalize))], dtype=torch.int32))
         # reciprocal of the length penalty in the precision of a division by a host scalar
-        inv_norm[1:T + 2].copy_(1.0 / torch.tensor([float(n) ** cfg.alpha if normalize else 1.0 for n in range(1, T + 2)], dtype=torch.float32))
+        penalty = bool(cfg.normalize and cfg.alpha > 0)
+        inv_norm[1:T + 2].copy_(1.0 / torch.tensor([float(n) ** cfg.alpha if penalty else 1.0 for n in range(1, T + 2)], dtype=torch.float32))
         max_rows.copy_(max_len_per)
         scores.fill_(float("-inf"))
         scores.view(B, K)[:, 0] = 0.0                       # only the first hypothesis is alive at step 0

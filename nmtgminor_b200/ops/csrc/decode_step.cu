@@ -552,7 +552,9 @@ beam_part_kernel(const T* __restrict__ logits, long ld, const uint8_t* __restric
 }
 
 // Everything that the search does between two steps, one CTA per sentence.
-//   ctl = {T, min_len, normalize}; inv_norm[n] = 1 / n^alpha for n = 1 .. T + 1 (1 without normalisation)
+//   ctl = {T, min_len, normalize}; inv_norm[n] = 1 / n^alpha for n = 1 .. T + 1 (1 without normalisation or with alpha <= 0).
+//   `normalize` chooses the stop rule: with it a sentence goes on until its best active hypothesis, at the longest length, cannot beat the
+//   worst finished one; without it the first K finished hypotheses end it
 __global__ void __launch_bounds__(256)
 beam_advance_kernel(const NmtgBeam s, const void* logits, int bf16, long ld, const float2* __restrict__ part_lse,
                     const Cand* __restrict__ part, int pieces, int V, int staged) {
@@ -670,7 +672,7 @@ beam_advance_kernel(const NmtgBeam s, const void* logits, int bf16, long ld, con
           const float v = top_val[j];
           if (row_tok[top_c[j]] != s.eos || !isfinite(v)) continue;
           ++ended;
-          const float score = normalize ? v * inv_here : v;
+          const float score = v * inv_here;
           int at = K;
           while (at > 0 && fs[at - 1] < score) --at;              // behind its equals
           if (at == K) continue;

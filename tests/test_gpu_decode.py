@@ -168,11 +168,7 @@ def test_step_cross_attention(B, K, heads, cap):
             assert (out[b * K:(b + 1) * K].double() - want).abs().max() <= 2 ** -8 * want.abs().max() + 1e-6
 
 
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("B,K,V,T,min_len,normalize", [(1, 1, 40, 6, 0, False), (3, 4, 50, 12, 1, False), (5, 4, 4097, 9, 3, True),
-                                                       (2, 6, 8200, 7, 0, True), (2, 32, 5000, 5, 1, False), (4, 3, 1000, 10, 10, True)])
-def test_device_search_matches_host_bookkeeping(dtype, B, K, V, T, min_len, normalize):
-    """The step kernels against the tensor statements of the same search, on logits that depend on the last word and the step."""
+def _compare_searches(dtype, B, K, V, T, min_len, normalize, alpha, end_bias=None):
     from types import SimpleNamespace
 
     from nmtgminor_b200.inference import beam_search as bs
@@ -181,6 +177,13 @@ def test_device_search_matches_host_bookkeeping(dtype, B, K, V, T, min_len, norm
     by_word = torch.randn(V, ld, device="cuda", generator=g)
     by_word[:, 3] += 1.5                                   # EOS is likely enough to end hypotheses early
     by_step = torch.randn(T + 2, ld, device="cuda", generator=g)
+    if end_bias is not None:                               # EOS is a weak continuation at first and a strong one from step 4 on
+        h = torch.Generator().manual_seed(V + T)
+        by_word, by_step = torch.randn(V, ld, generator=h), torch.randn(T + 2, ld, generator=h)
+        by_word[:, 3] += 1.5 + end_bias
+        by_word[torch.arange(V), torch.randint(4, V, (V,), generator=h)] += 6
+        by_step[:4, 3], by_step[4:, 3] = 0.0, by_step[4:, 3] + 12
+        by_word, by_step = by_word.cuda(), by_step.cuda()
     logits_of = lambda tok, step: (by_word[tok] + by_step[step]).to(dtype)[:, :V]
     lens = torch.randint(2, 9, (B,), device="cuda", generator=g)
 
@@ -197,7 +200,7 @@ def test_device_search_matches_host_bookkeeping(dtype, B, K, V, T, min_len, norm
     model = SimpleNamespace(supports_logits_step=True, decoder=torch.nn.Module(), create_decoder_state=lambda batch, k: State())
     model.step = lambda tokens, state, logits_only=False: {"logits": logits_of(tokens[:, -1], tokens.shape[1] - 1)}
     cfg = bs.BeamConfig(beam_size=K, n_best=K, max_len=T, min_len=min_len, dynamic_max_len=True, len_a=1.0, len_b=T - 8, normalize=normalize,
-                        alpha=0.6 if normalize else 0.0)
+                        alpha=alpha)
     want = bs.beam_search(model, None, cfg)
     limit = (lens.float() + T - 8).clamp(max=T).long()
 
@@ -215,6 +218,23 @@ def test_device_search_matches_host_bookkeeping(dtype, B, K, V, T, min_len, norm
             for x, y in zip(a, b):
                 assert abs(x.score - y.score) <= 2e-5 * max(1.0, abs(x.score)) or x.score == y.score
                 assert torch.allclose(torch.tensor(x.positional_scores), torch.tensor(y.positional_scores), atol=2e-4)
+    cfg.normalize = not normalize
+    return want, bs.beam_search(model, None, cfg)          # the same under the other stop rule
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,K,V,T,min_len,normalize", [(1, 1, 40, 6, 0, False), (3, 4, 50, 12, 1, False), (5, 4, 4097, 9, 3, True),
+                                                       (2, 6, 8200, 7, 0, True), (2, 32, 5000, 5, 1, False), (4, 3, 1000, 10, 10, True)])
+def test_device_search_matches_host_bookkeeping(dtype, B, K, V, T, min_len, normalize):
+    """The step kernels against the tensor statements of the same search, on logits that depend on the last word and the step."""
+    _compare_searches(dtype, B, K, V, T, min_len, normalize, 0.6 if normalize else 0.0)
+
+
+@pytest.mark.parametrize("B,K,V,alpha,end_bias", [(8, 2, 50, 0.0, 2.0), (6, 3, 50, 0.0, 2.0), (6, 3, 50, -0.5, 2.0), (8, 4, 300, 0.0, 3.0)])
+def test_device_search_stop_rule_without_penalty(B, K, V, alpha, end_bias):
+    """`normalize` without a length penalty: the search goes on after `beam` hypotheses have ended while a better one can still come."""
+    found, first_ended = _compare_searches(torch.float32, B, K, V, 24, 0, True, alpha, end_bias)
+    assert any([h.tokens for h in a] != [h.tokens for h in b] for a, b in zip(found, first_ended)), "the inputs must tell the two rules apart"
 
 
 @pytest.mark.parametrize("beam", [1, 2, 5])
