@@ -133,6 +133,38 @@ def _replayable(model, state) -> bool:
             and state.context.is_cuda and state.context.dtype == torch.bfloat16)
 
 
+class _StepPools:
+    """Table sets, and the graphs captured over them, of one model in one state.  A graph has the address of every tensor baked in that
+    its step reads besides its own tables; those tensors are held here, so that as long as the model has the same addresses it
+    has the same tensors.  A model that has others (a longer position table, a new weight store, a layer replaced) gets a new object."""
+
+    def __init__(self, state):
+        self.state = state
+        self.sets = {}
+
+    @classmethod
+    def of(cls, model, device):
+        emb = getattr(model.decoder, "embed", None)
+        table = emb._pos_table(device) if hasattr(emb, "_pos_table") else None
+        held, state = [table], []
+        for part in (model.decoder, getattr(model, "generator", None)):
+            for m in part.modules() if part is not None else ():
+                state.append(m.training)
+                for t in (*m._parameters.values(), *m._buffers.values()):
+                    if t is not None:
+                        held += (t, getattr(t, "work", None))
+        state += [(t.data_ptr(), t.shape) if t is not None else None for t in held]
+        pools = model.__dict__.get("_decode_pools")
+        if pools is None or pools.state != state:
+            pools = model.__dict__["_decode_pools"] = cls(state)
+            # the storage that is there now: a parameter can be pointed at another
+            pools.held = [t.detach() for t in held if t is not None]
+        return pools
+
+    def __reduce__(self):           # a copied or saved model starts without
+        return type(None), ()
+
+
 class _DeviceSearch:
     """A search whose steps never leave the device: embedding, decoder layers over preallocated caches, output projection, best
     continuations and all bookkeeping (finished hypotheses, next active set, ancestors of every cached position) read and
@@ -152,17 +184,14 @@ class _DeviceSearch:
         cap = (T + 2 + 63) // 64 * 64                    # the geometry of a batch, rounded so that batches share it
         emb = getattr(model.decoder, "embed", None)
         if emb is not None and hasattr(emb, "renew"):
-            before = id(getattr(emb, "pos", None))
             emb.renew(cap)
-            if id(getattr(emb, "pos", None)) != before:
-                model.__dict__.pop("_decode_pools", None)      # graphs captured against the old position table are stale
         from ..models.layers import SelfAttention
         widths = [m.dim for m in model.decoder.modules() if isinstance(m, SelfAttention)]
         cross = [b for b in state.buffers if "c_k" in b]
         src_cap = (max(b["c_k"].shape[1] for b in cross) + 63) // 64 * 64 if cross else 0
         self.key = (B, K, cap, src_cap, len(state.buffers), str(dev), cfg.pad, cfg.eos)
-        self.pools = model.__dict__.setdefault("_decode_pools", {})
-        pool = self.pools.pop(self.key, None)
+        self.pools = _StepPools.of(model, dev)
+        pool = self.pools.sets.pop(self.key, None)
         if pool is None:
             mk = lambda shape, dt: torch.zeros(shape, dtype=dt, device=dev)
             i32, f32, i64 = torch.int32, torch.float32, torch.int64
@@ -251,9 +280,9 @@ class _DeviceSearch:
         scores, last = tables[10][:, :n].cpu(), tables[11][:, :n].cpu()
         longest = int(last.masked_fill(scores == float("-inf"), 0).max()) + 1
         words, word_scores = words[:, :, :longest].cpu(), word_scores[:, :, :longest].cpu()
-        if len(self.pools) >= self.MAX_KEPT:
-            self.pools.pop(next(iter(self.pools)), None)
-        self.pools[self.key] = self.pool
+        if len(self.pools.sets) >= self.MAX_KEPT:
+            self.pools.sets.pop(next(iter(self.pools.sets)), None)
+        self.pools.sets[self.key] = self.pool
         results = []
         for b in range(self.B):
             hyps = []

@@ -237,17 +237,13 @@ def test_device_search_stop_rule_without_penalty(B, K, V, alpha, end_bias):
     assert any([h.tokens for h in a] != [h.tokens for h in b] for a, b in zip(found, first_ended)), "the inputs must tell the two rules apart"
 
 
-@pytest.mark.parametrize("beam", [1, 2, 5])
-def test_replayed_search_matches_the_stepwise_one(beam):
-    """Captured steps against the same search launched kernel by kernel, over enough steps and batches that the replays matter; with
-    one hypothesis per sentence the encoder's keys have as many rows as there are hypotheses."""
-    from nmtgminor_b200.data.dataset import collate
+def _successor_model(seed):
+    """A small Transformer on the GPU in which every word prefers one other word."""
     from nmtgminor_b200.data.synthetic import synthetic_dict
-    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
     from nmtgminor_b200.models.transformer import Transformer
     from nmtgminor_b200.options import default_options
     from nmtgminor_b200.parallel.flat import FlatParameterStore
-    torch.manual_seed(beam)
+    torch.manual_seed(seed)
     d = synthetic_dict(300)
     opt = default_options(["-model_size", "256", "-layers", "3", "-n_heads", "4", "-inner_size", "512", "-ffn_activation", "relu"])
     model = Transformer(opt, {"src": d, "tgt": d}).eval()
@@ -256,9 +252,19 @@ def test_replayed_search_matches_the_stepwise_one(beam):
         order = torch.randperm(296) + 4
         model.generator.weight[order] = 1.5 * model.decoder.embed.weight[order.roll(1)]
         model.generator.weight[order[0]] += 1.5 * model.decoder.embed.weight[2]
-    FlatParameterStore(model, "cuda")
+    model.store = FlatParameterStore(model, "cuda")
     for b in model.buffers():
         b.data = b.data.cuda()
+    return model
+
+
+@pytest.mark.parametrize("beam", [1, 2, 5])
+def test_replayed_search_matches_the_stepwise_one(beam):
+    """Captured steps against the same search launched kernel by kernel, over enough steps and batches that the replays matter; with
+    one hypothesis per sentence the encoder's keys have as many rows as there are hypotheses."""
+    from nmtgminor_b200.data.dataset import collate
+    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
+    model = _successor_model(beam)
     g = torch.Generator().manual_seed(3)
     for _ in range(3):
         src = [torch.randint(4, 300, (int(n),), generator=g) for n in torch.randint(3, 40, (7,), generator=g)]
@@ -268,4 +274,37 @@ def test_replayed_search_matches_the_stepwise_one(beam):
             assert a[0].tokens == b[0].tokens
             # the logits are bf16 of up to 32: one rounding that falls the other way moves a score by 2^-3; two of them
             assert abs(a[0].score - b[0].score) <= 0.25
+    assert ops.check_status() == 0
+
+
+def test_replayed_search_follows_the_model():
+    """A second search of the same geometry after the model moved: a longer position table, and a new weight store with other weights.  The
+    old tensors stay allocated and are overwritten, as if something else had been put there."""
+    from nmtgminor_b200.data.dataset import collate
+    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
+    from nmtgminor_b200.parallel.flat import FlatParameterStore
+    model = _successor_model(5)
+    g = torch.Generator().manual_seed(4)
+    src = [torch.randint(4, 300, (int(n),), generator=g) for n in (9, 20, 5)]
+    batch = collate(src, None, padded=True, packed=True, round_to=1).cuda("cuda")
+    search = lambda graph: [h[0] for h in beam_search(model, batch, BeamConfig(beam_size=2, max_len=30, min_len=20, cuda_graph=graph))]
+
+    def same():
+        for a, b in zip(search(True), search(False)):
+            assert a.tokens == b.tokens and abs(a.score - b.score) <= 0.25          # the tolerance of the test above
+    same()
+    first = [h.tokens for h in search(True)]
+    old = model.decoder.embed._pos_work
+    model.renew_buffer(5000)
+    old.normal_(0.0, 3.0)
+    same()
+    old = model.store
+    with torch.no_grad():
+        order = torch.randperm(296, generator=g) + 4
+        for p in (model.generator.weight, model.decoder.embed.weight):
+            p[4:] = p[order.to(p.device)]                  # words change their names
+    model.store = FlatParameterStore(model, "cuda")
+    old.work.zero_()
+    same()
+    assert [h.tokens for h in search(True)] != first
     assert ops.check_status() == 0
