@@ -20,6 +20,7 @@ Functional counterpart of the reference's ``FastTranslator._translate_batch``
 """
 from __future__ import annotations
 
+import threading
 from dataclasses import dataclass, field
 from typing import List, Optional
 
@@ -136,14 +137,35 @@ def _replayable(model, state) -> bool:
 class _StepPools:
     """Table sets, and the graphs captured over them, of one model in one state.  A graph has the address of every tensor baked in that
     its step reads besides its own tables; those tensors are held here, so that as long as the model has the same addresses it
-    has the same tensors.  A model that has others (a longer position table, a new weight store, a layer replaced) gets a new object."""
+    has the same tensors.  A model that has others (a longer position table, a new weight store, a layer replaced) gets a new object.
+
+    Searches may run in several threads: a set belongs to one search at a time, and the lock guards the sets and the captures."""
+
+    MAX_KEPT = 4
+    lock = threading.RLock()
 
     def __init__(self, state):
         self.state = state
         self.sets = {}
 
+    def take(self, key):
+        with self.lock:
+            return self.sets.pop(key, None)
+
+    def put(self, key, kept):
+        with self.lock:
+            self.sets.pop(key, None)             # of two searches of one geometry the later one's set stays
+            while len(self.sets) >= self.MAX_KEPT:
+                self.sets.pop(next(iter(self.sets)))
+            self.sets[key] = kept
+
     @classmethod
     def of(cls, model, device):
+        with cls.lock:
+            return cls._of(model, device)
+
+    @classmethod
+    def _of(cls, model, device):
         emb = getattr(model.decoder, "embed", None)
         table = emb._pos_table(device) if hasattr(emb, "_pos_table") else None
         held, state = [table], []
@@ -175,8 +197,6 @@ class _DeviceSearch:
     Tables, caches and the graph are kept on the model for later batches of the same geometry; a search takes its set out of the pool
     and puts it back when its results are on the host, so concurrent searches have sets of their own."""
 
-    MAX_KEPT = 4
-
     def __init__(self, model, state, cfg, K: int, B: int, T: int, max_len_per):
         dev = state.context.device
         R = B * K
@@ -191,7 +211,7 @@ class _DeviceSearch:
         src_cap = (max(b["c_k"].shape[1] for b in cross) + 63) // 64 * 64 if cross else 0
         self.key = (B, K, cap, src_cap, len(state.buffers), str(dev), cfg.pad, cfg.eos)
         self.pools = _StepPools.of(model, dev)
-        pool = self.pools.sets.pop(self.key, None)
+        pool = self.pools.take(self.key)
         if pool is None:
             mk = lambda shape, dt: torch.zeros(shape, dtype=dt, device=dev)
             i32, f32, i64 = torch.int32, torch.float32, torch.int64
@@ -248,12 +268,16 @@ class _DeviceSearch:
         if pool["warm"] < 2:                    # lazy initialisation happens outside the capture
             pool["warm"] += 1
             return self._body()
-        if pool["graph"] is None:
-            g = torch.cuda.CUDAGraph()
-            torch.cuda.synchronize()
-            with torch.cuda.graph(g, capture_error_mode="thread_local"):
-                self._body()
-            pool["graph"] = g                   # captured, not run
+        while pool["graph"] is None:
+            with _StepPools.lock:               # one capture at a time, on a stream of its own
+                self.pools = _StepPools.of(self.model, self.tok.device)
+                g = torch.cuda.CUDAGraph()
+                torch.cuda.synchronize()
+                with torch.cuda.graph(g, stream=torch.cuda.Stream(self.tok.device), capture_error_mode="thread_local"):
+                    self._body()                # captured, not run
+                # another thread may have renewed the position table meanwhile: then this graph is not what the pool holds
+                if _StepPools.of(self.model, self.tok.device) is self.pools:
+                    pool["graph"] = g
         pool["graph"].replay()
 
     def run(self):
@@ -280,9 +304,7 @@ class _DeviceSearch:
         scores, last = tables[10][:, :n].cpu(), tables[11][:, :n].cpu()
         longest = int(last.masked_fill(scores == float("-inf"), 0).max()) + 1
         words, word_scores = words[:, :, :longest].cpu(), word_scores[:, :, :longest].cpu()
-        if len(self.pools.sets) >= self.MAX_KEPT:
-            self.pools.sets.pop(next(iter(self.pools.sets)), None)
-        self.pools.sets[self.key] = self.pool
+        self.pools.put(self.key, self.pool)
         results = []
         for b in range(self.B):
             hyps = []

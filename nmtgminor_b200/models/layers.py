@@ -186,9 +186,10 @@ class Embedding(nn.Module):
             return self.pos
         if device.type != "cuda":
             return self.pos
-        if self._pos_work is None or self._pos_work.device != device:
-            self._pos_work = self.pos.to(device=device, dtype=torch.bfloat16)
-        return self._pos_work
+        pos, work = self.pos, self._pos_work          # another thread may renew the table at any time
+        if work is None or work.device != device or work.shape != pos.shape:
+            work = self._pos_work = pos.to(device=device, dtype=torch.bfloat16)
+        return work
 
     word_dropout = 0.0      # probability of dropping a whole vocabulary entry for one batch (training only)
 

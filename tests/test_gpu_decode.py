@@ -308,3 +308,28 @@ def test_replayed_search_follows_the_model():
     same()
     assert [h.tokens for h in search(True)] != first
     assert ops.check_status() == 0
+
+
+def test_searches_in_several_threads():
+    """Four threads with geometries of their own and one that two of them share: captures, a position table that grows under the others, and
+    a pool that overflows.  Every result is the one of a search alone."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from nmtgminor_b200.data.dataset import collate
+    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
+    g = torch.Generator().manual_seed(8)
+    jobs = []
+    for i, (n, beam, longest) in enumerate(((3, 2, 30), (5, 4, 70), (1, 3, 1100), (4, 1, 130), (2, 2, 30), (3, 2, 30))):
+        src = [torch.randint(4, 300, (int(m),), generator=g) for m in torch.randint(3, 40, (n,), generator=g)]
+        cfg = BeamConfig(beam_size=beam, max_len=longest, min_len=25)
+        jobs.append((collate(src, None, padded=True, packed=True, round_to=1).cuda("cuda"), cfg))
+    flat = lambda found: [(h.tokens, h.score) for hyps in found for h in hyps]
+    alone = _successor_model(9)
+    want = [flat(beam_search(alone, *job)) for job in jobs]
+    shared = _successor_model(9)
+    with ThreadPoolExecutor(4) as threads:
+        for _ in range(3):
+            got = [f.result(timeout=120) for f in [threads.submit(lambda j: flat(beam_search(shared, *j)), job) for job in jobs]]
+            assert got == want
+    assert len(shared.__dict__["_decode_pools"].sets) <= 4
+    assert ops.check_status() == 0
