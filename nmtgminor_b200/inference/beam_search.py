@@ -213,19 +213,20 @@ class _DeviceSearch:
         self.pools = _StepPools.of(model, dev)
         pool = self.pools.take(self.key)
         if pool is None:
-            mk = lambda shape, dt: torch.zeros(shape, dtype=dt, device=dev)
-            i32, f32, i64 = torch.int32, torch.float32, torch.int64
-            pool = {"graph": None, "warm": 0, "tables": [
-                mk(3, i32), mk(cap + 1, f32), mk(B, i32), mk(R, f32), mk(R, torch.uint8), mk(B, torch.uint8), mk(R, i64), mk(R, i64),
-                mk((R, cap), i32), mk(B, i32), mk((B, K), f32), mk((B, K), i32), mk((B, K), i32), mk((B, K), f32),
-                mk((cap, R), i32), mk((cap, R), i32), mk((cap, R), f32)], "layers": []}
-            for buf, H in zip(state.buffers, widths):
-                keep = {"k": torch.empty(R, cap, H, dtype=torch.bfloat16, device=dev), "v": torch.empty(R, cap, H, dtype=torch.bfloat16, device=dev)}
-                if "c_k" in buf:
-                    shape = (B, src_cap, buf["c_k"].shape[2])
-                    keep.update(c_k=mk(shape, torch.bfloat16), c_v=mk(shape, torch.bfloat16), c_len=mk(B, i32))
-                pool["layers"].append(keep)
-            pool["done_host"] = [torch.zeros(B, dtype=torch.uint8, pin_memory=True) for _ in range(2)]
+            with torch.inference_mode(False), torch.no_grad():      # kept tables serve callers in either mode
+                mk = lambda shape, dt: torch.zeros(shape, dtype=dt, device=dev)
+                i32, f32, i64 = torch.int32, torch.float32, torch.int64
+                pool = {"graph": None, "warm": 0, "tables": [
+                    mk(3, i32), mk(cap + 1, f32), mk(B, i32), mk(R, f32), mk(R, torch.uint8), mk(B, torch.uint8), mk(R, i64), mk(R, i64),
+                    mk((R, cap), i32), mk(B, i32), mk((B, K), f32), mk((B, K), i32), mk((B, K), i32), mk((B, K), f32),
+                    mk((cap, R), i32), mk((cap, R), i32), mk((cap, R), f32)], "layers": []}
+                for buf, H in zip(state.buffers, widths):
+                    keep = {name: torch.empty(R, cap, H, dtype=torch.bfloat16, device=dev) for name in ("k", "v")}
+                    if "c_k" in buf:
+                        shape = (B, src_cap, buf["c_k"].shape[2])
+                        keep.update(c_k=mk(shape, torch.bfloat16), c_v=mk(shape, torch.bfloat16), c_len=mk(B, i32))
+                    pool["layers"].append(keep)
+                pool["done_host"] = [torch.zeros(B, dtype=torch.uint8, pin_memory=True) for _ in range(2)]
         self.pool = pool
         (ctl, inv_norm, max_rows, scores, force, done, tok, pos_rows, anc, fin_count, fin_score) = pool["tables"][:11]
         self.tok, self.pos_rows, self.done = tok, pos_rows, done

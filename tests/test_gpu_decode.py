@@ -333,3 +333,17 @@ def test_searches_in_several_threads():
             assert got == want
     assert len(shared.__dict__["_decode_pools"].sets) <= 4
     assert ops.check_status() == 0
+
+
+def test_search_in_and_out_of_inference_mode():
+    """Tables that were made under torch.inference_mode serve a search outside of it."""
+    from nmtgminor_b200.data.dataset import collate
+    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
+    model = _successor_model(11)
+    batch = collate([torch.arange(4, 20)], None, padded=True, packed=True, round_to=1).cuda("cuda")
+    search = lambda: [(h.tokens, h.score) for h in beam_search(model, batch, BeamConfig(beam_size=2, max_len=20, min_len=10))[0]]
+    with torch.inference_mode():
+        want = search()
+    assert search() == want
+    with torch.inference_mode():
+        assert search() == want
