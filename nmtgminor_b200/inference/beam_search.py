@@ -197,11 +197,16 @@ class _DeviceSearch:
     Tables, caches and the graph are kept on the model for later batches of the same geometry; a search takes its set out of the pool
     and puts it back when its results are on the host, so concurrent searches have sets of their own."""
 
+    @staticmethod
+    def capacity(T: int) -> int:
+        """Cached positions for ``T`` steps, rounded so that batches share a geometry."""
+        return (T + 2 + 63) // 64 * 64
+
     def __init__(self, model, state, cfg, K: int, B: int, T: int, max_len_per):
         dev = state.context.device
         R = B * K
         self.model, self.state, self.cfg, self.K, self.B, self.T = model, state, cfg, K, B, T
-        cap = (T + 2 + 63) // 64 * 64                    # the geometry of a batch, rounded so that batches share it
+        cap = self.capacity(T)
         emb = getattr(model.decoder, "embed", None)
         if emb is not None and hasattr(emb, "renew"):
             emb.renew(cap)
@@ -336,7 +341,8 @@ def beam_search(model, batch, cfg: BeamConfig, prefix_tokens: Optional[torch.Ten
     fused = (device.type == "cuda" and cfg.fused_step and getattr(model, "supports_logits_step", False)
              and not cfg.sampling and cfg.no_repeat_ngram_size <= 0 and cfg.vocab_mask is None and 2 * K <= 64
              and cfg.diversity_rate <= 0)
-    if fused and cfg.cuda_graph and prefix_tokens is None and banned_first is None and _replayable(model, state):
+    if (fused and cfg.cuda_graph and prefix_tokens is None and banned_first is None and _replayable(model, state)
+            and B * K * _DeviceSearch.capacity(T) < 2 ** 31):       # cache rows are addressed with 32 bits
         return _DeviceSearch(model, state, cfg, K, B, T, max_len_per).run()
     R = B * K
     tokens = torch.full((R, T + 2), cfg.pad, dtype=torch.long, device=device)

@@ -241,6 +241,7 @@ Tensor decode_self(const Tensor& qkv, Tensor& k_cache, Tensor& v_cache, const Te
   const int R = qkv.size(0);
   TORCH_CHECK(k_cache.dim() == 3 && k_cache.sizes() == v_cache.sizes() && k_cache.size(0) == R && k_cache.size(2) == heads * 64);
   TORCH_CHECK(K > 0 && R % K == 0 && anc.dim() == 2 && anc.size(0) == R && anc.size(1) == k_cache.size(1) && pos_rows.numel() == R);
+  TORCH_CHECK(anc.numel() <= INT32_MAX, "decode_self: cache rows are addressed with 32 bits");
   c10::cuda::CUDAGuard guard(qkv.device());
   Tensor out = torch::empty({R, heads * 64}, qkv.options());
   ck(nmtg_decode_self(qkv.data_ptr(), qkv.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), anc.data_ptr<int>(),

@@ -239,8 +239,9 @@ decode_self_kernel(const __nv_bfloat16* __restrict__ qkv, long ld, __nv_bfloat16
   __shared__ __align__(16) float qs[KB][64];
   __shared__ float part[kStepWarps][KB][66];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int h = blockIdx.x, r0 = (blockIdx.y / groups) * K + (blockIdx.y % groups) * KB;
-  const int beams = min(KB, K - static_cast<int>(blockIdx.y % groups) * KB);
+  const int h = blockIdx.x % heads, item = blockIdx.x / heads;
+  const int r0 = (item / groups) * K + (item % groups) * KB;
+  const int beams = min(KB, K - (item % groups) * KB);
   const int hid = heads * 64;
   const int sub = lane >> 3, eighth = lane & 7, col = h * 64 + eighth * 8;
   pdl_trigger();
@@ -323,7 +324,8 @@ decode_cross_kernel(const __nv_bfloat16* __restrict__ q, long ld, const __nv_bfl
   __shared__ float part[kStepWarps][KB][66];
   __shared__ __align__(16) float mine[KB][68];      // this CTA's sums, read by the whole cluster
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int h = blockIdx.x, b = blockIdx.y / groups, k0 = (blockIdx.y % groups) * KB;
+  const int h = blockIdx.x % heads, item = blockIdx.x / heads;
+  const int b = item / groups, k0 = (item % groups) * KB;
   const int beams = min(KB, K - k0);
   const int share = blockIdx.z;
   const int hid = heads * 64;
@@ -457,12 +459,12 @@ template <> __device__ __forceinline__ float as_float<__nv_bfloat16>(__nv_bfloat
 template <typename T>
 __global__ void __launch_bounds__(kPartThreads)
 beam_part_kernel(const T* __restrict__ logits, long ld, const uint8_t* __restrict__ force, float2* __restrict__ part_lse,
-                 Cand* __restrict__ part, int K2, int V, int pad, int eos, int vec) {
+                 Cand* __restrict__ part, int pieces, int K2, int V, int pad, int eos, int vec) {
   __shared__ Cand list[kPartCols];
   __shared__ float red[2][kPartThreads / 32];
   __shared__ int count;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kPartThreads / 32;
-  const int r = blockIdx.y, piece = blockIdx.x;
+  const int r = blockIdx.x / pieces, piece = blockIdx.x - r * pieces;
   const int c0 = piece * kPartCols;
   pdl_trigger();
   pdl_wait();
@@ -540,7 +542,7 @@ beam_part_kernel(const T* __restrict__ logits, long ld, const uint8_t* __restric
   for (int i = 0; i < kPartEach; ++i)
     if ((takes >> i) & 1u) list[at++] = (static_cast<Cand>(key[i]) << 32) | (kNone - static_cast<uint32_t>(c0 + col[i / kPer] + i % kPer));
   __syncthreads();
-  const long o = static_cast<long>(r) * gridDim.x + piece;
+  const long o = static_cast<long>(r) * pieces + piece;
   if (threadIdx.x == kPartThreads - 1) {
     float s = 0.f;
     for (int w = 0; w < warps; ++w) s += red[1][w];
@@ -772,7 +774,7 @@ const char* launch_self(const void* qkv, long ld, void* kc, void* vc, const int*
                         int cap, float scale, int sms, cudaStream_t stream) {
   const int groups = (K + KB - 1) / KB;
   const int warps = step_warps(static_cast<long>(heads) * B * groups, cap, sms);
-  return launch(decode_self_kernel<KB>, dim3(heads, B * groups), dim3(32 * warps), 0, 1, stream, static_cast<const __nv_bfloat16*>(qkv), ld,
+  return launch(decode_self_kernel<KB>, dim3(heads * B * groups), dim3(32 * warps), 0, 1, stream, static_cast<const __nv_bfloat16*>(qkv), ld,
                 static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), anc, pos_rows, static_cast<__nv_bfloat16*>(out), K, groups,
                 heads, cap, scale);
 }
@@ -789,7 +791,7 @@ const char* launch_cross(const void* q, long ld, const void* ck, const void* cv,
   while (splits < 8 && ctas * splits < 4L * sms && cap >= splits * 2 * 128) splits *= 2;
   const int blocks = (cap / splits + 4 * keys_of<KB>() - 1) / (4 * keys_of<KB>());
   const int warps = cap > 512 ? 4 : step_warps(ctas * splits, blocks, sms);
-  return launch(decode_cross_kernel<KB>, dim3(heads, B * groups, splits), dim3(32 * warps), 0, splits, stream,
+  return launch(decode_cross_kernel<KB>, dim3(heads * B * groups, 1, splits), dim3(32 * warps), 0, splits, stream,
                 static_cast<const __nv_bfloat16*>(q), ld, static_cast<const __nv_bfloat16*>(ck), static_cast<const __nv_bfloat16*>(cv),
                 lengths, static_cast<__nv_bfloat16*>(out), K, groups, heads, cap, scale, splits);
 }
@@ -830,17 +832,16 @@ const char* nmtg_beam_step(const NmtgBeam* s, const void* logits, long ld, int d
   if (B <= 0 || K <= 0 || K > 32) return "beam_step: 1 to 32 hypotheses per sentence";
   if (K2 > V) return "beam_step: vocabulary smaller than twice the beam";
   if (ld < V) return "beam_step: row stride smaller than the vocabulary";
-  if (R > 65535) return "beam_step: too many hypotheses";
   const int vec = (ld * (dtype == 0 ? 4 : 2)) % 16 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
   float2* lse = static_cast<float2*>(part_lse);
   Cand* cand = static_cast<Cand*>(part);
   const char* e;
   if (dtype == 0)
-    e = launch(beam_part_kernel<float>, dim3(pieces, R), dim3(kPartThreads), 0, 1, stream, static_cast<const float*>(logits), ld, s->force, lse,
-               cand, K2, V, s->pad, s->eos, vec);
+    e = launch(beam_part_kernel<float>, dim3(pieces * R), dim3(kPartThreads), 0, 1, stream, static_cast<const float*>(logits), ld, s->force, lse,
+               cand, pieces, K2, V, s->pad, s->eos, vec);
   else
-    e = launch(beam_part_kernel<__nv_bfloat16>, dim3(pieces, R), dim3(kPartThreads), 0, 1, stream, static_cast<const __nv_bfloat16*>(logits),
-               ld, s->force, lse, cand, K2, V, s->pad, s->eos, vec);
+    e = launch(beam_part_kernel<__nv_bfloat16>, dim3(pieces * R), dim3(kPartThreads), 0, 1, stream, static_cast<const __nv_bfloat16*>(logits),
+               ld, s->force, lse, cand, pieces, K2, V, s->pad, s->eos, vec);
   if (e) return e;
   // the pieces' candidates are staged in shared memory unless a wide beam over a large vocabulary makes them many
   const size_t tables = static_cast<size_t>(K) * K2 * 16 + 4 * (2 * K2 + K + K * 256 + 7 * K), cands = static_cast<size_t>(K) * pieces * K2 * 8;

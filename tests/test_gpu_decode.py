@@ -230,6 +230,24 @@ def test_device_search_matches_host_bookkeeping(dtype, B, K, V, T, min_len, norm
     _compare_searches(dtype, B, K, V, T, min_len, normalize, 0.6 if normalize else 0.0)
 
 
+def test_steps_of_very_many_rows():
+    """More rows than a grid has blocks along its second dimension: attention over the past and over the source, and a whole search."""
+    R, hid = 66000, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    k, v, q = rnd(R, 16, hid), rnd(R, 16, hid), rnd(R, hid)
+    out = ops.ext().decode_cross(q, k, v, torch.full((R,), 16, dtype=torch.int32, device="cuda"), 1, 0.125)
+    want = torch.einsum("rj,rjd->rd", torch.softmax(torch.einsum("rd,rjd->rj", q.float(), k.float()) * 0.125, -1), v.float())
+    assert (out.float() - want).abs().max() <= 2 ** -7 * want.abs().max()          # one rounding to bf16, 32-bit sums on both sides
+    qkv = rnd(R, 3 * hid)
+    anc = torch.arange(R, dtype=torch.int32, device="cuda")[:, None].expand(R, 16).contiguous()
+    keys, vals = torch.cat([k[:, :15], qkv[:, None, hid:2 * hid]], 1).float(), torch.cat([v[:, :15], qkv[:, None, 2 * hid:]], 1).float()
+    out = ops.ext().decode_self(qkv, k, v, anc, torch.full((R,), 15, dtype=torch.long, device="cuda"), 1, 1, 0.125)
+    want = torch.einsum("rj,rjd->rd", torch.softmax(torch.einsum("rd,rjd->rj", qkv[:, :hid].float(), keys) * 0.125, -1), vals)
+    assert (out.float() - want).abs().max() <= 2 ** -7 * want.abs().max()
+    _compare_searches(torch.bfloat16, R // 2, 2, 40, 3, 0, False, 0.0)
+
+
 @pytest.mark.parametrize("B,K,V,alpha,end_bias", [(8, 2, 50, 0.0, 2.0), (6, 3, 50, 0.0, 2.0), (6, 3, 50, -0.5, 2.0), (8, 4, 300, 0.0, 3.0)])
 def test_device_search_stop_rule_without_penalty(B, K, V, alpha, end_bias):
     """`normalize` without a length penalty: the search goes on after `beam` hypotheses have ended while a better one can still come."""
