@@ -305,7 +305,7 @@ class _DeviceSearch:
                 event.record()
                 seen = (event, host)
         tables = self.pool["tables"]
-        n = min(cfg.n_best, K)
+        n = max(1, min(cfg.n_best, K))
         words, word_scores = ops.ext().beam_trace(tables, K, cfg.pad, cfg.eos, n)
         scores, last = tables[10][:, :n].cpu(), tables[11][:, :n].cpu()
         longest = int(last.masked_fill(scores == float("-inf"), 0).max()) + 1
@@ -314,7 +314,7 @@ class _DeviceSearch:
         results = []
         for b in range(self.B):
             hyps = []
-            for k in range(n):
+            for k in range(min(cfg.n_best, K)):
                 if torch.isfinite(scores[b, k]):
                     m = int(last[b, k]) + 1
                     hyps.append(Hypothesis(words[b, k, :m].tolist(), float(scores[b, k]), word_scores[b, k, :m].tolist()))

@@ -365,3 +365,15 @@ def test_search_in_and_out_of_inference_mode():
     assert search() == want
     with torch.inference_mode():
         assert search() == want
+
+
+@pytest.mark.parametrize("n_best", [-1, 0, 1, 9])
+def test_number_of_hypotheses_asked_for(n_best):
+    """None, one and more than the beam: the same lists from the replayed and the kernel-by-kernel search."""
+    from nmtgminor_b200.data.dataset import collate
+    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
+    model = _successor_model(12)
+    batch = collate([torch.arange(4, 20), torch.arange(30, 36)], None, padded=True, packed=True, round_to=1).cuda("cuda")
+    a, b = (beam_search(model, batch, BeamConfig(beam_size=2, n_best=n_best, max_len=20, min_len=10, cuda_graph=c)) for c in (True, False))
+    assert [len(x) for x in a] == [len(x) for x in b] == [max(1, min(n_best, 2))] * 2
+    assert [x[0].tokens for x in a] == [x[0].tokens for x in b]
