@@ -267,3 +267,15 @@ def test_pad_rows_matches_tensor_operations(dtype, width):
     too_long = PackedSeqs(seqs.tokens, seqs.positions, cu, 129)
     with pytest.raises(RuntimeError):
         too_long.pad(x)
+
+
+def test_pad_rows_of_lazily_conjugated_values():
+    """A conjugate or negative view shares the memory of its base: padding must give the view's values."""
+    from nmtgminor_b200.models.layers import PackedSeqs
+    z = torch.randn(6, 3, dtype=torch.complex64, device="cuda")
+    cu = torch.tensor([0, 2, 6], dtype=torch.int32, device="cuda")
+    seqs = PackedSeqs(torch.zeros(6, dtype=torch.long, device="cuda"), torch.zeros(6, dtype=torch.long, device="cuda"), cu, 4)
+    for x in (z, z.conj(), torch._neg_view(z.real.contiguous())):
+        got = seqs.pad(x, time_first=False)
+        assert torch.equal(got[0, :2], x[:2].resolve_conj().resolve_neg()) and torch.equal(got[1], x[2:].resolve_conj().resolve_neg())
+        assert not got[0, 2:].any()
