@@ -80,6 +80,7 @@ def _one_kernel_pad(x, cu) -> bool:
     """Plain GPU tensors that nothing differentiates through or transforms; the others are padded with tensor operations."""
     return (x.is_cuda and cu.device == x.device and cu.dtype == torch.int32 and cu.is_contiguous() and x.is_contiguous() and type(x) is torch.Tensor
             and not x.is_conj() and not x.is_neg()          # their memory holds other values
+            and torch._C._len_torch_dispatch_stack() == 0   # a mode (make_fx, a counter) wants to see every operation
             and not (torch.is_grad_enabled() and x.requires_grad) and not torch._C._functorch.is_functorch_wrapped_tensor(x)
             and torch.autograd.forward_ad._current_level < 0 and not torch.jit.is_tracing() and ops.extension_available())
 

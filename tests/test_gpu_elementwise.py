@@ -279,3 +279,15 @@ def test_pad_rows_of_lazily_conjugated_values():
         got = seqs.pad(x, time_first=False)
         assert torch.equal(got[0, :2], x[:2].resolve_conj().resolve_neg()) and torch.equal(got[1], x[2:].resolve_conj().resolve_neg())
         assert not got[0, 2:].any()
+
+
+def test_pad_rows_under_tracing():
+    """A trace of the padding must follow its input, not keep the result of the example."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    from nmtgminor_b200.models.layers import PackedSeqs
+    cu = torch.tensor([0, 2, 6], dtype=torch.int32, device="cuda")
+    seqs = PackedSeqs(torch.zeros(6, dtype=torch.long, device="cuda"), torch.zeros(6, dtype=torch.long, device="cuda"), cu, 4)
+    a, b = torch.randn(6, 8, device="cuda"), torch.randn(6, 8, device="cuda")
+    traced = make_fx(lambda x: seqs.pad(x, time_first=False))(a)
+    assert torch.equal(traced(b), seqs.pad(b, time_first=False))
