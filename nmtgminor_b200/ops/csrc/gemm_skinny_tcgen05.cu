@@ -290,7 +290,9 @@ bool skinny_takes(const GemmDesc* d, int sms) {
          (reinterpret_cast<uintptr_t>(d->bias) & 7) == 0;
 }
 
-const char* launch_gemm_skinny(const GemmDesc* d, int sms, cudaStream_t stream) {
+// `weights_settled`: no kernel that may still run writes the weights.  A gathered weight is not: the copy right before this launch
+// writes it, so that it is read after griddepcontrol.wait like everything else.
+const char* launch_gemm_skinny(const GemmDesc* d, int sms, bool weights_settled, cudaStream_t stream) {
   const bool pdl = step_overlap();
   const int nt = skinny_rows(d->M);
   CUtensorMap tw, tx;
@@ -303,7 +305,7 @@ const char* launch_gemm_skinny(const GemmDesc* d, int sms, cudaStream_t stream) 
   a.residual = reinterpret_cast<const __nv_bfloat16*>(d->residual); a.ld_res = d->ld_res;
   a.out = reinterpret_cast<__nv_bfloat16*>(d->out); a.ld_out = d->ld_out;
   a.act = d->act; a.status = d->status;
-  a.early = pdl ? 1 : 0;
+  a.early = pdl && weights_settled ? 1 : 0;
   const int tiles_n = (d->N + kSkinnyFeat - 1) / kSkinnyFeat, tiles_m = (d->M + nt - 1) / nt;
   // as many K slices as keep one wave of CTAs, at least two k-blocks each
   int split = 8;

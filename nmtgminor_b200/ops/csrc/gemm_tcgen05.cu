@@ -396,7 +396,7 @@ const char* launch_gemm_pair(const GemmDesc* d, const GemmArgs& a, int bn, cudaS
 const char* launch_gather_copy(const GemmDesc* d, cudaStream_t stream);
 bool plan_pair_gather(const GemmDesc* d, int bn, GatherArgs* g);
 bool skinny_takes(const GemmDesc* d, int sms);
-const char* launch_gemm_skinny(const GemmDesc* d, int sms, cudaStream_t stream);
+const char* launch_gemm_skinny(const GemmDesc* d, int sms, bool weights_settled, cudaStream_t stream);
 }
 using namespace b200;
 
@@ -505,8 +505,9 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   // down to 64 columns
   const bool skinny = g_gemm_variant == 0 && d->M <= 512 && !d->out_fp32 && d->force_bn == 0 && d->split_k <= 1 && !d->colsum;
   if (skinny) {
-    if (d->gather) { const char* e = gather_first(); if (e) return e; }
-    if (skinny_takes(d, sms)) return launch_gemm_skinny(d, sms, stream);
+    const bool gathered = d->gather != nullptr;
+    if (gathered) { const char* e = gather_first(); if (e) return e; }
+    if (skinny_takes(d, sms)) return launch_gemm_skinny(d, sms, !gathered, stream);
     const int num_m = (d->M + BM - 1) / BM;
     int bn = 64;
     if (static_cast<long>(num_m) * ((d->N + 255) / 256) >= sms) bn = 256;

@@ -63,8 +63,8 @@ void nmtg_set_gemm_variant(int v);
 // communication kernels placed on the free SMs (nmtg_reduce_unit with a negative CTA count) never share one with them.
 void nmtg_set_sm_reserve(int n);
 // While it is on for the calling thread, the kernels of a decoding step are launched so that each may set itself up (and read
-// weights, which no kernel of the step writes) while the one before it is still running; everything else they touch only after
-// that kernel has finished.  The first kernel of a step is always launched the ordinary way.
+// weights, which no kernel of the step writes; those of a gathered operand excepted) while the one before it is still running;
+// everything else they touch only after that kernel has finished.  The first kernel of a step is always launched the ordinary way.
 void nmtg_set_step_overlap(int on);
 // Timing aid for the short-sequence attention backward: bit mask of work to leave out (see the kernel); 0 = everything.
 void nmtg_set_attn_bwd_ablation(int bits);

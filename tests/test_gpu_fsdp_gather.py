@@ -94,3 +94,25 @@ def test_unfused_switch_gives_the_same_result():
         ops.ext().set_gemm_variant(51)
     torch.cuda.synchronize()
     assert torch.equal(a, b) and torch.equal(view, w)
+
+
+@pytest.mark.parametrize("m,n_out,n_in", [(4, 1024, 1024), (64, 512, 2048), (300, 256, 256)])
+def test_few_rows_wait_for_their_gathered_weight(m, n_out, n_in):
+    """Few-row products with launches that overlap: the copy right before the product writes its weight, which changes every time."""
+    from nmtgminor_b200 import ops
+    x = torch.randn(m, n_in, device="cuda").bfloat16()
+    got = torch.empty(m, n_out, device="cuda", dtype=torch.bfloat16)
+    want = torch.empty_like(got)
+    w, view, gather, counters, shards = _sharded_case(n_out, n_in, 2, seed=3)
+    for i in range(8):
+        for s in shards:
+            s.neg_()
+        w.neg_()
+        ops.gemm(x, w, want, allow_split_k=True)
+        ops.ext().set_step_overlap(True)
+        try:
+            ops.gemm(x, view, got, allow_split_k=True, gather=_Rec(gather))
+        finally:
+            ops.ext().set_step_overlap(False)
+        assert torch.equal(got, want), i
+    assert ops.check_status() == 0 and int(counters.abs().sum()) == 0
