@@ -28,7 +28,7 @@ struct GemmArgs {
   __nv_bfloat16* preact;   // optional [M, ld_out]: value after bias, before activation
   uint32_t* mask;          // optional [M, ld_mask] sign bits of the output (written, or read by kActMaskBwd)
   int ld_mask;
-  float* colsum;           // optional fp32 [N]: += column sums of the stored bf16 output (TMA-store epilogue)
+  float* colsum;           // optional fp32 [N]: += column sums of the stored bf16 output (from the staging tiles, or from registers: sum_here)
   int act;
   float dropout_p;
   unsigned long long seed, stream_id;
@@ -101,7 +101,7 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __ex
 constexpr uint32_t kEpiBias = 1u, kEpiPreact = 2u, kEpiActFwd = 4u, kEpiActBwd = 8u, kEpiMaskBwd = 16u, kEpiDrop = 32u,
                    kEpiMaskOut = 64u, kEpiRes = 128u, kEpiF32 = 256u, kEpiBf16 = 512u,
                    kEpiRagged = 1024u /* N not a multiple of 64: partial column chunks */,
-                   kEpiColsum = 2048u /* column sums of the output, pair kernel only */, kEpiAll = 4095u;
+                   kEpiColsum = 2048u /* column sums of the output */, kEpiAll = 4095u;
 
 // Features a problem needs (host side).
 inline uint32_t gemm_epilogue_features(const GemmArgs& a) {
@@ -147,7 +147,8 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
     tmem_ld32(taddr, r);
     tmem_ld_wait();
     const bool live = row_ok && p.ablate != 1;
-    // column sums straight from registers need every lane of the warp (single-CTA kernel; the host pairs them with the mask epilogue only)
+    // Column sums straight from registers (single-CTA kernel) need every lane of the warp, so that the lanes of rows past M go on to them.
+    // They must meet no operand or output of their row on the way: the host sends column sums here with the mask epilogue at most.
     const bool sum_here = (kFeat & kEpiColsum) && p.colsum != nullptr && stage_row == nullptr;
     if (!live && !sum_here) return;
     float v[32];

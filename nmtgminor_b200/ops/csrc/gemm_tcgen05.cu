@@ -547,8 +547,9 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
       (!d->colsum || (gemm_epilogue_features(a) & ~(kEpiBf16 | kEpiMaskBwd | kEpiColsum)) == 0))
     narrow_bn = one_wave_tile(d, sms, num_kb, &narrow_split);
   // ---- CTA-pair kernel (256-row tiles): the default for everything but very small M ----------------
-  if (d->colsum && d->M <= BM) return "gemm: the column-sum output needs more than 128 rows (CTA-pair kernel)";
-  if (g_gemm_variant != 1 && d->M > BM && narrow_bn == 0) {
+  if (d->colsum && d->M <= BM) return "gemm: the column-sum output needs more than 128 rows";
+  // (column sums elsewhere than in the narrow tiles above, whose epilogue has the mask at most: see sum_here)
+  if ((g_gemm_variant != 1 || d->colsum) && d->M > BM && narrow_bn == 0) {
     int bn = (d->N > 128) ? 256 : 128;
     if (d->force_bn == 128 || d->force_bn == 256) bn = d->force_bn;
     if (d->gather) {

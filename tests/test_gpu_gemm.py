@@ -340,3 +340,32 @@ def test_second_matrix_epilogues(M, N, K):
     assert ops.check_status() == 0
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 64, 128), (200, 256, 256), (1000, 1032, 264), (2300, 512, 128)])
+def test_column_sums_beside_every_operand(M, N, K):
+    """Column sums with rows past the last tile, next to an aux operand, the sign bits and dropout, with the single-CTA kernel asked for
+    and not: the product is the one without the sums, and a pre-activation beside them stays refused."""
+    e = ops.ext()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w, aux = rnd(M, K), rnd(N, K) * K ** -0.5, rnd(M, N)
+    bits = torch.randint(-2 ** 31, 2 ** 31 - 1, (M, (N + 31) // 32), device="cuda", generator=g).int()
+    try:
+        for variant in (0, 1):
+            for more in (dict(act=8, mask=bits), dict(act=6, aux=aux), dict(act=5, aux=aux, dropout_p=0.25, seed=3, stream_id=1), dict(residual=aux)):
+                e.set_gemm_variant(variant)
+                out, cs = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16), torch.ones(N, device="cuda")
+                ops.gemm(x, w, out, colsum=cs, **more)
+                e.set_gemm_variant(0)
+                want = torch.zeros_like(out)
+                ops.gemm(x, w, want, force_bn=256, **more)
+                assert torch.equal(out, want), more
+                # 32-bit sums of M values of order 1
+                assert (cs.double() - 1 - out.double().sum(0)).abs().max() < 2 ** -20 * M + 1e-4
+            e.set_gemm_variant(variant)
+            with pytest.raises(RuntimeError):
+                ops.gemm(x, w, out, colsum=cs, act=2, preact=torch.zeros_like(out))
+    finally:
+        e.set_gemm_variant(0)
+    assert ops.check_status() == 0
