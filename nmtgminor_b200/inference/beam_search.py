@@ -261,8 +261,9 @@ class _DeviceSearch:
         from .. import ops
         ops.ext().set_step_overlap(True)        # this thread's launches
         try:
-            hidden = self.model.decoder.step_static(self.tok, self.pos_rows, self.state)
-            logits = self.model.generator(hidden)
+            with ops.step_sums:
+                hidden = self.model.decoder.step_static(self.tok, self.pos_rows, self.state)
+                logits = self.model.generator(hidden)
             if logits.dtype not in (torch.float32, torch.bfloat16):
                 logits = logits.float()
             ops.ext().beam_step(logits, self.pool["tables"], self.K, self.cfg.pad, self.cfg.eos)

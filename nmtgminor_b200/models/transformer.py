@@ -435,7 +435,11 @@ class Seq2SeqBase(nn.Module):
         """input_t ``[B*beam, t]`` (all symbols so far) -> ``log_prob [B*beam, V]`` fp32 for the next symbol
         (``logits_only``: raw ``logits`` instead, for the fused log-softmax + top-k beam kernel)."""
         tokens = input_t[:, -1].contiguous()
-        hidden = self.decoder.step(tokens, input_t.shape[1] - 1, state)
+        with ops.step_sums:
+            return self._step(tokens, input_t.shape[1] - 1, state, logits_only)
+
+    def _step(self, tokens, position, state: DecodingState, logits_only: bool) -> Dict:
+        hidden = self.decoder.step(tokens, position, state)
         if getattr(self, "copy_generator", None) is not None and getattr(state, "src_tokens", None) is not None:
             state.position += 1
             logp = self.copy_generator(hidden[:, None, :], state.context, state.src_tokens, state.src_pad_mask).squeeze(1)

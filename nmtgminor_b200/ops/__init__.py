@@ -171,6 +171,23 @@ def gemm(a, b, out, *, a_mn_major=False, b_mn_major=False, bias=None, residual=N
     return out
 
 
+class _StepSums(threading.local):
+    """``with step_sums:`` - the forward products of this thread may cut their sum over K into parts whose number depends on the row
+    count (csrc/gemm_skinny_tcgen05.cu).  Searches use it for their decoding steps.  Everywhere else a row's result does not depend
+    on the rows beside it: a sentence is encoded and scored to the same bits alone and in a batch."""
+
+    depth = 0
+
+    def __enter__(self):
+        self.depth += 1
+
+    def __exit__(self, *exc):
+        self.depth -= 1
+
+
+step_sums = _StepSums()
+
+
 def _gather_of(weight):
     """The gather record of a fully sharded weight matrix, or None (replicated parameters)."""
     return getattr(weight, "_fsdp", None)
@@ -280,7 +297,7 @@ def linear(x, weight, bias=None, act="none", dropout_p=0.0, residual=None, train
         if not torch.is_grad_enabled() or not (need_dx or gw is not None):
             y = empty_rows(x.shape[0], weight.shape[0], x.device)
             return gemm(xin, weight.work, y, bias=b, residual=residual, act=act_id, dropout_p=p, seed=_Rng.seed,
-                        stream_id=sid, allow_split_k=True, gather=_gather_of(weight))
+                        stream_id=sid, allow_split_k=step_sums.depth > 0, gather=_gather_of(weight))
         return _LinearFn.apply(_track(xin), weight.work, b, residual, gw, gb, act_id, p, _Rng.seed, sid, need_dx,
                                _gather_of(weight))
     return ref.linear(x, weight, bias, act_id, p, residual)
@@ -361,9 +378,10 @@ def mlp(x, w1, b1, w2, b2, act="relu", dropout_p=0.0, out_dropout_p=0.0, residua
                                 b2.work if b2 is not None else None, residual, g, act_id, p1, p2, _Rng.seed, sid1, sid2,
                                 _gather_of(w1), _gather_of(w2))
         h = torch.empty((x.shape[0], w1.shape[0]), dtype=torch.bfloat16, device=x.device)
-        gemm(xin, w1.work, h, bias=b1.work if b1 is not None else None, act=act_id, allow_split_k=True, gather=_gather_of(w1))
+        split = step_sums.depth > 0
+        gemm(xin, w1.work, h, bias=b1.work if b1 is not None else None, act=act_id, allow_split_k=split, gather=_gather_of(w1))
         y = torch.empty((x.shape[0], w2.shape[0]), dtype=torch.bfloat16, device=x.device)
-        return gemm(h, w2.work, y, bias=b2.work if b2 is not None else None, residual=residual, allow_split_k=True, gather=_gather_of(w2))
+        return gemm(h, w2.work, y, bias=b2.work if b2 is not None else None, residual=residual, allow_split_k=split, gather=_gather_of(w2))
     h = ref.linear(x, w1, b1, act_id, p1, None)
     return ref.linear(h, w2, b2, 0, p2, residual)
 
@@ -812,7 +830,7 @@ def generator_cross_entropy(h, weight, bias, labels, smoothing=0.0, pad_idx=0, g
             return _GeneratorXentFn.apply(_track(hin), weight.work, b, gw, gb, labels.contiguous(), float(smoothing), int(pad_idx),
                                           grad_scale)
         logits = empty_rows(h.shape[0], weight.shape[0], h.device)
-        gemm(hin, weight.work, logits, bias=b, allow_split_k=True)
+        gemm(hin, weight.work, logits, bias=b)
         return cross_entropy(logits, labels, smoothing, pad_idx)
     logits = ref.linear(h, weight, bias, 0, 0.0, None)
     loss_sum, correct, row_loss = ref.cross_entropy(logits, labels, smoothing, pad_idx)

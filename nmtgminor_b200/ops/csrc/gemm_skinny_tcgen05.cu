@@ -278,7 +278,7 @@ static int skinny_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 
 // Whether the few-row kernel takes this problem: plain Linear products (both operands K-major) with bias, activation and
 // residual whose 128-feature x 64-row tiles fit the GPU at once (two CTAs to an SM), where the caller lets the sum over K be split:
-// inference does; training keeps one order of its forward sums whatever the batch size.  Measured (us, this kernel back to back
+// decoding steps do; training, scoring and encoding keep one order of their forward sums whatever the batch size.  Measured (us, this kernel back to back
 // with programmatic launch / the tiled kernel): 1024 x 1024, 4 rows
 // 3.6 / 8.4, 256 rows 7.2 / 9.3, 512 rows 7.5 / 9.3; 4096 x 1024, 64 rows 6.0 / 8.6; 1024 x 4096, 4 rows 5.4 / 22.8; 32000 x
 // 1024, 33 rows 13.9 / 20.3.  Beyond one wave (32000 x 1024 with 128 rows: 25 us against 19) the tiled kernel is the better one.

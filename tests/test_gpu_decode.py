@@ -377,3 +377,24 @@ def test_number_of_hypotheses_asked_for(n_best):
     a, b = (beam_search(model, batch, BeamConfig(beam_size=2, n_best=n_best, max_len=20, min_len=10, cuda_graph=c)) for c in (True, False))
     assert [len(x) for x in a] == [len(x) for x in b] == [max(1, min(n_best, 2))] * 2
     assert [x[0].tokens for x in a] == [x[0].tokens for x in b]
+
+
+def test_scores_do_not_depend_on_the_batch():
+    """A sentence is scored to the same bits alone (few rows, few tiles) and beside eleven others, and so are its encoder states."""
+    from nmtgminor_b200.data.dataset import collate
+    model = _successor_model(13)
+    g = torch.Generator().manual_seed(2)
+    ids = lambda n: torch.randint(4, 300, (int(n),), generator=g)
+    src = [ids(n) for n in torch.randint(20, 100, (12,), generator=g)]
+    tgt = [torch.cat([torch.tensor([2]), ids(n), torch.tensor([3])]) for n in torch.randint(20, 100, (12,), generator=g)]
+    pack = lambda s, t: collate(s, t, padded=True, packed=True, round_to=1).cuda("cuda")
+    _, _, tokens = model.decode(pack(src, tgt))
+    with torch.no_grad():
+        context, seqs = model.encode(pack(src, tgt))
+        for i in range(12):
+            _, _, alone = model.decode(pack(src[i:i + 1], tgt[i:i + 1]))
+            n = len(tgt[i]) - 1
+            assert torch.equal(alone[:n, 0], tokens[:n, i])
+            states, _ = model.encode(pack(src[i:i + 1], None))
+            at = int(seqs.cu[i])
+            assert torch.equal(states[:len(src[i])], context[at:at + len(src[i])])
