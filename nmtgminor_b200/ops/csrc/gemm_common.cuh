@@ -58,32 +58,40 @@ struct GatherArgs {
   int* counters;            // [0]: CTAs that have left the kernel, [1]: next unclaimed block, [2 + s]: finished blocks of segment s
 };
 
-// erfc(|x| / sqrt 2) / 2, the upper tail of the normal distribution, by the Chebyshev fit of Press et al., Numerical Recipes, section 6.2
-// (erfcc; relative error below 1.2e-7 everywhere): one reciprocal, one exponential, ten multiply-adds and no branch.  1 + erff(x)
-// is no closer in the middle, loses the lower tail to cancellation, and its two ranges cost an epilogue of 32 unrolled elements 16 us of
-// 44 (6144 x 2048 x 512 with the GELU gradient).
-__device__ __forceinline__ float normal_tail(float x) {
-  const float z = fabsf(x) * 0.70710678118654752f;
-  const float t = __fdividef(1.f, fmaf(0.5f, z, 1.f));
-  float q = fmaf(t, 0.17087277f, -0.82215223f);
-  q = fmaf(t, q, 1.48851587f);
-  q = fmaf(t, q, -1.13520398f);
-  q = fmaf(t, q, 0.27886807f);
-  q = fmaf(t, q, -0.18628806f);
-  q = fmaf(t, q, 0.09678418f);
-  q = fmaf(t, q, 0.37409196f);
-  q = fmaf(t, q, 1.00002368f);
-  q = fmaf(t, q, -1.26551223f);
-  return 0.5f * t * __expf(fmaf(-z, z, q));
+// Distribution function of the normal distribution, and exp(-x^2 / 2) beside it, without a branch: in the middle (|x| < 1.25) 1/2 + x P(x^2),
+// outside exp(-x^2 / 2) t Q(t) with t = 1 / (1 + 0.35 |x|) for the lower tail and one minus it above.  P and Q are minimax fits to the error
+// function (iteratively reweighted least squares in 64 bits against erf and the scaled erfc; 2e-9 absolute and, down to the smallest
+// normal float, 1.5e-8 relative).  Measured over 4 million points against 64 bits, largest and root mean square error, (1 + erff(x / sqrt 2)) / 2 in
+// brackets:  |x| < 0.5 4.0e-8, 1.4e-8 (5.1e-8, 1.5e-8);  to 1.25 5.3e-8, 1.5e-8 (6.3e-8, 1.8e-8);  1.25 to 3 6.1e-8, 1.8e-8 (6.3e-8, 2.4e-8);
+// relative in the lower tail 6e-7 at -3 (3e-5) and 2e-6 at -6 (all of it); the square in the exponent sets that.
+// The two ranges of erff, a branch, cost an epilogue of 32 unrolled elements 16 us of 44 (6144 x 2048 x 512 with the GELU gradient).
+__device__ __forceinline__ float normal_cdf(float x, float& bell) {
+  const float z = x * x, a = fabsf(x);
+  bell = exp2f(-0.72134752f * z);
+  const float t = __fdividef(1.f, fmaf(0.35f, a, 1.f));
+  float q = fmaf(t, 0.0444524474f, -0.111576788f);
+  q = fmaf(t, q, 0.0438466556f);
+  q = fmaf(t, q, 0.0324914902f);
+  q = fmaf(t, q, 0.0890091509f);
+  q = fmaf(t, q, 0.122769959f);
+  q = fmaf(t, q, 0.139575362f);
+  q = fmaf(t, q, 0.139633134f);
+  const float tail = q * t * bell;
+  float p = fmaf(z, -6.6448597e-06f, 0.000110327455f);
+  p = fmaf(z, p, -0.00118270959f);
+  p = fmaf(z, p, 0.00997150037f);
+  p = fmaf(z, p, -0.0664899871f);
+  p = fmaf(z, p, 0.398942262f);
+  return a < 1.25f ? fmaf(x, p, 0.5f) : x < 0.f ? tail : 1.f - tail;
 }
-__device__ __forceinline__ float normal_cdf(float x) {
-  const float tail = normal_tail(x);
-  return x < 0.f ? tail : 1.f - tail;
+__device__ __forceinline__ float gelu_f(float x) {
+  float bell;
+  return x * normal_cdf(x, bell);
 }
-__device__ __forceinline__ float gelu_f(float x) { return x * normal_cdf(x); }
 __device__ __forceinline__ float gelu_grad(float x) {
-  const float pdf = 0.3989422804014327f * __expf(-0.5f * x * x);
-  return normal_cdf(x) + x * pdf;
+  float bell;
+  const float cdf = normal_cdf(x, bell);
+  return cdf + x * (0.3989422804014327f * bell);
 }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 

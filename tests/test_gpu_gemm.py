@@ -369,3 +369,35 @@ def test_column_sums_beside_every_operand(M, N, K):
     finally:
         e.set_gemm_variant(0)
     assert ops.check_status() == 0
+
+
+def test_gelu_in_32_bits_is_as_close_as_erff():
+    """The epilogues' GELU and its gradient with 32-bit output against 64 bits, next to the formula with erff in 32 bits: no range of the input is
+    further off, and the lower tail keeps its relative accuracy."""
+    n, rows = 256, 288
+    x = (torch.arange(rows * n, device="cuda", dtype=torch.float64) - rows * n // 2) / 4096          # -9 to 9, at most 16 bits
+    # as a sum of two bf16 numbers, which a product with two stacked identities adds exactly
+    hi = x.bfloat16()
+    lo = (x - hi.double()).bfloat16()
+    assert torch.equal(x, hi.double() + lo.double())
+    eye = torch.eye(n, device="cuda").bfloat16()
+    out = torch.empty(rows, n, device="cuda")
+    ops.gemm(torch.cat([hi.view(rows, n), lo.view(rows, n)], 1), torch.cat([eye, eye], 1), out, act=2)
+    aux = torch.linspace(-9, 9, rows * n, device="cuda").bfloat16()
+    grad = torch.empty(rows, n, device="cuda")
+    ops.gemm(torch.ones(rows, n, device="cuda").bfloat16(), eye, grad, aux=aux.view(rows, n), act=6)
+    normal = lambda t: 0.5 * torch.erfc(-t / 2 ** 0.5)
+    bell = lambda t: torch.exp(-0.5 * t * t) / (2 * torch.pi) ** 0.5
+    with_erff = lambda t: 0.5 * (1.0 + torch.erf(t * 2 ** -0.5))
+    f, ad, af = x.float(), aux.double(), aux.float()
+    for name, t, got, want, plain in (("value", x, out.view(-1), x * normal(x), f * with_erff(f)),
+                                      ("gradient", ad, grad.view(-1), normal(ad) + ad * bell(ad), with_erff(af) + af * bell(af))):
+        err, ref = (got.double() - want).abs(), (plain.double() - want).abs()
+        for a, b in ((-9, -4), (-4, -2), (-2, -1.25), (-1.25, -0.5), (-0.5, 0.5), (0.5, 1.25), (1.25, 3), (3, 9)):
+            at = (t >= a) & (t < b)
+            rms, ref_rms = err[at].square().mean().sqrt(), ref[at].square().mean().sqrt()
+            assert rms <= 1.05 * ref_rms, (name, a, b, float(rms), float(ref_rms))
+            assert err[at].max() <= 2.0 ** -23 * max(1.0, b), (name, a, b, float(err[at].max()))     # two ulps of a result in [0.5, 1), or of x itself
+        low = (t > -8.5) & (t < -2)
+        assert (err[low] <= 4e-6 * want[low].abs()).all()
+    assert ops.check_status() == 0
