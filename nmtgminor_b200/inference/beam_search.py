@@ -289,6 +289,10 @@ class _DeviceSearch:
 
     def run(self):
         """All steps, then per sentence the ``n_best`` finished hypotheses, best first."""
+        with torch.cuda.device(self.tok.device):        # events and captures belong to the model's device, whichever is current
+            return self._run()
+
+    def _run(self):
         from .. import ops
         cfg, K = self.cfg, self.K
         seen = None

@@ -255,7 +255,7 @@ def test_device_search_stop_rule_without_penalty(B, K, V, alpha, end_bias):
     assert any([h.tokens for h in a] != [h.tokens for h in b] for a, b in zip(found, first_ended)), "the inputs must tell the two rules apart"
 
 
-def _successor_model(seed):
+def _successor_model(seed, device="cuda"):
     """A small Transformer on the GPU in which every word prefers one other word."""
     from nmtgminor_b200.data.synthetic import synthetic_dict
     from nmtgminor_b200.models.transformer import Transformer
@@ -270,9 +270,9 @@ def _successor_model(seed):
         order = torch.randperm(296) + 4
         model.generator.weight[order] = 1.5 * model.decoder.embed.weight[order.roll(1)]
         model.generator.weight[order[0]] += 1.5 * model.decoder.embed.weight[2]
-    model.store = FlatParameterStore(model, "cuda")
+    model.store = FlatParameterStore(model, device)
     for b in model.buffers():
-        b.data = b.data.cuda()
+        b.data = b.data.to(device)
     return model
 
 
@@ -398,3 +398,18 @@ def test_scores_do_not_depend_on_the_batch():
             states, _ = model.encode(pack(src[i:i + 1], None))
             at = int(seqs.cu[i])
             assert torch.equal(states[:len(src[i])], context[at:at + len(src[i])])
+
+
+def test_search_on_another_device_than_the_current_one():
+    """The flags that end a search early are waited for on the model's device."""
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    from nmtgminor_b200.data.dataset import collate
+    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
+    cfg = BeamConfig(beam_size=3, max_len=200, min_len=30)
+    batches = [collate([torch.arange(4, 4 + n), torch.arange(30, 36)], None, padded=True, packed=True, round_to=1) for n in (9, 20, 30)]
+    found = []
+    for device in ("cuda:0", "cuda:1"):
+        model = _successor_model(14, device)
+        found.append([[h[0].tokens for h in beam_search(model, b.cuda(device), cfg)] for b in batches])
+    assert found[0] == found[1]
