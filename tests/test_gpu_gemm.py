@@ -401,3 +401,24 @@ def test_gelu_in_32_bits_is_as_close_as_erff():
         low = (t > -8.5) & (t < -2)
         assert (err[low] <= 4e-6 * want[low].abs()).all()
     assert ops.check_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(200, 72, 128), (704, 1024, 256), (1000, 520, 264), (1920, 512, 512), (3840, 512, 1000)])
+def test_one_wave_tiles_of_data_gradients(M, N, K):
+    """The same narrow tiles with the weight as the [K, N] operand of a data gradient: plain, with the sign bits and their column sums, with an
+    activation gradient.  One accumulator per element, its products in the order of the CTA-pair kernel."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    dy, w, aux = rnd(M, K), rnd(K, N) * K ** -0.5, rnd(M, N)
+    bits = torch.randint(-2 ** 31, 2 ** 31 - 1, (M, (N + 31) // 32), device="cuda", generator=g).int()
+    got = []
+    for forced in (0, 256):
+        out = [torch.zeros(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(4)]
+        ops.gemm(dy, w, out[0], b_mn_major=True, force_bn=forced)
+        ops.gemm(dy, w, out[1], b_mn_major=True, act=8, mask=bits, alpha=1.25, colsum=torch.zeros(N, device="cuda"), force_bn=forced)
+        ops.gemm(dy, w, out[2], b_mn_major=True, act=6, aux=aux, force_bn=forced)
+        ops.gemm(dy, w, out[3], b_mn_major=True, act=7, aux=aux, dropout_p=0.25, seed=3, stream_id=2, force_bn=forced)
+        got.append(out)
+    assert ops.check_status() == 0
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
