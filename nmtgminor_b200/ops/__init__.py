@@ -162,7 +162,9 @@ def gemm(a, b, out, *, a_mn_major=False, b_mn_major=False, bias=None, residual=N
          mask=None, colsum=None, gather=None):
     """out[M,N] = epilogue(alpha * A B^T) on the tcgen05 kernel (see csrc/ops_api.h: GemmDesc).  ``mask`` (int32
     [M, ceil(N/32)]) receives the sign bits of the output, or supplies them when ``act`` is the mask-backward id 8.
-    ``colsum`` (fp32 [N]): the column sums of the bf16 output are added to it by the epilogue (bias gradients).
+    ``colsum`` (fp32 [N]): the column sums of the bf16 output are added to it by the epilogue (bias gradients; more than 128 rows).
+    ``allow_split_k``: the sum over K may be cut into parts (fp32 outputs, and few rows: see ``step_sums``); ``force_bn``: tile width, 128 or 256
+    (64 on the single-CTA kernel).
     ``gather``: record of a fully sharded weight (``parallel.fsdp.GatherInfo``) whose pieces this call pulls from
     their owners into ``b`` before (and while) it multiplies."""
     g = gather.pending() if gather is not None else None
@@ -346,7 +348,7 @@ class _MlpFn(torch.autograd.Function):
         dz1 = torch.empty_like(h)
         fused_gb1 = False
         if act == 1:   # the sign bits encode ReLU and the dropout mask; only the keep scale is missing
-            # with more than 128 rows the CTA-pair kernel runs, whose epilogue can also sum the columns (fc1 bias gradient)
+            # with more than 128 rows the epilogue can also sum the columns (fc1 bias gradient)
             fused_gb1 = gb1 is not None and dz2.shape[0] > 128 and dz1.shape[1] % 8 == 0
             gemm(dz2, w2, dz1, b_mn_major=True, act=8, mask=z, alpha=_keep_scale(p1), colsum=gb1 if fused_gb1 else None,
                  gather=ctx.gathers[1])

@@ -45,19 +45,21 @@ struct GemmDesc {
                           // epilogues (before the residual), read by kActMaskBwd
   int ld_mask;
   float* colsum;          // optional fp32 [N]: column sums of the (bf16-rounded) output are ADDED here (bias gradient of the
-                          // layer whose output gradient this GEMM produces); CTA-pair kernel with the TMA-store epilogue only
+                          // layer whose output gradient this GEMM produces); more than 128 rows, no stored pre-activation
   int act;
   float dropout_p; unsigned long long seed, stream_id;
   const unsigned long long* seed_dev;  // optional device word added to seed (lets graph replays draw new masks)
   int split_k;            // 0 = automatic (only when allow_split_k), else forced
-  int allow_split_k;      // the sum over K may be split: fp32 outputs (atomic adds), and bf16 outputs with few rows (CTA clusters)
-  int force_bn;           // 0 = automatic, 128 or 256
+  int allow_split_k;      // the sum over K may be split: fp32 outputs (atomic adds), and bf16 outputs with few rows (CTA clusters; the number of
+                          // parts then depends on M, so that a row's last bit depends on how many rows stand beside it)
+  int force_bn;           // 0 = automatic, 128 or 256, or 64 with the single-CTA kernel (nmtg_set_gemm_variant(1), M <= 128)
   int* status;            // device int, 0 = ok
   const NmtgGather* gather;  // optional: B is gathered from its owners by this call (see NmtgGather)
 };
 
 const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream);
-// 0 = automatic (CTA-pair kernel when M > 128), 1 = single-CTA kernel only, 2 = same as 0
+// 0 = automatic (CTA-pair kernel when M > 128, unless the problem is a few rows or less than a wave of narrow tiles), 1 = single-CTA kernel
+// (products with column sums excepted), 2 = CTA-pair kernel when M > 128
 void nmtg_set_gemm_variant(int v);
 // n (even) SMs are left free by every launcher of this library: persistent kernels size their grids for the rest, so that
 // communication kernels placed on the free SMs (nmtg_reduce_unit with a negative CTA count) never share one with them.
