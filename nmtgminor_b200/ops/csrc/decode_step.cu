@@ -233,13 +233,13 @@ __device__ __forceinline__ void attend_apart(Running (&run)[KB], const float (&q
 template <int KB>
 __global__ void __launch_bounds__(32 * kStepWarps, 2)
 decode_self_kernel(const __nv_bfloat16* __restrict__ qkv, long ld, __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc,
-                   const int* __restrict__ anc, const long* __restrict__ pos_rows, __nv_bfloat16* __restrict__ out, int K, int groups,
+                   const int* __restrict__ anc, const long* __restrict__ pos_rows, __nv_bfloat16* __restrict__ out, int first, int K, int groups,
                    int heads, int cap, float scale) {
   constexpr int KU = keys_of<KB>();
   __shared__ __align__(16) float qs[KB][64];
   __shared__ float part[kStepWarps][KB][66];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int h = blockIdx.x % heads, item = blockIdx.x / heads;
+  const int h = blockIdx.x, item = first + blockIdx.y;
   const int r0 = (item / groups) * K + (item % groups) * KB;
   const int beams = min(KB, K - (item % groups) * KB);
   const int hid = heads * 64;
@@ -317,14 +317,14 @@ decode_self_kernel(const __nv_bfloat16* __restrict__ qkv, long ld, __nv_bfloat16
 template <int KB>
 __global__ void __launch_bounds__(32 * kStepWarps, 2)
 decode_cross_kernel(const __nv_bfloat16* __restrict__ q, long ld, const __nv_bfloat16* __restrict__ ck, const __nv_bfloat16* __restrict__ cv,
-                    const int* __restrict__ lengths, __nv_bfloat16* __restrict__ out, int K, int groups, int heads, int cap, float scale,
-                    int splits) {
+                    const int* __restrict__ lengths, __nv_bfloat16* __restrict__ out, int first, int K, int groups, int heads, int cap,
+                    float scale, int splits) {
   constexpr int KU = keys_of<KB>();
   __shared__ __align__(16) float qs[KB][64];
   __shared__ float part[kStepWarps][KB][66];
   __shared__ __align__(16) float mine[KB][68];      // this CTA's sums, read by the whole cluster
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int h = blockIdx.x % heads, item = blockIdx.x / heads;
+  const int h = blockIdx.x, item = first + blockIdx.y;
   const int b = item / groups, k0 = (item % groups) * KB;
   const int beams = min(KB, K - k0);
   const int share = blockIdx.z;
@@ -459,12 +459,12 @@ template <> __device__ __forceinline__ float as_float<__nv_bfloat16>(__nv_bfloat
 template <typename T>
 __global__ void __launch_bounds__(kPartThreads)
 beam_part_kernel(const T* __restrict__ logits, long ld, const uint8_t* __restrict__ force, float2* __restrict__ part_lse,
-                 Cand* __restrict__ part, int pieces, int K2, int V, int pad, int eos, int vec) {
+                 Cand* __restrict__ part, int first, int K2, int V, int pad, int eos, int vec) {
   __shared__ Cand list[kPartCols];
   __shared__ float red[2][kPartThreads / 32];
   __shared__ int count;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kPartThreads / 32;
-  const int r = blockIdx.x / pieces, piece = blockIdx.x - r * pieces;
+  const int r = first + blockIdx.y, piece = blockIdx.x;
   const int c0 = piece * kPartCols;
   pdl_trigger();
   pdl_wait();
@@ -542,7 +542,7 @@ beam_part_kernel(const T* __restrict__ logits, long ld, const uint8_t* __restric
   for (int i = 0; i < kPartEach; ++i)
     if ((takes >> i) & 1u) list[at++] = (static_cast<Cand>(key[i]) << 32) | (kNone - static_cast<uint32_t>(c0 + col[i / kPer] + i % kPer));
   __syncthreads();
-  const long o = static_cast<long>(r) * pieces + piece;
+  const long o = static_cast<long>(r) * gridDim.x + piece;
   if (threadIdx.x == kPartThreads - 1) {
     float s = 0.f;
     for (int w = 0; w < warps; ++w) s += red[1][w];
@@ -769,14 +769,25 @@ int step_warps(long ctas, int blocks, int sms) {
   return w;
 }
 
+// go(first, n) for runs of at most 65535 rows, the most that a grid holds along its second dimension (rows and heads in one
+// dimension instead made the attention over 1500 frames take 52 us for 46, the wait for the kernel before it included)
+template <typename Go>
+const char* by_rows(int rows, Go go) {
+  for (int first = 0; first < rows; first += 65535)
+    if (const char* e = go(first, rows - first < 65535 ? rows - first : 65535)) return e;
+  return nullptr;
+}
+
 template <int KB>
 const char* launch_self(const void* qkv, long ld, void* kc, void* vc, const int* anc, const long* pos_rows, void* out, int B, int K, int heads,
                         int cap, float scale, int sms, cudaStream_t stream) {
   const int groups = (K + KB - 1) / KB;
   const int warps = step_warps(static_cast<long>(heads) * B * groups, cap, sms);
-  return launch(decode_self_kernel<KB>, dim3(heads * B * groups), dim3(32 * warps), 0, 1, stream, static_cast<const __nv_bfloat16*>(qkv), ld,
-                static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), anc, pos_rows, static_cast<__nv_bfloat16*>(out), K, groups,
-                heads, cap, scale);
+  return by_rows(B * groups, [&](int first, int n) {
+    return launch(decode_self_kernel<KB>, dim3(heads, n), dim3(32 * warps), 0, 1, stream, static_cast<const __nv_bfloat16*>(qkv), ld,
+                  static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), anc, pos_rows, static_cast<__nv_bfloat16*>(out), first, K,
+                  groups, heads, cap, scale);
+  });
 }
 
 template <int KB>
@@ -791,9 +802,11 @@ const char* launch_cross(const void* q, long ld, const void* ck, const void* cv,
   while (splits < 8 && ctas * splits < 4L * sms && cap >= splits * 2 * 128) splits *= 2;
   const int blocks = (cap / splits + 4 * keys_of<KB>() - 1) / (4 * keys_of<KB>());
   const int warps = cap > 512 ? 4 : step_warps(ctas * splits, blocks, sms);
-  return launch(decode_cross_kernel<KB>, dim3(heads * B * groups, 1, splits), dim3(32 * warps), 0, splits, stream,
-                static_cast<const __nv_bfloat16*>(q), ld, static_cast<const __nv_bfloat16*>(ck), static_cast<const __nv_bfloat16*>(cv),
-                lengths, static_cast<__nv_bfloat16*>(out), K, groups, heads, cap, scale, splits);
+  return by_rows(B * groups, [&](int first, int n) {
+    return launch(decode_cross_kernel<KB>, dim3(heads, n, splits), dim3(32 * warps), 0, splits, stream,
+                  static_cast<const __nv_bfloat16*>(q), ld, static_cast<const __nv_bfloat16*>(ck), static_cast<const __nv_bfloat16*>(cv),
+                  lengths, static_cast<__nv_bfloat16*>(out), first, K, groups, heads, cap, scale, splits);
+  });
 }
 
 }  // namespace
@@ -835,13 +848,13 @@ const char* nmtg_beam_step(const NmtgBeam* s, const void* logits, long ld, int d
   const int vec = (ld * (dtype == 0 ? 4 : 2)) % 16 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
   float2* lse = static_cast<float2*>(part_lse);
   Cand* cand = static_cast<Cand*>(part);
-  const char* e;
-  if (dtype == 0)
-    e = launch(beam_part_kernel<float>, dim3(pieces * R), dim3(kPartThreads), 0, 1, stream, static_cast<const float*>(logits), ld, s->force, lse,
-               cand, pieces, K2, V, s->pad, s->eos, vec);
-  else
-    e = launch(beam_part_kernel<__nv_bfloat16>, dim3(pieces * R), dim3(kPartThreads), 0, 1, stream, static_cast<const __nv_bfloat16*>(logits),
-               ld, s->force, lse, cand, pieces, K2, V, s->pad, s->eos, vec);
+  const char* e = by_rows(R, [&](int first, int n) {
+    if (dtype == 0)
+      return launch(beam_part_kernel<float>, dim3(pieces, n), dim3(kPartThreads), 0, 1, stream, static_cast<const float*>(logits), ld, s->force,
+                    lse, cand, first, K2, V, s->pad, s->eos, vec);
+    return launch(beam_part_kernel<__nv_bfloat16>, dim3(pieces, n), dim3(kPartThreads), 0, 1, stream, static_cast<const __nv_bfloat16*>(logits),
+                  ld, s->force, lse, cand, first, K2, V, s->pad, s->eos, vec);
+  });
   if (e) return e;
   // the pieces' candidates are staged in shared memory unless a wide beam over a large vocabulary makes them many
   const size_t tables = static_cast<size_t>(K) * K2 * 16 + 4 * (2 * K2 + K + K * 256 + 7 * K), cands = static_cast<size_t>(K) * pieces * K2 * 8;
