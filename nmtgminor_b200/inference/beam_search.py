@@ -160,27 +160,24 @@ class _StepPools:
             self.sets[key] = kept
 
     @classmethod
-    def of(cls, model, device):
-        with cls.lock:
-            return cls._of(model, device)
-
-    @classmethod
-    def _of(cls, model, device):
+    def of(cls, model, device, modules=None):
+        """The pool of ``model`` as it is now (``modules``: those of its decoder, if they are at hand)."""
         emb = getattr(model.decoder, "embed", None)
-        table = emb._pos_table(device) if hasattr(emb, "_pos_table") else None
-        held, state = [table], []
-        for part in (model.decoder, getattr(model, "generator", None)):
-            for m in part.modules() if part is not None else ():
-                state.append(m.training)
+        modules = list(model.decoder.modules()) if modules is None else modules
+        held = [emb._pos_table(device) if hasattr(emb, "_pos_table") else None]
+        generator = getattr(model, "generator", None)
+        for m in (*modules, *(generator.modules() if generator is not None else ())):
+            if m._parameters or m._buffers:
                 for t in (*m._parameters.values(), *m._buffers.values()):
-                    if t is not None:
-                        held += (t, getattr(t, "work", None))
-        state += [(t.data_ptr(), t.shape) if t is not None else None for t in held]
-        pools = model.__dict__.get("_decode_pools")
-        if pools is None or pools.state != state:
-            pools = model.__dict__["_decode_pools"] = cls(state)
-            # the storage that is there now: a parameter can be pointed at another
-            pools.held = [t.detach() for t in held if t is not None]
+                    held += (t, getattr(t, "work", None))
+        state = [m.training for m in modules]
+        state += [None if t is None else (t.data_ptr(), t.shape) for t in held]
+        with cls.lock:
+            pools = model.__dict__.get("_decode_pools")
+            if pools is None or pools.state != state:
+                pools = model.__dict__["_decode_pools"] = cls(state)
+                # the storage that is there now: a parameter can be pointed at another
+                pools.held = [t.detach() for t in held if t is not None]
         return pools
 
     def __reduce__(self):           # a copied or saved model starts without
@@ -211,11 +208,12 @@ class _DeviceSearch:
         if emb is not None and hasattr(emb, "renew"):
             emb.renew(cap)
         from ..models.layers import SelfAttention
-        widths = [m.dim for m in model.decoder.modules() if isinstance(m, SelfAttention)]
+        modules = list(model.decoder.modules())
+        widths = [m.dim for m in modules if isinstance(m, SelfAttention)]
         cross = [b for b in state.buffers if "c_k" in b]
         src_cap = (max(b["c_k"].shape[1] for b in cross) + 63) // 64 * 64 if cross else 0
         self.key = (B, K, cap, src_cap, len(state.buffers), str(dev), cfg.pad, cfg.eos)
-        self.pools = _StepPools.of(model, dev)
+        self.pools = _StepPools.of(model, dev, modules)
         pool = self.pools.take(self.key)
         if pool is None:
             with torch.inference_mode(False), torch.no_grad():      # kept tables serve callers in either mode
