@@ -136,8 +136,8 @@ def _replayable(model, state) -> bool:
 
 class _StepPools:
     """Table sets, and the graphs captured over them, of one model in one state.  A graph has the address of every tensor baked in that
-    its step reads besides its own tables; those tensors are held here, so that as long as the model has the same addresses it
-    has the same tensors.  A model that has others (a longer position table, a new weight store, a layer replaced) gets a new object.
+    its step reads besides its own tables.  The state is those addresses, so that a graph is replayed only on a model whose tensors
+    lie where they lay; one that has moved (a longer position table, a new weight store, a layer replaced) gets a new object.
 
     Searches may run in several threads: a set belongs to one search at a time, and the lock guards the sets and the captures."""
 
@@ -161,24 +161,23 @@ class _StepPools:
 
     @classmethod
     def of(cls, model, device, modules=None):
-        """The pool of ``model`` as it is now (``modules``: those of its decoder, if they are at hand)."""
+        """The pool of ``model`` as it is now, and the tensors that its steps read: a search holds on to them, since another thread may
+        replace the position table meanwhile.  ``modules``: those of the decoder, if they are at hand."""
         emb = getattr(model.decoder, "embed", None)
         modules = list(model.decoder.modules()) if modules is None else modules
-        held = [emb._pos_table(device) if hasattr(emb, "_pos_table") else None]
+        reads = [emb._pos_table(device) if hasattr(emb, "_pos_table") else None]
         generator = getattr(model, "generator", None)
         for m in (*modules, *(generator.modules() if generator is not None else ())):
             if m._parameters or m._buffers:
                 for t in (*m._parameters.values(), *m._buffers.values()):
-                    held += (t, getattr(t, "work", None))
+                    reads += (t, getattr(t, "work", None))
         state = [m.training for m in modules]
-        state += [None if t is None else (t.data_ptr(), t.shape) for t in held]
+        state += [None if t is None else (t.data_ptr(), t.shape, t.dtype) for t in reads]
         with cls.lock:
             pools = model.__dict__.get("_decode_pools")
             if pools is None or pools.state != state:
                 pools = model.__dict__["_decode_pools"] = cls(state)
-                # the storage that is there now: a parameter can be pointed at another
-                pools.held = [t.detach() for t in held if t is not None]
-        return pools
+        return pools, reads
 
     def __reduce__(self):           # a copied or saved model starts without
         return type(None), ()
@@ -213,7 +212,7 @@ class _DeviceSearch:
         cross = [b for b in state.buffers if "c_k" in b]
         src_cap = (max(b["c_k"].shape[1] for b in cross) + 63) // 64 * 64 if cross else 0
         self.key = (B, K, cap, src_cap, len(state.buffers), str(dev), cfg.pad, cfg.eos)
-        self.pools = _StepPools.of(model, dev, modules)
+        self.pools, self.reads = _StepPools.of(model, dev, modules)
         pool = self.pools.take(self.key)
         if pool is None:
             with torch.inference_mode(False), torch.no_grad():      # kept tables serve callers in either mode
@@ -275,13 +274,13 @@ class _DeviceSearch:
             return self._body()
         while pool["graph"] is None:
             with _StepPools.lock:               # one capture at a time, on a stream of its own
-                self.pools = _StepPools.of(self.model, self.tok.device)
+                self.pools, self.reads = _StepPools.of(self.model, self.tok.device)
                 g = torch.cuda.CUDAGraph()
                 torch.cuda.synchronize()
                 with torch.cuda.graph(g, stream=torch.cuda.Stream(self.tok.device), capture_error_mode="thread_local"):
                     self._body()                # captured, not run
-                # another thread may have renewed the position table meanwhile: then this graph is not what the pool holds
-                if _StepPools.of(self.model, self.tok.device) is self.pools:
+                # another thread may have renewed the position table meanwhile: then this graph reads another one than is held
+                if _StepPools.of(self.model, self.tok.device)[0] is self.pools:
                     pool["graph"] = g
         pool["graph"].replay()
 

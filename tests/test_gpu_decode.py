@@ -413,3 +413,23 @@ def test_search_on_another_device_than_the_current_one():
         model = _successor_model(14, device)
         found.append([[h[0].tokens for h in beam_search(model, b.cuda(device), cfg)] for b in batches])
     assert found[0] == found[1]
+
+
+def test_searches_keep_no_weights():
+    """Between searches nothing holds the weights that the captured steps read: a replaced store is freed."""
+    import gc
+
+    from nmtgminor_b200.data.dataset import collate
+    from nmtgminor_b200.inference.beam_search import BeamConfig, beam_search
+    from nmtgminor_b200.parallel.flat import FlatParameterStore
+    model = _successor_model(15)
+    batch = collate([torch.arange(4, 20)], None, padded=True, packed=True, round_to=1).cuda("cuda")
+    search = lambda: beam_search(model, batch, BeamConfig(beam_size=2, max_len=20, min_len=10))[0][0].tokens
+    want = search()
+    assert search() == want
+    gc.collect()
+    before = torch.cuda.memory_allocated()
+    model.store = FlatParameterStore(model, "cuda")
+    gc.collect()
+    assert torch.cuda.memory_allocated() - before < model.store.work.numel()
+    assert search() == want
