@@ -34,6 +34,7 @@ struct GemmArgs {
   unsigned long long seed, stream_id;
   const unsigned long long* seed_dev;
   int* status;
+  int by_element;          // an epilogue operand is not on a 16-byte boundary: nothing of it moves as vectors
   int tma_store;           // bf16 output leaves through shared memory and TMA stores (CTA-pair kernel)
   int tma_second;          // so does the pre-activation, and the aux operand comes in that way (see two_stagings)
   int ablate;              // profiling aid: 1 = read the accumulator but skip arithmetic and stores, 2 = skip the epilogue body,
@@ -108,7 +109,7 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __ex
 // rather than on arithmetic.  kEpiAll is the general kernel.
 constexpr uint32_t kEpiBias = 1u, kEpiPreact = 2u, kEpiActFwd = 4u, kEpiActBwd = 8u, kEpiMaskBwd = 16u, kEpiDrop = 32u,
                    kEpiMaskOut = 64u, kEpiRes = 128u, kEpiF32 = 256u, kEpiBf16 = 512u,
-                   kEpiRagged = 1024u /* N not a multiple of 64: partial column chunks */,
+                   kEpiRagged = 1024u /* N not a multiple of 64, or unaligned operands: column chunks element by element */,
                    kEpiColsum = 2048u /* column sums of the output */, kEpiAll = 4095u;
 
 // Features a problem needs (host side).
@@ -123,7 +124,7 @@ inline uint32_t gemm_epilogue_features(const GemmArgs& a) {
   if (a.mask && a.act != kActMaskBwd) f |= kEpiMaskOut;
   if (a.residual) f |= kEpiRes;
   f |= a.out_fp32 ? kEpiF32 : kEpiBf16;
-  if (a.N % 64) f |= kEpiRagged;
+  if (a.N % 64 || a.by_element) f |= kEpiRagged;
   if (a.colsum) f |= kEpiColsum;
   return f;
 }
@@ -134,7 +135,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
                                                     uint8_t* stage_row = nullptr, const int stage_half = 0,
                                                     const int stage_r = 0, uint8_t* pre_row = nullptr,
                                                     const bool aux_staged = false) {
-    const bool full_cols = !(kFeat & kEpiRagged) || (col0 + 32 <= p.N);
+    const bool full_cols = !(kFeat & kEpiRagged) || (!p.by_element && col0 + 32 <= p.N);
     // global operands of the epilogue are requested BEFORE the TMEM load so their latency overlaps it
     uint4 aux_v[4], res_v[4];
     const bool aux_vec = (kFeat & kEpiActBwd) && !aux_staged && row_ok && full_cols && p.act >= kActReluBwd && p.act != kActMaskBwd && (p.ld_aux & 7) == 0;

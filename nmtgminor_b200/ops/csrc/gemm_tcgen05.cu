@@ -476,6 +476,8 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   a.preact = reinterpret_cast<__nv_bfloat16*>(d->preact);
   a.mask = reinterpret_cast<uint32_t*>(d->mask); a.ld_mask = d->ld_mask;
   a.colsum = d->colsum;
+  a.by_element = ((reinterpret_cast<uintptr_t>(d->bias) | reinterpret_cast<uintptr_t>(d->residual) | reinterpret_cast<uintptr_t>(d->aux) |
+                   reinterpret_cast<uintptr_t>(d->preact)) & 15) != 0;
   a.ablate = g_gemm_ablate;
   a.stream_k = 0;
   a.trace = g_gemm_trace;

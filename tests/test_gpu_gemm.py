@@ -422,3 +422,25 @@ def test_one_wave_tiles_of_data_gradients(M, N, K):
     assert ops.check_status() == 0
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M,N,K", [(4, 128, 64), (200, 256, 128), (700, 512, 256), (5000, 1024, 64)])
+@pytest.mark.parametrize("off", [1, 4])
+def test_epilogue_operands_off_their_boundary(M, N, K, off):
+    """Residual, bias, aux operand and pre-activation that start inside a 16-byte unit: the results of aligned copies."""
+    g = torch.Generator(device="cuda").manual_seed(M + off)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w = rnd(M, K), rnd(N, K) * K ** -0.5
+    res, bias, pre = rnd(M, N + 8)[:, off:off + N], rnd(N + 8)[off:off + N], torch.zeros(M * N + 8, device="cuda").bfloat16()[off:off + M * N].view(M, N)
+    new = lambda: torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+    for kw in (dict(residual=res), dict(bias=bias), dict(bias=bias, act=2), dict(aux=res, act=6), dict(aux=res, act=5, dropout_p=0.25, seed=3, stream_id=1),
+               dict(bias=bias, act=1, preact=pre, dropout_p=0.25, seed=3, stream_id=1)):
+        for split in (False, True):
+            a, b = new(), new()
+            ops.gemm(x, w, a, allow_split_k=split, **kw)
+            whole = {k: v.clone() if torch.is_tensor(v) else v for k, v in kw.items()}
+            ops.gemm(x, w, b, **whole)
+            assert torch.allclose(a.float(), b.float(), rtol=2 ** -7, atol=2 ** -9) if split else torch.equal(a, b), list(kw)
+            if "preact" in kw:
+                assert torch.equal(kw["preact"], whole["preact"])
+    assert ops.check_status() == 0
