@@ -23,6 +23,11 @@ int dtype_code(const Tensor& t) {
 void need(const Tensor& t, at::ScalarType ty, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == ty, name, ": wrong device, layout or dtype");
 }
+// [rows, cap, heads * 64] caches, read with 16-byte loads
+void need_cache(const Tensor& t, const char* name) {
+  need(t, at::kBFloat16, name);
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, name, " must start on a 16-byte boundary");
+}
 const long* off_ptr(const OptTensor& t) {
   if (!t.has_value()) return nullptr;
   need(*t, at::kLong, "batch_offset");
@@ -199,11 +204,12 @@ void gather_rows(const Tensor& src, Tensor& dst, const Tensor& index, int64_t co
 Tensor decode_attn(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const OptTensor& lengths, int64_t len,
                    int64_t heads, double scale) {
   TORCH_CHECK(q.is_cuda() && q.scalar_type() == at::kBFloat16 && q.dim() == 2 && q.stride(1) == 1);
-  need(k_cache, at::kBFloat16, "k_cache"); need(v_cache, at::kBFloat16, "v_cache");
+  need_cache(k_cache, "k_cache"); need_cache(v_cache, "v_cache");
   TORCH_CHECK(k_cache.dim() == 3 && k_cache.sizes() == v_cache.sizes() && k_cache.size(2) == heads * 64 && q.size(1) == heads * 64);
   c10::cuda::CUDAGuard guard(q.device());
   const int R = q.size(0), cap = k_cache.size(1);
-  TORCH_CHECK(R % k_cache.size(0) == 0, "query rows must be a multiple of cache rows");
+  TORCH_CHECK(k_cache.size(0) > 0 && R % k_cache.size(0) == 0, "query rows must be a multiple of cache rows");
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(q.data_ptr()) & 15) == 0, "q must start on a 16-byte boundary");
   const int kv_div = R / k_cache.size(0);
   const int* lp = nullptr;
   if (lengths.has_value()) { need(*lengths, at::kInt, "lengths"); TORCH_CHECK(lengths->numel() == k_cache.size(0)); lp = lengths->data_ptr<int>(); }
@@ -216,8 +222,10 @@ Tensor decode_attn(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache
 void cache_append(const Tensor& k_new, const Tensor& v_new, Tensor& k_cache, Tensor& v_cache, int64_t pos) {
   TORCH_CHECK(k_new.is_cuda() && k_new.scalar_type() == at::kBFloat16 && k_new.dim() == 2 && k_new.stride(1) == 1);
   TORCH_CHECK(v_new.scalar_type() == at::kBFloat16 && v_new.stride(1) == 1 && v_new.stride(0) == k_new.stride(0) && v_new.sizes() == k_new.sizes());
-  need(k_cache, at::kBFloat16, "k_cache"); need(v_cache, at::kBFloat16, "v_cache");
-  TORCH_CHECK(k_cache.dim() == 3 && k_cache.size(0) >= k_new.size(0) && k_cache.size(2) == k_new.size(1) && k_new.size(1) % 64 == 0);
+  need_cache(k_cache, "k_cache"); need_cache(v_cache, "v_cache");
+  TORCH_CHECK(((reinterpret_cast<uintptr_t>(k_new.data_ptr()) | reinterpret_cast<uintptr_t>(v_new.data_ptr())) & 15) == 0,
+              "new keys and values must start on a 16-byte boundary");
+  TORCH_CHECK(k_cache.dim() == 3 && k_cache.sizes() == v_cache.sizes() && k_cache.size(0) >= k_new.size(0) && k_cache.size(2) == k_new.size(1) && k_new.size(1) % 64 == 0);
   c10::cuda::CUDAGuard guard(k_new.device());
   ck(nmtg_cache_append(k_new.data_ptr(), v_new.data_ptr(), k_new.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
                        static_cast<int>(k_new.size(0)), static_cast<int>(k_new.size(1) / 64), static_cast<int>(k_cache.size(1)),
@@ -228,7 +236,7 @@ Tensor decode_self(const Tensor& qkv, Tensor& k_cache, Tensor& v_cache, const Te
                    double scale) {
   TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == at::kBFloat16 && qkv.dim() == 2 && qkv.stride(1) == 1 && qkv.size(1) == 3 * heads * 64 &&
               (reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 15) == 0);
-  need(k_cache, at::kBFloat16, "k_cache"); need(v_cache, at::kBFloat16, "v_cache"); need(anc, at::kInt, "anc"); need(pos_rows, at::kLong, "pos_rows");
+  need_cache(k_cache, "k_cache"); need_cache(v_cache, "v_cache"); need(anc, at::kInt, "anc"); need(pos_rows, at::kLong, "pos_rows");
   const int R = qkv.size(0);
   TORCH_CHECK(k_cache.dim() == 3 && k_cache.sizes() == v_cache.sizes() && k_cache.size(0) == R && k_cache.size(2) == heads * 64);
   TORCH_CHECK(K > 0 && R % K == 0 && anc.dim() == 2 && anc.size(0) == R && anc.size(1) == k_cache.size(1) && pos_rows.numel() == R);
@@ -243,7 +251,7 @@ Tensor decode_self(const Tensor& qkv, Tensor& k_cache, Tensor& v_cache, const Te
 
 Tensor decode_cross(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& lengths, int64_t heads, double scale) {
   TORCH_CHECK(q.is_cuda() && q.scalar_type() == at::kBFloat16 && q.dim() == 2 && q.stride(1) == 1 && q.size(1) == heads * 64);
-  need(k_cache, at::kBFloat16, "k_cache"); need(v_cache, at::kBFloat16, "v_cache"); need(lengths, at::kInt, "lengths");
+  need_cache(k_cache, "k_cache"); need_cache(v_cache, "v_cache"); need(lengths, at::kInt, "lengths");
   TORCH_CHECK(k_cache.dim() == 3 && k_cache.sizes() == v_cache.sizes() && k_cache.size(2) == heads * 64);
   const int R = q.size(0), B = k_cache.size(0);
   TORCH_CHECK(B > 0 && R % B == 0 && lengths.numel() == B, "query rows must be a multiple of cache rows");

@@ -433,3 +433,17 @@ def test_searches_keep_no_weights():
     gc.collect()
     assert torch.cuda.memory_allocated() - before < model.store.work.numel()
     assert search() == want
+
+
+def test_unaligned_caches_are_refused():
+    """The caches are read with 16-byte loads: one that starts inside such a unit is an error on the host."""
+    e, R, hid = ops.ext(), 4, 128
+    flat = torch.zeros(R * 8 * hid + 8, device="cuda").bfloat16()
+    good, bad = flat[:R * 8 * hid].view(R, 8, hid), flat[1:R * 8 * hid + 1].view(R, 8, hid)
+    q, qkv, lens = torch.zeros(R, hid, device="cuda").bfloat16(), torch.zeros(R, 3 * hid, device="cuda").bfloat16(), torch.ones(R, dtype=torch.int32, device="cuda")
+    anc, pos = torch.zeros(R, 8, dtype=torch.int32, device="cuda"), torch.zeros(R, dtype=torch.long, device="cuda")
+    for k, v in ((bad, good), (good, bad)):
+        for call in (lambda: e.decode_cross(q, k, v, lens, 2, 0.125), lambda: e.decode_attn(q, k, v, lens, 8, 2, 0.125),
+                     lambda: e.decode_self(qkv, k, v, anc, pos, 2, 2, 0.125), lambda: e.cache_append(q, q, k, v, 0)):
+            with pytest.raises(RuntimeError, match="16-byte"):
+                call()
