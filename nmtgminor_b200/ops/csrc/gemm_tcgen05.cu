@@ -422,6 +422,45 @@ void nmtg_set_gemm_variant(int v) {
   else g_gemm_variant = v;
 }
 
+// largest split <= requested whose last part is not empty
+static int fix_split(int split, int num_kb) {
+  if (split > num_kb) split = num_kb;
+  while (split > 1 && (split - 1) * ((num_kb + split - 1) / split) >= num_kb) --split;
+  return split < 1 ? 1 : split;
+}
+
+// How the CTA-pair kernel would sum over K: parts of whole tiles, or (weight gradients: fp32, accumulating, where the tiles do not fill the
+// clusters evenly) an equal run of k-blocks for every cluster instead of whole tiles
+// (measured: a gain where whole tiles leave a fifth or more of the clusters idle, and for many-wave problems such
+// as the generator; a loss of 5-15 % from the extra partial-tile reductions where the tiles nearly fill a wave)
+struct PairPlan {
+  int split, stream_k;
+  long chain;          // k-blocks that one accumulator adds up
+};
+static PairPlan plan_pair(const GemmDesc* d, int sms, int num_kb, int bn) {
+  const long tiles = static_cast<long>((d->M + 2 * BM - 1) / (2 * BM)) * ((d->N + bn - 1) / bn);
+  const int clusters = sms / 2;
+  int split = 1;
+  if (d->split_k > 0) split = d->split_k;
+  else if (d->out_fp32 && d->allow_split_k) {
+    while (tiles * split * 2 <= clusters && num_kb / (split * 2) >= 8) split *= 2;
+  }
+  PairPlan p;
+  p.split = fix_split(split, num_kb);
+  p.stream_k = 0;
+  p.chain = (num_kb + p.split - 1) / p.split;
+  const long units = tiles * p.split;
+  const double wave_fill = static_cast<double>(units) / (static_cast<double>((units + clusters - 1) / clusters) * clusters);
+  if (g_stream_k && d->out_fp32 && d->accumulate && d->allow_split_k && d->split_k <= 0 && (units % clusters) != 0 &&
+      tiles * num_kb / clusters >= 16 && (wave_fill < 0.8 || tiles >= 4L * clusters)) {
+    p.split = 1;
+    p.stream_k = 1;
+    const long run = (tiles * num_kb + clusters - 1) / clusters;
+    p.chain = run < num_kb ? run : num_kb;
+  }
+  return p;
+}
+
 // Tile width (64 or 128 columns, one CTA each) for a problem that is smaller than a wave of such tiles, or 0 for the CTA-pair kernel.
 // A 64-deep step of the main loop takes much the same time in all three kernels when a CTA has one tile to work on (0.31 us,
 // 0.36 us for a pair: latency, not bandwidth), so what counts is the fixed cost - set-up, and an epilogue that nothing hides,
@@ -429,6 +468,8 @@ void nmtg_set_gemm_variant(int v) {
 // dropout and residual 12.5 / 7.3 / 8.8, 704 x 1024 x 256 with ReLU, dropout and mask 11.5 / 6.2 / 7.5, 3840 x 512 x 2048 22.7 / 25.3 (two
 // waves) / 17.7, weight gradient 512 x 512 x 1920 14.1 / 8.7 / 10.0; beyond one wave the pair wins: 3840 x 1024 x 1024 16.2 / 26.4 /
 // 17.6.  The estimates below are fitted to such measurements for widths 256 to 1024 and 704 to 5632 rows.
+// An accumulator's rounding grows with the k-blocks that it adds up, so a weight gradient is taken only with chains no longer than the
+// pair kernel's: 1256 x 896 over 4439 rows in two parts was 2.3e-6 off 64 bits (rms, relative), 1.1e-6 in the pair kernel's runs of 19 blocks.
 static int one_wave_tile(const GemmDesc* d, int sms, int num_kb, int* split) {
   const bool sums = d->out_fp32 && d->allow_split_k && d->accumulate;
   if (d->out_fp32 && !sums) return 0;
@@ -437,6 +478,7 @@ static int one_wave_tile(const GemmDesc* d, int sms, int num_kb, int* split) {
   long pair_split = 1;
   while (sums && pairs * pair_split * 2 <= clusters && num_kb / (pair_split * 2) >= 8) pair_split *= 2;
   const long waves = (pairs * pair_split + clusters - 1) / clusters;
+  const long pair_chain = plan_pair(d, sms, num_kb, bn_pair).chain;
   double best = (sums ? 9.5 : 8.0) + 0.36 * static_cast<double>((num_kb + pair_split - 1) / pair_split) * waves - 0.5;
   int bn = 0;
   for (int w = 64; w <= 128; w += 64) {
@@ -446,6 +488,7 @@ static int one_wave_tile(const GemmDesc* d, int sms, int num_kb, int* split) {
     if (sums) {                          // at least six steps for a CTA: the partial tiles meet in atomic adds
       s = sms / tiles < num_kb / 6 ? sms / tiles : num_kb / 6;
       if (s < 1) s = 1;
+      if ((num_kb + s - 1) / s > pair_chain) continue;
     }
     const double t = (w == 64 ? 5.2 : 6.0) + (sums ? 0.4 : 0.0) + 0.31 * static_cast<double>((num_kb + s - 1) / s);
     if (t < best) {
@@ -497,11 +540,6 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   };
   const int sms = gemm_sms();
   const int num_kb = (d->K + BK - 1) / BK;
-  auto fix_split = [&](int split) {   // largest split <= requested whose last part is not empty
-    if (split > num_kb) split = num_kb;
-    while (split > 1 && (split - 1) * ((num_kb + split - 1) / split) >= num_kb) --split;
-    return split < 1 ? 1 : split;
-  };
   // ---- skinny problems (incremental decoding: a few hundred rows): the weight matrix is streamed once, so the
   // only lever is the number of CTAs pulling it in; take the widest tile that still gives every SM a tile,
   // down to 64 columns
@@ -558,27 +596,10 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
       GatherArgs probe;
       if (g_fused_gather == 0 || !plan_pair_gather(d, bn, &probe)) { const char* e = gather_first(); if (e) return e; }
     }
-    const long tiles = static_cast<long>((d->M + 2 * BM - 1) / (2 * BM)) * ((d->N + bn - 1) / bn);
-    int split = 1;
-    if (d->split_k > 0) split = d->split_k;
-    else if (d->out_fp32 && d->allow_split_k) {
-      const int clusters = sms / 2;
-      while (tiles * split * 2 <= clusters && num_kb / (split * 2) >= 8) split *= 2;
-    }
-    if (split > 1 && !d->out_fp32) return "gemm: split-K needs an fp32 output";
-    a.split_k = fix_split(split);
-    // weight gradients (fp32, accumulating): when the tiles do not fill the clusters evenly, hand every cluster an
-    // equal run of k-blocks instead of whole tiles
-    // (measured: a gain where whole tiles leave a fifth or more of the clusters idle, and for many-wave problems such
-    // as the generator; a loss of 5-15 % from the extra partial-tile reductions where the tiles nearly fill a wave)
-    const int clusters = sms / 2;
-    const long units = tiles * a.split_k;
-    const double wave_fill = static_cast<double>(units) / (static_cast<double>((units + clusters - 1) / clusters) * clusters);
-    if (g_stream_k && d->out_fp32 && d->accumulate && d->allow_split_k && d->split_k <= 0 && (units % clusters) != 0 &&
-        tiles * num_kb / clusters >= 16 && (wave_fill < 0.8 || tiles >= 4L * clusters)) {
-      a.split_k = 1;
-      a.stream_k = 1;
-    }
+    const PairPlan plan = plan_pair(d, sms, num_kb, bn);
+    if (plan.split > 1 && !d->out_fp32) return "gemm: split-K needs an fp32 output";
+    a.split_k = plan.split;
+    a.stream_k = plan.stream_k;
     return launch_gemm_pair(d, a, bn, stream);
   }
   // ---- single-CTA kernel: tile width 256 when it does not waste a wave, else 128 -------------------
@@ -602,7 +623,7 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
     while (tiles * split * 2 <= sms && num_kb / (split * 2) >= 8) split *= 2;
   }
   if (split > 1 && !d->out_fp32) return "gemm: split-K needs an fp32 output";
-  a.split_k = fix_split(split);
+  a.split_k = fix_split(split, num_kb);
 
   CUtensorMap ta, tb;
   bool ok;

@@ -444,3 +444,19 @@ def test_epilogue_operands_off_their_boundary(M, N, K, off):
             if "preact" in kw:
                 assert torch.equal(kw["preact"], whole["preact"])
     assert ops.check_status() == 0
+
+
+@pytest.mark.parametrize("T,O,I", [(4439, 1256, 896), (3835, 1128, 848), (5020, 1320, 152), (4850, 536, 752), (1920, 512, 512), (704, 256, 1024), (5632, 1024, 1024)])
+def test_weight_gradients_are_no_further_off_than_the_pair_kernels(T, O, I):
+    """32-bit sums over thousands of rows: narrow tiles may not add up longer chains than the kernel that they stand in for."""
+    ops.ext().set_gemm_variant(0)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    dy, x = rnd(T, O), rnd(T, I)
+    want = dy.double().t() @ x.double()
+    err = []
+    for forced in (0, 256):
+        dw = torch.zeros(O, I, device="cuda")
+        ops.gemm(dy, x, dw, a_mn_major=True, b_mn_major=True, accumulate=True, allow_split_k=True, force_bn=forced)
+        err.append(float((dw.double() - want).square().mean().sqrt()))
+    assert err[0] <= 1.1 * err[1], err          # a million values each: the two figures are known to a part in a hundred
