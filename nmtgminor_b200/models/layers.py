@@ -15,6 +15,7 @@ onmt/modules/optimized/feed_forward.py:13-207), ``PrePostProcessing``
 from __future__ import annotations
 
 import math
+import threading
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -153,6 +154,9 @@ def quantize_linears_for_cpu(model: nn.Module) -> int:
     return n
 
 
+_renewing = threading.Lock()
+
+
 class Embedding(nn.Module):
     """Token embedding * scale + (sinusoidal | learned) position row, then dropout, in one kernel."""
 
@@ -178,8 +182,10 @@ class Embedding(nn.Module):
 
     def renew(self, n_pos: int):
         if self.use_pos and not self.learned_pos and n_pos > self.pos.shape[0]:
-            self.pos = sinusoidal_table(n_pos, self.pos.shape[1]).to(self.pos.device)
-            self._pos_work = None
+            with _renewing:                    # of two threads the one with the shorter table must not come last
+                if n_pos > self.pos.shape[0]:
+                    self.pos = sinusoidal_table(n_pos, self.pos.shape[1]).to(self.pos.device)
+                    self._pos_work = None
 
     def _pos_table(self, device):
         if not self.use_pos:

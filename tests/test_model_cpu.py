@@ -165,3 +165,25 @@ def test_learning_rate_schedules():
     assert math.isclose(learning_rate_at(5, cos, 1.0), 0.5)
     assert learning_rate_at(60, cos, 1.0) == pytest.approx(0.5, abs=1e-6)
     assert learning_rate_at(110, cos, 1.0) == pytest.approx(0.0, abs=1e-6)
+
+
+def test_position_table_never_shrinks(monkeypatch):
+    """Two threads lengthen the table at once: whoever finishes last, it holds the longer one."""
+    import threading
+    import time
+
+    from nmtgminor_b200.models import layers
+    emb, started, make = layers.Embedding(10, 8, max_pos=16), threading.Event(), layers.sinusoidal_table
+
+    def slow(n_pos, dim):
+        if n_pos == 32:
+            started.set()
+            time.sleep(0.3)
+        return make(n_pos, dim)
+    monkeypatch.setattr(layers, "sinusoidal_table", slow)
+    first = threading.Thread(target=emb.renew, args=(32,))
+    first.start()
+    assert started.wait(5)
+    emb.renew(64)
+    first.join(5)
+    assert emb.pos.shape == (64, 8) and torch.equal(emb.pos, make(64, 8))
