@@ -157,6 +157,12 @@ def quantize_linears_for_cpu(model: nn.Module) -> int:
 _renewing = threading.Lock()
 
 
+def _settle(t: torch.Tensor) -> None:
+    """Wait until ``t`` has been written, before other threads and streams may see it."""
+    if t.is_cuda and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream(t.device).synchronize()
+
+
 class Embedding(nn.Module):
     """Token embedding * scale + (sinusoidal | learned) position row, then dropout, in one kernel."""
 
@@ -184,7 +190,9 @@ class Embedding(nn.Module):
         if self.use_pos and not self.learned_pos and n_pos > self.pos.shape[0]:
             with _renewing:                    # of two threads the one with the shorter table must not come last
                 if n_pos > self.pos.shape[0]:
-                    self.pos = sinusoidal_table(n_pos, self.pos.shape[1]).to(self.pos.device)
+                    pos = sinusoidal_table(n_pos, self.pos.shape[1]).to(self.pos.device)
+                    _settle(pos)
+                    self.pos = pos
                     self._pos_work = None
 
     def _pos_table(self, device):
@@ -196,7 +204,11 @@ class Embedding(nn.Module):
             return self.pos
         pos, work = self.pos, self._pos_work          # another thread may renew the table at any time
         if work is None or work.device != device or work.shape != pos.shape:
-            work = self._pos_work = pos.to(device=device, dtype=torch.bfloat16)
+            work = pos.to(device=device, dtype=torch.bfloat16)
+            # the conversion of a captured call runs at its replays only, and in its graph's memory: it is not for the others
+            if not torch.cuda.is_current_stream_capturing():
+                _settle(work)
+                self._pos_work = work
         return work
 
     word_dropout = 0.0      # probability of dropping a whole vocabulary entry for one batch (training only)

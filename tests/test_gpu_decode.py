@@ -447,3 +447,21 @@ def test_unaligned_caches_are_refused():
                      lambda: e.decode_self(qkv, k, v, anc, pos, 2, 2, 0.125), lambda: e.cache_append(q, q, k, v, 0)):
             with pytest.raises(RuntimeError, match="16-byte"):
                 call()
+
+
+def test_position_table_first_needed_in_a_capture():
+    """A captured call that meets a renewed table converts it for itself: calls outside of the graph must not get its memory, which only
+    a replay fills."""
+    from nmtgminor_b200.models.layers import PackedSeqs
+    emb = _successor_model(16).decoder.embed
+    at = torch.arange(50, device="cuda")
+    seqs = PackedSeqs(torch.full((50,), 7, device="cuda"), at, torch.tensor([0, 50], dtype=torch.int32, device="cuda"), 50)
+    with torch.no_grad():
+        want = emb(seqs)
+        emb.renew(3000)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = emb(seqs)
+        assert torch.equal(emb(seqs), want)
+        graph.replay()
+        assert torch.equal(out, want) and torch.equal(emb(seqs), want)
