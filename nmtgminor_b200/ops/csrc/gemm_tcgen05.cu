@@ -254,7 +254,11 @@ static bool make_tmap_2d(CUtensorMap* out, const void* base, long rows, long col
   // (autograd's backward thread when the first thing it does is build a descriptor) has none: bind the primary one.
   static thread_local bool context_bound = false;
   if (bind_context && !context_bound) {
+    // the thread may be capturing, and its capture would not survive this call
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     cudaFree(nullptr);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     context_bound = true;
   }
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};

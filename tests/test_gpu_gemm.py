@@ -460,3 +460,27 @@ def test_weight_gradients_are_no_further_off_than_the_pair_kernels(T, O, I):
         ops.gemm(dy, x, dw, a_mn_major=True, b_mn_major=True, accumulate=True, allow_split_k=True, force_bn=forced)
         err.append(float((dw.double() - want).square().mean().sqrt()))
     assert err[0] <= 1.1 * err[1], err          # a million values each: the two figures are known to a part in a hundred
+
+
+def test_first_product_of_a_thread_inside_a_capture():
+    """A thread whose first product is a captured one, on operands that no descriptor has been made for yet."""
+    import threading
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x, w = torch.randn(200, 512, device="cuda", generator=g).bfloat16(), torch.randn(256, 512, device="cuda", generator=g).bfloat16()
+    want, out = torch.empty(200, 256, device="cuda").bfloat16(), torch.empty(200, 256, device="cuda").bfloat16()
+    ops.gemm(x.clone(), w.clone(), want)             # the kernel is loaded
+    graph, errors = torch.cuda.CUDAGraph(), []
+
+    def capture():
+        try:
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph, stream=torch.cuda.Stream(), capture_error_mode="thread_local"):
+                ops.gemm(x, w, out)
+        except Exception as exc:
+            errors.append(exc)
+    t = threading.Thread(target=capture)
+    t.start()
+    t.join(60)
+    assert not errors, errors
+    graph.replay()
+    assert torch.equal(out, want)
