@@ -143,6 +143,16 @@ class _StepPools:
 
     MAX_KEPT = 4
     lock = threading.RLock()
+    streams = {}             # device index -> the stream that captures run on
+
+    @classmethod
+    def capture_stream(cls, device):
+        """A stream of the process that no other thread can be working on: its launches would end up in the graph."""
+        from .. import ops
+        with cls.lock:
+            if device.index not in cls.streams:
+                cls.streams[device.index] = torch.cuda.ExternalStream(ops.ext().make_stream(device.index), device=device)
+            return cls.streams[device.index]
 
     def __init__(self, state):
         self.state = state
@@ -273,11 +283,11 @@ class _DeviceSearch:
             pool["warm"] += 1
             return self._body()
         while pool["graph"] is None:
-            with _StepPools.lock:               # one capture at a time, on a stream of its own
+            with _StepPools.lock:               # one capture at a time
                 self.pools, self.reads = _StepPools.of(self.model, self.tok.device)
                 g = torch.cuda.CUDAGraph()
                 torch.cuda.synchronize()
-                with torch.cuda.graph(g, stream=torch.cuda.Stream(self.tok.device), capture_error_mode="thread_local"):
+                with torch.cuda.graph(g, stream=_StepPools.capture_stream(self.tok.device), capture_error_mode="thread_local"):
                     self._body()                # captured, not run
                 # another thread may have renewed the position table meanwhile: then this graph reads another one than is held
                 if _StepPools.of(self.model, self.tok.device)[0] is self.pools:

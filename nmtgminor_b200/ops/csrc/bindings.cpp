@@ -551,6 +551,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         pybind11::arg("dropout_p"), pybind11::arg("seed"), pybind11::arg("stream_id"), pybind11::arg("alpha"), pybind11::arg("accumulate"),
         pybind11::arg("allow_split_k"), pybind11::arg("split_k"), pybind11::arg("force_bn"), pybind11::arg("mask") = pybind11::none(),
         pybind11::arg("colsum") = pybind11::none(), pybind11::arg("gather") = pybind11::none());
+  // a stream that nobody else has: torch hands its own out in turn, so that two owners may meet on one
+  m.def("make_stream", [](int64_t device) {
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+    cudaStream_t s = nullptr;
+    const cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    TORCH_CHECK(e == cudaSuccess, "cudaStreamCreateWithFlags: ", cudaGetErrorString(e));
+    return reinterpret_cast<int64_t>(s);
+  });
   m.def("set_step_overlap", [](bool on) { nmtg_set_step_overlap(on); });
   m.def("set_gemm_variant", [](int64_t v) { nmtg_set_gemm_variant(static_cast<int>(v)); });
   m.def("set_sm_reserve", [](int64_t n) { nmtg_set_sm_reserve(static_cast<int>(n)); });

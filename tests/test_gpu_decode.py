@@ -465,3 +465,13 @@ def test_position_table_first_needed_in_a_capture():
         assert torch.equal(emb(seqs), want)
         graph.replay()
         assert torch.equal(out, want) and torch.equal(emb(seqs), want)
+
+
+def test_captures_have_a_stream_of_their_own():
+    """torch hands out 32 streams of a priority in turn: none of them may be the one that searches capture on, since another thread's launches
+    on it would be captured instead of run."""
+    from nmtgminor_b200.inference.beam_search import _StepPools
+    device = torch.device("cuda", torch.cuda.current_device())
+    others = {torch.cuda.Stream(priority=p).cuda_stream for p in (0, -1) for _ in range(80)} | {torch.cuda.current_stream().cuda_stream}
+    assert _StepPools.capture_stream(device).cuda_stream not in others
+    assert _StepPools.capture_stream(device) is _StepPools.capture_stream(device)

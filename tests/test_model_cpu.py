@@ -187,3 +187,14 @@ def test_position_table_never_shrinks(monkeypatch):
     emb.renew(64)
     first.join(5)
     assert emb.pos.shape == (64, 8) and torch.equal(emb.pos, make(64, 8))
+
+
+def test_a_model_is_copied_without_its_search_tables():
+    import pickle
+    import threading
+
+    from nmtgminor_b200.inference.beam_search import _StepPools
+    pools = _StepPools(["state"])
+    pools.put("geometry", {"graph": threading.Lock()})          # as little to be copied as a captured graph
+    assert copy.deepcopy({"_decode_pools": pools}) == {"_decode_pools": None} and pickle.loads(pickle.dumps(pools)) is None
+
