@@ -168,6 +168,39 @@ def test_step_cross_attention(B, K, heads, cap):
             assert (out[b * K:(b + 1) * K].double() - want).abs().max() <= 2 ** -8 * want.abs().max() + 1e-6
 
 
+@pytest.mark.parametrize("K,pos", [(1, 15), (1, 16), (3, 17), (5, 255), (7, 256), (8, 31), (8, 513), (9, 257), (17, 16)])
+def test_step_attention_tiles(K, pos):
+    """Edges of the key blocks (16), of the staged ancestors (256) and of the eight queries of a CTA, with a past that the hypotheses
+    share at first; a hypothesis whose past is not a number leaves the others of its sentence alone."""
+    g = torch.Generator(device="cuda").manual_seed(pos * K)
+    B, heads = 2, 2
+    R, hid, cap = B * K, heads * 64, (pos + 64) // 64 * 64
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    qkv, kc, vc = rnd(R, 3 * hid), rnd(R, cap, hid), rnd(R, cap, hid)
+    own = torch.arange(R, device="cuda").view(B, K, 1)
+    anc = torch.where(torch.arange(cap, device="cuda") < pos // 2, own[:, :1], own).int().view(R, cap).contiguous()
+    if K > 1:
+        vc[1, pos // 2:], kc[1, pos // 2:] = float("nan"), float("nan")
+    out = ops.ext().decode_self(qkv, kc.clone(), vc.clone(), anc, torch.full((R,), pos, dtype=torch.long, device="cuda"), K, heads, 0.125)
+    q, k, v = (t.double().view(R, heads, 64) for t in qkv.split(hid, 1))
+    take = lambda c: torch.stack([c[anc[:, j].long(), j] for j in range(pos)], 1).double().view(R, pos, heads, 64)
+    keys, vals = torch.cat([take(kc), k[:, None]], 1), torch.cat([take(vc), v[:, None]], 1)
+    want = torch.einsum("rhj,rjhd->rhd", torch.softmax(torch.einsum("rhd,rjhd->rhj", q, keys) * 0.125, -1), vals).reshape(R, hid)
+    if K > 1:
+        assert out[1].isnan().all()
+        out[1], want[1] = 0, 0
+    assert (out.double() - want).abs().max() < 2 ** -8 * want.abs().max()          # one rounding to bf16 of a 32-bit result
+    # the same queries over keys that all of them share, from rows that do not start on 16 bytes
+    shift = torch.zeros(R, hid + 8, dtype=torch.bfloat16, device="cuda")[:, 3:hid + 3]
+    shift.copy_(qkv[:, :hid])
+    kb, vb = rnd(B, pos, hid), rnd(B, pos, hid)
+    out = ops.ext().decode_cross(shift, kb, vb, torch.tensor([pos, pos - 3], dtype=torch.int32, device="cuda"), heads, 0.125)
+    for b, n in enumerate((pos, pos - 3)):
+        qb, kk, vv = q[b * K:(b + 1) * K], kb[b, :n].double().view(n, heads, 64), vb[b, :n].double().view(n, heads, 64)
+        want = torch.einsum("khj,jhd->khd", torch.softmax(torch.einsum("khd,jhd->khj", qb, kk) * 0.125, -1), vv).reshape(K, hid)
+        assert (out[b * K:(b + 1) * K].double() - want).abs().max() < 2 ** -8 * want.abs().max()
+
+
 def _compare_searches(dtype, B, K, V, T, min_len, normalize, alpha, end_bias=None):
     from types import SimpleNamespace
 
