@@ -25,8 +25,9 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// VPL = 16-byte vectors per lane (row length <= VPL * 256 elements)
-template <int VPL>
+// VPL = 16-byte vectors per lane (row length <= VPL * 256 elements).  kStep: a decoding step's launch (nmtg_set_step_overlap), whose gain
+// and bias are fetched while the kernel before it runs; behind the row's statistics they were one more round trip of a chain of them.
+template <int VPL, bool kStep = false>
 __global__ void __launch_bounds__(kLnWarps * 32)
 ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
               const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y, float* __restrict__ mean,
@@ -35,6 +36,15 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   const int warp = threadIdx.x >> 5;
   const int nvec = hidden >> 3;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // decoding steps: see nmtg_set_step_overlap
+  uint4 gain[kStep ? VPL : 1], shift[kStep ? VPL : 1];
+  if constexpr (kStep) {
+#pragma unroll
+    for (int i = 0; i < VPL; ++i)
+      if (lane + i * 32 < nvec) {
+        gain[i] = __ldg(reinterpret_cast<const uint4*>(gamma) + lane + i * 32);
+        shift[i] = __ldg(reinterpret_cast<const uint4*>(beta) + lane + i * 32);
+      }
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int row = blockIdx.x * kLnWarps + warp; row < rows; row += gridDim.x * kLnWarps) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * hidden);
@@ -80,8 +90,8 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
     for (int i = 0; i < VPL; ++i) {
       const int vi = lane + i * 32;
       if (vi < nvec) {
-        uint4 g = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
-        uint4 b = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
+        uint4 g = kStep ? gain[kStep ? i : 0] : __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
+        uint4 b = kStep ? shift[kStep ? i : 0] : __ldg(reinterpret_cast<const uint4*>(beta) + vi);
         const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&g);
         const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
         uint4 o;
@@ -428,7 +438,8 @@ const char* nmtg_layernorm_fwd(const void* x, const void* gamma, const void* bet
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = step_overlap() ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, ln_fwd_kernel<decltype(vpl)::value>, reinterpret_cast<const __nv_bfloat16*>(x),
+    auto kern = step_overlap() ? ln_fwd_kernel<decltype(vpl)::value, true> : ln_fwd_kernel<decltype(vpl)::value>;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, reinterpret_cast<const __nv_bfloat16*>(x),
                                        reinterpret_cast<const __nv_bfloat16*>(gamma), reinterpret_cast<const __nv_bfloat16*>(beta),
                                        reinterpret_cast<__nv_bfloat16*>(y), mean, rstd, rows, hidden, eps);
     return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
