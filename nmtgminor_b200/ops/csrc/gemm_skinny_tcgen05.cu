@@ -83,8 +83,14 @@ __device__ __forceinline__ float4 skinny_act(float4 v, int act) {
 template <int kSplit, int kRows>
 __device__ __forceinline__ void skinny_finish(const SkinnyArgs& p, const uint8_t* smem, int rank, int warp, int lane, int rows, int m0, int n0) {
   const int col = n0 + lane * 4;
-  const bool col_ok = col < p.N;               // N is a multiple of 4
-  const float4 bias = (p.bias && col_ok) ? unpack4(*reinterpret_cast<const uint2*>(p.bias + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool col_ok = col < p.N, four = col + 4 <= p.N;
+  float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (p.bias && four) bias = unpack4(*reinterpret_cast<const uint2*>(p.bias + col));
+  else if (p.bias && col_ok) {
+    bias.x = __bfloat162float(p.bias[col]);
+    if (col + 1 < p.N) bias.y = __bfloat162float(p.bias[col + 1]);
+    if (col + 2 < p.N) bias.z = __bfloat162float(p.bias[col + 2]);
+  }
   const uint32_t red = smem_u32(smem) + lane * 16;
   for (int j0 = rank + kSplit * kRows * warp; j0 < rows; j0 += kSplit * kRows * 4) {
     float4 acc[kRows];
@@ -119,7 +125,13 @@ __device__ __forceinline__ void skinny_finish(const SkinnyArgs& p, const uint8_t
       __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
       o.x = *reinterpret_cast<uint32_t*>(&lo);
       o.y = *reinterpret_cast<uint32_t*>(&hi);
-      *reinterpret_cast<uint2*>(p.out + static_cast<size_t>(m0 + j) * p.ld_out + col) = o;
+      __nv_bfloat16* to = p.out + static_cast<size_t>(m0 + j) * p.ld_out + col;
+      if (four) *reinterpret_cast<uint2*>(to) = o;
+      else {                                     // N is no multiple of 4 (no residual then)
+        to[0] = lo.x;
+        if (col + 1 < p.N) to[1] = lo.y;
+        if (col + 2 < p.N) to[2] = hi.x;
+      }
     }
   }
 }
@@ -172,7 +184,11 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         mbar_expect_tx(&full_bar[i], S::kStageBytes);
         tma_load_2d(smem + i * S::kStageBytes, &tmap_w, &full_bar[i], (kb0 + i) * BK, n0);
       }
-      if (p.early) pdl_wait();
+      if (p.early) {
+        // what the ring does not hold yet waits in L2
+        for (int i = first; i < n_kb; ++i) tma_prefetch_2d(&tmap_w, (kb0 + i) * BK, n0);
+        pdl_wait();
+      }
       for (int i = 0; i < first; ++i)
         tma_load_2d(smem + i * S::kStageBytes + S::kWBytes, &tmap_x, &full_bar[i], (kb0 + i) * BK, m0);
       int stage = 0;
@@ -284,12 +300,13 @@ static int skinny_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 // decoding steps do; training, scoring and encoding keep one order of their forward sums whatever the batch size.  Measured (us, this kernel back to back
 // with programmatic launch / the tiled kernel): 1024 x 1024, 4 rows
 // 3.6 / 8.4, 256 rows 7.2 / 9.3, 512 rows 7.5 / 9.3; 4096 x 1024, 64 rows 6.0 / 8.6; 1024 x 4096, 4 rows 5.4 / 22.8; 32000 x
-// 1024, 33 rows 13.9 / 20.3.  Beyond one wave (32000 x 1024 with 128 rows: 25 us against 19) the tiled kernel is the better one.
+// 1024, 33 rows 13.9 / 20.3.  Beyond one wave (32000 x 1024 with 128 rows: 25 us against 19) the tiled kernel is the better one; up to 32 rows
+// two waves are no slower (51865 x 1280, 4 rows 30.4 / 36.1, 20 rows 32.5 / 35.0, 32 rows 32.9 / 32.6, 48 rows 36.6 / 30.6).
 bool skinny_takes(const GemmDesc* d, int sms) {
   const long tiles = static_cast<long>((d->N + kSkinnyFeat - 1) / kSkinnyFeat) * ((d->M + skinny_rows(d->M) - 1) / skinny_rows(d->M));
-  return d->allow_split_k && d->M <= 512 && tiles <= 2L * sms && !d->out_fp32 && !d->a_mn_major && !d->b_mn_major && !d->gather && !d->preact && !d->mask &&
+  return d->allow_split_k && d->M <= 512 && tiles <= (d->M <= 32 ? 4L : 2L) * sms && !d->out_fp32 && !d->a_mn_major && !d->b_mn_major && !d->gather && !d->preact && !d->mask &&
          !d->colsum && !d->aux && d->act >= 0 && d->act <= kActSilu && d->dropout_p <= 0.f && d->split_k <= 1 && d->force_bn == 0 &&
-         d->N % 4 == 0 && (!d->residual || (d->ld_res % 4 == 0 && (reinterpret_cast<uintptr_t>(d->residual) & 7) == 0)) &&
+         d->ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(d->out) & 7) == 0 && (!d->residual || d->N % 4 == 0) && (!d->residual || (d->ld_res % 4 == 0 && (reinterpret_cast<uintptr_t>(d->residual) & 7) == 0)) &&
          (reinterpret_cast<uintptr_t>(d->bias) & 7) == 0;
 }
 
