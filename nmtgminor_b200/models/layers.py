@@ -133,6 +133,20 @@ class Linear(nn.Module):
         return ops.linear(x, self.weight, self.bias, act, dropout_p, residual, self.training)
 
 
+def _plain(m, cls) -> bool:
+    """Whether calling ``m`` is calling ``cls.forward`` and nothing else."""
+    return type(m) is cls and not (m._forward_hooks or m._forward_pre_hooks or nn.modules.module._has_any_global_hook())
+
+
+def _normed(norm, linear, x):
+    """``linear(norm(x))``, in one kernel where the modules are the plain ones (``norm`` None: ``x`` is normalised already)."""
+    if norm is None:
+        return linear(x)
+    if _plain(norm, LayerNorm) and _plain(linear, Linear) and getattr(linear, "_int8", None) is None:
+        return ops.norm_linear(x, norm.weight, norm.bias, norm.eps, linear.weight, linear.bias)
+    return linear(norm(x))
+
+
 def quantize_linears_for_cpu(model: nn.Module) -> int:
     """Attach an int8 dynamically quantised twin (per-tensor weight scale, activations quantised on the fly) to every
     ``Linear`` of ``model`` for CPU inference; returns how many were converted.  The fp32 weights stay in place, so the
@@ -292,11 +306,12 @@ class SelfAttention(nn.Module):
         return self.out(ctx, dropout_p=dropout_p, residual=residual)
 
     # -- incremental decoding: x [B, H] is ONE new position per hypothesis --------------------------
-    def step(self, x, cache: dict, residual=None):
+    # ``norm``: LayerNorm of the sub-layer, if ``x`` has not been through it
+    def step(self, x, cache: dict, residual=None, norm=None):
         if self.rotary:
             raise NotImplementedError("rotary positions are built for encoder stacks (no incremental step)")
         H, h = self.dim, self.heads
-        qkv = self.qkv(x)
+        qkv = _normed(norm, self.qkv, x)
         q, k, v = qkv[:, :H], qkv[:, H:2 * H], qkv[:, 2 * H:]
         B = x.shape[0]
         if _fused_decode(qkv, H, h) and cache.get("cap"):
@@ -347,8 +362,8 @@ class CrossAttention(nn.Module):
         kv = self.kv(memory_padded.reshape(B * T, Hm)).view(B, T, 2 * self.dim)
         return kv[..., :self.dim].contiguous(), kv[..., self.dim:].contiguous()
 
-    def step(self, x, cache: dict, mem_mask, residual=None):
-        q = self.q(x)
+    def step(self, x, cache: dict, mem_mask, residual=None, norm=None):
+        q = _normed(norm, self.q, x)
         ck, cv = cache["c_k"], cache["c_v"]
         if "c_len" in cache and _fused_decode(q, self.dim, self.heads):
             # one cache row per sentence, shared by its hypotheses
@@ -410,6 +425,13 @@ class FeedForward(nn.Module):
             return self.fc2(h, dropout_p=dropout_p, residual=residual)
         return ops.mlp(x, self.fc1.weight, self.fc1.bias, self.fc2.weight, self.fc2.bias, self.activation, self.dropout,
                        dropout_p, residual, self.training)
+
+    def step(self, x, norm):
+        """``x + ffn(norm(x))`` of a decoding step."""
+        if self.glu or self.training or not _plain(norm, LayerNorm) or ops.ACT_IDS[self.activation] not in (1, 2, 3):
+            return self(norm(x), residual=x)
+        h = ops.norm_linear(x, norm.weight, norm.bias, norm.eps, self.fc1.weight, self.fc1.bias, self.activation)
+        return ops.linear(h, self.fc2.weight, self.fc2.bias, "none", 0.0, x, False)
 
 
 def _sub(layer, fn, inp, residual, p, seqs, *args):
@@ -655,12 +677,17 @@ class DecoderLayer(nn.Module, _LayerOptions):
             if not self.ignore_source:
                 x = self.cross_norm(x + self.cross_attn.step(x, cache, mem_mask))
             return self.ffn_norm(self.ffn(x, residual=x))
-        x = self.self_attn.step(self.self_norm(x), cache, residual=x)      # residual add in the GEMM epilogue
+        # LayerNorm in front of the projections, residual add in their epilogues
+        x = self.self_attn.step(x, cache, residual=x, norm=self.self_norm)
         if self.interleaved_ffn:
-            x = self.mid_ffn(self.mid_norm(x), residual=x)
+            x = _ffn_step(self.mid_ffn, x, self.mid_norm)
         if not self.ignore_source:
-            x = self.cross_attn.step(self.cross_norm(x), cache, mem_mask, residual=x)
-        return self.ffn(self.ffn_norm(x), residual=x)
+            x = self.cross_attn.step(x, cache, mem_mask, residual=x, norm=self.cross_norm)
+        return _ffn_step(self.ffn, x, self.ffn_norm)
+
+
+def _ffn_step(ffn, x, norm):
+    return ffn.step(x, norm) if _plain(ffn, FeedForward) else ffn(norm(x), residual=x)
 
 
 def _decoder_step_general(self, x, cache: dict, mem_mask):

@@ -297,12 +297,35 @@ def linear(x, weight, bias=None, act="none", dropout_p=0.0, residual=None, train
         need_dx = x.requires_grad
         xin = (x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)).contiguous()
         if not torch.is_grad_enabled() or not (need_dx or gw is not None):
+            if step_sums.depth > 0 and p == 0.0:
+                y = _step_linear(xin, weight, b, residual, act_id)
+                if y is not None:
+                    return y
             y = empty_rows(x.shape[0], weight.shape[0], x.device)
             return gemm(xin, weight.work, y, bias=b, residual=residual, act=act_id, dropout_p=p, seed=_Rng.seed,
                         stream_id=sid, allow_split_k=step_sums.depth > 0, gather=_gather_of(weight))
         return _LinearFn.apply(_track(xin), weight.work, b, residual, gw, gb, act_id, p, _Rng.seed, sid, need_dx,
                                _gather_of(weight))
     return ref.linear(x, weight, bias, act_id, p, residual)
+
+
+def _step_linear(x, weight, bias, residual, act_id, norm=None, eps=0.0):
+    """The product of a decoding step with few rows, LayerNorm (gain and bias) included, in one kernel; None where that one does not
+    take it.  ``x`` bf16 rows, ``bias`` and ``norm`` working copies."""
+    if x.shape[0] > 32 or x.dim() != 2 or _gather_of(weight) is not None:
+        return None
+    gamma, beta = norm if norm is not None else (None, None)
+    return ext().step_linear(x, gamma, beta, float(eps), weight.work, bias, residual, act_id)
+
+
+def norm_linear(x, norm_weight, norm_bias, eps, weight, bias=None, act="none", residual=None):
+    """``linear(layer_norm(x))``; one kernel in a decoding step with few rows."""
+    if (step_sums.depth > 0 and not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous()
+            and fused_param(weight) and fused_param(norm_weight)):
+        y = _step_linear(x, weight, bias.work if bias is not None else None, residual, ACT_IDS[act], (norm_weight.work, norm_bias.work), eps)
+        if y is not None:
+            return y
+    return linear(layer_norm(x, norm_weight, norm_bias, eps), weight, bias, act, 0.0, residual, False)
 
 
 class _MlpFn(torch.autograd.Function):
@@ -379,11 +402,12 @@ def mlp(x, w1, b1, w2, b2, act="relu", dropout_p=0.0, out_dropout_p=0.0, residua
             return _MlpFn.apply(_track(xin), w1.work, b1.work if b1 is not None else None, w2.work,
                                 b2.work if b2 is not None else None, residual, g, act_id, p1, p2, _Rng.seed, sid1, sid2,
                                 _gather_of(w1), _gather_of(w2))
+        if step_sums.depth > 0:
+            return linear(linear(xin, w1, b1, act_id, 0.0, None, False), w2, b2, 0, 0.0, residual, False)
         h = torch.empty((x.shape[0], w1.shape[0]), dtype=torch.bfloat16, device=x.device)
-        split = step_sums.depth > 0
-        gemm(xin, w1.work, h, bias=b1.work if b1 is not None else None, act=act_id, allow_split_k=split, gather=_gather_of(w1))
+        gemm(xin, w1.work, h, bias=b1.work if b1 is not None else None, act=act_id, gather=_gather_of(w1))
         y = torch.empty((x.shape[0], w2.shape[0]), dtype=torch.bfloat16, device=x.device)
-        return gemm(h, w2.work, y, bias=b2.work if b2 is not None else None, residual=residual, allow_split_k=split, gather=_gather_of(w2))
+        return gemm(h, w2.work, y, bias=b2.work if b2 is not None else None, residual=residual, gather=_gather_of(w2))
     h = ref.linear(x, w1, b1, act_id, p1, None)
     return ref.linear(h, w2, b2, 0, p2, residual)
 

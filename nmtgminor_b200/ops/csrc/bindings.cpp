@@ -59,6 +59,33 @@ const unsigned long long* seed_ptr(const Tensor& like) {
 Tensor get_seed_tensor(int64_t device) { return seed_tensor(static_cast<int>(device)); }
 
 // C[M,N] = epilogue(alpha * A B^T) ; see GemmDesc
+// [residual +] act([LayerNorm](x) W^T + bias) of a decoding step, or nothing where the kernel does not take these operands.
+std::optional<Tensor> step_linear(const Tensor& x, const OptTensor& gamma, const OptTensor& beta, double eps, const Tensor& w, const OptTensor& bias,
+                                  const OptTensor& residual, int64_t act) {
+  const auto rows_of = [](const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.stride(1) == 1 && t.stride(0) % 8 == 0 &&
+           (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  };
+  const auto vector_of = [&](const OptTensor& t, int64_t n) {
+    return !t.has_value() || (t->device() == x.device() && t->scalar_type() == at::kBFloat16 && t->numel() == n && t->is_contiguous() &&
+                              (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0);
+  };
+  if (!rows_of(x) || !rows_of(w) || w.device() != x.device() || w.size(1) != x.size(1) || w.size(0) % 8 || gamma.has_value() != beta.has_value())
+    return std::nullopt;
+  const int M = static_cast<int>(x.size(0)), N = static_cast<int>(w.size(0)), K = static_cast<int>(x.size(1));
+  if (!vector_of(gamma, K) || !vector_of(beta, K) || !vector_of(bias, N)) return std::nullopt;
+  if (residual.has_value() && (!rows_of(*residual) || residual->device() != x.device() || residual->size(0) != M || residual->size(1) != N))
+    return std::nullopt;
+  c10::cuda::CUDAGuard guard(x.device());
+  if (!nmtg_step_linear_takes(M, N, K, gamma.has_value())) return std::nullopt;
+  Tensor out = torch::empty({M, N}, x.options());
+  ck(nmtg_step_linear(x.data_ptr(), static_cast<int>(x.stride(0)), opt_ptr(gamma), opt_ptr(beta), static_cast<float>(eps), w.data_ptr(),
+                      static_cast<int>(w.stride(0)), opt_ptr(bias), opt_ptr(residual),
+                      residual.has_value() ? static_cast<int>(residual->stride(0)) : 0, out.data_ptr(), N, M, N, K, static_cast<int>(act),
+                      cur_stream()));
+  return out;
+}
+
 void gemm(const Tensor& a, bool a_mn_major, const Tensor& b, bool b_mn_major, Tensor& out, const OptTensor& bias,
           const OptTensor& residual, const OptTensor& aux, const OptTensor& preact, int64_t act, double dropout_p,
           int64_t seed, int64_t stream_id, double alpha, bool accumulate, bool allow_split_k, int64_t split_k,
@@ -559,6 +586,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     TORCH_CHECK(e == cudaSuccess, "cudaStreamCreateWithFlags: ", cudaGetErrorString(e));
     return reinterpret_cast<int64_t>(s);
   });
+  m.def("step_linear", &step_linear);
   m.def("set_step_overlap", [](bool on) { nmtg_set_step_overlap(on); });
   m.def("set_gemm_variant", [](int64_t v) { nmtg_set_gemm_variant(static_cast<int>(v)); });
   m.def("set_sm_reserve", [](int64_t n) { nmtg_set_sm_reserve(static_cast<int>(n)); });

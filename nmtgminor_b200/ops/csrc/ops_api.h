@@ -58,6 +58,11 @@ struct GemmDesc {
 };
 
 const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream);
+// out[M, N] = [residual +] act([LayerNorm](x) W^T + bias) for the few rows of a decoding step (step_linear.cu).  gamma / beta null: no
+// LayerNorm.  The sum over K is cut into parts, as in a product that allows split_k.
+int nmtg_step_linear_takes(int M, int N, int K, int norm);
+const char* nmtg_step_linear(const void* x, int ldx, const void* gamma, const void* beta, float eps, const void* w, int ldw, const void* bias,
+                             const void* residual, int ld_res, void* out, int ld_out, int M, int N, int K, int act, cudaStream_t stream);
 // 0 = automatic (CTA-pair kernel when M > 128, unless the problem is a few rows or less than a wave of narrow tiles), 1 = single-CTA kernel
 // (products with column sums excepted), 2 = CTA-pair kernel when M > 128
 void nmtg_set_gemm_variant(int v);

@@ -508,3 +508,33 @@ def test_captures_have_a_stream_of_their_own():
     others = {torch.cuda.Stream(priority=p).cuda_stream for p in (0, -1) for _ in range(80)} | {torch.cuda.current_stream().cuda_stream}
     assert _StepPools.capture_stream(device).cuda_stream not in others
     assert _StepPools.capture_stream(device) is _StepPools.capture_stream(device)
+
+
+@pytest.mark.parametrize("M,N,K,norm,act", [(1, 8, 8, True, "none"), (8, 24, 40, True, "relu"), (7, 3072, 256, True, "none"), (6, 4096, 1024, True, "gelu"), (16, 4096, 1024, False, "gelu"),
+                                            (8, 5120, 1280, True, "silu"), (17, 5120, 1280, False, "silu"), (32, 1280, 1272, False, "silu"), (4, 2056, 512, True, "relu"), (4, 9472, 768, True, "none"), (12, 9472, 768, False, "none"),
+                                            (5, 512, 512, False, "none"), (8, 1280, 1280, False, "relu"), (3, 1024, 4096, False, "none"), (8, 2368, 5120, False, "none"),
+                                            (1, 256, 1544, False, "gelu"), (7, 768, 3072, False, "none"), (32, 520, 520, False, "none"), (13, 1280, 1280, False, "none")])
+def test_step_linear(M, N, K, norm, act):
+    """LayerNorm, product, bias, activation and residual of a decoding step in one kernel: ragged tiles of rows, features and K."""
+    g = torch.Generator(device="cuda").manual_seed(M * N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w, bias, res, gamma, beta = rnd(M, K), rnd(N, K) * K ** -0.5, rnd(N), rnd(M, N), rnd(K), rnd(K)
+    for b, r in ((bias, res), (None, None)):
+        out = ops.ext().step_linear(x, gamma if norm else None, beta if norm else None, 1e-5, w, b, r, ops.ACT_IDS[act])
+        h = ops.ext().layernorm_fwd(x, gamma, beta, 1e-5)[0] if norm else x          # the same bf16 values
+        y = h.double() @ w.double().t() + (b.double() if b is not None else 0)
+        y = {"none": lambda t: t, "relu": torch.relu, "gelu": torch.nn.functional.gelu, "silu": torch.nn.functional.silu}[act](y)
+        y = y + (r.double() if r is not None else 0)
+        # one rounding to bf16 of a 32-bit sum of K products (2^-24 each step, of the sum of magnitudes)
+        size = h.double().abs() @ w.double().abs().t()
+        assert ((out.double() - y).abs() <= 2 ** -8 * y.abs() + K ** 0.5 * 2 ** -22 * size + 1e-5).all()
+    assert ops.ext().step_linear(x.float(), None, None, 0.0, w, None, None, 0) is None
+    assert ops.ext().step_linear(rnd(33, K), None, None, 0.0, w, None, None, 0) is None
+
+
+def test_step_linear_normalises_as_the_layernorm_kernel_does():
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for K in (8, 256, 520, 1024, 1280):
+        x, gamma, beta = (torch.randn(*s, device="cuda", generator=g).bfloat16() for s in ((7, K), (K,), (K,)))
+        eye = torch.eye(K, device="cuda").bfloat16()
+        assert torch.equal(ops.ext().step_linear(x * 3 + 1, gamma, beta, 1e-5, eye, None, None, 0), ops.ext().layernorm_fwd(x * 3 + 1, gamma, beta, 1e-5)[0])
