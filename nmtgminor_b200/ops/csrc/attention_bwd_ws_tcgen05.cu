@@ -400,6 +400,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_word) {
+#pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }

@@ -90,6 +90,26 @@ __device__ __forceinline__ void zero_tail_bwd(const AttnArgs& p) {
   zero_tail_rows(p.dv, p.ld_dv, w, k_end, p.total_k);
 }
 
+// nk UMMA k-steps issued by the elected lane of a converged warp; nk and the descriptors uniform.
+template <int kAStep, int kBStep>
+__device__ __forceinline__ void umma_steps_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int nk) {
+#pragma unroll 1
+  for (int k = 0; k < nk; ++k) {
+    if (elect_one()) umma_bf16(d_tmem, adesc, bdesc, idesc, k > 0 ? 1u : 0u);
+    adesc += kAStep >> 4;
+    bdesc += kBStep >> 4;
+  }
+}
+// A of 64-column slabs (P or dS, K-major), B MN-major
+__device__ __forceinline__ void umma_slabs_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int nk) {
+#pragma unroll 1
+  for (int k = 0; k < nk; ++k) {
+    if (elect_one()) umma_bf16(d_tmem, adesc, bdesc, idesc, k > 0 ? 1u : 0u);
+    adesc += (k & 3) == 3 ? (kTileBytes - 96) >> 4 : 2;
+    bdesc += 2048 >> 4;
+  }
+}
+
 // nk UMMA k-steps reading A from a_addr (+ k * a_step bytes) and B from b_addr (+ k * b_step bytes)
 __device__ __forceinline__ void umma_steps(uint32_t d_tmem, uint32_t a_addr, uint32_t a_lbo, uint32_t a_step,
                                            uint32_t b_addr, uint32_t b_lbo, uint32_t b_step, uint32_t idesc, int nk,

@@ -7,12 +7,16 @@
 // so that per-item latencies (global loads, MMA completion, TMEM reads) are hidden instead of summed, which
 // is what dominates when a sentence has only 20..100 tokens.
 //
-// forward : two softmax groups alternate items (TMEM: S0 S1 | O0 O1), three Q/K/V slots.
+// forward : four items in flight, each with a Q/K/V slot, 128 TMEM columns (S, then O) and a softmax group of its own.
 // backward: 256 math threads (query row x half of the key columns) on one item, a warpgroup that prepares D / log-sum-exp
 //           of the next item and writes dQ, dK, dV of the previous one; TMEM holds two sets (S dP, reused for dV dQ dK),
 //           two Q/K/V/dO slots; P and dS are staged once in shared memory and consumed K-major (dQ = dS K) and MN-major
 //           (dV = P^T dO, dK = dS^T Q).
 // MMA reduction lengths are trimmed to the real sequence lengths (multiples of 16).
+// What bounds these kernels is the fetching of instructions: all roles run at once, each in code of its own, and the SMs of a GPC share
+// what their own caches cannot hold (CTAs on a GPC with fewer of them ran 1.4 times as fast).  So a loop body is there once: one 32-column
+// chunk a turn, dropout a template argument, MMA steps and gradient matrices in loops that are not unrolled.  The backward pass went from
+// 157 KB and 83.6 us (136 sentences of 20 to 100 words x 16 heads, dropout) to 70 KB and 67.1; unrolling its MMA steps alone cost 12 us.
 // Same numerics, dropout counters and interfaces as the general kernels in attention_tcgen05.cu.
 #include "attention_common.cuh"
 #include "bounds_check.cuh"
@@ -44,256 +48,258 @@ __device__ __forceinline__ Item get_item(const AttnArgs& p, int item) {
 // ---------------------------------------------------------------------------------------------------
 // forward
 // ---------------------------------------------------------------------------------------------------
-constexpr int kFwdSlots = 3;
+// Four items are in flight, each in a slot and with a softmax group of its own: an item is a chain of waits (S, two passes over it, P,
+// O, about 5500 cycles for 60 keys with dropout) that one or two warps of a scheduler cannot fill.  To fit, P overwrites the Q and K
+// tiles (S = Q K^T is complete when a group starts) and O the columns of S.  Only the producer looks items up: the look-up is a
+// round trip to memory, and in the MMA warp it took 1300 of the 3260 cycles that an item took with two groups.  136 sentences of 20 to
+// 100 words x 16 heads, two groups (157 KB of code) / four (39): without dropout 40.3 / 26.2 us, with it 50.9 / 32.3.
 constexpr int kFwdSlotBytes = 3 * kTileBytes;
-constexpr int kFwdShortThreads = 320;   // warps 0-3 / 4-7: softmax groups, warp 8: TMA producer, warp 9: MMA issuer
-constexpr int kFwdShortSmem = kFwdSlots * kFwdSlotBytes + 2 * kPBytes + 256 + 1024;
+constexpr int fwd_short_threads(int groups) { return groups * 128 + 64; }   // softmax groups, TMA producer warp, MMA warp
+constexpr int fwd_short_smem(int groups) { return groups * kFwdSlotBytes + 512 + 1024; }
+constexpr uint32_t kIssuePolls = 1u << 22;   // polls of the MMA warp without progress before it gives up
 
-__global__ void __launch_bounds__(kFwdShortThreads, 1)
+// Up to 64 queries leave two of a group's four warps without work, and a warp's number decides both its rows (TMEM lanes) and its
+// scheduler: odd groups take such items in rows 64 .. 127 (the tile starts 64 rows early; a load may start before the matrix).
+__device__ __forceinline__ int row_shift(int group, int q_len) { return (group & 1) && q_len <= 64 ? 64 : 0; }
+
+// Bounded wait of a warp that polls several barriers: counts polls without progress, false when it is time to give up.
+__device__ __forceinline__ bool keep_polling(uint32_t& idle, volatile int* abort_word, int* status) {
+  if (++idle > 4096) {        // a few microseconds of plain polling first: a sleep here delays every waiter
+    if (*abort_word) return false;
+    if (idle > kIssuePolls) {
+      *abort_word = 1;
+      if (status) atomicCAS(status, 0, static_cast<int>(kTimeoutTmemEmpty));
+      return false;
+    }
+    __nanosleep(idle > 65536 ? 256 : 32);
+  }
+  return true;
+}
+
+template <int kFwdGroups, bool kDrop>
+__global__ void __launch_bounds__(fwd_short_threads(kFwdGroups), 1)
 attn_fwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const AttnArgs p, const int num_items) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sSlots = smem;
-  uint8_t* sP = smem + kFwdSlots * kFwdSlotBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + 2 * kPBytes);
-  uint64_t* slot_full = bars;
-  uint64_t* slot_empty = bars + 3;
-  uint64_t* s_full = bars + 6;
-  uint64_t* s_empty = bars + 8;
-  uint64_t* p_full = bars + 10;
-  uint64_t* o_full = bars + 12;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint8_t* sSlots = smem;            // [4][Q K V]; P over Q and K
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kFwdGroups * kFwdSlotBytes);
+  uint64_t* slot_full = bars;                       // TMA (and the item's descriptor) -> everybody
+  uint64_t* slot_empty = bars + kFwdGroups;         // P V done -> TMA
+  uint64_t* s_full = bars + 2 * kFwdGroups;         // S ready -> softmax group
+  uint64_t* p_full = bars + 3 * kFwdGroups;         // P staged -> MMA
+  uint64_t* o_full = bars + 4 * kFwdGroups;         // O ready -> softmax group
+  uint64_t* o_read = bars + 5 * kFwdGroups;         // O read -> MMA may write the next S
+  int4* desc = reinterpret_cast<int4*>(bars + 6 * kFwdGroups);      // q0, k0, head, (q_len << 8) | k_len; 0 lengths: no more items
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(desc + kFwdGroups);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   zero_tail_fwd(p);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 3; ++i) { mbar_init(&slot_full[i], 1); mbar_init(&slot_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kFwdGroups; ++i) {
+      mbar_init(&slot_full[i], 1);
+      mbar_init(&slot_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], 128);
       mbar_init(&p_full[i], 128);
       mbar_init(&o_full[i], 1);
+      mbar_init(&o_read[i], 128);
     }
     *abort_word = 0;
     mbar_fence_init();
   }
-  if (warp == 9) tmem_alloc(tmem_slot, 512);
+  constexpr int kProducer = kFwdGroups * 4, kMma = kProducer + 1;
+  if (warp == kMma) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 8) {
+  if (warp == kProducer) {
     if (lane == 0) {
       int it = 0;
+      bool ok = true;
+      Item nxt = static_cast<int>(blockIdx.x) < num_items ? get_item(p, blockIdx.x) : Item{};
       for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
-        const Item w = get_item(p, item);
+        const Item w = nxt;
+        if (item + static_cast<int>(gridDim.x) < num_items) nxt = get_item(p, item + gridDim.x);
         if (!w.valid) continue;
-        const int slot = it % kFwdSlots;
-        if (!mbar_wait(&slot_empty[slot], ((it / kFwdSlots) & 1) ^ 1, abort_word, p.status, kTimeoutSmemEmpty)) break;
+        const int slot = it % kFwdGroups;
+        if (!mbar_wait(&slot_empty[slot], ((it / kFwdGroups) & 1) ^ 1, abort_word, p.status, kTimeoutSmemEmpty)) { ok = false; break; }
+        desc[slot] = make_int4(w.q0, w.k0, w.h, (w.q_len << 8) | w.k_len);
         uint8_t* s = sSlots + slot * kFwdSlotBytes;
         mbar_expect_tx(&slot_full[slot], kFwdSlotBytes);
-        tma_load_2d(s, &tmap_q, &slot_full[slot], w.h * kHd, w.q0);
+        tma_load_2d(s, &tmap_q, &slot_full[slot], w.h * kHd, w.q0 - row_shift(slot, w.q_len));
         tma_load_2d(s + kTileBytes, &tmap_k, &slot_full[slot], w.h * kHd, w.k0);
         tma_load_2d(s + 2 * kTileBytes, &tmap_v, &slot_full[slot], w.h * kHd, w.k0);
         ++it;
       }
-    }
-  } else if (warp == 9) {
-    if (lane == 0) {
-      const uint32_t idesc_s = make_idesc_bf16(kTile, kTile, 0, 0);
-      const uint32_t idesc_o = make_idesc_bf16(kTile, kHd, 0, 1);
-      int it = 0;
-      bool have_prev = false, ok = true;
-      int prev_it = 0, prev_klen = 0;
-      auto issue_pv = [&](int j, int k_len) -> bool {
-        const int g = j & 1, slot = j % kFwdSlots;
-        if (!mbar_wait(&p_full[g], (j >> 1) & 1, abort_word, p.status, kTimeoutTmemEmpty)) return false;
-        tc_fence_after_sync();
-        const uint32_t pa = smem_u32(sP + g * kPBytes);
-        const uint32_t va = smem_u32(sSlots + slot * kFwdSlotBytes + 2 * kTileBytes);
-        const uint32_t tO = tmem_base + 256 + g * kHd;
-        const int nk = (k_len + 15) >> 4;
-        for (int k = 0; k < nk; ++k) {
-          const uint64_t ad = make_smem_desc_sw128(pa + (k >> 2) * kTileBytes + (k & 3) * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc_sw128(va + k * 2048, 8192, 1024);
-          umma_bf16(tO, ad, bd, idesc_o, k > 0 ? 1u : 0u);
-        }
-        umma_commit(&o_full[g]);
-        umma_commit(&slot_empty[slot]);
-        return true;
-      };
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        const Item w = get_item(p, item);
-        if (!w.valid) continue;
-        const int slot = it % kFwdSlots, g = it & 1;
-        if (!mbar_wait(&slot_full[slot], (it / kFwdSlots) & 1, abort_word, p.status, kTimeoutTmaFull)) { ok = false; break; }
-        if (!mbar_wait(&s_empty[g], ((it >> 1) & 1) ^ 1, abort_word, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
-        tc_fence_after_sync();
-        const uint32_t qa = smem_u32(sSlots + slot * kFwdSlotBytes);
-        umma_steps(tmem_base + g * kTile, qa, 16, 32, qa + kTileBytes, 16, 32, idesc_s, kHd / 16, false);
-        umma_commit(&s_full[g]);
-        if (have_prev) ok = issue_pv(prev_it, prev_klen);
-        have_prev = true;
-        prev_it = it;
-        prev_klen = w.k_len;
-        ++it;
+      for (int e = 0; e < kFwdGroups && ok; ++e, ++it) {
+        const int slot = it % kFwdGroups;
+        if (!mbar_wait(&slot_empty[slot], ((it / kFwdGroups) & 1) ^ 1, abort_word, p.status, kTimeoutSmemEmpty)) break;
+        desc[slot] = make_int4(0, 0, 0, 0);
+        mbar_arrive(&slot_full[slot]);
       }
-      if (ok && have_prev) issue_pv(prev_it, prev_klen);
     }
-  } else if (warp < 8) {
+  } else if (warp == kMma) {
+    const uint32_t idesc_s = make_idesc_bf16(kTile, kTile, 0, 0);
+    const uint32_t idesc_o = make_idesc_bf16(kTile, kHd, 0, 1);
+    const uint32_t tmem = uniform(tmem_base), slots = uniform(smem_u32(sSlots));
+    // two queues, served in whichever order their inputs arrive: S of item s_it, P V of item o_it
+    int s_it = 0, o_it = 0;
+    uint32_t steps = 0;                       // 16-key steps of the items in flight, 4 bits each
+    bool more = true;
+    uint32_t idle = 0;
+    while (more || o_it < s_it) {
+      bool progressed = false;
+      if (o_it < s_it && all_lanes(mbar_test_wait(&p_full[o_it % kFwdGroups], (o_it / kFwdGroups) & 1))) {
+        tc_fence_after_sync();
+        const int g = o_it % kFwdGroups;
+        const uint32_t pa = slots + g * kFwdSlotBytes, tO = tmem + g * kTile;
+        const uint64_t ad = make_smem_desc_sw128(pa, 16, 1024), bd = make_smem_desc_sw128(pa + 2 * kTileBytes, 8192, 1024);
+        const int nk = static_cast<int>((steps >> (4 * g)) & 15u);
+        umma_slabs_warp(tO, ad, bd, idesc_o, nk);
+        if (elect_one()) {
+          umma_commit(&o_full[g]);
+          umma_commit(&slot_empty[g]);
+        }
+        ++o_it;
+        progressed = true;
+      }
+      if (more && s_it - o_it < kFwdGroups && all_lanes(mbar_test_wait(&slot_full[s_it % kFwdGroups], (s_it / kFwdGroups) & 1) &&
+                                                        mbar_test_wait(&o_read[s_it % kFwdGroups], ((s_it / kFwdGroups) & 1) ^ 1))) {
+        tc_fence_after_sync();
+        const int g = s_it % kFwdGroups;
+        const int lens = uniform(desc[g].w);
+        if (lens == 0) more = false;
+        else {
+          const uint32_t qa = slots + g * kFwdSlotBytes;
+          umma_steps_warp<32, 32>(tmem + g * kTile, make_smem_desc_sw128(qa, 16, 1024), make_smem_desc_sw128(qa + kTileBytes, 16, 1024), idesc_s, kHd / 16);
+          if (elect_one()) umma_commit(&s_full[g]);
+          steps = (steps & ~(15u << (4 * g))) | (static_cast<uint32_t>(((lens & 255) + 15) >> 4) << (4 * g));
+          ++s_it;
+        }
+        progressed = true;
+      }
+      if (progressed) idle = 0;
+      else if (!all_lanes(keep_polling(idle, abort_word, p.status))) break;
+    }
+  } else {
     const int g = warp >> 2;
     const int t = (warp & 3) * 32 + lane;
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem_base + g * kTile, tO = tmem_base + 256 + g * kHd;
-    uint8_t* myP = sP + g * kPBytes;
+    const uint32_t tS = tmem_base + g * kTile + lane_sel;      // S, then O in its first 64 columns
+    uint8_t* myP = sSlots + g * kFwdSlotBytes;
     const float scale_log2 = p.scale * 1.4426950408889634f;
-    const bool do_drop = p.dropout_p > 0.f;
-    const unsigned long long seed = p.seed + ((do_drop && p.seed_dev) ? *p.seed_dev : 0ull);
-    int it = 0;
-    int item = blockIdx.x;
-    Item nxt = item < num_items ? get_item(p, item) : Item{};
-    while (item < num_items) {
-      const Item w = nxt;
-      item += gridDim.x;
-      if (item < num_items) nxt = get_item(p, item);   // loads for the next item overlap this item's work
-      if (!w.valid) continue;
-      const int my = ((it & 1) == g);
-      const uint32_t ph = (it >> 1) & 1;
-      ++it;
-      if (!my) continue;
+    const unsigned long long seed = p.seed + ((kDrop && p.seed_dev) ? *p.seed_dev : 0ull);
+    for (uint32_t ph = 0;; ph ^= 1) {
+      if (!mbar_wait(&slot_full[g], ph, abort_word, p.status, kTimeoutTmaFull)) break;
+      const int4 d = desc[g];
+      const int q_len = d.w >> 8, k_len = d.w & 255;
+      if (d.w == 0) break;
       if (!mbar_wait(&s_full[g], ph, abort_word, p.status, kTimeoutTmemFull)) break;
       tc_fence_after_sync();
-      const bool warp_active = (warp & 3) * 32 < w.q_len;
-      const int nchunks = (w.k_len + 31) >> 5;
+      const int tq = t - row_shift(g, q_len);               // this thread's query
+      const int first = (warp & 3) * 32 - row_shift(g, q_len);
+      const bool warp_active = first >= 0 && first < q_len;
+      const int nchunks = (k_len + 31) >> 5;
       float row_sum = 0.f, row_max = kNegBig;
       if (warp_active) {
-        const DropRng rng(seed, (p.stream_id << 16) | static_cast<unsigned long long>(w.h), p.dropout_p);
-        // two column chunks (64 scores) per round: both TMEM loads are in flight before the single wait
+        const DropRng rng(seed, (p.stream_id << 16) | static_cast<unsigned long long>(d.z), p.dropout_p);
+        // raw-score maximum (scale > 0: scaling commutes with the maximum)
+        const int limit = p.causal ? min(k_len, tq + 1) : k_len;
 #pragma unroll 1
-        for (int c0 = 0; c0 < nchunks; c0 += 2) {
-          uint32_t r0[32], r1[32];
-          tmem_ld32(tS + lane_sel + c0 * 32, r0);
-          if (c0 + 1 < nchunks) tmem_ld32(tS + lane_sel + (c0 + 1) * 32, r1);
+        for (int c = 0; c < nchunks; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tS + c * 32, r);
           tmem_ld_wait();
-          // raw-score maximum (scale > 0: scaling commutes with the maximum); a chunk whose 32 key columns all exist
-          // (and no causal mask) needs no per-element test
+          const int left = limit - c * 32;
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int c = c0 + half;
-            if (c >= nchunks) break;
-            if (!p.causal && (c + 1) * 32 <= w.k_len) {
-              float m0 = kNegBig, m1 = kNegBig, m2 = kNegBig, m3 = kNegBig;
-#pragma unroll
-              for (int j = 0; j < 32; j += 4) {
-                m0 = fmaxf(m0, __uint_as_float(half == 0 ? r0[j] : r1[j]));
-                m1 = fmaxf(m1, __uint_as_float(half == 0 ? r0[j + 1] : r1[j + 1]));
-                m2 = fmaxf(m2, __uint_as_float(half == 0 ? r0[j + 2] : r1[j + 2]));
-                m3 = fmaxf(m3, __uint_as_float(half == 0 ? r0[j + 3] : r1[j + 3]));
-              }
-              row_max = fmaxf(row_max, fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)));
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const int col = c * 32 + j;
-                const bool valid = col < w.k_len && (!p.causal || col <= t);
-                row_max = fmaxf(row_max, valid ? __uint_as_float(half == 0 ? r0[j] : r1[j]) : kNegBig);
-              }
-            }
-          }
+          for (int j = 0; j < 32; ++j) row_max = fmaxf(row_max, j < left ? __uint_as_float(r[j]) : kNegBig);
         }
         row_max *= scale_log2;         // from here on in the base-2 domain: P = 2^(S * scale * log2 e - row_max)
 #pragma unroll 1
-        for (int c0 = 0; c0 < nchunks; c0 += 2) {
-          uint32_t r0[32], r1[32];
-          tmem_ld32(tS + lane_sel + c0 * 32, r0);
-          if (c0 + 1 < nchunks) tmem_ld32(tS + lane_sel + (c0 + 1) * 32, r1);
+        for (int c = 0; c < nchunks; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tS + c * 32, r);
           tmem_ld_wait();
+          float pv[32];
+          const int left = limit - c * 32;
+          if (left >= 32) {            // no per-element test
+            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int c = c0 + half;
-            if (c >= nchunks) break;
-            float pv[32];
-            if (!p.causal && (c + 1) * 32 <= w.k_len) {
-              float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-              for (int j = 0; j < 32; j += 4) {
-                pv[j] = ex2_approx(fmaf(__uint_as_float(half == 0 ? r0[j] : r1[j]), scale_log2, -row_max));
-                pv[j + 1] = ex2_approx(fmaf(__uint_as_float(half == 0 ? r0[j + 1] : r1[j + 1]), scale_log2, -row_max));
-                pv[j + 2] = ex2_approx(fmaf(__uint_as_float(half == 0 ? r0[j + 2] : r1[j + 2]), scale_log2, -row_max));
-                pv[j + 3] = ex2_approx(fmaf(__uint_as_float(half == 0 ? r0[j + 3] : r1[j + 3]), scale_log2, -row_max));
-                s0 += pv[j];
-                s1 += pv[j + 1];
-                s2 += pv[j + 2];
-                s3 += pv[j + 3];
-              }
-              row_sum += (s0 + s1) + (s2 + s3);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const int col = c * 32 + j;
-                const bool valid = col < w.k_len && (!p.causal || col <= t);
-                const float sv = __uint_as_float(half == 0 ? r0[j] : r1[j]);
-                const float e = valid ? ex2_approx(fmaf(sv, scale_log2, -row_max)) : 0.f;
-                row_sum += e;
-                pv[j] = e;
-              }
+            for (int j = 0; j < 32; j += 4) {
+              pv[j] = ex2_approx(fmaf(__uint_as_float(r[j]), scale_log2, -row_max));
+              pv[j + 1] = ex2_approx(fmaf(__uint_as_float(r[j + 1]), scale_log2, -row_max));
+              pv[j + 2] = ex2_approx(fmaf(__uint_as_float(r[j + 2]), scale_log2, -row_max));
+              pv[j + 3] = ex2_approx(fmaf(__uint_as_float(r[j + 3]), scale_log2, -row_max));
+              s0 += pv[j];
+              s1 += pv[j + 1];
+              s2 += pv[j + 2];
+              s3 += pv[j + 3];
             }
-            if (do_drop) apply_dropout32(rng, static_cast<unsigned long long>(w.q0 + t) * p.kstride + c * 32, pv);
+            row_sum += (s0 + s1) + (s2 + s3);
+          } else {
 #pragma unroll
-            for (int g4 = 0; g4 < 4; ++g4) {
-              uint4 o;
-              __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(pv[g4 * 8 + 2 * j], pv[g4 * 8 + 2 * j + 1]);
-              const int chunk = c * 4 + g4;
-              *reinterpret_cast<uint4*>(myP + (chunk >> 3) * kTileBytes + sw128_offset(t, chunk & 7)) = o;
+            for (int j = 0; j < 32; ++j) {
+              const float e = j < left ? ex2_approx(fmaf(__uint_as_float(r[j]), scale_log2, -row_max)) : 0.f;
+              row_sum += e;
+              pv[j] = e;
             }
+          }
+          if constexpr (kDrop) apply_dropout32(rng, static_cast<unsigned long long>(d.x + tq) * p.kstride + c * 32, pv);
+#pragma unroll
+          for (int g4 = 0; g4 < 4; ++g4) {
+            uint4 o;
+            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(pv[g4 * 8 + 2 * j], pv[g4 * 8 + 2 * j + 1]);
+            const int chunk = c * 4 + g4;
+            *reinterpret_cast<uint4*>(myP + (chunk >> 3) * kTileBytes + sw128_offset(t, chunk & 7)) = o;
           }
         }
       }
       tc_fence_before_sync();
       fence_async_smem();
       mbar_arrive(&p_full[g]);
-      mbar_arrive(&s_empty[g]);
       if (!mbar_wait(&o_full[g], ph, abort_word, p.status, kTimeoutTmemFull)) break;
       tc_fence_after_sync();
       if (warp_active) {
         const float inv = row_sum > 0.f ? 1.f / row_sum : 0.f;
-        __nv_bfloat16* orow = p.out + static_cast<size_t>(w.q0 + t) * p.ld_out + w.h * kHd;
-        uint32_t r0[32], r1[32];
-        tmem_ld32(tO + lane_sel, r0);
-        tmem_ld32(tO + lane_sel + 32, r1);
-        tmem_ld_wait();
-        if (t < w.q_len) {
+        __nv_bfloat16* orow = p.out + static_cast<size_t>(d.x + tq) * p.ld_out + d.z * kHd;
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          uint32_t r[32];
+          tmem_ld32(tS + half * 32, r);
+          tmem_ld_wait();
+          if (tq < q_len) {
 #pragma unroll
-          for (int g4 = 0; g4 < 8; ++g4) {
-            uint4 o;
-            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+            for (int g4 = 0; g4 < 4; ++g4) {
+              uint4 o;
+              __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int e = (g4 & 3) * 8 + 2 * j;
-              const float a = __uint_as_float(g4 < 4 ? r0[e] : r1[e]), b = __uint_as_float(g4 < 4 ? r0[e + 1] : r1[e + 1]);
-              o2[j] = __floats2bfloat162_rn(a * inv, b * inv);
+              for (int j = 0; j < 4; ++j)
+                o2[j] = __floats2bfloat162_rn(__uint_as_float(r[g4 * 8 + 2 * j]) * inv, __uint_as_float(r[g4 * 8 + 2 * j + 1]) * inv);
+              reinterpret_cast<uint4*>(orow)[half * 4 + g4] = o;
             }
-            reinterpret_cast<uint4*>(orow)[g4] = o;
           }
-          if (p.lse) p.lse[static_cast<size_t>(w.h) * p.lse_stride + w.q0 + t] = row_sum > 0.f ? (row_max + __log2f(row_sum)) * 0.6931471805599453f : 0.f;
         }
+        if (p.lse && tq < q_len)
+          p.lse[static_cast<size_t>(d.z) * p.lse_stride + d.x + tq] = row_sum > 0.f ? (row_max + __log2f(row_sum)) * 0.6931471805599453f : 0.f;
       }
       tc_fence_before_sync();
+      mbar_arrive(&o_read[g]);
     }
   }
 
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_word) {
+#pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 9) {
+  if (warp == kMma) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
@@ -307,7 +313,8 @@ attn_fwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 //                     32-column chunk c, so all 256 threads work on the SAME item and each holds few values at a time
 //                     (the math is issue-bound: with one warp per scheduler and most registers tied up in TMEM chunks the
 //                     compiler could not interleave independent elements, which is what made the one-group version slow)
-//   warps 8-11        D = rowsum(dO * O) and the log-sum-exp of item i+1 into shared memory, then dQ / dK / dV of item i-1
+//   warps 8-11        D = rowsum(dO * O) (dO from its tile, O from one loaded for this) and the log-sum-exp of item i+1 into shared memory,
+//                     then dQ / dK / dV of item i-1
 //   warp 12           TMA producer          warp 13   MMA issuer
 // TMEM holds two sets of 256 columns, set = item & 1:
 //   columns   0..127  S  = Q K^T          later  dV (0..63) and dQ (64..127)
@@ -319,16 +326,16 @@ constexpr int kBwdSlots = 2;
 constexpr int kBwdSlotBytes = 4 * kTileBytes;   // Q, K, V, dO
 constexpr int kBwdShortThreads = 448;
 constexpr int kBwdRowBytes = 2 * 2 * kTile * 4; // D and log-sum-exp of two items in flight
-constexpr int kBwdShortSmem = kBwdSlots * kBwdSlotBytes + 2 * kPBytes + kBwdRowBytes + 256 + 1024;
-constexpr uint32_t kBwdIssuePolls = 1u << 22;   // polls of the MMA warp without progress before it gives up
+constexpr int kBwdShortSmem = kBwdSlots * kBwdSlotBytes + 2 * kPBytes + kTileBytes + kBwdRowBytes + 256 + 1024;
 
-// One gradient row (64 fp32 accumulator columns of this thread's TMEM lane) scaled, packed to bf16 and stored.
-__device__ __forceinline__ void bwd_store_row(uint32_t taddr, __nv_bfloat16* drow, float osc, bool store) {
+// One gradient row per thread (64 fp32 accumulator columns of its TMEM lane) scaled, packed to bf16 and stored.
+__device__ __forceinline__ void bwd_store_rows(uint32_t taddr, __nv_bfloat16* base, int ld, int rows, float osc, int lane) {
   uint32_t r0[32], r1[32];
   tmem_ld32(taddr, r0);
   tmem_ld32(taddr + 32, r1);
   tmem_ld_wait();
-  if (store) {
+  if (lane < rows) {
+    __nv_bfloat16* drow = base + static_cast<size_t>(lane) * ld;
 #pragma unroll
     for (int g4 = 0; g4 < 8; ++g4) {
       uint4 o;
@@ -343,10 +350,11 @@ __device__ __forceinline__ void bwd_store_row(uint32_t taddr, __nv_bfloat16* dro
   }
 }
 
+template <bool kDrop>
 __global__ void __launch_bounds__(kBwdShortThreads, 1)
 attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
-                      const AttnArgs p, const int num_items, const int ablate) {
+                      const __grid_constant__ CUtensorMap tmap_o, const AttnArgs p, const int num_items, const int ablate) {
   // `ablate` (0 in production) switches parts of the work off while keeping every barrier hand-shake, so that a timing run
   // can tell which role bounds the item rate (results are then meaningless):
   //   1 no P / dS math   2 no gradient read-out   4 no gradient MMAs   8 no S / dP MMAs   16 no TMA loads
@@ -356,9 +364,10 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint8_t* sSlots = smem;
   uint8_t* sP = smem + kBwdSlots * kBwdSlotBytes;
   uint8_t* sDS = sP + kPBytes;
-  float* sD = reinterpret_cast<float*>(sDS + kPBytes);   // [2][128] rowsum(dO * O) of the items in flight
+  uint8_t* sO = sDS + kPBytes;                           // O of the item whose D comes next
+  float* sD = reinterpret_cast<float*>(sO + kTileBytes);   // [2][128] rowsum(dO * O) of the items in flight
   float* sL = sD + 2 * kTile;                            // [2][128] log-sum-exp * log2 e (+inf for rows past the sequence)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + kPBytes + kBwdRowBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + kTileBytes + kBwdRowBytes);
   uint64_t* slot_full = bars;        // [2] TMA -> MMA
   uint64_t* slot_empty = bars + 2;   // [2] gradient MMAs done -> TMA
   uint64_t* sdp_full = bars + 4;     // [2] S / dP ready -> math group
@@ -368,7 +377,9 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint64_t* pds_free = bars + 11;    // gradient MMAs done -> math threads may overwrite P / dS
   uint64_t* d_full = bars + 12;      // [2] D / log-sum-exp rows written -> math threads
   uint64_t* d_free = bars + 14;      // [2] rows read -> may be overwritten
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* o_full = bars + 16;      // O loaded -> D
+  uint64_t* o_free = bars + 17;      // O read -> TMA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   zero_tail_bwd(p);
@@ -385,6 +396,8 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     }
     mbar_init(pds_full, 256);
     mbar_init(pds_free, 1);
+    mbar_init(o_full, 1);
+    mbar_init(o_free, 128);
     *abort_word = 0;
     mbar_fence_init();
   }
@@ -405,6 +418,7 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         uint8_t* s = sSlots + slot * kBwdSlotBytes;
         if (ablate & 16) {
           mbar_arrive(&slot_full[slot]);
+          mbar_arrive(o_full);
           ++it;
           continue;
         }
@@ -413,92 +427,84 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         tma_load_2d(s + kTileBytes, &tmap_k, &slot_full[slot], w.h * kHd, w.k0);
         tma_load_2d(s + 3 * kTileBytes, &tmap_do, &slot_full[slot], w.h * kHd, w.q0);
         tma_load_2d(s + 2 * kTileBytes, &tmap_v, &slot_full[slot], w.h * kHd, w.k0);
+        if (!mbar_wait(o_free, (it & 1) ^ 1, abort_word, p.status, kTimeoutSmemEmpty)) break;
+        mbar_expect_tx(o_full, kTileBytes);
+        tma_load_2d(sO, &tmap_o, o_full, w.h * kHd, w.q0);
         ++it;
       }
     }
   } else if (warp == 13) {
-    if (lane == 0) {
-      const uint32_t idesc_s = make_idesc_bf16(kTile, kTile, 0, 0);
-      const uint32_t idesc_dq = make_idesc_bf16(kTile, kHd, 0, 1);
-      const uint32_t idesc_dkv = make_idesc_bf16(kTile, kHd, 1, 1);
-      // Two queues served in whichever order their inputs arrive: S / dP of item s_it (needs its tiles and a free TMEM
-      // set) and the gradients of item g_it (needs P / dS).  Blocking on one would hold back the other: the tiles of item
-      // i + 1 land about a TMA round trip after the gradients of item i - 1 completed.
-      int s_it = 0, g_it = 0;
-      unsigned long long lens = 0;   // (q_len, k_len) bytes of items g_it .. s_it (at most three alive), 16 bits per item
-      int item = blockIdx.x;
-      auto next_valid = [&]() {
-        while (item < num_items) {
-          const Item w = get_item(p, item);
-          if (w.valid) {
-            const int sh = (s_it & 3) * 16;
-            lens = (lens & ~(0xFFFFull << sh)) | (static_cast<unsigned long long>((w.q_len << 8) | w.k_len) << sh);
-            return true;
-          }
-          item += gridDim.x;
+    const uint32_t idesc_s = make_idesc_bf16(kTile, kTile, 0, 0);
+    const uint32_t idesc_dq = make_idesc_bf16(kTile, kHd, 0, 1);
+    const uint32_t idesc_dkv = make_idesc_bf16(kTile, kHd, 1, 1);
+    const uint32_t tmem = uniform(tmem_base), slots = uniform(smem_u32(sSlots)), pa = uniform(smem_u32(sP)), dsa = uniform(smem_u32(sDS));
+    // Two queues served in whichever order their inputs arrive: S / dP of item s_it (needs its tiles and a free TMEM
+    // set) and the gradients of item g_it (needs P / dS).  Blocking on one would hold back the other: the tiles of item
+    // i + 1 land about a TMA round trip after the gradients of item i - 1 completed.
+    int s_it = 0, g_it = 0;
+    uint32_t steps = 0;            // 16-row steps of queries (low 4 bits) and keys of the items in flight, a byte each
+    int item = blockIdx.x;
+    Item nxt = item < num_items ? get_item(p, item) : Item{};        // of `item`; fetched one ahead, a round trip to memory otherwise
+    auto next_valid = [&]() {
+      while (item < num_items) {
+        const Item w = nxt;
+        if (item + static_cast<int>(gridDim.x) < num_items) nxt = get_item(p, item + gridDim.x);
+        const int lens = uniform(w.valid ? (w.q_len << 8) | w.k_len : 0);
+        if (lens != 0) {
+          const int sh = (s_it & 3) * 8;
+          steps = (steps & ~(0xffu << sh)) | (static_cast<uint32_t>((((lens >> 8) + 15) >> 4) | ((((lens & 255) + 15) >> 4) << 4)) << sh);
+          return true;
         }
-        return false;
-      };
-      bool more = next_valid();
-      uint32_t idle = 0;
-      while (more || g_it < s_it) {
-        bool progressed = false;
-        if (g_it < s_it && mbar_test_wait(pds_full, g_it & 1)) {
-          tc_fence_after_sync();
-          const int s = g_it & 1;
-          const uint32_t set = tmem_base + s * 256;
-          const uint32_t base = smem_u32(sSlots + s * kBwdSlotBytes);
-          const uint32_t qa = base, ka = base + kTileBytes, doa = base + 3 * kTileBytes;
-          const uint32_t pa = smem_u32(sP), dsa = smem_u32(sDS);
-          const uint32_t lw = static_cast<uint32_t>(lens >> ((g_it & 3) * 16)) & 0xFFFFu;
-          const int nkq = ((lw >> 8) + 15) >> 4, nkk = ((lw & 0xFFu) + 15) >> 4;
+        item += gridDim.x;
+      }
+      return false;
+    };
+    bool more = next_valid();
+    uint32_t idle = 0;
+    while (more || g_it < s_it) {
+      bool progressed = false;
+      if (g_it < s_it && all_lanes(mbar_test_wait(pds_full, g_it & 1))) {
+        tc_fence_after_sync();
+        const int s = g_it & 1;
+        const uint32_t set = tmem + s * 256;
+        const uint32_t qa = slots + s * kBwdSlotBytes, ka = qa + kTileBytes, doa = qa + 3 * kTileBytes;
+        const uint32_t lw = (steps >> ((g_it & 3) * 8)) & 0xffu;
+        const int nkq = lw & 15, nkk = lw >> 4;
+        if (!(ablate & 4)) {
           // dV = P^T dO, dK = dS^T Q : A read MN-major (keys = M, two 64-key slabs), reduction over query rows
-          if (!(ablate & 4)) {
-            umma_steps(set, pa, kTileBytes, 2048, doa, 8192, 2048, idesc_dkv, nkq, false);
-            umma_steps(set + 128, dsa, kTileBytes, 2048, qa, 8192, 2048, idesc_dkv, nkq, false);
-          }
+          umma_steps_warp<2048, 2048>(set, make_smem_desc_sw128(pa, kTileBytes, 1024), make_smem_desc_sw128(doa, 8192, 1024), idesc_dkv, nkq);
+          umma_steps_warp<2048, 2048>(set + 128, make_smem_desc_sw128(dsa, kTileBytes, 1024), make_smem_desc_sw128(qa, 8192, 1024), idesc_dkv, nkq);
           // dQ = dS K : A K-major (slab per 64 keys), B = K tile MN-major, reduction over keys
-          for (int k = 0; k < ((ablate & 4) ? 0 : nkk); ++k) {
-            const uint64_t ad = make_smem_desc_sw128(dsa + (k >> 2) * kTileBytes + (k & 3) * 32, 16, 1024);
-            const uint64_t bd = make_smem_desc_sw128(ka + k * 2048, 8192, 1024);
-            umma_bf16(set + 64, ad, bd, idesc_dq, k > 0 ? 1u : 0u);
-          }
+          const uint64_t ad = make_smem_desc_sw128(dsa, 16, 1024), bd = make_smem_desc_sw128(ka, 8192, 1024);
+          umma_slabs_warp(set + 64, ad, bd, idesc_dq, nkk);
+        }
+        if (elect_one()) {
           umma_commit(pds_free);
           umma_commit(&grads_full[s]);
           umma_commit(&slot_empty[s]);
-          ++g_it;
-          progressed = true;
         }
-        if (more && s_it - g_it < 2 && mbar_test_wait(&slot_full[s_it & 1], (s_it >> 1) & 1) &&
-            mbar_test_wait(&set_free[s_it & 1], ((s_it >> 1) & 1) ^ 1)) {
-          tc_fence_after_sync();
-          const int s = s_it & 1;
-          const uint32_t set = tmem_base + s * 256;
-          const uint32_t base = smem_u32(sSlots + s * kBwdSlotBytes);
-          if (!(ablate & 8)) {
-            umma_steps(set, base, 16, 32, base + kTileBytes, 16, 32, idesc_s, kHd / 16, false);                              // Q K^T
-            umma_steps(set + 128, base + 3 * kTileBytes, 16, 32, base + 2 * kTileBytes, 16, 32, idesc_s, kHd / 16, false);   // dO V^T
-          }
-          umma_commit(&sdp_full[s]);
-          ++s_it;
-          item += gridDim.x;
-          more = next_valid();
-          progressed = true;
-        }
-        if (progressed) {
-          idle = 0;
-        } else {
-          if (++idle > 4096) {        // a few microseconds of plain polling first: a sleep here delays every waiter
-            if (*abort_word) break;
-            if (idle > kBwdIssuePolls) {
-              *abort_word = 1;
-              if (p.status) atomicCAS(p.status, 0, static_cast<int>(kTimeoutTmemEmpty));
-              break;
-            }
-            __nanosleep(idle > 65536 ? 256 : 32);
-          }
-        }
+        ++g_it;
+        progressed = true;
       }
+      if (more && s_it - g_it < 2 && all_lanes(mbar_test_wait(&slot_full[s_it & 1], (s_it >> 1) & 1) &&
+                                               mbar_test_wait(&set_free[s_it & 1], ((s_it >> 1) & 1) ^ 1))) {
+        tc_fence_after_sync();
+        const int s = s_it & 1;
+        const uint32_t set = tmem + s * 256;
+        const uint32_t base = slots + s * kBwdSlotBytes;
+        if (!(ablate & 8)) {
+          umma_steps_warp<32, 32>(set, make_smem_desc_sw128(base, 16, 1024), make_smem_desc_sw128(base + kTileBytes, 16, 1024), idesc_s, kHd / 16);   // Q K^T
+          umma_steps_warp<32, 32>(set + 128, make_smem_desc_sw128(base + 3 * kTileBytes, 16, 1024),
+                                  make_smem_desc_sw128(base + 2 * kTileBytes, 16, 1024), idesc_s, kHd / 16);                                          // dO V^T
+        }
+        if (elect_one()) umma_commit(&sdp_full[s]);
+        ++s_it;
+        item += gridDim.x;
+        more = next_valid();
+        progressed = true;
+      }
+      if (progressed) idle = 0;
+      else if (!all_lanes(keep_polling(idle, abort_word, p.status))) break;
     }
   } else if (warp < 8) {
     // ---- math threads: P and dS of every item, 16 of every 32 key columns each ---------------------------------------
@@ -506,8 +512,7 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     const int t = (warp & 3) * 32 + lane;
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const float scale_log2 = p.scale * 1.4426950408889634f;
-    const bool do_drop = p.dropout_p > 0.f && !(ablate & 64);
-    const unsigned long long seed = p.seed + ((do_drop && p.seed_dev) ? *p.seed_dev : 0ull);
+    const unsigned long long seed = p.seed + ((kDrop && p.seed_dev) ? *p.seed_dev : 0ull);
     int it = 0;
     int item = blockIdx.x;
     Item nxt = item < num_items ? get_item(p, item) : Item{};
@@ -530,37 +535,23 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       if (warp_writes) {
         const DropRng rng(seed, (p.stream_id << 16) | static_cast<unsigned long long>(w.h), p.dropout_p);
         const unsigned long long row_base = static_cast<unsigned long long>(w.q0 + t) * p.kstride + half * 16;
-        // two chunks (2 x 16 columns of this thread) per round: four TMEM loads in flight before the single wait
 #pragma unroll 1
-        for (int c = 0; c < nchunks; c += 2) {
-          const bool two = c + 1 < nchunks;
-          uint32_t s0[16], d0[16], s1[16], d1[16];
-          tmem_ld16(set + c * 32, s0);
-          tmem_ld16(set + 128 + c * 32, d0);
-          if (two) {
-            tmem_ld16(set + (c + 1) * 32, s1);
-            tmem_ld16(set + 128 + (c + 1) * 32, d1);
-          }
-          uint32_t km0 = 0xffffu, km1 = 0xffffu;
-          if (do_drop) {   // the mask words are hashed while the TMEM loads are in flight
-            km0 = drop_mask16(rng, row_base + c * 32);
-            if (two) km1 = drop_mask16(rng, row_base + (c + 1) * 32);
-          }
+        for (int c = 0; c < nchunks; ++c) {
+          uint32_t sc[16], dp[16];
+          tmem_ld16(set + c * 32, sc);
+          tmem_ld16(set + 128 + c * 32, dp);
+          uint32_t km = 0xffffu;
+          if constexpr (kDrop) km = drop_mask16(rng, row_base + c * 32);     // hashed while the TMEM loads are in flight
           tmem_ld_wait();
-          // all of the arithmetic comes before the wait for the staging tiles: it overlaps the previous item's gradient MMAs
-          uint4 p0[2], e0[2], p1[2], e1[2];
-          bwd_compute16(s0, d0, km0, do_drop, rng.scale, Drow, scale_log2, lse2, c * 32 + half * 16, w.k_len, p.causal != 0,
-                        c * 32 + half * 16, t, p0, e0);
-          if (two)
-            bwd_compute16(s1, d1, km1, do_drop, rng.scale, Drow, scale_log2, lse2, (c + 1) * 32 + half * 16, w.k_len,
-                          p.causal != 0, (c + 1) * 32 + half * 16, t, p1, e1);
+          // the arithmetic comes before the wait for the staging tiles: it overlaps the previous item's gradient MMAs
+          uint4 pr[2], ds[2];
+          bwd_compute16(sc, dp, km, kDrop, rng.scale, Drow, scale_log2, lse2, c * 32 + half * 16, w.k_len, p.causal != 0, c * 32 + half * 16, t, pr, ds);
           if (!may_store) {   // the gradient MMAs of the previous item still read the staging tiles
             ok = __all_sync(0xffffffffu, mbar_wait(pds_free, (it - 1) & 1, abort_word, p.status, kTimeoutSmemEmpty));
             if (!ok) break;
             may_store = true;
           }
-          bwd_store16(p0, e0, c * 32 + half * 16, t, sP, sDS);
-          if (two) bwd_store16(p1, e1, (c + 1) * 32 + half * 16, t, sP, sDS);
+          bwd_store16(pr, ds, c * 32 + half * 16, t, sP, sDS);
         }
       }
       if (ok && !may_store) {
@@ -592,13 +583,16 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       if (!__all_sync(0xffffffffu, mbar_wait(&grads_full[s], (j >> 1) & 1, abort_word, p.status, kTimeoutTmemFull))) return false;
       tc_fence_after_sync();
       if (!(ablate & 2)) {
-        const size_t col = static_cast<size_t>(w.h) * kHd;
-        if (wq * 32 < w.q_len)
-          bwd_store_row(set + 64, p.dq + static_cast<size_t>(w.q0 + t) * p.ld_dq + col, p.scale, t < w.q_len);
-        if (wq * 32 < w.k_len) {
-          // dK carries the softmax scale that dS left out
-          bwd_store_row(set + 128, p.dk + static_cast<size_t>(w.k0 + t) * p.ld_dk + col, p.scale, t < w.k_len);
-          bwd_store_row(set, p.dv + static_cast<size_t>(w.k0 + t) * p.ld_dv + col, 1.f, t < w.k_len);
+        // dQ, dK, dV; dQ and dK carry the softmax scale that dS left out
+        const int row0 = wq * 32;
+#pragma unroll 1
+        for (int m = 0; m < 3; ++m) {
+          const int len = m == 0 ? w.q_len : w.k_len, first = m == 0 ? w.q0 : w.k0;
+          if (row0 >= len) continue;
+          __nv_bfloat16* base = m == 0 ? p.dq : m == 1 ? p.dk : p.dv;
+          const int ld = m == 0 ? p.ld_dq : m == 1 ? p.ld_dk : p.ld_dv;
+          bwd_store_rows(set + (m == 0 ? 64 : m == 1 ? 128 : 0), base + static_cast<size_t>(first + row0) * ld + static_cast<size_t>(w.h) * kHd, ld,
+                         len - row0, m == 2 ? 1.f : p.scale, lane);
         }
       }
       tc_fence_before_sync();
@@ -608,28 +602,22 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     while (item < num_items && ok) {
       const Item w = nxt;
       item += gridDim.x;
-      if (item < num_items) {
-        nxt = get_item(p, item);
-        if (nxt.valid && t < nxt.q_len) {   // the rows this thread reads in the next iteration, on their way to L2 now
-          prefetch_l2(p.o + static_cast<size_t>(nxt.q0 + t) * p.ld_o + nxt.h * kHd);
-          prefetch_l2(p.d_o + static_cast<size_t>(nxt.q0 + t) * p.ld_do + nxt.h * kHd);
-        }
-      }
+      if (item < num_items) nxt = get_item(p, item);
       if (!w.valid) continue;
       const int s = it & 1;
       float Drow = 0.f, lse2 = kInf;
+      if (t < w.q_len) lse2 = (ablate & 32) ? 0.f : p.lse[static_cast<size_t>(w.h) * p.lse_stride + w.q0 + t] * 1.4426950408889634f;
+      if (!__all_sync(0xffffffffu, mbar_wait(o_full, it & 1, abort_word, p.status, kTimeoutTmaFull) &&
+                                       mbar_wait(&slot_full[s], (it >> 1) & 1, abort_word, p.status, kTimeoutTmaFull))) { ok = false; break; }
       if (t < w.q_len && !(ablate & 32)) {
-        const uint4* orow = reinterpret_cast<const uint4*>(p.o + static_cast<size_t>(w.q0 + t) * p.ld_o + w.h * kHd);
-        const uint4* drow = reinterpret_cast<const uint4*>(p.d_o + static_cast<size_t>(w.q0 + t) * p.ld_do + w.h * kHd);
-        uint4 a[8], d[8];
-#pragma unroll
-        for (int g4 = 0; g4 < 8; ++g4) { a[g4] = orow[g4]; d[g4] = drow[g4]; }
-        lse2 = p.lse[static_cast<size_t>(w.h) * p.lse_stride + w.q0 + t] * 1.4426950408889634f;
+        const uint8_t* so = sO;
+        const uint8_t* sdo = sSlots + s * kBwdSlotBytes + 3 * kTileBytes;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int g4 = 0; g4 < 8; ++g4) {
-          const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a[g4]);
-          const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&d[g4]);
+          const uint4 a = *reinterpret_cast<const uint4*>(so + sw128_offset(t, g4)), d = *reinterpret_cast<const uint4*>(sdo + sw128_offset(t, g4));
+          const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
+          const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&d);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const float2 x = __bfloat1622float2(a2[j]), y = __bfloat1622float2(d2[j]);
@@ -637,9 +625,8 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           }
         }
         Drow = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-      } else if (t < w.q_len) {
-        lse2 = 0.f;
       }
+      mbar_arrive(o_free);
       // the rows of item it - 2 have been read by every math thread
       if (!__all_sync(0xffffffffu, mbar_wait(&d_free[s], ((it >> 1) & 1) ^ 1, abort_word, p.status, kTimeoutSmemEmpty))) { ok = false; break; }
       sD[s * kTile + t] = Drow;
@@ -655,6 +642,7 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_word) {
+#pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
@@ -668,32 +656,50 @@ static int g_attn_bwd_ablate = 0;
 void set_attn_bwd_ablation(int bits) { g_attn_bwd_ablate = bits; }
 int get_attn_bwd_ablation() { return g_attn_bwd_ablate; }
 
-const char* launch_attn_fwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a,
-                                  int num_items, cudaStream_t stream) {
+template <int kGroups, bool kDrop>
+static const char* launch_fwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, int num_items,
+                                    cudaStream_t stream) {
+  auto kern = attn_fwd_short_kernel<kGroups, kDrop>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t ce = cudaFuncSetAttribute(attn_fwd_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdShortSmem);
+    cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_short_smem(kGroups));
     if (ce != cudaSuccess) return cudaGetErrorString(ce);
     configured = true;
   }
   const int grid = num_items < num_sms() ? num_items : num_sms();
-  attn_fwd_short_kernel<<<grid, kFwdShortThreads, kFwdShortSmem, stream>>>(tq, tk, tv, a, num_items);
+  kern<<<grid, fwd_short_threads(kGroups), fwd_short_smem(kGroups), stream>>>(tq, tk, tv, a, num_items);
+  cudaError_t ce = cudaGetLastError();
+  return ce == cudaSuccess ? nullptr : cudaGetErrorString(ce);
+}
+
+const char* launch_attn_fwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a,
+                                  int num_items, cudaStream_t stream) {
+  const bool drop = a.dropout_p > 0.f;
+  // up to two items to a CTA: two groups
+  if (num_items <= 2 * num_sms())
+    return drop ? launch_fwd_short<2, true>(tq, tk, tv, a, num_items, stream) : launch_fwd_short<2, false>(tq, tk, tv, a, num_items, stream);
+  return drop ? launch_fwd_short<4, true>(tq, tk, tv, a, num_items, stream) : launch_fwd_short<4, false>(tq, tk, tv, a, num_items, stream);
+}
+
+template <bool kDrop>
+static const char* launch_bwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                                    const CUtensorMap& to, const AttnArgs& a, int num_items, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t ce = cudaFuncSetAttribute(attn_bwd_short_kernel<kDrop>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdShortSmem);
+    if (ce != cudaSuccess) return cudaGetErrorString(ce);
+    configured = true;
+  }
+  const int grid = num_items < num_sms() ? num_items : num_sms();
+  attn_bwd_short_kernel<kDrop><<<grid, kBwdShortThreads, kBwdShortSmem, stream>>>(tq, tk, tv, tdo, to, a, num_items, g_attn_bwd_ablate);
   cudaError_t ce = cudaGetLastError();
   return ce == cudaSuccess ? nullptr : cudaGetErrorString(ce);
 }
 
 const char* launch_attn_bwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                                  const AttnArgs& a, int num_items, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t ce = cudaFuncSetAttribute(attn_bwd_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdShortSmem);
-    if (ce != cudaSuccess) return cudaGetErrorString(ce);
-    configured = true;
-  }
-  const int grid = num_items < num_sms() ? num_items : num_sms();
-  attn_bwd_short_kernel<<<grid, kBwdShortThreads, kBwdShortSmem, stream>>>(tq, tk, tv, tdo, a, num_items, g_attn_bwd_ablate);
-  cudaError_t ce = cudaGetLastError();
-  return ce == cudaSuccess ? nullptr : cudaGetErrorString(ce);
+                                  const CUtensorMap& to, const AttnArgs& a, int num_items, cudaStream_t stream) {
+  const bool drop = a.dropout_p > 0.f && !(g_attn_bwd_ablate & 64);
+  return drop ? launch_bwd_short<true>(tq, tk, tv, tdo, to, a, num_items, stream) : launch_bwd_short<false>(tq, tk, tv, tdo, to, a, num_items, stream);
 }
 
 }  // namespace b200

@@ -264,6 +264,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_word) {
+#pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
@@ -585,6 +586,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_word) {
+#pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
@@ -646,7 +648,7 @@ namespace b200 {
 const char* launch_attn_fwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a,
                                   int num_items, cudaStream_t stream);
 const char* launch_attn_bwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                                  const AttnArgs& a, int num_items, cudaStream_t stream);
+                                  const CUtensorMap& to, const AttnArgs& a, int num_items, cudaStream_t stream);
 const char* launch_attn_fwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, int max_q,
                                cudaStream_t stream);
 const char* launch_attn_bwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
@@ -672,6 +674,7 @@ const char* nmtg_attn_fwd(const AttnDesc* d, cudaStream_t stream) {
       (e = check_ptr(d->out, d->ld_out)))
     return e;
   const int width = d->num_heads * kHd;
+  const bool one_tile = g_attn_variant == 0 && d->max_q <= kTile && d->max_k <= kTile && !d->bias;
   CUtensorMap tq, tk, tv;
   if (!cached_tmap(&tq, d->q, d->total_q, width, d->ld_q, kTile, kHd)) return "attention: tensor map (q) failed";
   if (!cached_tmap(&tk, d->k, d->total_k, width, d->ld_k, kTile, kHd)) return "attention: tensor map (k) failed";
@@ -683,8 +686,7 @@ const char* nmtg_attn_fwd(const AttnDesc* d, cudaStream_t stream) {
   a.lse = d->lse; a.lse_stride = d->lse_stride;
   a.p_debug = nullptr; a.total_q = d->total_q; a.total_k = d->total_k; a.batch = d->batch; a.status = d->status;
   a.bias = d->bias; a.bias_sb = d->bias_sb; a.bias_sh = d->bias_sh; a.bias_sq = d->bias_sq; a.dbias = nullptr;
-  if (g_attn_variant == 0 && d->max_q <= kTile && d->max_k <= kTile && !d->bias)
-    return launch_attn_fwd_short(tq, tk, tv, a, d->batch * d->num_heads, stream);
+  if (one_tile) return launch_attn_fwd_short(tq, tk, tv, a, d->batch * d->num_heads, stream);
   // Long sequences without attention dropout: the warp-specialised kernel (attention_fwd_ws_tcgen05.cu), two query tiles
   // per CTA.  Measured against the kernel below: 0.233 / 0.264 ms on 8 x 1500 x 20 heads, but 0.070 / 0.053 ms on
   // 8 x 448 causal (too few CTAs of 256 queries for 148 SMs), hence the length threshold; variant 1 ignores it (tests).
@@ -715,6 +717,7 @@ const char* nmtg_attn_bwd(const AttnDesc* d, cudaStream_t stream) {
   if (d->max_k > kTile && !d->dq_acc) return "attention backward: sequences above 128 keys need the fp32 dq buffer";
   const int width = d->num_heads * kHd;
   CUtensorMap tq, tk, tv, tdo;
+  const bool one_tile = g_attn_variant == 0 && d->max_q <= kTile && d->max_k <= kTile && !d->bias;
   if (!cached_tmap(&tq, d->q, d->total_q, width, d->ld_q, kTile, kHd)) return "attention: tensor map (q) failed";
   if (!cached_tmap(&tk, d->k, d->total_k, width, d->ld_k, kTile, kHd)) return "attention: tensor map (k) failed";
   if (!cached_tmap(&tv, d->v, d->total_k, width, d->ld_v, kTile, kHd)) return "attention: tensor map (v) failed";
@@ -731,8 +734,11 @@ const char* nmtg_attn_bwd(const AttnDesc* d, cudaStream_t stream) {
   a.dq_acc = d->dq_acc; a.ld_dqacc = d->ld_dqacc;
   a.total_q = d->total_q; a.total_k = d->total_k; a.batch = d->batch; a.status = d->status;
   a.bias = d->bias; a.bias_sb = d->bias_sb; a.bias_sh = d->bias_sh; a.bias_sq = d->bias_sq; a.dbias = d->dbias;
-  if (g_attn_variant == 0 && d->max_q <= kTile && d->max_k <= kTile && !d->bias)
-    return launch_attn_bwd_short(tq, tk, tv, tdo, a, d->batch * d->num_heads, stream);
+  if (one_tile) {
+    CUtensorMap to;
+    if (!cached_tmap(&to, d->out, d->total_q, width, d->ld_out, kTile, kHd)) return "attn_bwd: cuTensorMapEncodeTiled failed for O";
+    return launch_attn_bwd_short(tq, tk, tv, tdo, to, a, d->batch * d->num_heads, stream);
+  }
   static bool configured = false;
   if (!configured) {
     cudaError_t ce = cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);

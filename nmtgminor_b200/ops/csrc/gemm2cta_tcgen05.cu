@@ -456,6 +456,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_word) {
+#pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }

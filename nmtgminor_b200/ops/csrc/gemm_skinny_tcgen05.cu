@@ -257,6 +257,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   if (p.split > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   else __syncthreads();
   if (*abort_word) {
+#pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);      // copies in flight land before shared memory is released
     __syncthreads();
   }

@@ -115,6 +115,43 @@ def test_many_items_per_cta_pipeline():
     assert _err(qkv.grad, q32.grad) < 3e-2
 
 
+@pytest.mark.parametrize("heads,copies", [(2, 1), (2, 9), (9, 3)])
+@pytest.mark.parametrize("p", [0.0, 0.3])
+@pytest.mark.parametrize("causal", [False, True])
+def test_single_tile_kernels_agree_with_the_general_ones(heads, copies, p, causal):
+    """One, two and many items to a CTA (two and four softmax groups, both row halves), queries and keys at the edges of the 16-row
+    reductions, 32-column chunks and 64-row halves, empty sequences among them; the same dropout masks.  Both kernels round P and dS to
+    bf16 and sum in 32 bits."""
+    g = torch.Generator(device=DEV).manual_seed(heads)
+    lq, lk = [1, 16, 0, 17, 64, 65, 31, 128, 32, 33, 100, 63] * copies, [5, 128, 3, 15, 33, 64, 32, 127, 1, 96, 97, 16] * copies
+    lk = lq if causal else lk
+    W, nq, nk = heads * 64, sum(lq), sum(lk)
+    rnd = lambda n: torch.randn(n, W, device=DEV, generator=g).bfloat16()
+    q, k, v, dout, cu_q, cu_k = rnd(nq + 8), rnd(nk + 8), rnd(nk + 8), rnd(nq + 8), _cu(lq), _cu(lk)
+    res = []
+    for kind in (0, 2):
+        ops.ext().set_attention_variant(kind)
+        try:
+            _poison()
+            out, lse = torch.empty_like(q), torch.empty(heads, nq + 8, device=DEV)
+            grads = [torch.empty_like(t) for t in (q, k, v)]
+            acc = torch.zeros(nq + 8, W, device=DEV)
+            ops.ext().attn_fwd(q, k, v, out, lse, cu_q, cu_k, heads, 128, 128, causal, 0.125, p, 7, 3)
+            ops.ext().attn_bwd(q, k, v, out, lse, dout, *grads, acc, cu_q, cu_k, heads, 128, 128, causal, 0.125, p, 7, 3)
+            torch.cuda.synchronize()
+        finally:
+            ops.ext().set_attention_variant(0)
+        res.append([out[:nq], lse[:, :nq]] + [t[:n] for t, n in zip(grads, (nq, nk, nk))])
+    assert ops.check_status() == 0
+    keep = torch.ones(nk, dtype=torch.bool, device=DEV)           # keys of a sequence without queries get no gradient from the kernels
+    for i, n in enumerate(lq):
+        keep[int(cu_k[i]):int(cu_k[i + 1])] = n > 0
+    for a, b, rel in zip(res[0], res[1], (2e-2, 1e-4, 2e-2, 2e-2, 2e-2)):
+        if a.shape[0] == nk and not causal:
+            a, b = a[keep], b[keep]
+        assert _err(a, b) < rel
+
+
 def test_attention_dropout_is_replayed_in_backward(variant):
     """With dropout the op must stay a deterministic function of (seed, stream): finite differences of the
     forward agree with the analytic backward only if backward regenerates the forward mask."""
