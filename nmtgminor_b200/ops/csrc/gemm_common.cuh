@@ -96,6 +96,54 @@ __device__ __forceinline__ float gelu_grad(float x) {
 }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 
+// Two elements at a time: the 32-bit pairs of sm_100 (one instruction, both halves rounded as the single one rounds).
+struct Pair {
+  uint64_t v;
+  __device__ __forceinline__ Pair() {}
+  __device__ __forceinline__ Pair(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi)); }
+  __device__ __forceinline__ explicit Pair(float both) : Pair(both, both) {}
+  __device__ __forceinline__ float2 split() const {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+  }
+};
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair d;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return d;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  Pair d;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+// normal_cdf of two values, the same operations
+__device__ __forceinline__ Pair normal_cdf2(Pair x, Pair& bell) {
+  const float2 f = x.split();
+  const float a0 = fabsf(f.x), a1 = fabsf(f.y);
+  const Pair z = mul2(x, x);
+  const float2 e = mul2(z, Pair(-0.72134752f)).split();
+  bell = Pair(exp2f(e.x), exp2f(e.y));
+  const float2 d = fma2(Pair(0.35f), Pair(a0, a1), Pair(1.f)).split();
+  const Pair t(__fdividef(1.f, d.x), __fdividef(1.f, d.y));
+  Pair q = fma2(t, Pair(0.0444524474f), Pair(-0.111576788f));
+  q = fma2(t, q, Pair(0.0438466556f));
+  q = fma2(t, q, Pair(0.0324914902f));
+  q = fma2(t, q, Pair(0.0890091509f));
+  q = fma2(t, q, Pair(0.122769959f));
+  q = fma2(t, q, Pair(0.139575362f));
+  q = fma2(t, q, Pair(0.139633134f));
+  const float2 tail = mul2(mul2(q, t), bell).split();
+  Pair p = fma2(z, Pair(-6.6448597e-06f), Pair(0.000110327455f));
+  p = fma2(z, p, Pair(-0.00118270959f));
+  p = fma2(z, p, Pair(0.00997150037f));
+  p = fma2(z, p, Pair(-0.0664899871f));
+  p = fma2(z, p, Pair(0.398942262f));
+  const float2 mid = fma2(x, p, Pair(0.5f)).split();
+  return Pair(a0 < 1.25f ? mid.x : f.x < 0.f ? tail.x : 1.f - tail.x, a1 < 1.25f ? mid.y : f.y < 0.f ? tail.y : 1.f - tail.y);
+}
+
 // One thread = one accumulator row; processes columns [col0, col0 + 32) read from TMEM address `taddr`:
 // alpha, bias, optional pre-activation store, activation or activation gradient, dropout, residual, store
 // (bf16, fp32, fp32 accumulate, or fp32 red.add for split-K).  Warp-collective (contains a tcgen05.ld).
@@ -241,7 +289,14 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
         for (int j = 0; j < 32; ++j) v[j] *= av[j] > 0.f ? 1.f : 0.f;
       } else if (p.act == kActGeluBwd) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] *= gelu_grad(av[j]);
+        for (int j = 0; j < 32; j += 2) {
+          const Pair x(av[j], av[j + 1]);
+          Pair bell;
+          const Pair cdf = normal_cdf2(x, bell);
+          const float2 d = fma2(x, mul2(Pair(0.3989422804014327f), bell), cdf).split();
+          v[j] *= d.x;
+          v[j + 1] *= d.y;
+        }
       } else {
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
@@ -254,7 +309,13 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
       for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
     } else if ((kFeat & kEpiActFwd) && p.act == kActGelu) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = gelu_f(v[j]);
+      for (int j = 0; j < 32; j += 2) {
+        const Pair x(v[j], v[j + 1]);
+        Pair bell;
+        const float2 f = mul2(x, normal_cdf2(x, bell)).split();
+        v[j] = f.x;
+        v[j + 1] = f.y;
+      }
     } else if ((kFeat & kEpiActFwd) && p.act == kActSilu) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoid_f(v[j]);
