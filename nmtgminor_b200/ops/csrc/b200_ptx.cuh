@@ -179,7 +179,8 @@ __device__ __forceinline__ bool elect_one() {
 template <typename T>
 __device__ __forceinline__ T uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
 // the same answer for all lanes
-__device__ __forceinline__ bool all_lanes(bool v) { return __all_sync(0xffffffffu, v); }
+template <bool kWarp = true>
+__device__ __forceinline__ bool all_lanes(bool v) { return kWarp ? __all_sync(0xffffffffu, v) != 0 : v; }
 
 // D[tmem] (+)= A[smem] * B[smem]; one thread issues.  accumulate = 0 overwrites D.
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,

@@ -74,8 +74,10 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc,
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
+// the mbarriers at this offset of both CTAs of the pair
+__device__ __forceinline__ void umma_commit_both(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"(static_cast<uint16_t>(3)) : "memory");
 }
 
 template <int BN, bool kTrace, uint32_t kFeat>
@@ -175,6 +177,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const long left = g.units - static_cast<long>(sgm) * g.seg_units;
         const int need = left < g.seg_units ? static_cast<int>(left) : g.seg_units;
         const int* ctr = g.counters + 2 + sgm;
+#pragma unroll 1
         for (uint32_t i = 0; i < B200_WAIT_POLLS; ++i) {
           if (ld_acquire_gpu(ctr) >= need) {
             fence_proxy_async_all();     // the copies were ordinary stores; the loads below go through the async proxy
@@ -219,7 +222,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------- UMMA issuer (leader only) -------------------------------
-    if (leader && lane == 0) {
+    // All lanes, see elect_one; one lane for weight gradients, whose partial tiles then meet in the output less often at the same time
+    // (5120 x 1280 over 1800 rows: 32 us so, 35.5 with all lanes; 8192 rows 59 both ways)
+    constexpr bool kWarp = kFeat != kEpiF32;
+    if (leader && (kWarp || lane == 0)) {
       const uint32_t idesc = make_idesc_bf16(2 * BM, BN, p.a_mn_major, p.b_mn_major);
       const uint32_t a_lbo = p.a_mn_major ? BK * 128 : 16, b_lbo = p.b_mn_major ? BK * 128 : 16;
       const uint32_t a_kstep = p.a_mn_major ? (16 * 128) >> 4 : 32 >> 4;
@@ -238,36 +244,36 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         long long t0 = kTrace ? clock64() : 0;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_word, p.status, kTimeoutTmemEmpty)) break;
+        if (!all_lanes<kWarp>(mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_word, p.status, kTimeoutTmemEmpty))) break;
         if (kTrace) t_wait_acc += clock64() - t0;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = (kWarp ? uniform(tmem_base) : tmem_base) + acc * BN;
         for (int kb = kb_begin; kb < kb_end; ++kb) {
           t0 = kTrace ? clock64() : 0;
-          if (!mbar_wait(&full_bar[stage], phase, abort_word, p.status, kTimeoutTmaFull)) { ok = false; break; }
+          if (!all_lanes<kWarp>(mbar_wait(&full_bar[stage], phase, abort_word, p.status, kTimeoutTmaFull))) { ok = false; break; }
           if (kTrace) {
             const long long t1 = clock64();
             t_wait_ops += t1 - t0;
             if (t_first == 0) t_first = t1 - t_begin;
           }
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * S::kStageBytes);
+          const uint32_t sa = (kWarp ? uniform(smem_u32(smem)) : smem_u32(smem)) + stage * S::kStageBytes;
           const uint32_t sb = sa + S::kABytes;
           const uint64_t adesc = make_smem_desc_sw128(sa, a_lbo, 1024);
           const uint64_t bdesc = make_smem_desc_sw128(sb, b_lbo, 1024);
-          if (!kTrace || p.ablate != 3) {     // traced ablation 3: stream the operands only, no tensor-core work
+          if (!kWarp || elect_one()) {
+            if (!kTrace || p.ablate != 3) {     // traced ablation 3: stream the operands only, no tensor-core work
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k)
-              umma_bf16_pair(d_tmem, adesc + static_cast<uint64_t>(k * a_kstep), bdesc + static_cast<uint64_t>(k * b_kstep), idesc,
-                             (kb > kb_begin || k > 0) ? 1u : 0u);
+              for (int k = 0; k < BK / 16; ++k)
+                umma_bf16_pair(d_tmem, adesc + static_cast<uint64_t>(k * a_kstep), bdesc + static_cast<uint64_t>(k * b_kstep), idesc,
+                               (kb > kb_begin || k > 0) ? 1u : 0u);
+            }
+            umma_commit_both(smem_u32(&empty_bar[stage]));
           }
-          umma_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 0));
-          umma_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 1));
           if (++stage == S::kStages) { stage = 0; phase ^= 1; }
         }
         if (ok) {
-          umma_commit_pair(map_to_cta(smem_u32(&tmem_full[acc]), 0));
-          umma_commit_pair(map_to_cta(smem_u32(&tmem_full[acc]), 1));
+          if (!kWarp || elect_one()) umma_commit_both(smem_u32(&tmem_full[acc]));
         }
       }
       if (kTrace && p.trace) {
@@ -387,15 +393,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
           __syncwarp();
           const long long c1 = tracing ? clock64() : 0;
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + g * 64;
+#pragma unroll 1          // the body once: twice as much code is fetched more slowly than it runs
+          for (int half = 0; half < 2; ++half)
             if (col0 + half * 32 < p.N)
-              gemm_epilogue_chunk<kFeat>(p, rng, do_drop, row, row_ok, col0 + half * 32,
-                                  tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + g * 64 + half * 32,
-                                  stage + lane * 128, half, lane,
-                                  (kTwo && (kFeat & kEpiPreact) && p.tma_second) ? my_stage + 32 * 128 + lane * 128 : nullptr,
-                                  kAuxTma && p.tma_second);
-          }
+              gemm_epilogue_chunk<kFeat>(p, rng, do_drop, row, row_ok, col0 + half * 32, taddr + half * 32, stage + lane * 128, half, lane,
+                                         (kTwo && (kFeat & kEpiPreact) && p.tma_second) ? my_stage + 32 * 128 + lane * 128 : nullptr,
+                                         kAuxTma && p.tma_second);
           const long long c2 = tracing ? clock64() : 0;
           fence_async_smem();
           __syncwarp();

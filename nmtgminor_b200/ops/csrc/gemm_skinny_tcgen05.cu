@@ -202,26 +202,27 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (++stage == S::kStages) { stage = 0; phase ^= 1; }
       }
     }
-  } else if (warp == 5) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(kSkinnyFeat, NT, 0, 0);
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(&full_bar[stage], phase, abort_word, p.status, kTimeoutTmaFull)) { ok = false; break; }
-        tc_fence_after_sync();
-        const uint32_t sw = smem_u32(smem + stage * S::kStageBytes);
-        const uint64_t wdesc = make_smem_desc_sw128(sw, 16, 1024);
-        const uint64_t xdesc = make_smem_desc_sw128(sw + S::kWBytes, 16, 1024);
+  } else if (warp == 5) {                // all lanes: see elect_one
+    constexpr uint32_t idesc = make_idesc_bf16(kSkinnyFeat, NT, 0, 0);
+    const uint32_t tmem = uniform(tmem_base), smem0 = uniform(smem_u32(smem));
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!all_lanes(mbar_wait(&full_bar[stage], phase, abort_word, p.status, kTimeoutTmaFull))) { ok = false; break; }
+      tc_fence_after_sync();
+      const uint32_t sw = smem0 + stage * S::kStageBytes;
+      const uint64_t wdesc = make_smem_desc_sw128(sw, 16, 1024);
+      const uint64_t xdesc = make_smem_desc_sw128(sw + S::kWBytes, 16, 1024);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k)
-          umma_bf16(tmem_base, wdesc + static_cast<uint64_t>(k * 2), xdesc + static_cast<uint64_t>(k * 2), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+          umma_bf16(tmem, wdesc + static_cast<uint64_t>(k * 2), xdesc + static_cast<uint64_t>(k * 2), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
         umma_commit(&empty_bar[stage]);
-        if (++stage == S::kStages) { stage = 0; phase ^= 1; }
       }
-      if (ok) umma_commit(done_bar);
+      if (++stage == S::kStages) { stage = 0; phase ^= 1; }
     }
+    if (ok && elect_one()) umma_commit(done_bar);
   } else {
     pdl_wait();        // the residual is an earlier kernel's output, and so may be the buffer that is written
     const bool ok = mbar_wait(done_bar, 0, abort_word, p.status, kTimeoutTmemFull);
