@@ -30,7 +30,6 @@ namespace b200 {
 
 constexpr int kWsThreads = 448;
 constexpr int kWsSmem = 2 * kTileBytes + 6 * kTileBytes + 3 * kPBytes + 256 + 1024;
-constexpr uint32_t kWsIssuePolls = 1u << 22;   // polls of the MMA warp without progress before it gives up
 
 // Time stamps (SM clock) of CTA (0, 0, 0) when ablation bit 128 is set: [tile][16] = math warp 0: S lo ready, loaded,
 // computed, stored, S hi ready, loaded, computed, stored | MMA warp: S lo issued, S hi issued, products issued | dQ warps:
@@ -149,11 +148,14 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     }
   } else if (warp == 13) {
     // ---- MMA issuer ----------------------------------------------------------------------------------------------
-    if (lane == 0 && n_tiles > 0 && mbar_wait(kv_full, 0, abort_word, p.status, kTimeoutTmaFull)) {
+    // all lanes (see elect_one): 40 MMAs a tile, of 32 clocks each, cost one lane 150 to 200 clocks each to issue
+    if (n_tiles > 0 && all_lanes(mbar_wait(kv_full, 0, abort_word, p.status, kTimeoutTmaFull))) {
       const uint32_t idesc_s = make_idesc_bf16(kTile, 64, 0, 0);       // S, dP halves: K-major x K-major, N = 64 keys
       const uint32_t idesc_dq = make_idesc_bf16(kTile, kHd, 0, 1);     // dQ    : K-major A, MN-major B
       const uint32_t idesc_dkv = make_idesc_bf16(kTile, kHd, 1, 1);    // dK,dV : MN-major A and B
-      const uint32_t ka = smem_u32(sK), va = smem_u32(sV);
+      const uint32_t tmem = uniform(tmem_base), base = uniform(smem_u32(smem));
+      const uint32_t ka = base, va = base + kTileBytes, qd = base + 2 * kTileBytes, pa = base + 8 * kTileBytes, dsa0 = pa + kPBytes;
+      const uint32_t uS = tmem, uDP = tmem + 128, uDK = tmem + 256, uDV = tmem + 320, uDQ = tmem + 384;
       // Two queues served in whichever order their inputs arrive: the halves of S / dP of tile s_it, and the gradient
       // products of tile g_it.  The S queue is polled first: the math threads wait for nothing else.
       int s_it = 0, s_half = 0, g_it = 0;
@@ -162,17 +164,17 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         bool progressed = false;
         if (s_it < n_tiles) {
           const int s = s_it % 3;
-          const bool ready = (s_half == 1 || mbar_test_wait(&qdo_full[s], (s_it / 3) & 1)) &&
-                             (s_it == 0 || mbar_test_wait(&s_free[s_half], (s_it - 1) & 1));
+          const bool ready = all_lanes((s_half == 1 || mbar_test_wait(&qdo_full[s], (s_it / 3) & 1)) &&
+                                       (s_it == 0 || mbar_test_wait(&s_free[s_half], (s_it - 1) & 1)));
           if (ready) {
             tc_fence_after_sync();
-            const uint32_t qa = smem_u32(sQD + s * 2 * kTileBytes), doa = qa + kTileBytes;
+            const uint32_t qa = qd + s * 2 * kTileBytes, doa = qa + kTileBytes;
             const uint32_t koff = s_half * 64 * 128;     // keys 64..127 start 64 rows (of 128 bytes) into the K / V tiles
             if (!(ablate & 8)) {
-              umma_steps(tS + s_half * 64, qa, 16, 32, ka + koff, 16, 32, idesc_s, kHd / 16, false);      // Q K^T
-              umma_steps(tDP + s_half * 64, doa, 16, 32, va + koff, 16, 32, idesc_s, kHd / 16, false);    // dO V^T
+              umma_steps_warp<32, 32>(uS + s_half * 64, make_smem_desc_sw128(qa, 16, 1024), make_smem_desc_sw128(ka + koff, 16, 1024), idesc_s, kHd / 16);      // Q K^T
+              umma_steps_warp<32, 32>(uDP + s_half * 64, make_smem_desc_sw128(doa, 16, 1024), make_smem_desc_sw128(va + koff, 16, 1024), idesc_s, kHd / 16);    // dO V^T
             }
-            umma_commit(&s_full[s_half]);
+            if (elect_one()) umma_commit(&s_full[s_half]);
             WS_STAMP(s_it, 8 + s_half);
             if (s_half == 1) ++s_it;
             s_half ^= 1;
@@ -181,41 +183,28 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         if (g_it < s_it) {
           const int s = g_it & 1;
-          if (mbar_test_wait(&pds_full[s], (g_it >> 1) & 1) && (g_it < 2 || mbar_test_wait(&dq_free[s], ((g_it >> 1) & 1) ^ 1))) {
+          if (all_lanes(mbar_test_wait(&pds_full[s], (g_it >> 1) & 1) && (g_it < 2 || mbar_test_wait(&dq_free[s], ((g_it >> 1) & 1) ^ 1)))) {
             tc_fence_after_sync();
             const int qb = g_it % 3;
-            const uint32_t qa = smem_u32(sQD + qb * 2 * kTileBytes), doa = qa + kTileBytes;
-            const uint32_t pa = smem_u32(sPst), dsa = smem_u32(sDSst + s * kPBytes);
-            const uint32_t dq = tDQ + s * 64;
+            const uint32_t qa = qd + qb * 2 * kTileBytes, doa = qa + kTileBytes;
+            const uint32_t dsa = dsa0 + s * kPBytes;
             // dV += P^T dO, dK += dS^T Q : A read MN-major (M = keys: two 64-key slabs), reduction over the 128 query rows
-            if (!(ablate & 4)) {
-              umma_steps(tDV, pa, kTileBytes, 2048, doa, 8192, 2048, idesc_dkv, 8, g_it > 0);
-            }
-            umma_commit(p_free);            // dV is the only reader of the P staging tile
-            if (!(ablate & 4)) umma_steps(tDK, dsa, kTileBytes, 2048, qa, 8192, 2048, idesc_dkv, 8, g_it > 0);
-            umma_commit(&qdo_free[qb]);    // dV and dK were the last readers of the Q / dO tiles: the tile after next can be fetched
-            if (!(ablate & 4)) {
-              // dQ = dS K : A = dS K-major (two slabs of 4 k-steps), B = K tile MN-major
-              umma_steps(dq, dsa, 16, 32, ka, 8192, 2048, idesc_dq, 4, false);
-              umma_steps(dq, dsa + kTileBytes, 16, 32, ka + 4 * 2048, 8192, 2048, idesc_dq, 4, true);
-            }
-            umma_commit(&grads_full[s]);
+            if (!(ablate & 4))
+              umma_steps_warp<2048, 2048>(uDV, make_smem_desc_sw128(pa, kTileBytes, 1024), make_smem_desc_sw128(doa, 8192, 1024), idesc_dkv, 8, g_it > 0);
+            if (elect_one()) umma_commit(p_free);            // dV is the only reader of the P staging tile
+            if (!(ablate & 4))
+              umma_steps_warp<2048, 2048>(uDK, make_smem_desc_sw128(dsa, kTileBytes, 1024), make_smem_desc_sw128(qa, 8192, 1024), idesc_dkv, 8, g_it > 0);
+            if (elect_one()) umma_commit(&qdo_free[qb]);    // dV and dK were the last readers of the Q / dO tiles: the tile after next can be fetched
+            // dQ = dS K : A = dS K-major (two slabs of 4 k-steps), B = K tile MN-major
+            if (!(ablate & 4)) umma_slabs_warp(uDQ + s * 64, make_smem_desc_sw128(dsa, 16, 1024), make_smem_desc_sw128(ka, 8192, 1024), idesc_dq, 8);
+            if (elect_one()) umma_commit(&grads_full[s]);
             WS_STAMP(g_it, 10);
             ++g_it;
             progressed = true;
           }
         }
-        if (progressed) {
-          idle = 0;
-        } else if (++idle > 4096) {      // a few microseconds of plain polling first: a sleep here delays every waiter
-          if (*abort_word) break;
-          if (idle > kWsIssuePolls) {
-            *abort_word = 1;
-            if (p.status) atomicCAS(p.status, 0, static_cast<int>(kTimeoutTmemEmpty));
-            break;
-          }
-          __nanosleep(idle > 65536 ? 256 : 32);
-        }
+        if (progressed) idle = 0;
+        else if (!all_lanes(keep_polling(idle, abort_word, p.status))) break;
       }
     }
   } else if (warp < 8) {

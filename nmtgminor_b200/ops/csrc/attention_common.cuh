@@ -90,12 +90,29 @@ __device__ __forceinline__ void zero_tail_bwd(const AttnArgs& p) {
   zero_tail_rows(p.dv, p.ld_dv, w, k_end, p.total_k);
 }
 
+constexpr uint32_t kIssuePolls = 1u << 22;   // polls of the MMA warp without progress before it gives up
+
+// Bounded wait of a warp that polls several barriers: counts polls without progress, false when it is time to give up.
+__device__ __forceinline__ bool keep_polling(uint32_t& idle, volatile int* abort_word, int* status) {
+  if (++idle > 4096) {        // a few microseconds of plain polling first: a sleep here delays every waiter
+    if (*abort_word) return false;
+    if (idle > kIssuePolls) {
+      *abort_word = 1;
+      if (status) atomicCAS(status, 0, static_cast<int>(kTimeoutTmemEmpty));
+      return false;
+    }
+    __nanosleep(idle > 65536 ? 256 : 32);
+  }
+  return true;
+}
+
 // nk UMMA k-steps issued by the elected lane of a converged warp; nk and the descriptors uniform.
 template <int kAStep, int kBStep>
-__device__ __forceinline__ void umma_steps_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int nk) {
+__device__ __forceinline__ void umma_steps_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int nk,
+                                                bool accumulate_first = false) {
 #pragma unroll 1
   for (int k = 0; k < nk; ++k) {
-    if (elect_one()) umma_bf16(d_tmem, adesc, bdesc, idesc, k > 0 ? 1u : 0u);
+    if (elect_one()) umma_bf16(d_tmem, adesc, bdesc, idesc, accumulate_first || k > 0 ? 1u : 0u);
     adesc += kAStep >> 4;
     bdesc += kBStep >> 4;
   }

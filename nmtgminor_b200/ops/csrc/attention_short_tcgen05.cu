@@ -56,25 +56,10 @@ __device__ __forceinline__ Item get_item(const AttnArgs& p, int item) {
 constexpr int kFwdSlotBytes = 3 * kTileBytes;
 constexpr int fwd_short_threads(int groups) { return groups * 128 + 64; }   // softmax groups, TMA producer warp, MMA warp
 constexpr int fwd_short_smem(int groups) { return groups * kFwdSlotBytes + 512 + 1024; }
-constexpr uint32_t kIssuePolls = 1u << 22;   // polls of the MMA warp without progress before it gives up
 
 // Up to 64 queries leave two of a group's four warps without work, and a warp's number decides both its rows (TMEM lanes) and its
 // scheduler: odd groups take such items in rows 64 .. 127 (the tile starts 64 rows early; a load may start before the matrix).
 __device__ __forceinline__ int row_shift(int group, int q_len) { return (group & 1) && q_len <= 64 ? 64 : 0; }
-
-// Bounded wait of a warp that polls several barriers: counts polls without progress, false when it is time to give up.
-__device__ __forceinline__ bool keep_polling(uint32_t& idle, volatile int* abort_word, int* status) {
-  if (++idle > 4096) {        // a few microseconds of plain polling first: a sleep here delays every waiter
-    if (*abort_word) return false;
-    if (idle > kIssuePolls) {
-      *abort_word = 1;
-      if (status) atomicCAS(status, 0, static_cast<int>(kTimeoutTmemEmpty));
-      return false;
-    }
-    __nanosleep(idle > 65536 ? 256 : 32);
-  }
-  return true;
-}
 
 template <int kFwdGroups, bool kDrop>
 __global__ void __launch_bounds__(fwd_short_threads(kFwdGroups), 1)
