@@ -714,20 +714,26 @@ def _decoder_step_general(self, x, cache: dict, mem_mask):
 DecoderLayer._step_general = _decoder_step_general
 
 
-def pack_padded(x_bt, lengths, capacity=None):
-    """Right-padded ``[B, T, ...]`` + lengths -> packed ``[N, ...]`` and a ``PackedSeqs`` descriptor (tokens unused)."""
+def pack_padded(x_bt, lengths, capacity=None, total=None):
+    """Right-padded ``[B, T, ...]`` + lengths -> packed ``[N, ...]`` and a ``PackedSeqs`` descriptor (tokens unused).  ``total``: the sum of
+    the lengths (none above T), if the caller has it on the host; otherwise the host waits for the device here, and kernels that
+    it could have launched meanwhile come late."""
     B, T = x_bt.shape[0], x_bt.shape[1]
     lengths = lengths.to(torch.int64).clamp(max=T)
     ar = torch.arange(T, device=x_bt.device)
-    mask = ar[None, :] < lengths[:, None]
-    packed = x_bt[mask]
-    total = packed.shape[0]
+    if total is not None:
+        rows = torch.repeat_interleave(torch.arange(B, device=x_bt.device), lengths, output_size=total)
+        pos = torch.arange(total, device=x_bt.device) - (torch.cumsum(lengths, 0) - lengths)[rows]
+        packed = x_bt.flatten(0, 1).index_select(0, rows * T + pos)
+    else:
+        mask = ar[None, :] < lengths[:, None]
+        packed, pos = x_bt[mask], ar[None, :].expand(B, T)[mask]
+        total = packed.shape[0]
     cap = capacity if capacity is not None else total
     if cap > total:
         packed = torch.cat([packed, packed.new_zeros((cap - total,) + tuple(packed.shape[1:]))], 0)
     cu = torch.zeros(B + 1, dtype=torch.int32, device=x_bt.device)
     cu[1:] = torch.cumsum(lengths, 0).to(torch.int32)
-    pos = ar[None, :].expand(B, T)[mask]
     if cap > total:
         pos = torch.cat([pos, pos.new_zeros(cap - total)])
     seqs = PackedSeqs(torch.ones(cap, dtype=torch.int64, device=x_bt.device), pos, cu, int(T), lengths)

@@ -239,6 +239,9 @@ class Wav2Vec2Encoder(nn.Module):
             raise ValueError("this encoder has language adapters: the batch must carry its source language id")
         feats, lengths = split_audio_batch(source)
         wav = feats[:, :, 0].float()
+        # the number of frames is asked for before the front end runs: the host then launches ahead of the device all the way
+        frames = int(self.extractor.output_lengths(torch.tensor(wav.shape[1])))
+        total = int(self.extractor.output_lengths(lengths).clamp(max=frames).sum()) if wav.is_cuda else None
         if self.freeze_extractor:
             with torch.no_grad():
                 x = self.extractor(wav)
@@ -259,7 +262,7 @@ class Wav2Vec2Encoder(nn.Module):
             x = x.masked_fill(cm.unsqueeze(1), 0.0)
         x = x * valid.unsqueeze(-1)
         x = x + self.pos_conv(x)
-        packed, seqs = pack_padded(x, out_len)
+        packed, seqs = pack_padded(x, out_len, total=total if T == frames else None)
         packed = packed.to(torch.bfloat16) if (packed.is_cuda and ops.fused_param(self.input_norm.weight)) else packed
         if not self.layer_norm_first:
             packed = self.input_norm(packed)
@@ -289,6 +292,8 @@ class WhisperEncoder(nn.Module):
 
     def forward(self, source):
         feats, lengths = split_audio_batch(source)           # [B, T, n_mels]
+        frames = (feats.shape[1] + 1) // 2
+        total = int(torch.div(lengths + 1, 2, rounding_mode="floor").clamp(max=frames).sum()) if feats.is_cuda else None      # see Wav2Vec2Encoder
         assert feats.shape[-1] == self.n_mels, "expected %d mel bins (+1 padding channel), got %d" % (self.n_mels, feats.shape[-1])
         if feats.is_cuda and ops.fused_param(self.conv1.weight) and self.n_mels % 8 == 0:
             from ..ops.conv import conv1d                       # both stem layers as GEMMs with GELU in the epilogue
@@ -301,7 +306,7 @@ class WhisperEncoder(nn.Module):
         if x.shape[1] > self.positions.shape[0]:
             self.positions = sinusoidal_table(x.shape[1], self.dim).to(x.device)
         x = x + self.positions[:x.shape[1]].to(x.dtype)
-        packed, seqs = pack_padded(x, out_len)
+        packed, seqs = pack_padded(x, out_len, total=total if x.shape[1] == frames else None)
         packed = packed.to(torch.bfloat16) if (packed.is_cuda and ops.fused_param(self.final_norm.weight)) else packed
         for layer in self.layers:
             packed = layer(packed, seqs)

@@ -396,10 +396,13 @@ class Seq2SeqBase(nn.Module):
     def decode(self, batch):
         """Gold scoring: per-sentence sum of target log-probabilities ``[B]`` and per-token scores ``[T, B]``."""
         was_training = self.training
-        self.eval()
+        switched = any(m.training for m in self.modules())      # the two walks that set the mode took a seventh of the host's time
+        if switched:
+            self.eval()
         out = self.forward(batch, compute_loss=True)
         padded = out["tgt"].pad((-out["row_loss"])[:, None]).squeeze(-1)
-        self.train(was_training)
+        if switched:
+            self.train(was_training)
         return batch.get("target_output"), padded.sum(0), padded
 
     @torch.no_grad()

@@ -277,7 +277,8 @@ class TrainEngine:
         With ``cuda_graph`` the first batch of every shape class (packed capacities, sentence count, length bounds: see
         ``data.dataset.bucket_capacity``) runs kernel by kernel and is then captured; later batches of the class replay
         the graph.  The returned tensors are overwritten by the next step."""
-        self.model.train()
+        if not all(m.training for m in self.model.modules()):
+            self.model.train()
         if not (self.use_graph and self.optim.fused) or not update:
             return self._eager_step(batch, update)
         if hasattr(self.reducer, "active"):

@@ -198,3 +198,16 @@ def test_a_model_is_copied_without_its_search_tables():
     pools.put("geometry", {"graph": threading.Lock()})          # as little to be copied as a captured graph
     assert copy.deepcopy({"_decode_pools": pools}) == {"_decode_pools": None} and pickle.loads(pickle.dumps(pools)) is None
 
+
+
+@pytest.mark.parametrize("lengths,capacity", [([3, 9, 0, 1, 20], None), ([3, 9, 0, 1, 20], 32), ([0, 0], None), ([9], 9)])
+def test_packing_with_the_total_known(lengths, capacity):
+    """The rows, their positions and their gradients are those of the packing that looks for the total itself."""
+    from nmtgminor_b200.models.layers import pack_padded
+    n = torch.tensor(lengths)
+    x = torch.randn(len(lengths), 9, 3).transpose(0, 1).contiguous().transpose(0, 1).requires_grad_(True)
+    a, sa = pack_padded(x, n, capacity)
+    b, sb = pack_padded(x, n, capacity, total=int(n.clamp(max=9).sum()))
+    assert torch.equal(a, b) and torch.equal(sa.positions, sb.positions) and torch.equal(sa.cu, sb.cu) and sa.max_len == sb.max_len
+    w = torch.randn_like(a)
+    assert torch.equal(torch.autograd.grad((a * w).sum(), x)[0], torch.autograd.grad((b * w).sum(), x)[0])
