@@ -210,7 +210,7 @@ attn_fwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           tmem_ld_wait();
           float pv[32];
           const int left = limit - c * 32;
-          if (left >= 32) {            // no per-element test
+          if (!p.causal && left >= 32) {            // no per-element test
             float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
