@@ -484,3 +484,16 @@ def test_first_product_of_a_thread_inside_a_capture():
     assert not errors, errors
     graph.replay()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 4096), (129, 264, 5001), (300, 512, 8000), (512, 1024, 4100), (900, 8, 20000)])
+def test_long_sums_of_small_outputs(M, N, K):
+    """Generator data gradients whose sum over the vocabulary is cut over the GPU: one rounding to bf16 of a 32-bit sum."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    dz = ops.empty_rows(M, K, torch.device("cuda"))
+    dz.copy_(torch.randn(M, K, device="cuda", generator=g))
+    w = torch.randn(K, N, device="cuda", generator=g).bfloat16()
+    out = ops._long_sum_gemm(dz, w)
+    want, size = dz.double() @ w.double(), dz.double().abs() @ w.double().abs()
+    assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + K ** 0.5 * 2 ** -22 * size).all()
+    assert ops.check_status() == 0
