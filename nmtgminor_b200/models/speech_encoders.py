@@ -94,9 +94,13 @@ class ConvFeatureExtractor(nn.Module):
 
 
     def _forward_gemm(self, wav):
-        """Channels-last path: the single-channel first layer stays a library convolution, every later layer is one
-        tcgen05 GEMM over overlapping rows (``ops.conv.conv1d``) with GELU in its epilogue when no norm intervenes."""
-        from ..ops.conv import conv1d
+        """Channels-last path.  Without gradients ``ops.conv.frozen_front_end`` takes the layers that it can; else the
+        single-channel first layer stays a library convolution and every later layer is one tcgen05 GEMM over overlapping rows (``ops.conv.conv1d``) with GELU in its epilogue when no norm intervenes."""
+        from ..ops.conv import conv1d, frozen_front_end
+        if self.mode == "layer_norm":
+            x = frozen_front_end(wav, self.convs, self.norms)
+            if x is not None:
+                return x.float()
         conv, norm = self.convs[0], self.norms[0]
         x = F.conv1d(wav.unsqueeze(1).to(conv.weight.dtype), conv.weight, conv.bias, stride=conv.stride[0])
         if isinstance(norm, nn.LayerNorm):

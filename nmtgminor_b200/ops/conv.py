@@ -135,3 +135,62 @@ def conv1d(x, weight, bias=None, stride: int = 1, act: str = "none", padding: in
         gw = gb = None
     return _Conv1dFn.apply(xin, weight.work, bias.work if bias is not None else None, gw, gb, int(stride), act_id,
                            bool(x.requires_grad and torch.is_grad_enabled()))
+
+
+def _front_end_layer(i, conv, norm, channels: int, device) -> bool:
+    """Whether layer ``i`` is of the kind that the kernels of csrc/frontend.cu take."""
+    if not (type(conv) is torch.nn.Conv1d and type(norm) is torch.nn.LayerNorm and tuple(norm.normalized_shape) == (channels,)
+            and norm.weight is not None and norm.bias is not None and not (norm._forward_hooks or norm._forward_pre_hooks)):
+        return False
+    w = conv.weight
+    if not all(p.dtype == torch.float32 and p.device == device for p in (norm.weight, norm.bias, w)):
+        return False
+    if conv.out_channels != channels or conv.groups != 1 or conv.dilation != (1,) or conv.padding != (0,):
+        return False
+    if i == 0:
+        return conv.in_channels == 1 and conv.kernel_size[0] <= 16 and conv.stride[0] <= 64
+    return conv.in_channels == channels and fused_param(w) and (conv.bias is None or fused_param(conv.bias))
+
+
+def frozen_front_end(wav, convs, norms):
+    """Strided convolutions over ``wav`` [B, samples], LayerNorm over the channels and GELU behind each, without gradients: ``[B, T, C]``
+    (bf16).  The first convolution, every norm and every GELU run in the kernels of csrc/frontend.cu, which leave their frames where the
+    next convolution's overlapping rows are read.  None for layers that these do not take (256 or 512 channels as one or two 16-byte
+    vectors a lane) and under the tracers and modes that have to see tensor operations."""
+    C = convs[0].out_channels
+    if (torch.is_grad_enabled() or torch.is_autocast_enabled() or type(wav) is not torch.Tensor or not wav.is_cuda or wav.dim() != 2
+            or wav.shape[0] == 0 or C not in (256, 512) or _OVERLAP_OK[0] is False or torch.autograd.forward_ad._current_level >= 0
+            or torch.nn.modules.module._has_any_global_hook()):
+        return None
+    T = wav.shape[1]
+    for i, (conv, norm) in enumerate(zip(convs, norms)):
+        if not _front_end_layer(i, conv, norm, C, wav.device) or T < conv.kernel_size[0]:
+            return None
+        T = (T - conv.kernel_size[0]) // conv.stride[0] + 1
+    B, T = wav.shape
+    for i, (conv, norm) in enumerate(zip(convs, norms)):
+        k, s = conv.kernel_size[0], conv.stride[0]
+        T = (T - k) // s + 1
+        # rows for the next convolution: whole strides of every utterance, and the overhang of the last one's frames.  Those past T are
+        # never read by a frame that is kept
+        nk, ns = (convs[i + 1].kernel_size[0], convs[i + 1].stride[0]) if i + 1 < len(convs) else (0, 1)
+        rows = -(-T // ns) * ns
+        out = torch.empty((B * rows + nk, C), dtype=torch.bfloat16, device=wav.device)
+        affine = (norm.weight.detach().contiguous(), norm.bias.detach().contiguous(), norm.eps)
+        if i == 0:
+            bias = conv.bias.detach().float() if conv.bias is not None else None
+            ext().conv_norm_gelu(wav.detach().float().contiguous(), conv.weight.detach().contiguous(), bias, *affine, out, rows, T, s)
+        else:
+            y = empty_rows(B * had // s, C, wav.device)
+            taps = conv.weight.work.permute(0, 2, 1).reshape(C, k * C).contiguous()
+            try:
+                gemm(_overlap_view(buf, y.shape[0], k, s, C), taps, y, bias=conv.bias.work if conv.bias is not None else None)
+                _OVERLAP_OK[0] = True
+            except RuntimeError as exc:
+                if "cuTensorMapEncodeTiled" not in str(exc):
+                    raise
+                _OVERLAP_OK[0] = False
+                return None
+            ext().norm_gelu(y, B, had // s, *affine, out, rows, T)
+        buf, had = out, rows
+    return buf[:B * had].view(B, had, C)

@@ -34,6 +34,34 @@ const long* off_ptr(const OptTensor& t) {
   return reinterpret_cast<const long*>(t->data_ptr<int64_t>());
 }
 
+// LayerNorm + GELU of the convolution of wav [B, samples] with w [C, 1, taps]; out: at least B * out_rows rows [.., C]
+void conv_norm_gelu(const Tensor& wav, const Tensor& w, const OptTensor& bias, const Tensor& gamma, const Tensor& beta, double eps, Tensor& out,
+                    int64_t out_rows, int64_t T, int64_t stride) {
+  TORCH_CHECK(wav.is_cuda() && wav.scalar_type() == at::kFloat && wav.dim() == 2 && wav.stride(1) == 1, "wav must be fp32 rows");
+  need(w, at::kFloat, "w"); need(gamma, at::kFloat, "gamma"); need(beta, at::kFloat, "beta"); need(out, at::kBFloat16, "out");
+  if (bias.has_value()) need(*bias, at::kFloat, "bias");
+  const int64_t C = out.size(-1), taps = w.numel() / C;
+  TORCH_CHECK(w.numel() == C * taps && gamma.numel() == C && beta.numel() == C && (!bias.has_value() || bias->numel() == C));
+  TORCH_CHECK(out.numel() >= wav.size(0) * out_rows * C && T <= out_rows && (reinterpret_cast<uintptr_t>(out.data_ptr()) & 15) == 0);
+  c10::cuda::CUDAGuard guard(wav.device());
+  ck(nmtg_conv_norm_gelu(wav.data_ptr<float>(), wav.stride(0), w.data_ptr<float>(), bias.has_value() ? bias->data_ptr<float>() : nullptr,
+                         gamma.data_ptr<float>(), beta.data_ptr<float>(), static_cast<float>(eps), out.data_ptr(), static_cast<int>(wav.size(0)),
+                         static_cast<int>(wav.size(1)), static_cast<int>(T), static_cast<int>(out_rows), static_cast<int>(C),
+                         static_cast<int>(taps), static_cast<int>(stride), cur_stream()));
+}
+
+// LayerNorm + GELU of the first T of the in_rows rows of every utterance
+void norm_gelu(const Tensor& x, int64_t B, int64_t in_rows, const Tensor& gamma, const Tensor& beta, double eps, Tensor& out, int64_t out_rows,
+               int64_t T) {
+  need(x, at::kBFloat16, "x"); need(gamma, at::kFloat, "gamma"); need(beta, at::kFloat, "beta"); need(out, at::kBFloat16, "out");
+  const int64_t C = x.size(-1);
+  TORCH_CHECK(out.size(-1) == C && gamma.numel() == C && beta.numel() == C && x.numel() >= B * in_rows * C && out.numel() >= B * out_rows * C);
+  TORCH_CHECK(((reinterpret_cast<uintptr_t>(out.data_ptr()) | reinterpret_cast<uintptr_t>(x.data_ptr())) & 15) == 0);
+  c10::cuda::CUDAGuard guard(x.device());
+  ck(nmtg_norm_gelu(x.data_ptr(), gamma.data_ptr<float>(), beta.data_ptr<float>(), static_cast<float>(eps), out.data_ptr(), static_cast<int>(B),
+                    static_cast<int>(T), static_cast<int>(in_rows), static_cast<int>(out_rows), static_cast<int>(C), cur_stream()));
+}
+
 Tensor joint_fwd(const Tensor& f, const Tensor& g, const Tensor& f_len, const Tensor& g_len, const OptTensor& batch_offset,
                  int64_t packed_rows, bool relu, double p, int64_t seed, int64_t stream_id) {
   TORCH_CHECK(f.is_cuda() && f.is_contiguous() && g.is_contiguous() && f.dim() == 3 && g.dim() == 3);
@@ -362,6 +390,8 @@ void bind_sequence_ops(pybind11::module& m) {
   m.def("softmax_dropout_fwd", &softmax_dropout_fwd);
   m.def("softmax_dropout_bwd", &softmax_dropout_bwd);
   m.def("beam_topk", &beam_topk);
+  m.def("conv_norm_gelu", &conv_norm_gelu);
+  m.def("norm_gelu", &norm_gelu);
   namespace py = pybind11;
   m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("dst"), py::arg("index"), py::arg("copy_elems"));
   m.def("decode_attn", &decode_attn, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("lengths"), py::arg("len"),

@@ -7,6 +7,14 @@
 
 extern "C" {
 
+// ---- front end of raw audio, without gradients (frontend.cu): 256 or 512 channels, rows of utterance b at b * out_rows ----------
+// wav fp32 [B, samples] (row stride wav_stride), w fp32 [channels][taps], bias optional; out bf16 frames t < T
+const char* nmtg_conv_norm_gelu(const float* wav, long wav_stride, const float* w, const float* bias, const float* gamma, const float* beta,
+                                float eps, void* out, int B, int samples, int T, int out_rows, int channels, int taps, int stride,
+                                cudaStream_t stream);
+const char* nmtg_norm_gelu(const void* x, const float* gamma, const float* beta, float eps, void* out, int B, int T, int in_rows, int out_rows,
+                           int channels, cudaStream_t stream);
+
 // ---- transducer joint: h[b,t,u,:] = act(f[b,t,:] + g[b,u,:]) ------------------------------------------------
 // dtype: 0 = fp32, 1 = bf16.  packed: rows of sentence b start at (b ? batch_offset[b-1] : 0) and are laid
 // out [t][u] with u running over g_len[b]; dense: [B, T, U, H] with rows outside the lengths zeroed.

@@ -1,6 +1,7 @@
 """Convolution-as-GEMM (overlapping-row TMA view) against F.conv1d."""
 import pytest
 import torch
+import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,56 @@ def test_feature_extractor_gemm_path_matches_library_path():
         got = fe(wav)
         assert got.shape == want.shape
         assert (got.float() - want).abs().max().item() / want.abs().max().item() < 5e-2
+
+
+@pytest.mark.parametrize("channels,taps,stride,B,samples,bias", [(256, 1, 1, 1, 1, True), (512, 10, 5, 1, 10, False), (512, 10, 5, 3, 2347, True),
+                                                                 (256, 16, 64, 2, 1105, False), (512, 3, 2, 5, 64, True)])
+def test_front_end_kernels(channels, taps, stride, B, samples, bias):
+    """Convolution + LayerNorm + GELU and LayerNorm + GELU against 64 bits: results differ by their rounding to the
+    8 significant bits of bf16 (at most 2^-8 of the value) and by the 32-bit
+    sums, whose error in a unit-variance row stays below 2^-23 * (taps + channels) over the deviation of the row."""
+    g = torch.Generator().manual_seed(taps * channels + samples)
+    rand = lambda *s: torch.randn(*s, generator=g).cuda()
+    wav, w, b = rand(B, samples), rand(channels, 1, taps), rand(channels) if bias else None
+    norm = torch.nn.LayerNorm(channels).cuda()
+    with torch.no_grad():
+        norm.weight.copy_(1 + 0.2 * rand(channels))
+        norm.bias.copy_(0.3 * rand(channels))
+    T = (samples - taps) // stride + 1
+    rows = T + 3
+
+    def want(y):
+        return F.gelu(F.layer_norm(y, (channels,), norm.weight.double(), norm.bias.double(), norm.eps))
+
+    def check(got, ref):
+        error = (got.double() - ref).abs()
+        assert (error <= ref.abs() * 2 ** -8 + 2 ** -23 * (taps + channels) * 8).all(), error.max()
+    out = torch.full((B * rows, channels), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.ext().conv_norm_gelu(wav, w, b, norm.weight, norm.bias, norm.eps, out, rows, T, stride)
+    check(out.view(B, rows, channels)[:, :T], want(F.conv1d(wav.double().unsqueeze(1), w.double(), None if b is None else b.double(), stride=stride)
+                                                   .transpose(1, 2)))
+    assert (out.view(B, rows, channels)[:, T:] == 7).all()
+    x, then = rand(B * rows, channels).bfloat16(), torch.full_like(out[:B * (T + 1)], 7.0)
+    ops.ext().norm_gelu(x, B, rows, norm.weight, norm.bias, norm.eps, then, T + 1, T)
+    check(then.view(B, T + 1, channels)[:, :T], want(x.view(B, rows, channels)[:, :T].double()))
+    assert (then.view(B, T + 1, channels)[:, T:] == 7).all()
+
+
+@pytest.mark.parametrize("samples", [400, 719, 4001])
+@pytest.mark.parametrize("conv_bias", [False, True])
+def test_frozen_front_end_matches_the_general_path(samples, conv_bias):
+    """The same layers with and without gradients; strides 5, 2, 2, 3 leave tails of every length behind an utterance."""
+    from nmtgminor_b200.models.speech_encoders import ConvFeatureExtractor
+    torch.manual_seed(samples)
+    fe = ConvFeatureExtractor([(256, 10, 5), (256, 3, 2), (256, 2, 2), (256, 4, 3)], conv_bias=conv_bias).cuda()
+    FlatParameterStore(fe, "cuda")
+    wav = torch.randn(3, samples + 8, device="cuda")[:, 3:3 + samples]
+    want = fe(wav)
+    with torch.no_grad():
+        assert C.frozen_front_end(wav, fe.convs, fe.norms) is not None
+        got = fe(wav)
+    assert got.shape == want.shape and got.dtype == want.dtype
+    assert (got - want).abs().max().item() / want.abs().max().item() < 5e-2
+    fe.norms[0].register_forward_hook(lambda *a: None)           # a hook that has to be called
+    with torch.no_grad():
+        assert C.frozen_front_end(wav, fe.convs, fe.norms) is None
