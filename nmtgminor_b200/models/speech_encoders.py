@@ -95,7 +95,8 @@ class ConvFeatureExtractor(nn.Module):
 
     def _forward_gemm(self, wav):
         """Channels-last path.  Without gradients ``ops.conv.frozen_front_end`` takes the layers that it can; else the
-        single-channel first layer stays a library convolution and every later layer is one tcgen05 GEMM over overlapping rows (``ops.conv.conv1d``) with GELU in its epilogue when no norm intervenes."""
+        single-channel first layer stays a library convolution and every later layer is one tcgen05 GEMM over overlapping
+        rows (``ops.conv.conv1d``) with GELU in its epilogue when no norm intervenes."""
         from ..ops.conv import conv1d, frozen_front_end
         if self.mode == "layer_norm":
             x = frozen_front_end(wav, self.convs, self.norms)
@@ -129,7 +130,9 @@ class ConvPositionalEmbedding(nn.Module):
         self.trim = 1 if kernel % 2 == 0 else 0
 
     def forward(self, x_bt):          # [B, T, C]
-        y = self.conv(x_bt.transpose(1, 2))
+        from ..ops.conv import weight_normed
+        w = weight_normed(self.conv)
+        y = self.conv(x_bt.transpose(1, 2)) if w is None else self.conv._conv_forward(x_bt.transpose(1, 2), w, self.conv.bias)
         if self.trim:
             y = y[:, :, :-self.trim]
         return F.gelu(y).transpose(1, 2)

@@ -137,10 +137,20 @@ def conv1d(x, weight, bias=None, stride: int = 1, act: str = "none", padding: in
                            bool(x.requires_grad and torch.is_grad_enabled()))
 
 
+def _watched() -> bool:
+    """Whether a mode or a hook of all modules has to see the tensor operations that a kernel would replace."""
+    return (torch.is_autocast_enabled() or torch.jit.is_tracing() or torch._C._are_functorch_transforms_active()
+            or torch.autograd.forward_ad._current_level >= 0 or torch.nn.modules.module._has_any_global_hook())
+
+
+def _hooked(*modules) -> bool:
+    return any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in modules)
+
+
 def _front_end_layer(i, conv, norm, channels: int, device) -> bool:
     """Whether layer ``i`` is of the kind that the kernels of csrc/frontend.cu take."""
     if not (type(conv) is torch.nn.Conv1d and type(norm) is torch.nn.LayerNorm and tuple(norm.normalized_shape) == (channels,)
-            and norm.weight is not None and norm.bias is not None and not (norm._forward_hooks or norm._forward_pre_hooks)):
+            and norm.weight is not None and norm.bias is not None and not _hooked(norm)):
         return False
     w = conv.weight
     if not all(p.dtype == torch.float32 and p.device == device for p in (norm.weight, norm.bias, w)):
@@ -158,9 +168,8 @@ def frozen_front_end(wav, convs, norms):
     next convolution's overlapping rows are read.  None for layers that these do not take (256 or 512 channels as one or two 16-byte
     vectors a lane) and under the tracers and modes that have to see tensor operations."""
     C = convs[0].out_channels
-    if (torch.is_grad_enabled() or torch.is_autocast_enabled() or type(wav) is not torch.Tensor or not wav.is_cuda or wav.dim() != 2
-            or wav.shape[0] == 0 or C not in (256, 512) or _OVERLAP_OK[0] is False or torch.autograd.forward_ad._current_level >= 0
-            or torch.nn.modules.module._has_any_global_hook()):
+    if (torch.is_grad_enabled() or _watched() or type(wav) is not torch.Tensor or not wav.is_cuda or wav.dim() != 2 or wav.shape[0] == 0
+            or C not in (256, 512) or _OVERLAP_OK[0] is False):
         return None
     T = wav.shape[1]
     for i, (conv, norm) in enumerate(zip(convs, norms)):
@@ -194,3 +203,43 @@ def frozen_front_end(wav, convs, norms):
             ext().norm_gelu(y, B, had // s, *affine, out, rows, T)
         buf, had = out, rows
     return buf[:B * had].view(B, had, C)
+
+
+class _WeightNormFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, v, gain):
+        w, norm = ext().weight_norm_fwd(v, gain)
+        ctx.save_for_backward(v, gain, norm)
+        return w
+
+    @staticmethod
+    def backward(ctx, dw):
+        v, gain, norm = ctx.saved_tensors
+        if torch.is_grad_enabled():          # a graph of the gradient is wanted: the same as differentiable operations
+            dims = tuple(range(v.dim() - 1))
+            n = v.square().sum(dims, keepdim=True).sqrt()
+            dot = (dw * v).sum(dims, keepdim=True)
+            return (gain / n) * (dw - v * (dot / n.square())), (dot / n).view_as(gain)
+        dw = dw.contiguous()
+        if dw.data_ptr() % 16:
+            dw = dw.clone()
+        return ext().weight_norm_bwd(dw, v, gain, norm)
+
+
+def weight_normed(conv):
+    """Weight of a convolution under ``parametrizations.weight_norm(conv, dim=last)`` from the kernels of csrc/weight_norm.cu; None where
+    something else parametrises it, or a form, mode or tracer needs the tensor operations."""
+    from torch.nn.utils import parametrizations, parametrize
+    chain = getattr(conv, "parametrizations", None)
+    if chain is None or set(chain.keys()) != {"weight"} or len(chain.weight) != 1 or parametrize._cache_enabled:
+        return None
+    norm, gain, v = chain.weight[0], chain.weight.original0, chain.weight.original1
+    if type(norm) is not parametrizations._WeightNorm or norm.dim not in (v.dim() - 1, -1):
+        return None
+    lanes = v.shape[-1] // 4
+    if (_watched() or _hooked(conv, norm, chain.weight)
+            or not all(type(p) in (torch.Tensor, torch.nn.Parameter) and p.is_cuda and p.dtype == torch.float32 and p.is_contiguous()
+                       and p.data_ptr() % 16 == 0 for p in (v, gain))
+            or v.device != gain.device or gain.numel() != v.shape[-1] or v.numel() == 0 or v.shape[-1] % 4 or lanes > 256 or lanes & (lanes - 1)):
+        return None
+    return _WeightNormFn.apply(v, gain)

@@ -62,6 +62,34 @@ void norm_gelu(const Tensor& x, int64_t B, int64_t in_rows, const Tensor& gamma,
                     static_cast<int>(T), static_cast<int>(in_rows), static_cast<int>(out_rows), static_cast<int>(C), cur_stream()));
 }
 
+constexpr int kNormTable = 512;      // rows of partial sums: blocks at most
+
+void need_aligned(const Tensor& t, const char* what) {
+  need(t, at::kFloat, what);
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, what, " must start on a 16-byte boundary");
+}
+// v [.., cols], gain of cols elements -> (w as v, norm [cols])
+std::tuple<Tensor, Tensor> weight_norm_fwd(const Tensor& v, const Tensor& gain) {
+  need_aligned(v, "v"); need_aligned(gain, "gain");
+  const int64_t cols = v.size(-1);
+  TORCH_CHECK(gain.numel() == cols);
+  c10::cuda::CUDAGuard guard(v.device());
+  Tensor w = at::empty_like(v), norm = at::empty({cols}, v.options()), table = at::empty({kNormTable, cols}, v.options());
+  ck(nmtg_weight_norm(v.data_ptr<float>(), gain.data_ptr<float>(), w.data_ptr<float>(), norm.data_ptr<float>(), table.data_ptr<float>(), kNormTable,
+                      v.numel() / cols, static_cast<int>(cols), cur_stream()));
+  return {w, norm};
+}
+std::tuple<Tensor, Tensor> weight_norm_bwd(const Tensor& dw, const Tensor& v, const Tensor& gain, const Tensor& norm) {
+  need_aligned(dw, "dw"); need_aligned(v, "v"); need_aligned(gain, "gain"); need_aligned(norm, "norm");
+  const int64_t cols = v.size(-1);
+  TORCH_CHECK(dw.sizes() == v.sizes() && gain.numel() == cols && norm.numel() == cols);
+  c10::cuda::CUDAGuard guard(v.device());
+  Tensor dv = at::empty_like(v), dg = at::empty_like(gain), table = at::empty({kNormTable, cols}, v.options());
+  ck(nmtg_weight_norm_bwd(dw.data_ptr<float>(), v.data_ptr<float>(), gain.data_ptr<float>(), norm.data_ptr<float>(), dv.data_ptr<float>(),
+                          dg.data_ptr<float>(), table.data_ptr<float>(), kNormTable, v.numel() / cols, static_cast<int>(cols), cur_stream()));
+  return {dv, dg};
+}
+
 Tensor joint_fwd(const Tensor& f, const Tensor& g, const Tensor& f_len, const Tensor& g_len, const OptTensor& batch_offset,
                  int64_t packed_rows, bool relu, double p, int64_t seed, int64_t stream_id) {
   TORCH_CHECK(f.is_cuda() && f.is_contiguous() && g.is_contiguous() && f.dim() == 3 && g.dim() == 3);
@@ -392,6 +420,8 @@ void bind_sequence_ops(pybind11::module& m) {
   m.def("beam_topk", &beam_topk);
   m.def("conv_norm_gelu", &conv_norm_gelu);
   m.def("norm_gelu", &norm_gelu);
+  m.def("weight_norm_fwd", &weight_norm_fwd);
+  m.def("weight_norm_bwd", &weight_norm_bwd);
   namespace py = pybind11;
   m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("dst"), py::arg("index"), py::arg("copy_elems"));
   m.def("decode_attn", &decode_attn, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("lengths"), py::arg("len"),

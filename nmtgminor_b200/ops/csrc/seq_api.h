@@ -15,6 +15,13 @@ const char* nmtg_conv_norm_gelu(const float* wav, long wav_stride, const float* 
 const char* nmtg_norm_gelu(const void* x, const float* gamma, const float* beta, float eps, void* out, int B, int T, int in_rows, int out_rows,
                            int channels, cudaStream_t stream);
 
+// ---- weight normalisation of the columns of v fp32 [rows, cols], cols / 4 a power of two up to 256 (weight_norm.cu) ----------------
+// table: fp32 [table_rows, cols] of partial sums; norm [cols] is kept for the gradient; all pointers 16-byte aligned
+const char* nmtg_weight_norm(const float* v, const float* gain, float* w, float* norm, float* table, int table_rows, long rows, int cols,
+                             cudaStream_t stream);
+const char* nmtg_weight_norm_bwd(const float* dw, const float* v, const float* gain, const float* norm, float* dv, float* dg, float* table,
+                                 int table_rows, long rows, int cols, cudaStream_t stream);
+
 // ---- transducer joint: h[b,t,u,:] = act(f[b,t,:] + g[b,u,:]) ------------------------------------------------
 // dtype: 0 = fp32, 1 = bf16.  packed: rows of sentence b start at (b ? batch_offset[b-1] : 0) and are laid
 // out [t][u] with u running over g_len[b]; dense: [B, T, U, H] with rows outside the lengths zeroed.

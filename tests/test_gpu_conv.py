@@ -106,3 +106,31 @@ def test_frozen_front_end_matches_the_general_path(samples, conv_bias):
     fe.norms[0].register_forward_hook(lambda *a: None)           # a hook that has to be called
     with torch.no_grad():
         assert C.frozen_front_end(wav, fe.convs, fe.norms) is None
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 4), (3, 5, 8), (48, 3, 128), (1024, 64, 128), (2, 7, 1024)])
+def test_weight_norm_kernels(shape):
+    """Weight and gradients against 64 bits; the columns' sums are of rows = shape[0] * shape[1] products in 32 bits, whose error stays below
+    2^-24 * rows times the sum of their sizes."""
+    torch.manual_seed(shape[0])
+    conv = torch.nn.utils.parametrizations.weight_norm(torch.nn.Conv1d(shape[1], shape[0], shape[2]).cuda(), dim=2)
+    gain, v = conv.parametrizations.weight.original0, conv.parametrizations.weight.original1
+    with torch.no_grad():
+        gain.mul_(1 + 0.3 * torch.randn_like(gain))
+    w = C.weight_normed(conv)
+    dw = torch.randn_like(w)
+    dv, dg = torch.autograd.grad(w, (v, gain), dw, retain_graph=True)
+    vd, gd = v.detach().double().requires_grad_(), gain.detach().double().requires_grad_()
+    n = vd.square().sum((0, 1), keepdim=True).sqrt()
+    want = vd * (gd / n)
+    wv, wg = torch.autograd.grad(want, (vd, gd), dw.double())
+    part = 2 ** -24 * (shape[0] * shape[1] + 8)
+    size = (dw.double() * vd).abs().sum((0, 1), keepdim=True) / n       # what the terms of dg add up to without their signs
+    assert ((w - want).abs() <= part * want.abs()).all()
+    assert ((dg - wg).abs() <= 2 * part * size).all()
+    assert ((dv - wv).abs() <= 2 * part * (gd / n).abs() * (dw.abs() + vd.abs() * size / n)).all()
+    # a second derivative: the gradient as differentiable operations
+    dv2, dg2 = torch.autograd.grad(w, (v, gain), dw, create_graph=True)
+    assert dv2.requires_grad and torch.allclose(dv2, dv, rtol=1e-4, atol=1e-5) and torch.allclose(dg2, dg, rtol=1e-4, atol=1e-4)
+    conv.register_forward_hook(lambda *a: None)
+    assert C.weight_normed(conv) is None
