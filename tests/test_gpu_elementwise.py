@@ -42,6 +42,31 @@ def test_layernorm_fwd_bwd(rows, hidden):
     _close(dbeta, bf.grad, 0.02 * math.sqrt(rows) + 0.05, 2e-2, "ln dbeta")
 
 
+@pytest.mark.parametrize("rows,hidden,residual", [(511, 1024, True), (512, 8, False), (517, 264, True), (2500, 512, False), (2369, 1000, True),
+                                                  (2073, 1280, True), (1, 1288, False), (3000, 2040, True), (9000, 256, True)])
+def test_layernorm_bwd_of_many_rows(rows, hidden, residual):
+    """Gradients against 64 bits: dx differs by its rounding to 8 significant bits and by 32-bit sums of `hidden` terms, the affine gradients by
+    those of `rows` terms in any order (2^-24 a term of what the terms add up to without their signs, a few roundings more in each)."""
+    g = torch.Generator().manual_seed(rows + hidden)
+    rand = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    x, dy, gamma = (rand(rows, hidden) * 2 + 0.5).bfloat16(), rand(rows, hidden).bfloat16(), (1 + 0.2 * rand(hidden)).bfloat16()
+    dres = rand(rows, hidden).bfloat16() if residual else None
+    xd, d = x.double(), dy.double()
+    mean, rstd = xd.mean(-1).float(), (xd.var(-1, unbiased=False) + 1e-5).rsqrt().float()
+    xh = (xd - mean.double()[:, None]) * rstd.double()[:, None]
+    t = d * gamma.double()
+    want = rstd.double()[:, None] * (t - t.mean(-1, keepdim=True) - xh * (t * xh).mean(-1, keepdim=True))
+    if residual:
+        want = want + dres.double()
+    dgamma, dbeta = torch.ones(hidden, device=DEV), torch.ones(hidden, device=DEV)
+    dx = ops.ext().layernorm_bwd(dy, x, mean, rstd, gamma, dres, dgamma, dbeta)
+    part = 2 ** -24 * (hidden + 32)
+    size = rstd.double()[:, None] * (t.abs() + t.abs().mean(-1, keepdim=True) + xh.abs() * (t * xh).abs().mean(-1, keepdim=True))
+    assert ((dx.double() - want).abs() <= 2 ** -8 * want.abs() + 2 * part * size).all()
+    for got, terms in ((dgamma, d * xh), (dbeta, d)):
+        assert ((got.double() - 1 - terms.sum(0)).abs() <= 2 ** -24 * (rows + 32) * (1 + terms.abs().sum(0))).all()
+
+
 @pytest.mark.parametrize("rows,vocab", [(64, 8000), (129, 32000), (16, 51865 + 7), (8, 250056)])
 @pytest.mark.parametrize("smoothing", [0.0, 0.1])
 def test_xent_fused(rows, vocab, smoothing):
