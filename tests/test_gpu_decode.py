@@ -201,7 +201,7 @@ def test_step_attention_tiles(K, pos):
         assert (out[b * K:(b + 1) * K].double() - want).abs().max() < 2 ** -8 * want.abs().max()
 
 
-def _compare_searches(dtype, B, K, V, T, min_len, normalize, alpha, end_bias=None):
+def _compare_searches(dtype, B, K, V, T, min_len, normalize, alpha, end_bias=None, open_words=None):
     from types import SimpleNamespace
 
     from nmtgminor_b200.inference import beam_search as bs
@@ -217,6 +217,10 @@ def _compare_searches(dtype, B, K, V, T, min_len, normalize, alpha, end_bias=Non
         by_word[torch.arange(V), torch.randint(4, V, (V,), generator=h)] += 6
         by_step[:4, 3], by_step[4:, 3] = 0.0, by_step[4:, 3] + 12
         by_word, by_step = by_word.cuda(), by_step.cuda()
+    if open_words is not None:                             # all other words are impossible
+        closed = torch.ones(ld, dtype=torch.bool, device="cuda")
+        closed[open_words] = False
+        by_word[:, closed] = float("-inf")
     logits_of = lambda tok, step: (by_word[tok] + by_step[step]).to(dtype)[:, :V]
     lens = torch.randint(2, 9, (B,), device="cuda", generator=g)
 
@@ -261,6 +265,14 @@ def _compare_searches(dtype, B, K, V, T, min_len, normalize, alpha, end_bias=Non
 def test_device_search_matches_host_bookkeeping(dtype, B, K, V, T, min_len, normalize):
     """The step kernels against the tensor statements of the same search, on logits that depend on the last word and the step."""
     _compare_searches(dtype, B, K, V, T, min_len, normalize, 0.6 if normalize else 0.0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K,V,count", [(1, 4096, 4), (4, 9000, 12), (4, 13000, 60), (16, 9000, 40)])
+def test_device_search_among_few_possible_words(dtype, K, V, count):
+    """Pieces of the vocabulary without a possible word, and warps with fewer of them than are wanted."""
+    words = torch.cat([torch.tensor([3]), torch.linspace(4, V - 1, count).long()])
+    _compare_searches(dtype, 3, K, V, 8, 1, False, 0.0, open_words=words.cuda())
 
 
 def test_steps_of_very_many_rows():
