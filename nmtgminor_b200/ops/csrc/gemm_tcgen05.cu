@@ -547,18 +547,25 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   const int sms = gemm_sms();
   const int num_kb = (d->K + BK - 1) / BK;
   // ---- skinny problems (incremental decoding: a few hundred rows): the weight matrix is streamed once, so the
-  // only lever is the number of CTAs pulling it in; take the widest tile that still gives every SM a tile,
-  // down to 64 columns
+  // only lever is the number of CTAs pulling it in: the narrowest tiles that are one wave (us, two waves of 64 columns / one of 128:
+  // 256 x 8192 x 1024 14.5 / 10.5, 128 x 12288 x 4096 39.6 / 25.5; two of 128 / one of 256: 300 x 12288 x 4096 45.8 / 36.4), else the widest
   const bool skinny = g_gemm_variant == 0 && d->M <= 512 && !d->out_fp32 && d->force_bn == 0 && d->split_k <= 1 && !d->colsum;
   if (skinny) {
     const bool gathered = d->gather != nullptr;
     if (gathered) { const char* e = gather_first(); if (e) return e; }
     if (skinny_takes(d, sms)) return launch_gemm_skinny(d, sms, !gathered, stream);
     const int num_m = (d->M + BM - 1) / BM;
-    int bn = 64;
-    if (static_cast<long>(num_m) * ((d->N + 255) / 256) >= sms) bn = 256;
-    else if (static_cast<long>(num_m) * ((d->N + 127) / 128) >= sms) bn = 128;
+    auto tiles_of = [&](int w) { return static_cast<long>(num_m) * ((d->N + w - 1) / w); };
+    const int bn = tiles_of(64) <= sms ? 64 : tiles_of(128) <= sms ? 128 : 256;
     a.split_k = 1;
+    // Where 128 columns are more than one wave, the 256-row tiles of the CTA-pair kernel read every weight once instead of once per 128 rows
+    // (us, here / pairs: 256 x 32000 x 1024 25.6 / 20.5, 256 x 250056 x 1024 157 / 129, 512 x 32000 x 512 29.6 / 21.5, 400 x 6144 x 2048
+    // 25.9 / 17.2).  Not with an odd number of 128-row halves beyond one wave of pairs (320 x 250056 x 1024 199 / 208), nor with a second
+    // wave of a few tiles (400 x 10000 x 512 15.3 / 16.7); in one wave the narrow tiles are sooner done (256 x 4096 x 1024 8.9 / 11.8).
+    if (d->M > BM && tiles_of(128) > sms) {
+      const long pairs = static_cast<long>((num_m + 1) / 2) * ((d->N + 255) / 256), clusters = sms / 2;
+      if (pairs <= clusters || (num_m % 2 == 0 && (pairs > 2 * clusters || 4 * pairs >= 5 * clusters))) return launch_gemm_pair(d, a, 256, stream);
+    }
     CUtensorMap ta, tb;
     bool ok;
     if (!d->a_mn_major) ok = cached_tmap(&ta, d->a, d->M, d->K, d->lda, BM, BK);
@@ -567,8 +574,7 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
     if (!d->b_mn_major) ok = cached_tmap(&tb, d->b, d->N, d->K, d->ldb, bn, BK);
     else ok = cached_tmap(&tb, d->b, d->K, d->N, d->ldb, BK, 64);
     if (!ok) return "gemm: cuTensorMapEncodeTiled failed for B";
-    const long tiles = static_cast<long>(num_m) * ((d->N + bn - 1) / bn);
-    const int grid = static_cast<int>(tiles < sms ? tiles : sms);
+    const int grid = static_cast<int>(tiles_of(bn) < sms ? tiles_of(bn) : sms);
     // decoding steps are latency bound: short specialised epilogues (see gemm_common.cuh) for their two shapes
     constexpr uint32_t kLinear = kEpiBf16 | kEpiBias | kEpiRes;
     constexpr uint32_t kActivated = kEpiBf16 | kEpiBias | kEpiActFwd;

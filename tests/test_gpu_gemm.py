@@ -497,3 +497,35 @@ def test_long_sums_of_small_outputs(M, N, K):
     want, size = dz.double() @ w.double(), dz.double().abs() @ w.double().abs()
     assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + K ** 0.5 * 2 ** -22 * size).all()
     assert ops.check_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 4744, 72), (129, 9544, 64), (257, 6400, 136), (300, 12288, 64), (512, 9984, 64), (512, 12003, 200),
+                                   (100, 20000, 80), (256, 51865, 64)])
+@pytest.mark.parametrize("epilogue", ["plain", "residual", "gelu"])
+def test_wide_outputs_of_few_rows(M, N, K, epilogue):
+    """Up to 512 rows on either side of every line between the tile widths and the CTA pairs: one rounding to bf16 of a 32-bit sum, and the
+    sum itself the same whatever the tiles are."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, w, b = rnd(M, K).bfloat16(), (rnd(N, K) * K ** -0.5).bfloat16(), rnd(N).bfloat16()
+    kw, want = {}, x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T + 1
+    if epilogue != "plain":
+        kw["bias"], want, size = b, want + b.double(), size + b.double().abs()
+    if epilogue == "residual":
+        kw["residual"] = ops.empty_rows(M, N, x.device)
+        kw["residual"].copy_(rnd(M, N))
+        want, size = want + kw["residual"].double(), size + kw["residual"].double().abs()
+    if epilogue == "gelu":
+        kw["act"], want = 2, torch.nn.functional.gelu(want)
+    outs = []
+    try:
+        for variant in (0, 1):
+            ops.ext().set_gemm_variant(variant)
+            outs.append(ops.empty_rows(M, N, x.device))
+            ops.gemm(x, w, outs[-1], **kw)
+    finally:
+        ops.ext().set_gemm_variant(0)
+    assert ((outs[0].double() - want).abs() <= 2 ** -8 * want.abs() + K ** 0.5 * 2 ** -22 * size).all()
+    assert torch.equal(*outs)
+    assert ops.check_status() == 0
