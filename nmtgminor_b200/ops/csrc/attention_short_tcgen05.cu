@@ -20,6 +20,7 @@
 // Same numerics, dropout counters and interfaces as the general kernels in attention_tcgen05.cu.
 #include "attention_common.cuh"
 #include "bounds_check.cuh"
+#include "launch.cuh"
 
 namespace b200 {
 
@@ -79,7 +80,6 @@ attn_fwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(desc + kFwdGroups);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  zero_tail_fwd(p);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kFwdGroups; ++i) {
@@ -94,10 +94,13 @@ attn_fwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     mbar_fence_init();
   }
   constexpr int kProducer = kFwdGroups * 4, kMma = kProducer + 1;
+  wait_for_previous();
+  zero_tail_fwd(p);
   if (warp == kMma) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  let_next_start();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == kProducer) {
@@ -367,7 +370,6 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  zero_tail_bwd(p);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -386,10 +388,13 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     *abort_word = 0;
     mbar_fence_init();
   }
+  wait_for_previous();
+  zero_tail_bwd(p);
   if (warp == 13) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  let_next_start();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 12) {
@@ -652,9 +657,7 @@ static const char* launch_fwd_short(const CUtensorMap& tq, const CUtensorMap& tk
     configured = true;
   }
   const int grid = num_items < num_sms() ? num_items : num_sms();
-  kern<<<grid, fwd_short_threads(kGroups), fwd_short_smem(kGroups), stream>>>(tq, tk, tv, a, num_items);
-  cudaError_t ce = cudaGetLastError();
-  return ce == cudaSuccess ? nullptr : cudaGetErrorString(ce);
+  return launch_overlapped(kern, grid, fwd_short_threads(kGroups), fwd_short_smem(kGroups), stream, tq, tk, tv, a, num_items);
 }
 
 const char* launch_attn_fwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a,
@@ -676,9 +679,8 @@ static const char* launch_bwd_short(const CUtensorMap& tq, const CUtensorMap& tk
     configured = true;
   }
   const int grid = num_items < num_sms() ? num_items : num_sms();
-  attn_bwd_short_kernel<kDrop><<<grid, kBwdShortThreads, kBwdShortSmem, stream>>>(tq, tk, tv, tdo, to, a, num_items, g_attn_bwd_ablate);
-  cudaError_t ce = cudaGetLastError();
-  return ce == cudaSuccess ? nullptr : cudaGetErrorString(ce);
+  return launch_overlapped(attn_bwd_short_kernel<kDrop>, grid, kBwdShortThreads, kBwdShortSmem, stream, tq, tk, tv, tdo, to, a, num_items,
+                           g_attn_bwd_ablate);
 }
 
 const char* launch_attn_bwd_short(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,

@@ -21,6 +21,7 @@
 // bias_cuda.cu:22-612, softmax_apex.h) and its bundled FlashAttention-v1 mma.sync kernels
 // (onmt/modules/extensions/flashattn/src/fmha_fprop_kernel_1xN.h, fmha_dgrad_kernel_1xN_loop.h).
 #include "attention_common.cuh"
+#include "launch.cuh"
 
 namespace b200 {
 
@@ -44,6 +45,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+  wait_for_previous();
   zero_tail_fwd(p);
   const int b = blockIdx.z, h = blockIdx.y, qt = blockIdx.x;
   const int q_begin = p.cu_q[b], q_end = p.cu_q[b + 1];
@@ -66,6 +68,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  let_next_start();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tS = tmem_base;         // 128 columns
   const uint32_t tO = tmem_base + 128;   // 64 columns
@@ -299,6 +302,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+  wait_for_previous();
   zero_tail_bwd(p);
   const int b = blockIdx.z, h = blockIdx.y, kt = blockIdx.x;
   const int q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
@@ -323,6 +327,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  let_next_start();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tS = tmem_base, tDP = tmem_base + 128, tDQ = tmem_base + 256, tDK = tmem_base + 320,
                  tDV = tmem_base + 384;
@@ -600,6 +605,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 // 128-byte runs
 __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, int ld_o, const __nv_bfloat16* __restrict__ d_o, int ld_do,
                                   float* __restrict__ delta, long stride, int total_q, int heads) {
+  let_next_start();
+  wait_for_previous();
   const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= static_cast<long>(total_q) * heads) return;
   const int row = static_cast<int>(i / heads), h = static_cast<int>(i % heads);
@@ -623,6 +630,8 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, int ld_o,
 // dq (bf16) = dq_acc (fp32) for rows of sequences with more than one key tile
 __global__ void attn_dq_convert_kernel(const float* __restrict__ acc, int ld_acc, __nv_bfloat16* __restrict__ dq, int ld_dq,
                                        const int* __restrict__ cu_q, const int* __restrict__ cu_k, int width) {
+  let_next_start();
+  wait_for_previous();
   const int b = blockIdx.y;
   if (cu_k[b + 1] - cu_k[b] <= kTile) return;
   const int q_begin = cu_q[b], q_end = cu_q[b + 1];
@@ -700,10 +709,7 @@ const char* nmtg_attn_fwd(const AttnDesc* d, cudaStream_t stream) {
     configured = true;
   }
   dim3 grid((d->max_q + kTile - 1) / kTile, d->num_heads, d->batch);
-  if (d->bias) attn_fwd_kernel<true><<<grid, 256, kFwdSmem, stream>>>(tq, tk, tv, a);
-  else attn_fwd_kernel<false><<<grid, 256, kFwdSmem, stream>>>(tq, tk, tv, a);
-  cudaError_t ce = cudaGetLastError();
-  return ce == cudaSuccess ? nullptr : cudaGetErrorString(ce);
+  return launch_overlapped(d->bias ? attn_fwd_kernel<true> : attn_fwd_kernel<false>, grid, 256, kFwdSmem, stream, tq, tk, tv, a);
 }
 
 const char* nmtg_attn_bwd(const AttnDesc* d, cudaStream_t stream) {
@@ -748,8 +754,9 @@ const char* nmtg_attn_bwd(const AttnDesc* d, cudaStream_t stream) {
   }
   if (d->delta && d->max_k > kTile) {
     const long n = static_cast<long>(d->total_q) * d->num_heads;
-    attn_delta_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, stream>>>(a.o, a.ld_o, a.d_o, a.ld_do, d->delta, d->lse_stride,
-                                                                            d->total_q, d->num_heads);
+    if ((e = launch_overlapped(attn_delta_kernel, static_cast<int>((n + 255) / 256), 256, 0, stream, a.o, a.ld_o, a.d_o, a.ld_do, d->delta,
+                               d->lse_stride, d->total_q, d->num_heads)))
+      return e;
     a.delta = d->delta;
   }
   CUtensorMap tdq = tq;       // placeholder when the reductions go through red.add
@@ -758,23 +765,18 @@ const char* nmtg_attn_bwd(const AttnDesc* d, cudaStream_t stream) {
       cached_tmap_f32(&tdq, d->dq_acc, d->total_q, width, d->ld_dqacc, kTile, 32))
     a.dq_tma = 1;
   dim3 grid((d->max_k + kTile - 1) / kTile, d->num_heads, d->batch);
-  cudaError_t ce = cudaSuccess;
   if (!d->bias && a.delta && a.dq_tma && g_attn_variant != 2 && (g_attn_variant == 1 || d->max_k > 4 * kTile)) {
     // long sequences: the warp-specialised, pipelined kernel (attention_bwd_ws_tcgen05.cu); 0.587 / 0.664 ms on 8 x 1500 x 20
     // heads and 0.313 / 0.336 ms on 8 x 1000 x 16 heads against the kernel below, level with it at 448 tokens
     if ((e = launch_attn_bwd_ws(tq, tk, tv, tdo, tdq, a, grid, stream))) return e;
   } else {
-    if (d->bias) attn_bwd_kernel<true><<<grid, 256, kBwdSmem, stream>>>(tq, tk, tv, tdo, tdq, a);
-    else attn_bwd_kernel<false><<<grid, 256, kBwdSmem, stream>>>(tq, tk, tv, tdo, tdq, a);
-    ce = cudaGetLastError();
-    if (ce != cudaSuccess) return cudaGetErrorString(ce);
+    if ((e = launch_overlapped(d->bias ? attn_bwd_kernel<true> : attn_bwd_kernel<false>, grid, 256, kBwdSmem, stream, tq, tk, tv, tdo, tdq, a)))
+      return e;
   }
   if (d->max_k > kTile) {
     dim3 g2(64, d->batch);
-    attn_dq_convert_kernel<<<g2, 256, 0, stream>>>(d->dq_acc, d->ld_dqacc, reinterpret_cast<__nv_bfloat16*>(d->dq), d->ld_dq,
-                                                   d->cu_q, d->cu_k, width);
-    ce = cudaGetLastError();
-    if (ce != cudaSuccess) return cudaGetErrorString(ce);
+    return launch_overlapped(attn_dq_convert_kernel, g2, 256, 0, stream, d->dq_acc, d->ld_dqacc, reinterpret_cast<__nv_bfloat16*>(d->dq), d->ld_dq,
+                             d->cu_q, d->cu_k, width);
   }
   return nullptr;
 }

@@ -11,6 +11,13 @@
 
 namespace b200 {
 
+// Launch overlap inside a chain of kernels (launch_overlapped): a block sets itself up while the kernel before it ends, waits for that
+// kernel, and lets the next one be scheduled.  Nothing that another kernel writes or reads is touched before the wait; tensor memory is
+// allocated after it and before the next kernel is let in, so that blocks of two kernels never wait for each other's columns.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+
 // ---------------------------------------------------------------------------------------------
 // status word written by kernels (0 = ok)
 // ---------------------------------------------------------------------------------------------

@@ -12,6 +12,7 @@
 #include "b200_ptx.cuh"
 #include "ops_api.h"
 #include "bounds_check.cuh"
+#include "launch.cuh"
 
 namespace b200 {
 
@@ -41,6 +42,8 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 __global__ void dropout_add_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                                    __nv_bfloat16* __restrict__ y, long n16, float p, unsigned long long seed,
                                    unsigned long long stream_id, const unsigned long long* seed_dev) {
+  let_next_start();
+  wait_for_previous();
   const DropRng rng(seed + (seed_dev ? *seed_dev : 0ull), stream_id, p);
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n16;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -110,6 +113,8 @@ dropout_colsum_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __rest
                       float p, unsigned long long seed, unsigned long long stream_id, const unsigned long long* seed_dev) {
   constexpr int kRowsPerIter = 256 / kGroups;
   __shared__ float part[kRowsPerIter][kGroups * 16 + 1];
+  let_next_start();
+  wait_for_previous();
   const DropRng rng(seed + (seed_dev ? *seed_dev : 0ull), stream_id, p);
   const int c = threadIdx.x % kGroups, rsub = threadIdx.x / kGroups;
   float acc[16];
@@ -331,10 +336,9 @@ const char* nmtg_dropout_add(const void* x, const void* residual, void* y, long 
   long blocks = (n16 + 255) / 256;
   const long cap = static_cast<long>(num_sms()) * 8;
   if (blocks > cap) blocks = cap;
-  dropout_add_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(residual),
-      reinterpret_cast<__nv_bfloat16*>(y), n16, p, seed, stream_id, seed_dev);
-  return last_err();
+  return launch_overlapped(
+      dropout_add_kernel, static_cast<int>(blocks), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x),
+      reinterpret_cast<const __nv_bfloat16*>(residual), reinterpret_cast<__nv_bfloat16*>(y), n16, p, seed, stream_id, seed_dev);
 }
 
 const char* nmtg_act_backward(const void* dy, const void* z, void* dz, long n, int act, float p, unsigned long long seed,
@@ -362,19 +366,19 @@ const char* nmtg_dropout_colsum(const void* x, void* y, float* colsum, int rows,
   const long cap = static_cast<long>(num_sms()) * 4;
   if (blocks > cap) blocks = cap;
   auto go = [&](auto tag) {
-    dropout_colsum_kernel<decltype(tag)::value><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<__nv_bfloat16*>(y), colsum, rows, p, seed, stream_id, seed_dev);
+    return launch_overlapped(dropout_colsum_kernel<decltype(tag)::value>, static_cast<int>(blocks), 256, 0, stream,
+                             reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<__nv_bfloat16*>(y), colsum, rows, p, seed, stream_id,
+                             seed_dev);
   };
   switch (groups) {
-    case 256: go(std::integral_constant<int, 256>()); break;
-    case 128: go(std::integral_constant<int, 128>()); break;
-    case 64: go(std::integral_constant<int, 64>()); break;
-    case 32: go(std::integral_constant<int, 32>()); break;
-    case 16: go(std::integral_constant<int, 16>()); break;
-    case 8: go(std::integral_constant<int, 8>()); break;
+    case 256: return go(std::integral_constant<int, 256>());
+    case 128: return go(std::integral_constant<int, 128>());
+    case 64: return go(std::integral_constant<int, 64>());
+    case 32: return go(std::integral_constant<int, 32>());
+    case 16: return go(std::integral_constant<int, 16>());
+    case 8: return go(std::integral_constant<int, 8>());
     default: return "dropout_colsum: unsupported column count";
   }
-  return last_err();
 }
 
 const char* nmtg_embed_fwd(const int64_t* tokens, const int64_t* positions, const void* table, const void* pos_table,

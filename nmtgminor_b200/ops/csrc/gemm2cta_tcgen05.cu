@@ -15,6 +15,7 @@
 // Every wait is bounded; all exits go through the final cluster barrier so a CTA never leaves while its peer
 // may still touch its shared memory.
 #include "gemm_common.cuh"
+#include "launch.cuh"
 
 namespace b200 {
 
@@ -148,7 +149,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       for (int i = 0; i < 2 * kEpilogueWarps; ++i) mbar_init(&aux_full[i], 1);
     *abort_word = 0;
     mbar_fence_init();
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
   }
+  wait_for_previous();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * BN) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -157,13 +161,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   __syncthreads();
   cluster_sync_all();      // barriers of both CTAs are initialised and TMEM is allocated before anyone proceeds
   tc_fence_after_sync();
+  if (g.n_seg == 0) let_next_start();      // a gathering kernel waits for other GPUs: nothing takes its SMs meanwhile
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
     // ------------------------------- TMA producer (both CTAs) --------------------------------
     if (lane == 0) {
-      tma_prefetch_desc(&tmap_a);
-      tma_prefetch_desc(&tmap_b);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -492,6 +495,7 @@ static const char* launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, con
     if (e != cudaSuccess) return cudaGetErrorString(e);
     configured = true;
   }
+  if (g.n_seg == 0) return launch_overlapped(gemm_pair_kernel<BN, kTrace, kFeat>, grid, kPairThreads, kSmem, stream, ta, tb, tc, t2, args, g);
   gemm_pair_kernel<BN, kTrace, kFeat><<<grid, kPairThreads, kSmem, stream>>>(ta, tb, tc, t2, args, g);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);

@@ -15,6 +15,7 @@
 // (onmt/modules/extensions/mlp/mlp_relu_cuda.cu:82-190,445-1292; mlp_blaslt/mlp_gelu_cuda.cu:212-471;
 // multihead_attn/self_multihead_attn_cuda.cu:91,284; dropout_add/dropout.h:21-160).
 #include "gemm_common.cuh"
+#include "launch.cuh"
 
 #include <mutex>
 #include <unordered_map>
@@ -69,18 +70,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     *abort_word = 0;
     mbar_fence_init();
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
   }
+  wait_for_previous();
   if (warp == 1) tmem_alloc(tmem_slot, 2 * BN);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  let_next_start();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------------------
     if (lane == 0) {
-      tma_prefetch_desc(&tmap_a);
-      tma_prefetch_desc(&tmap_b);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -353,6 +356,9 @@ int num_sms() {
 }
 void set_sm_reserve(int n) { g_sm_reserve = n < 0 ? 0 : (n & ~1); }
 
+// SMs set aside for communication must stay free of blocks that wait for their turn.
+bool launch_overlap() { return g_sm_reserve == 0 && g_gemm_sm_reserve == 0; }
+
 int gemm_sms() {
   const int n = num_sms() - g_gemm_sm_reserve;
   return n < 2 ? 2 : n;
@@ -368,9 +374,7 @@ static const char* launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, con
     if (e != cudaSuccess) return cudaGetErrorString(e);
     configured = true;
   }
-  gemm_tcgen05_kernel<BN, kFeat><<<grid, kGemmThreads, GemmSmem<BN>::kTotal, stream>>>(ta, tb, args);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
+  return launch_overlapped(gemm_tcgen05_kernel<BN, kFeat>, grid, kGemmThreads, GemmSmem<BN>::kTotal, stream, ta, tb, args);
 }
 
 // The epilogues of the shapes a training step is made of (as in the CTA-pair kernel); anything else takes the general one.

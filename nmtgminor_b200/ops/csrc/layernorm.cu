@@ -12,6 +12,8 @@
 #include <type_traits>
 #include <cstdlib>
 #include "ops_api.h"
+#include "b200_ptx.cuh"
+#include "launch.cuh"
 
 namespace b200 {
 
@@ -121,6 +123,8 @@ ln_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
   const int nvec = hidden >> 3;
   for (int i = threadIdx.x; i < kLnWarps * 2 * hidden; i += blockDim.x) s_acc[i] = 0.f;
   __syncthreads();
+  let_next_start();
+  wait_for_previous();
   float* wg = s_acc + warp * 2 * hidden;  // lanes own disjoint columns: plain read-modify-write
   float* wb = wg + hidden;
   // narrow rows keep the affine-gradient partial sums in registers; wide rows use the shared-memory slice
@@ -331,6 +335,8 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 #pragma unroll
     for (int j = 0; j < 8; ++j) ag[i][j] = ab[i][j] = 0.f;
 
+  let_next_start();
+  wait_for_previous();
   const int step = gridDim.x * kWarps, row0 = blockIdx.x * kWarps + warp;
   auto fetch = [&](int row, int stage) {
     if (row < rows) {
@@ -563,7 +569,7 @@ const char* nmtg_layernorm_fwd(const void* x, const void* gamma, const void* bet
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = step_overlap() ? 1 : 0;
+    cfg.numAttrs = step_overlap() || launch_overlap() ? 1 : 0;
     auto kern = step_overlap() ? ln_fwd_kernel<decltype(vpl)::value, true> : ln_fwd_kernel<decltype(vpl)::value>;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, reinterpret_cast<const __nv_bfloat16*>(x),
                                        reinterpret_cast<const __nv_bfloat16*>(gamma), reinterpret_cast<const __nv_bfloat16*>(beta),
@@ -578,12 +584,10 @@ static const char* launch_ln_bwd(const void* dy, const void* x, const float* mea
   const int grid = (rows + kLnWarps - 1) / kLnWarps;
   const size_t smem = kLnWarps * 2 * static_cast<size_t>(hidden) * sizeof(float);
   auto run = [&](auto kern) -> const char* {
-    kern<<<grid, kLnWarps * 32, smem, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x), mean, rstd,
+    return launch_overlapped(
+        kern, grid, kLnWarps * 32, smem, stream, reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x), mean, rstd,
         reinterpret_cast<const __nv_bfloat16*>(gamma), reinterpret_cast<const __nv_bfloat16*>(dres),
         reinterpret_cast<__nv_bfloat16*>(dx), dgamma, dbeta, rows, hidden);
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
   };
   if (hidden <= 256) return run(ln_bwd_kernel<1>);
   if (hidden <= 512) return run(ln_bwd_kernel<2>);
@@ -600,12 +604,10 @@ static const char* launch_ln_bwd_stream(const void* dy, const void* x, const flo
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return cudaGetErrorString(e);
   const int need = (rows + kWarps - 1) / kWarps;
-  kern<<<need < num_sms() ? need : num_sms(), kWarps * 32, smem, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x), mean, rstd,
+  return launch_overlapped(
+      kern, need < num_sms() ? need : num_sms(), kWarps * 32, smem, stream, reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x), mean, rstd,
       reinterpret_cast<const __nv_bfloat16*>(gamma), reinterpret_cast<const __nv_bfloat16*>(dres), reinterpret_cast<__nv_bfloat16*>(dx), dgamma,
       dbeta, rows, hidden);
-  e = cudaGetLastError();
-  return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
 
 const char* nmtg_layernorm_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const void* gamma,
