@@ -37,7 +37,7 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int nvec = hidden >> 3;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // decoding steps: see nmtg_set_step_overlap
+  let_next_start();
   uint4 gain[kStep ? VPL : 1], shift[kStep ? VPL : 1];
   if constexpr (kStep) {
 #pragma unroll
@@ -47,7 +47,7 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
         shift[i] = __ldg(reinterpret_cast<const uint4*>(beta) + lane + i * 32);
       }
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_for_previous();
   for (int row = blockIdx.x * kLnWarps + warp; row < rows; row += gridDim.x * kLnWarps) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * hidden);
     float v[VPL][8];
