@@ -547,7 +547,7 @@ template <> __device__ __forceinline__ float as_float<__nv_bfloat16>(__nv_bfloat
 // in shared memory, one CTA per row: 43 us for 4 rows of 32000, which one pass over eight pieces does in a tenth.  256 rows of 32000 are
 // bound by instructions: comparing floats against the highest of the warps' bounds takes 14.1 us, where every column was ranked as an
 // integer, masked and checked against the end, and each warp used its own bound, 21.9.
-template <typename T>
+template <typename T, bool kWarm>
 __global__ void __launch_bounds__(kPartThreads)
 beam_part_kernel(const T* __restrict__ logits, long ld, const uint8_t* __restrict__ force, float2* __restrict__ part_lse,
                  Cand* __restrict__ part, int first, int K2, int V, int pad, int eos, int vec) {
@@ -558,109 +558,115 @@ beam_part_kernel(const T* __restrict__ logits, long ld, const uint8_t* __restric
   const int r = first + blockIdx.y, piece = blockIdx.x;
   const int c0 = piece * kPartCols;
   pdl_trigger();
-  pdl_wait();
   const T* x = logits + static_cast<long>(r) * ld + c0;
   constexpr int kPer = 16 / sizeof(T);
-  const int cols = min(kPartCols, V - c0);
-  float f[kPartEach];
-  int col[kPartEach / kPer];
+  // kWarm: once over no columns, storing nothing, before the wait; a step runs these instructions once, and fetching them took longer than
+  // running them (4 rows of 32000 in a search 6.6 us, 4.3 so; not where the blocks are several waves: 256 rows 13.5 and 16.5)
+#pragma unroll 1
+  for (int pass = kWarm ? 0 : 1; pass < 2; ++pass) {
+    if (pass == 1) pdl_wait();
+    const int cols = pass == 1 ? min(kPartCols, V - c0) : 0;
+    float f[kPartEach];
+    int col[kPartEach / kPer];
 #pragma unroll
-  for (int i = 0; i < kPartEach / kPer; ++i) {
-    col[i] = (i * kPartThreads + threadIdx.x) * kPer;
-    if (vec && col[i] + kPer <= cols) {
-      const uint4 u = *reinterpret_cast<const uint4*>(x + col[i]);
-      const T* e = reinterpret_cast<const T*>(&u);
+    for (int i = 0; i < kPartEach / kPer; ++i) {
+      col[i] = (i * kPartThreads + threadIdx.x) * kPer;
+      if (vec && col[i] + kPer <= cols) {
+        const uint4 u = *reinterpret_cast<const uint4*>(x + col[i]);
+        const T* e = reinterpret_cast<const T*>(&u);
 #pragma unroll
-      for (int j = 0; j < kPer; ++j) f[i * kPer + j] = as_float<T>(e[j]);
-    } else {
+        for (int j = 0; j < kPer; ++j) f[i * kPer + j] = as_float<T>(e[j]);
+      } else {
 #pragma unroll
-      for (int j = 0; j < kPer; ++j) f[i * kPer + j] = col[i] + j < cols ? as_float<T>(x[col[i] + j]) : -INFINITY;
+        for (int j = 0; j < kPer; ++j) f[i * kPer + j] = col[i] + j < cols ? as_float<T>(x[col[i] + j]) : -INFINITY;
+      }
     }
-  }
-  float top = -INFINITY;                                   // of this thread
+    float top = -INFINITY;                                   // of this thread
 #pragma unroll
-  for (int i = 0; i < kPartEach; ++i) top = fmaxf(top, f[i]);
-  float mx = warp_max(top);
-  if (lane == 0) red[0][warp] = mx;
-  if (threadIdx.x == 0) count = 0;
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < warps; ++w) mx = fmaxf(mx, red[0][w]);
-  float sum = 0.f;
-  if (mx != -INFINITY) {                                   // columns past the end hold -inf, whose weight is zero
-#pragma unroll
-    for (int i = 0; i < kPartEach; ++i) sum += __expf(f[i] - mx);
-  } else {
-#pragma unroll
-    for (int i = 0; i < kPartEach; ++i)
-      if (f[i] != f[i]) sum = f[i];                        // no number here: NaN stays NaN
-  }
-  sum = warp_sum(sum);
-  if (lane == 0) red[1][warp] = sum;
-  // masks: the padding word, and EOS where the control byte bans it
-  const bool ban = force != nullptr && force[r] == 2;
-  auto owns = [&](int word) { return word >= c0 && word - c0 < cols && (word - c0) / kPer % kPartThreads == threadIdx.x; };
-  if (owns(pad) || (ban && owns(eos))) {
-    top = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < kPartEach; ++i) {
-      const int c = c0 + col[i / kPer] + i % kPer;
-      if (c == pad || (ban && c == eos)) f[i] = -INFINITY;
-      top = fmaxf(top, f[i]);
-    }
-  }
-  // The K2-th largest of a warp's 32 lane maxima is a lower bound of the piece's K2-th largest value, so only what reaches the highest of
-  // these bounds can be chosen: a handful of candidates, collected in shared memory (all of them where K2 exceeds the lanes, or where the
-  // bound excludes nothing: then NaN may be wanted too).
-  float bar = -INFINITY;
-  if (K2 <= 32) {
-    uint32_t rest = rank_of(top), best = 0;
-    for (int j = 0; j < K2; ++j) {
-      best = __reduce_max_sync(0xffffffffu, rest);
-      const uint32_t who = __ballot_sync(0xffffffffu, rest == best);
-      if (lane == __ffs(who) - 1) rest = 0;
-    }
-    if (best != 0) bar = value_of(best);
-    if (lane == 0) red[2][warp] = bar;
+    for (int i = 0; i < kPartEach; ++i) top = fmaxf(top, f[i]);
+    float mx = warp_max(top);
+    if (lane == 0) red[0][warp] = mx;
+    if (threadIdx.x == 0) count = 0;
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < warps; ++w) bar = fmaxf(bar, red[2][w]);
-  }
-  uint32_t takes = 0;
-  if (bar != -INFINITY) {
-    if (top >= bar) {
+    for (int w = 0; w < warps; ++w) mx = fmaxf(mx, red[0][w]);
+    float sum = 0.f;
+    if (mx != -INFINITY) {                                   // columns past the end hold -inf, whose weight is zero
+#pragma unroll
+      for (int i = 0; i < kPartEach; ++i) sum += __expf(f[i] - mx);
+    } else {
 #pragma unroll
       for (int i = 0; i < kPartEach; ++i)
-        if (f[i] >= bar) takes |= 1u << i;
+        if (f[i] != f[i]) sum = f[i];                        // no number here: NaN stays NaN
     }
-  } else {
+    sum = warp_sum(sum);
+    if (lane == 0) red[1][warp] = sum;
+    // masks: the padding word, and EOS where the control byte bans it
+    const bool ban = pass == 1 && force != nullptr && force[r] == 2;
+    auto owns = [&](int word) { return word >= c0 && word - c0 < cols && (word - c0) / kPer % kPartThreads == threadIdx.x; };
+    if (owns(pad) || (ban && owns(eos))) {
+      top = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < kPartEach; ++i) {
+        const int c = c0 + col[i / kPer] + i % kPer;
+        if (c == pad || (ban && c == eos)) f[i] = -INFINITY;
+        top = fmaxf(top, f[i]);
+      }
+    }
+    // The K2-th largest of a warp's 32 lane maxima is a lower bound of the piece's K2-th largest value, so only what reaches the highest of
+    // these bounds can be chosen: a handful of candidates, collected in shared memory (all of them where K2 exceeds the lanes, or where the
+    // bound excludes nothing: then NaN may be wanted too).
+    float bar = -INFINITY;
+    if (K2 <= 32) {
+      uint32_t rest = rank_of(top), best = 0;
+      for (int j = 0; j < K2; ++j) {
+        best = __reduce_max_sync(0xffffffffu, rest);
+        const uint32_t who = __ballot_sync(0xffffffffu, rest == best);
+        if (lane == __ffs(who) - 1) rest = 0;
+      }
+      if (best != 0) bar = value_of(best);
+      if (lane == 0) red[2][warp] = bar;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < warps; ++w) bar = fmaxf(bar, red[2][w]);
+    }
+    uint32_t takes = 0;
+    if (bar != -INFINITY) {
+      if (top >= bar) {
+#pragma unroll
+        for (int i = 0; i < kPartEach; ++i)
+          if (f[i] >= bar) takes |= 1u << i;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPartEach; ++i)
+        if (col[i / kPer] + i % kPer < cols) takes |= 1u << i;
+    }
+    const int mine = __popc(takes);
+    int before = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += t;
+    }
+    int at = 0;
+    if (lane == 31) at = atomicAdd(&count, before);
+    at = __shfl_sync(0xffffffffu, at, 31) + before - mine;
 #pragma unroll
     for (int i = 0; i < kPartEach; ++i)
-      if (col[i / kPer] + i % kPer < cols) takes |= 1u << i;
+      if ((takes >> i) & 1u) list[at++] = cand_of(f[i], c0 + col[i / kPer] + i % kPer);
+    __syncthreads();
+    const long o = static_cast<long>(r) * gridDim.x + piece;
+    if (threadIdx.x == kPartThreads - 1 && pass == 1) {
+      float s = 0.f;
+      for (int w = 0; w < warps; ++w) s += red[1][w];
+      part_lse[o] = make_float2(mx, s);
+    }
+    const int n = count;
+    for (int j = n + threadIdx.x; j < K2 && pass == 1; j += kPartThreads) part[o * K2 + j] = 0;
+    take_best(list, n, K2, kPartThreads, [&](int place, Cand c) { part[o * K2 + place] = c; });
+    if (kWarm && pass == 0) __syncthreads();
   }
-  const int mine = __popc(takes);
-  int before = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, before, o);
-    if (lane >= o) before += t;
-  }
-  int at = 0;
-  if (lane == 31) at = atomicAdd(&count, before);
-  at = __shfl_sync(0xffffffffu, at, 31) + before - mine;
-#pragma unroll
-  for (int i = 0; i < kPartEach; ++i)
-    if ((takes >> i) & 1u) list[at++] = cand_of(f[i], c0 + col[i / kPer] + i % kPer);
-  __syncthreads();
-  const long o = static_cast<long>(r) * gridDim.x + piece;
-  if (threadIdx.x == kPartThreads - 1) {
-    float s = 0.f;
-    for (int w = 0; w < warps; ++w) s += red[1][w];
-    part_lse[o] = make_float2(mx, s);
-  }
-  const int n = count;
-  for (int j = n + threadIdx.x; j < K2; j += kPartThreads) part[o * K2 + j] = 0;
-  take_best(list, n, K2, kPartThreads, [&](int place, Cand c) { part[o * K2 + place] = c; });
 }
 
 // Everything that the search does between two steps, one CTA per sentence.
@@ -951,13 +957,14 @@ const char* nmtg_beam_step(const NmtgBeam* s, const void* logits, long ld, int d
   if (K2 > V) return "beam_step: vocabulary smaller than twice the beam";
   if (ld < V) return "beam_step: row stride smaller than the vocabulary";
   const int vec = (ld * (dtype == 0 ? 4 : 2)) % 16 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  const bool warm = step_overlap() && static_cast<long>(pieces) * R <= 2L * num_sms();      // blocks that wait together
   float2* lse = static_cast<float2*>(part_lse);
   Cand* cand = static_cast<Cand*>(part);
   const char* e = by_rows(R, [&](int first, int n) {
     if (dtype == 0)
-      return launch(beam_part_kernel<float>, dim3(pieces, n), dim3(kPartThreads), 0, 1, stream, static_cast<const float*>(logits), ld, s->force,
+      return launch(warm ? beam_part_kernel<float, true> : beam_part_kernel<float, false>, dim3(pieces, n), dim3(kPartThreads), 0, 1, stream, static_cast<const float*>(logits), ld, s->force,
                     lse, cand, first, K2, V, s->pad, s->eos, vec);
-    return launch(beam_part_kernel<__nv_bfloat16>, dim3(pieces, n), dim3(kPartThreads), 0, 1, stream, static_cast<const __nv_bfloat16*>(logits),
+    return launch(warm ? beam_part_kernel<__nv_bfloat16, true> : beam_part_kernel<__nv_bfloat16, false>, dim3(pieces, n), dim3(kPartThreads), 0, 1, stream, static_cast<const __nv_bfloat16*>(logits),
                   ld, s->force, lse, cand, first, K2, V, s->pad, s->eos, vec);
   });
   if (e) return e;

@@ -47,9 +47,13 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
         shift[i] = __ldg(reinterpret_cast<const uint4*>(beta) + lane + i * 32);
       }
   }
-  wait_for_previous();
-  for (int row = blockIdx.x * kLnWarps + warp; row < rows; row += gridDim.x * kLnWarps) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * hidden);
+  // In a step the loop is run once over the gain, storing nothing, before the wait: its instructions are then in the caches when the row
+  // arrives (in searches 7.2 / 4.5 us where a step has one such launch, 3.05 / 2.19 where it has 19 of 256 rows).
+  bool real = !kStep;
+  if constexpr (!kStep) wait_for_previous();
+#pragma unroll 1
+  for (int row = blockIdx.x * kLnWarps + warp; row < rows;) {
+    const uint4* xr = reinterpret_cast<const uint4*>(real ? x + static_cast<size_t>(row) * hidden : gamma);
     float v[VPL][8];
     float s = 0.f;
 #pragma unroll
@@ -83,7 +87,7 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       }
     }
     const float rs = rsqrtf(warp_sum(sq) / hidden + eps);
-    if (lane == 0) {
+    if (lane == 0 && real) {
       if (mean) mean[row] = mu;
       if (rstd) rstd[row] = rs;
     }
@@ -104,8 +108,14 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
           o2[j] = __floats2bfloat162_rn((v[i][2 * j] - mu) * rs * gf.x + bf.x,
                                         (v[i][2 * j + 1] - mu) * rs * gf.y + bf.y);
         }
-        yr[vi] = o;
+        if (real) yr[vi] = o;
       }
+    }
+    if (real) {
+      row += gridDim.x * kLnWarps;
+    } else {
+      wait_for_previous();
+      real = true;
     }
   }
 }
