@@ -550,3 +550,39 @@ def test_step_linear_normalises_as_the_layernorm_kernel_does():
         x, gamma, beta = (torch.randn(*s, device="cuda", generator=g).bfloat16() for s in ((7, K), (K,), (K,)))
         eye = torch.eye(K, device="cuda").bfloat16()
         assert torch.equal(ops.ext().step_linear(x * 3 + 1, gamma, beta, 1e-5, eye, None, None, 0), ops.ext().layernorm_fwd(x * 3 + 1, gamma, beta, 1e-5)[0])
+
+
+def _opposite_pairs(rows, T, hid, g):
+    """Keys in pairs of equal rows, anywhere in the past, whose values have opposite signs: attention over them is exactly 0."""
+    at = torch.randperm(T, device="cuda", generator=g)
+    k, v = (torch.randn(rows, T // 2, hid, device="cuda", generator=g).bfloat16() for _ in range(2))
+    keys, values = (torch.empty(rows, T, hid, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    keys[:, at], values[:, at] = torch.cat([k, k], 1), torch.cat([v, -v], 1)
+    return keys, values
+
+
+@pytest.mark.parametrize("kind,B,K,heads,T,adds", [("cross", 64, 4, 16, 200, 9), ("cross", 16, 4, 20, 1500, 18), ("self", 64, 4, 16, 82, 5),
+                                                   ("self", 4, 1, 8, 1002, 16)])
+def test_step_attention_sums_in_32_bits(kind, B, K, heads, T, adds):
+    """What is left of an exact 0 is the rounding of the sums.  `adds` 32-bit additions (blocks of 16 keys of a warp, then warps and shares)
+    round to nearest, 0.58 x 2^-24 of the sum so far each (root mean square); the sums so far are a random walk to the root of the terms'
+    squares.  A quarter more for what a block loses inside."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    e, hid, total, size = ops.ext(), heads * 64, 0.0, 0.0
+    for _ in range(3):
+        rows = B if kind == "cross" else B * K
+        keys, values = _opposite_pairs(rows, T, hid, g)
+        qkv = torch.randn(B * K, 3 * hid, device="cuda", generator=g).bfloat16()
+        if kind == "cross":
+            out = e.decode_cross(qkv[:, :hid].contiguous(), keys, values, torch.full((B,), T, dtype=torch.int32, device="cuda"), heads, 0.125)
+            keys, values = keys.repeat_interleave(K, 0), values.repeat_interleave(K, 0)
+        else:
+            qkv[:, hid:2 * hid], qkv[:, 2 * hid:] = keys[:, -1], values[:, -1]
+            anc = torch.arange(B * K, dtype=torch.int32, device="cuda")[:, None].expand(B * K, T + 6).contiguous()
+            kc, vc = (torch.cat([t, t.new_zeros(rows, 6, hid)], 1) for t in (keys, values))
+            out = e.decode_self(qkv, kc, vc, anc, torch.full((B * K,), T - 1, device="cuda"), K, heads, 0.125)
+        split = lambda t: t.float().view(B * K, T, heads, 64)
+        w = (torch.einsum("rhd,rjhd->rhj", qkv[:, :hid].float().view(B * K, heads, 64), split(keys)) * 0.125).softmax(-1)
+        size += torch.einsum("rhj,rjhd->rhd", w.square(), split(values).square()).mean().item()
+        total += out.double().square().mean().item()
+    assert total ** 0.5 <= 1.25 * 0.58 * 2 ** -24 * (size * adds / 2) ** 0.5
