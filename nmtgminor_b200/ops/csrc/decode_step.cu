@@ -92,6 +92,12 @@ __device__ __forceinline__ uint32_t transpose8(uint32_t x) {
   asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
   return y;
 }
+// x, or the largest number with some sign for what is none
+__device__ __forceinline__ float in_range(float x) {
+  float y;
+  asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(3.402823466e38f));
+  return y;
+}
 __device__ __forceinline__ uint4 zero4() { return make_uint4(0u, 0u, 0u, 0u); }
 __device__ __forceinline__ uint4 load8(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
 
@@ -177,6 +183,8 @@ struct WarpTile {
   // output += values x weights.  kOne: the values are those of query `only`, and the other queries' columns stay as they are, whatever
   // its values hold (0 x NaN).  A block's sum, smallest parts first, meets the output in an ordinary addition, which rounds to nearest; the
   // instruction cuts off, and summed through it alone outputs were 1.5 to 3 times as far from 64 bits (1500 keys 1.5e-8, 4.1e-9 so).
+  // The smaller parts of a weight are often zero, and under an infinite value their sum is then no number: it is brought into range,
+  // and what the largest part makes of such a value counts.
   template <bool kOne>
   __device__ __forceinline__ void add(const Values& v, const Weights& w, int only, int lane) {
     const uint32_t* v0 = reinterpret_cast<const uint32_t*>(&v.x[0][0]);
@@ -191,6 +199,8 @@ struct WarpTile {
       float d[4] = {0.f, 0.f, 0.f, 0.f};
       mma_bf16(d, a0, a1, a2, a3, w.x[2][0], w.x[2][1]);
       mma_bf16(d, a0, a1, a2, a3, w.x[1][0], w.x[1][1]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d[i] = in_range(d[i]);
       mma_bf16(d, a0, a1, a2, a3, w.x[0][0], w.x[0][1]);
 #pragma unroll
       for (int i = 0; i < 4; ++i)

@@ -586,3 +586,28 @@ def test_step_attention_sums_in_32_bits(kind, B, K, heads, T, adds):
         size += torch.einsum("rhj,rjhd->rhd", w.square(), split(values).square()).mean().item()
         total += out.double().square().mean().item()
     assert total ** 0.5 <= 1.25 * 0.58 * 2 ** -24 * (size * adds / 2) ** 0.5
+
+
+@pytest.mark.parametrize("K", [1, 3, 9])
+def test_infinite_values_of_a_step(K):
+    """An infinite value under a positive weight makes its own output infinite and no other one."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    B, heads, T, e = 2, 2, 40, ops.ext()
+    R, hid, inf = B * K, heads * 64, float("inf")
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    q, k, v = rnd(R, hid), rnd(B, T, hid), rnd(B, T, hid)
+    clean = e.decode_cross(q, k, v, torch.full((B,), T, dtype=torch.int32, device="cuda"), heads, 0.125).view(R, hid)
+    v[0, 5, 70], v[1, 39, 3] = inf, -inf
+    out = e.decode_cross(q, k, v, torch.full((B,), T, dtype=torch.int32, device="cuda"), heads, 0.125).view(R, hid)
+    want = clean.clone()
+    want[:K, 70], want[K:, 3] = inf, -inf
+    assert torch.equal(out, want)
+    qkv, kc, vc = rnd(R, 3 * hid), rnd(R, 64, hid), rnd(R, 64, hid)
+    anc = torch.arange(R, dtype=torch.int32, device="cuda")[:, None].expand(R, 64).contiguous()
+    anc[:, :32] = anc[:, :32] // K * K                       # a beginning that a sentence's hypotheses share
+    pos = torch.full((R,), T - 1, device="cuda")
+    step = lambda: e.decode_self(qkv, kc.clone(), vc.clone(), anc, pos, K, heads, 0.125).view(R, hid)
+    want = step()
+    vc[0, 20, 7], vc[R - 1, 35, 100], qkv[K - 1, 2 * hid + 9] = inf, inf, -inf
+    want[:K, 7], want[R - 1, 100], want[K - 1, 9] = inf, inf, -inf
+    assert torch.equal(step(), want)
