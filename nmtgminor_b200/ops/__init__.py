@@ -767,19 +767,13 @@ def cross_entropy(logits, labels, smoothing=0.0, pad_idx=0):
 
 
 def _long_sum_gemm(dz, w):
-    """``dz @ w`` (bf16) of the generator's data gradient.  The sum runs over the vocabulary and the output is small: where its 256 x 256
-    tiles leave half of the CTA pairs idle, the sum is cut over all of them into a 32-bit buffer that is rounded once (us: 3842 x 512 over
-    32000, 32 tiles, 143 / 104; 906 x 256 over 8000 36 / 15; 400 x 1024 over 250054 985 / 206; but 1856 x 1280 over 51865, 40 tiles, 262 /
-    301).  A tile's parts meet with atomic additions, as in weight gradients; against 64 bits no further off (1.657e-3 both, the last of
-    the long ones 1.688e-3 / 1.662e-3)."""
-    M, N = dz.shape[0], w.shape[1]
-    tiles = -(-M // 256) * -(-N // 256)
-    out = torch.empty((M, N), dtype=torch.bfloat16, device=dz.device)
-    if tiles * 4 > torch.cuda.get_device_properties(dz.device).multi_processor_count or w.shape[0] < 4096 or (M * N) % 8 or N % 8:
-        return gemm(dz, w, out, b_mn_major=True)
-    acc = torch.zeros((M, N), dtype=torch.float32, device=dz.device)
-    gemm(dz, w, acc, b_mn_major=True, accumulate=True, allow_split_k=True)
-    ext().cast_f32_bf16(acc, out)
+    """``dz @ w`` (bf16) of the generator's data gradient: the sum runs over the vocabulary, and where the output is small it is cut into
+    parts (csrc/gemm_tcgen05.cu: nmtg_gemm_parts).  They are added up in one order, so that a step repeats to the last bit whatever its
+    lower layers make of it; against 64 bits no further off than one sum (1.657e-3 both, the last of the long ones 1.688e-3 / 1.662e-3)."""
+    out = ext().gemm_in_parts(dz, w)
+    if out is None:
+        return gemm(dz, w, torch.empty((dz.shape[0], w.shape[1]), dtype=torch.bfloat16, device=dz.device), b_mn_major=True)
+    LAUNCHES[0] += 2
     return out
 
 

@@ -166,6 +166,27 @@ void gemm(const Tensor& a, bool a_mn_major, const Tensor& b, bool b_mn_major, Te
   ck(nmtg_gemm_bf16(&d, cur_stream()));
 }
 
+// a [M, K] times b [K, N] in bf16, the sum cut into parts that are added up in one order; nothing where it is not to be cut
+std::optional<Tensor> gemm_in_parts(const Tensor& a, const Tensor& b) {
+  need_bf16(a, "a"); need_bf16(b, "b");
+  need_rowmajor2d(a, "a"); need_rowmajor2d(b, "b");
+  TORCH_CHECK(a.size(1) == b.size(0), "gemm: reduction sizes differ (", a.size(1), " vs ", b.size(0), ")");
+  c10::cuda::CUDAGuard guard(a.device());
+  GemmDesc d = {};
+  d.M = static_cast<int>(a.size(0)); d.N = static_cast<int>(b.size(1)); d.K = static_cast<int>(a.size(1));
+  d.split_k = nmtg_gemm_parts(d.M, d.N, d.K, &d.force_bn);
+  if (d.split_k == 0) return std::nullopt;
+  Tensor parts = torch::empty({d.split_k, d.M, d.N}, a.options().dtype(torch::kFloat)), out = torch::empty({d.M, d.N}, a.options());
+  d.a = a.data_ptr(); d.lda = static_cast<int>(a.stride(0));
+  d.b = b.data_ptr(); d.ldb = static_cast<int>(b.stride(0)); d.b_mn_major = 1;
+  d.alpha = 1.f;
+  d.out = parts.data_ptr(); d.ld_out = d.N; d.out_fp32 = 1; d.part_rows = d.M;
+  d.status = status_ptr(a);
+  ck(nmtg_gemm_bf16(&d, cur_stream()));
+  ck(nmtg_sum_parts(parts.data_ptr<float>(), d.split_k, out.data_ptr(), out.numel(), cur_stream()));
+  return out;
+}
+
 std::vector<Tensor> layernorm_fwd(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps) {
   need_bf16(x, "x"); need_bf16(gamma, "gamma"); need_bf16(beta, "beta");
   TORCH_CHECK(x.is_contiguous() && x.dim() == 2);
@@ -587,6 +608,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return reinterpret_cast<int64_t>(s);
   });
   m.def("step_linear", &step_linear);
+  m.def("gemm_in_parts", &gemm_in_parts);
   m.def("set_step_overlap", [](bool on) { nmtg_set_step_overlap(on); });
   m.def("set_gemm_variant", [](int64_t v) { nmtg_set_gemm_variant(static_cast<int>(v)); });
   m.def("set_sm_reserve", [](int64_t n) { nmtg_set_sm_reserve(static_cast<int>(n)); });

@@ -39,6 +39,42 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 
 // One thread handles 16 consecutive elements (two 16-byte vectors, four hash words).
+// Parts of a long sum, added up in one order: the same bits whichever part was ready first.  Four elements to a thread; of many parts every
+// fourth of a warp takes a quarter, and the quarters meet in a fixed order, too.
+template <bool kMany>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float4* __restrict__ parts, int count, uint2* __restrict__ out, long n4) {
+  let_next_start();
+  wait_for_previous();
+  const int lane = threadIdx.x & 31, quarter = kMany ? lane >> 3 : 0;
+  const int each = kMany ? (count + 3) / 4 : count, begin = quarter * each, end = min(count, begin + each);
+  const long threads = static_cast<long>(gridDim.x) * blockDim.x, id = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  const long step = kMany ? threads / 4 : threads, first = kMany ? (id >> 5) * 8 + (lane & 7) : id;
+  for (long i0 = first - (kMany ? lane & 7 : 0); i0 < n4; i0 += step) {
+    const long i = i0 + (kMany ? lane & 7 : 0);
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n4) {
+#pragma unroll 8
+      for (int s = begin; s < end; ++s) {
+        const float4 a = parts[s * n4 + i];
+        f.x += a.x; f.y += a.y; f.z += a.z; f.w += a.w;
+      }
+    }
+    if constexpr (kMany) {
+#pragma unroll
+      for (int o = 8; o < 32; o <<= 1) {
+        f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
+        f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
+        f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
+        f.w += __shfl_xor_sync(0xffffffffu, f.w, o);
+      }
+    }
+    if (i < n4 && quarter == 0) {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
+      out[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+}
+
 __global__ void dropout_add_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                                    __nv_bfloat16* __restrict__ y, long n16, float p, unsigned long long seed,
                                    unsigned long long stream_id, const unsigned long long* seed_dev) {
@@ -326,6 +362,15 @@ using namespace b200;
 static const char* last_err() {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
+}
+
+const char* nmtg_sum_parts(const float* parts, int count, void* out, long n, cudaStream_t stream) {
+  if (n <= 0) return nullptr;
+  if (n % 8 || ((reinterpret_cast<uintptr_t>(parts) | reinterpret_cast<uintptr_t>(out)) & 15)) return "sum_parts: 16-byte pieces";
+  const bool many = count > 4;
+  const long blocks = (n / 4 * (many ? 4 : 1) + 255) / 256, cap = static_cast<long>(num_sms()) * 8;
+  return launch_overlapped(many ? sum_parts_kernel<true> : sum_parts_kernel<false>, static_cast<int>(blocks < cap ? blocks : cap), 256, 0, stream,
+                           reinterpret_cast<const float4*>(parts), count, reinterpret_cast<uint2*>(out), n / 4);
 }
 
 const char* nmtg_dropout_add(const void* x, const void* residual, void* y, long n, float p, unsigned long long seed,

@@ -369,8 +369,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_word, p.status, kTimeoutTmemFull)) break;
       if (tracing) { e_last = clock64(); e_wait += e_last - e0; }
       tc_fence_after_sync();
-      const int row = m0 + q * 32 + lane;
-      const bool row_ok = row < p.M;
+      const bool row_ok = m0 + q * 32 + lane < p.M;
+      const int row = m0 + q * 32 + lane + ((kFeat & kEpiF32) && p.part_rows ? kb_begin / kb_per_split * p.part_rows : 0);
       if ((kFeat & kEpiBf16) && p.tma_store) {
         // 64-column groups: both 32-column halves go to this warp's staging tile, one TMA store per group writes
         // full 128-byte lines (rows / columns outside the matrix are clipped by the copy engine)

@@ -13,7 +13,8 @@ constexpr int kEpilogueWarps = 8;   // two warps per TMEM lane quarter, interlea
 struct GemmArgs {
   int M, N, K;
   int a_mn_major, b_mn_major;
-  int split_k;             // >= 1; > 1 requires out_fp32 and atomic accumulation
+  int split_k;             // >= 1; > 1 requires out_fp32, and atomic accumulation or part_rows
+  int part_rows;           // > 0: part s of the sum over K is stored at row s * part_rows of the output, by itself
   int stream_k;            // CTA-pair kernel, fp32 accumulating output: equal runs of (tile, k-block) pairs per cluster
   float alpha;
   const __nv_bfloat16* bias;      // [N] or null
@@ -358,7 +359,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
     if ((kFeat & kEpiF32) && (p.out_fp32 || !(kFeat & kEpiBf16))) {
       float* op = reinterpret_cast<float*>(p.out) + static_cast<size_t>(row) * p.ld_out + col0;
       // accumulation into an existing fp32 buffer goes through the L2 reduction unit as well: no read round trip
-      if (p.split_k > 1 || p.accumulate || p.stream_k) {
+      if ((p.split_k > 1 && p.part_rows == 0) || p.accumulate || p.stream_k) {
         if (full_cols) {
 #pragma unroll
           for (int g = 0; g < 8; ++g)

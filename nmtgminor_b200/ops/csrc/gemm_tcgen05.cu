@@ -189,8 +189,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const uint32_t acc_phase = (it >> 1) & 1;
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_word, p.status, kTimeoutTmemFull)) break;
       tc_fence_after_sync();
-      const int row = m0 + q * 32 + lane;
-      const bool row_ok = row < p.M;
+      const bool row_ok = m0 + q * 32 + lane < p.M;
+      const int row = m0 + q * 32 + lane + ((kFeat & kEpiF32) && p.part_rows ? tile / (num_m * num_n) * p.part_rows : 0);
 #pragma unroll 1
       for (int c = chunk_par; c < BN / 32; c += kEpilogueWarps / 4) {
         const int col0 = n0 + c * 32;
@@ -510,6 +510,49 @@ static int one_wave_tile(const GemmDesc* d, int sms, int num_kb, int* split) {
   return bn;
 }
 
+// How a bf16 product with a long sum and a small output is cut into parts: their number, and the tile width (256: CTA pairs beyond 128 rows).  0 parts where
+// its 256 x 256 tiles occupy half of the CTA pairs or more: us, whole / in parts that are added up: 3842 x 512 over 32000, 32 tiles, 143 /
+// 107; 906 x 256 over 8000 36 / 13; 400 x 1024 over 250054 985 / 201; but 1856 x 1280 over 51865, 40 tiles, 262 / 301.  The widths are
+// weighed as in one_wave_tile.
+int nmtg_gemm_parts(int M, int N, int K, int* bn) {
+  const int sms = gemm_sms(), num_kb = (K + BK - 1) / BK;
+  const long pairs = static_cast<long>((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
+  if (M < 1 || N < 1 || pairs * 4 > sms || K < 4096 || N % 8) return 0;
+  int parts = 1;
+  double best = 1e30;
+  for (int w = 64; w <= 256; w *= 2) {
+    const bool pair = w == 256 && M > BM;
+    const long tiles = pair ? pairs : static_cast<long>((M + BM - 1) / BM) * ((N + w - 1) / w), slots = pair ? sms / 2 : sms;
+    if (tiles > slots) continue;
+    const long most = num_kb / (pair ? 8 : 6);
+    const int s = fix_split(static_cast<int>(slots / tiles < most ? slots / tiles : most), num_kb);
+    const double t = (w == 64 ? 5.6 : w == 128 ? 6.4 : pair ? 9.5 : 8.0) + (pair ? 0.36 : 0.31) * ((num_kb + s - 1) / s);
+    if (t < best) {
+      best = t;
+      parts = s;
+      *bn = w;
+    }
+  }
+  return parts > 1 ? parts : 0;
+}
+
+// Single-CTA kernel; bn = 64, 128 or 256, no part of the sum empty.
+static const char* launch_gemm_single(const GemmDesc* d, const GemmArgs& a, int bn, int sms, cudaStream_t stream) {
+  CUtensorMap ta, tb;
+  bool ok;
+  if (!d->a_mn_major) ok = cached_tmap(&ta, d->a, d->M, d->K, d->lda, BM, BK);
+  else ok = cached_tmap(&ta, d->a, d->K, d->M, d->lda, BK, 64);
+  if (!ok) return "gemm: cuTensorMapEncodeTiled failed for A";
+  if (!d->b_mn_major) ok = cached_tmap(&tb, d->b, d->N, d->K, d->ldb, bn, BK);
+  else ok = cached_tmap(&tb, d->b, d->K, d->N, d->ldb, BK, 64);
+  if (!ok) return "gemm: cuTensorMapEncodeTiled failed for B";
+  const long tiles = static_cast<long>((d->M + BM - 1) / BM) * ((d->N + bn - 1) / bn) * a.split_k;
+  const int grid = static_cast<int>(tiles < sms ? tiles : sms);
+  if (bn == 256) return launch_gemm<256>(ta, tb, a, grid, stream);
+  if (bn == 64) return launch_gemm_special<64>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
+  return launch_gemm_special<128>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
+}
+
 // Returns nullptr on success, else a static error string.
 const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   if (d->M <= 0 || d->N <= 0 || d->K <= 0) return nullptr;
@@ -533,6 +576,7 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
                    reinterpret_cast<uintptr_t>(d->preact)) & 15) != 0;
   a.ablate = g_gemm_ablate;
   a.stream_k = 0;
+  a.part_rows = d->part_rows;
   a.trace = g_gemm_trace;
   if (d->act == kActMaskBwd && !d->mask) return "gemm: the mask-backward epilogue needs a mask";
   a.act = d->act; a.dropout_p = d->dropout_p; a.seed = d->seed; a.stream_id = d->stream_id; a.seed_dev = d->seed_dev;
@@ -550,6 +594,13 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   };
   const int sms = gemm_sms();
   const int num_kb = (d->K + BK - 1) / BK;
+  if (d->part_rows) {      // nmtg_gemm_parts has chosen the kernel and the number of parts
+    if (!d->out_fp32 || d->accumulate || d->gather || d->bias || d->residual || d->aux || d->preact || d->mask || d->colsum || d->act || d->dropout_p > 0.f ||
+        d->part_rows < d->M || d->split_k < 1 || fix_split(d->split_k, num_kb) != d->split_k || (d->force_bn != 64 && d->force_bn != 128 && d->force_bn != 256))
+      return "gemm: a sum in parts is a plain fp32 product with no empty part";
+    a.split_k = d->split_k;
+    return d->force_bn == 256 && d->M > BM ? launch_gemm_pair(d, a, 256, stream) : launch_gemm_single(d, a, d->force_bn, sms, stream);
+  }
   // ---- skinny problems (incremental decoding: a few hundred rows): the weight matrix is streamed once, so the
   // only lever is the number of CTAs pulling it in: the narrowest tiles that are one wave (us, two waves of 64 columns / one of 128:
   // 256 x 8192 x 1024 14.5 / 10.5, 128 x 12288 x 4096 39.6 / 25.5; two of 128 / one of 256: 300 x 12288 x 4096 45.8 / 36.4), else the widest
@@ -640,19 +691,5 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
   }
   if (split > 1 && !d->out_fp32) return "gemm: split-K needs an fp32 output";
   a.split_k = fix_split(split, num_kb);
-
-  CUtensorMap ta, tb;
-  bool ok;
-  if (!d->a_mn_major) ok = cached_tmap(&ta, d->a, d->M, d->K, d->lda, BM, BK);
-  else ok = cached_tmap(&ta, d->a, d->K, d->M, d->lda, BK, 64);
-  if (!ok) return "gemm: cuTensorMapEncodeTiled failed for A";
-  if (!d->b_mn_major) ok = cached_tmap(&tb, d->b, d->N, d->K, d->ldb, bn, BK);
-  else ok = cached_tmap(&tb, d->b, d->K, d->N, d->ldb, BK, 64);
-  if (!ok) return "gemm: cuTensorMapEncodeTiled failed for B";
-
-  long tiles = static_cast<long>(num_m) * num_n * split;
-  int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  if (bn == 256) return launch_gemm<256>(ta, tb, a, grid, stream);
-  if (bn == 64) return launch_gemm_special<64>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
-  return launch_gemm_special<128>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
+  return launch_gemm_single(d, a, bn, sms, stream);
 }

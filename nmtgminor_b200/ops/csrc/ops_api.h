@@ -52,12 +52,17 @@ struct GemmDesc {
   int split_k;            // 0 = automatic (only when allow_split_k), else forced
   int allow_split_k;      // the sum over K may be split: fp32 outputs (atomic adds), and bf16 outputs with few rows (CTA clusters; the number of
                           // parts then depends on M, so that a row's last bit depends on how many rows stand beside it)
+  int part_rows;          // > 0: the split_k parts of the sum are stored by themselves, part s at row s * part_rows of an fp32 output (nmtg_gemm_parts)
   int force_bn;           // 0 = automatic, 128 or 256, or 64 with the single-CTA kernel (nmtg_set_gemm_variant(1), M <= 128)
   int* status;            // device int, 0 = ok
   const NmtgGather* gather;  // optional: B is gathered from its owners by this call (see NmtgGather)
 };
 
 const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream);
+// Parts (0: none) and tile width for a product whose sum is long and whose output is small; nmtg_sum_parts adds them up.
+int nmtg_gemm_parts(int M, int N, int K, int* bn);
+// out (bf16, n elements, n % 8 == 0) = parts[0] + parts[1] + ..., in this order, in 32 bits
+const char* nmtg_sum_parts(const float* parts, int count, void* out, long n, cudaStream_t stream);
 // out[M, N] = [residual +] act([LayerNorm](x) W^T + bias) for the few rows of a decoding step (step_linear.cu).  gamma / beta null: no
 // LayerNorm.  The sum over K is cut into parts, as in a product that allows split_k.
 int nmtg_step_linear_takes(int M, int N, int K, int norm);

@@ -499,6 +499,22 @@ def test_long_sums_of_small_outputs(M, N, K):
     assert ops.check_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(906, 256, 8000), (400, 1024, 30011), (100, 512, 4100), (130, 64, 60000)])
+def test_long_sums_repeat(M, N, K):
+    """The parts of a long sum meet in one order: the same bits every time, whatever else keeps the GPU busy."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    dz = ops.empty_rows(M, K, torch.device("cuda"))
+    dz.copy_(torch.randn(M, K, device="cuda", generator=g))
+    w = torch.randn(K, N, device="cuda", generator=g).bfloat16()
+    want, side = ops._long_sum_gemm(dz, w), torch.cuda.Stream()
+    for i in range(12):
+        with torch.cuda.stream(side):
+            busy = torch.randn(1 << (14 + i % 6), device="cuda").sort()
+        assert torch.equal(ops._long_sum_gemm(dz, w), want)
+    torch.cuda.synchronize()
+    assert ops.check_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(129, 4744, 72), (129, 9544, 64), (257, 6400, 136), (300, 12288, 64), (512, 9984, 64), (512, 12003, 200),
                                    (100, 20000, 80), (256, 51865, 64)])
 @pytest.mark.parametrize("epilogue", ["plain", "residual", "gelu"])
