@@ -138,8 +138,11 @@ def conv1d(x, weight, bias=None, stride: int = 1, act: str = "none", padding: in
 
 
 def _watched() -> bool:
-    """Whether a mode or a hook of all modules has to see the tensor operations that a kernel would replace."""
-    return (torch.is_autocast_enabled() or torch.jit.is_tracing() or torch._C._are_functorch_transforms_active()
+    """Whether a mode or a hook of all modules has to see the tensor operations that a kernel would replace.  (The mode of a default
+    device only looks at calls that make tensors.)"""
+    return (torch._C._len_torch_dispatch_stack() > 0
+            or any(type(m) is not torch.utils._device.DeviceContext for m in torch.overrides._get_current_function_mode_stack())
+            or torch.is_autocast_enabled() or torch.jit.is_tracing() or torch._C._are_functorch_transforms_active()
             or torch.autograd.forward_ad._current_level >= 0 or torch.nn.modules.module._has_any_global_hook())
 
 
@@ -215,7 +218,7 @@ class _WeightNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dw):
         v, gain, norm = ctx.saved_tensors
-        if torch.is_grad_enabled():          # a graph of the gradient is wanted: the same as differentiable operations
+        if torch.is_grad_enabled() or _watched():          # a graph of the gradient is wanted, or its operations: the same as those
             dims = tuple(range(v.dim() - 1))
             n = v.square().sum(dims, keepdim=True).sqrt()
             dot = (dw * v).sum(dims, keepdim=True)

@@ -134,3 +134,48 @@ def test_weight_norm_kernels(shape):
     assert dv2.requires_grad and torch.allclose(dv2, dv, rtol=1e-4, atol=1e-5) and torch.allclose(dg2, dg, rtol=1e-4, atol=1e-4)
     conv.register_forward_hook(lambda *a: None)
     assert C.weight_normed(conv) is None
+
+
+def test_modes_see_the_operations_that_kernels_replace():
+    """Under a dispatch or function mode (a counter, a trace) the normalisation of the weights and the front end are tensor operations."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from nmtgminor_b200.models.speech_encoders import ConvFeatureExtractor, ConvPositionalEmbedding
+
+    class Dispatched(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    class Called(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    seen, pos = [], ConvPositionalEmbedding(128, 16, 2).cuda()
+    x = torch.randn(2, 40, 128, device="cuda")
+    want = torch.autograd.grad(pos(x).square().sum(), list(pos.parameters()))
+    with Dispatched():
+        loss = pos(x).square().sum()
+        assert any("norm" in name for name in seen)
+        del seen[:]
+        got = torch.autograd.grad(loss, list(pos.parameters()))
+        assert any("norm" in name for name in seen)
+    for a, b in zip(got, want):
+        # the library's convolution rounds its operands to 11 bits (2^-11 each), and weights a last bit apart round differently
+        assert (a - b).norm() <= 2 ** -10 * b.norm()
+    fe = ConvFeatureExtractor([(256, 10, 5), (256, 3, 2)]).cuda()
+    FlatParameterStore(fe, "cuda")
+    wav = torch.randn(2, 4000, device="cuda")
+    with torch.no_grad():
+        for mode in (Dispatched(), Called()):
+            with mode:
+                assert C.weight_normed(pos.conv) is None and C.frozen_front_end(wav, fe.convs, fe.norms) is None
+        with torch.device("cuda"):            # a default device is no such mode
+            assert C.weight_normed(pos.conv) is not None and C.frozen_front_end(wav, fe.convs, fe.norms) is not None
+    # a graph that is recorded under the mode's eyes later: the forward pass ran outside
+    loss = pos(x).square().sum()
+    del seen[:]
+    with Dispatched():
+        torch.autograd.grad(loss, list(pos.parameters()))
+    assert any("sum" in name for name in seen)
