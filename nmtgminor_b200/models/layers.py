@@ -678,12 +678,19 @@ class DecoderLayer(nn.Module, _LayerOptions):
                 x = self.cross_norm(x + self.cross_attn.step(x, cache, mem_mask))
             return self.ffn_norm(self.ffn(x, residual=x))
         # LayerNorm in front of the projections, residual add in their epilogues
-        x = self.self_attn.step(x, cache, residual=x, norm=self.self_norm)
+        x = _attn_step(self.self_attn, SelfAttention, self.self_norm, x, cache)
         if self.interleaved_ffn:
             x = _ffn_step(self.mid_ffn, x, self.mid_norm)
         if not self.ignore_source:
-            x = self.cross_attn.step(x, cache, mem_mask, residual=x, norm=self.cross_norm)
+            x = _attn_step(self.cross_attn, CrossAttention, self.cross_norm, x, cache, mem_mask)
         return _ffn_step(self.ffn, x, self.ffn_norm)
+
+
+def _attn_step(attn, cls, norm, x, *rest):
+    """``x + attn(norm(x))`` of a decoding step; a class (or an object) with a ``step`` of its own gets normalised rows."""
+    if getattr(attn.step, "__func__", None) is cls.step:
+        return attn.step(x, *rest, residual=x, norm=norm)
+    return attn.step(norm(x), *rest, residual=x)
 
 
 def _ffn_step(ffn, x, norm):

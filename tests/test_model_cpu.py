@@ -211,3 +211,38 @@ def test_packing_with_the_total_known(lengths, capacity):
     assert torch.equal(a, b) and torch.equal(sa.positions, sb.positions) and torch.equal(sa.cu, sb.cu) and sa.max_len == sb.max_len
     w = torch.randn_like(a)
     assert torch.equal(torch.autograd.grad((a * w).sum(), x)[0], torch.autograd.grad((b * w).sum(), x)[0])
+
+
+def _steps(model, tokens=4):
+    """Hidden states of the decoder's steps over a fixed target."""
+    batch = collate([torch.arange(4, 12)], [torch.arange(2, 2 + tokens + 2)], padded=True, packed=True, round_to=1)
+    state = model.create_decoder_state(batch, beam_size=1)
+    ids = torch.arange(2, 2 + tokens)[None]
+    with torch.no_grad():
+        return torch.stack([model.step(ids[:, :i + 1], state, logits_only=True)["logits"] for i in range(tokens)])
+
+
+@pytest.fixture
+def small_model():
+    d = synthetic_dict(60)
+    torch.manual_seed(3)
+    return build_model(default_options(["-model", "transformer", "-model_size", "64", "-layers", "2", "-n_heads", "1", "-inner_size", "128",
+                                        "-ffn_activation", "relu"]), {"src": d, "tgt": d}).eval()
+
+
+def test_attention_with_a_step_of_its_own(small_model):
+    """An attention class whose ``step`` knows nothing of norms is handed normalised rows."""
+    from nmtgminor_b200.models.layers import CrossAttention, SelfAttention
+    want = _steps(small_model)
+
+    class Own(SelfAttention):
+        def step(self, x, cache, residual=None):
+            return super().step(x, cache, residual=residual)
+
+    class OwnCross(CrossAttention):
+        def step(self, x, cache, mem_mask, residual=None):
+            return super().step(x, cache, mem_mask, residual=residual)
+
+    for layer in small_model.decoder.layers:
+        layer.self_attn.__class__, layer.cross_attn.__class__ = Own, OwnCross
+    assert torch.equal(_steps(small_model), want)
