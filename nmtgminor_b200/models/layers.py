@@ -135,7 +135,8 @@ class Linear(nn.Module):
 
 def _plain(m, cls) -> bool:
     """Whether calling ``m`` is calling ``cls.forward`` and nothing else."""
-    return type(m) is cls and not (m._forward_hooks or m._forward_pre_hooks or nn.modules.module._has_any_global_hook())
+    return (type(m) is cls and "forward" not in m.__dict__
+            and not (m._forward_hooks or m._forward_pre_hooks or nn.modules.module._has_any_global_hook()))
 
 
 def _normed(norm, linear, x):

@@ -230,6 +230,34 @@ def small_model():
                                         "-ffn_activation", "relu"]), {"src": d, "tgt": d}).eval()
 
 
+def test_a_decoding_step_calls_hooked_modules(small_model):
+    """Norms, projections and feed-forward blocks of a step run their hooks, and a hook's output counts."""
+    want = _steps(small_model)
+    layer = small_model.decoder.layers[1]
+    for module in (layer.self_norm, layer.self_attn.qkv, layer.cross_norm, layer.cross_attn.q, layer.ffn_norm, layer.ffn):
+        calls = []
+        for kind, register in (("pre", module.register_forward_pre_hook), ("post", module.register_forward_hook)):
+            hook = register(lambda *a: calls.append(kind))
+            assert torch.equal(_steps(small_model), want)
+            hook.remove()
+        assert calls == ["pre"] * 4 + ["post"] * 4
+        hook = module.register_forward_hook(lambda m, a, out: out * 0.5)
+        assert not torch.allclose(_steps(small_model), want)
+        hook.remove()
+
+
+def test_a_decoding_step_calls_a_replaced_forward(small_model):
+    """A module whose ``forward`` was replaced on the object (as adapters and quantisers do) is called through it."""
+    want = _steps(small_model)
+    layer = small_model.decoder.layers[0]
+    for module in (layer.self_norm, layer.self_attn.qkv, layer.cross_norm, layer.cross_attn.q, layer.ffn_norm, layer.ffn):
+        inner = module.forward
+        module.forward = lambda *a, **k: inner(*a, **k) * 0.5
+        assert not torch.allclose(_steps(small_model), want)
+        del module.forward
+    assert torch.equal(_steps(small_model), want)
+
+
 def test_attention_with_a_step_of_its_own(small_model):
     """An attention class whose ``step`` knows nothing of norms is handed normalised rows."""
     from nmtgminor_b200.models.layers import CrossAttention, SelfAttention
