@@ -408,6 +408,7 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         uint8_t* s = sSlots + slot * kBwdSlotBytes;
         if (ablate & 16) {
           mbar_arrive(&slot_full[slot]);
+          if (!mbar_wait(o_free, (it & 1) ^ 1, abort_word, p.status, kTimeoutSmemEmpty)) break;
           mbar_arrive(o_full);
           ++it;
           continue;

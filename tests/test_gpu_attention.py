@@ -389,3 +389,24 @@ def test_pipelined_backward_replays_the_dropout_mask_on_long_sequences():
     lhs = (o_dir.float() * do.float()).sum().item()
     rhs = (dv * dirv.float()).sum().item()
     assert abs(lhs - rhs) <= 3e-2 * max(1.0, abs(lhs)), (lhs, rhs)
+
+
+@pytest.mark.parametrize("bits", [1, 2, 4, 8, 16, 32, 19, 31])
+def test_ablated_backward_keeps_its_hand_shakes(bits):
+    """With parts of the work switched off for timing no wait of the one-tile backward pass runs out."""
+    e, heads, W, lens = ops.ext(), 4, 256, [5, 100, 128, 33, 64, 1, 77, 20] * 24
+    cu = torch.tensor([0] + lens).cumsum(0).int().cuda()
+    n = int(cu[-1])
+    qkv, dout = torch.randn(n, 3 * W, device="cuda").bfloat16(), torch.randn(n, W, device="cuda").bfloat16()
+    out, lse = torch.empty(n, W, dtype=torch.bfloat16, device="cuda"), torch.empty(heads, n, device="cuda")
+    q, k, v = qkv[:, :W], qkv[:, W:2 * W], qkv[:, 2 * W:]
+    e.attn_fwd(q, k, v, out, lse, cu, cu, heads, 128, 128, False, 0.125, 0.1, 1, 1)
+    grads = torch.zeros_like(qkv)
+    try:
+        e.set_attn_bwd_ablation(bits)
+        for _ in range(3):
+            e.attn_bwd(q, k, v, out, lse, dout, grads[:, :W], grads[:, W:2 * W], grads[:, 2 * W:], None, cu, cu, heads, 128, 128, False, 0.125, 0.1, 1, 1)
+        torch.cuda.synchronize()
+    finally:
+        e.set_attn_bwd_ablation(0)
+    assert ops.check_status() == 0
