@@ -31,7 +31,8 @@ struct Item {
   bool valid = false;
 };
 
-__device__ __forceinline__ Item get_item(const AttnArgs& p, int item) {
+// `report`: this thread's look-ups are the ones that the debug build counts bad offsets in (one thread of a CTA that looks at every item)
+__device__ __forceinline__ Item get_item(const AttnArgs& p, int item, bool report = false) {
   Item it;
   const int b = item / p.num_heads;
   it.h = item - b * p.num_heads;
@@ -42,7 +43,7 @@ __device__ __forceinline__ Item get_item(const AttnArgs& p, int item) {
   it.valid = it.q_len > 0 && it.k_len > 0 && it.q_len <= kTile && it.k_len <= kTile;
   // a sequence that does not fit one tile (or offsets that run backwards) is skipped by every role of the kernel; the host
   // dispatch sends such batches to the general kernels, so meeting one here means the offsets are wrong
-  if (!it.valid && (it.q_len < 0 || it.k_len < 0 || it.q_len > kTile || it.k_len > kTile) && threadIdx.x == 0) NMTG_BOUNDS_HIT();
+  if (!it.valid && (it.q_len < 0 || it.k_len < 0 || it.q_len > kTile || it.k_len > kTile) && report) NMTG_BOUNDS_HIT();
   return it;
 }
 
@@ -107,10 +108,10 @@ attn_fwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     if (lane == 0) {
       int it = 0;
       bool ok = true;
-      Item nxt = static_cast<int>(blockIdx.x) < num_items ? get_item(p, blockIdx.x) : Item{};
+      Item nxt = static_cast<int>(blockIdx.x) < num_items ? get_item(p, blockIdx.x, true) : Item{};
       for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
         const Item w = nxt;
-        if (item + static_cast<int>(gridDim.x) < num_items) nxt = get_item(p, item + gridDim.x);
+        if (item + static_cast<int>(gridDim.x) < num_items) nxt = get_item(p, item + gridDim.x, true);
         if (!w.valid) continue;
         const int slot = it % kFwdGroups;
         if (!mbar_wait(&slot_empty[slot], ((it / kFwdGroups) & 1) ^ 1, abort_word, p.status, kTimeoutSmemEmpty)) { ok = false; break; }
@@ -401,7 +402,7 @@ attn_bwd_short_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     if (lane == 0) {
       int it = 0;
       for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
-        const Item w = get_item(p, item);
+        const Item w = get_item(p, item, true);
         if (!w.valid) continue;
         const int slot = it & 1;
         if (!mbar_wait(&slot_empty[slot], ((it >> 1) & 1) ^ 1, abort_word, p.status, kTimeoutSmemEmpty)) break;

@@ -410,3 +410,33 @@ def test_ablated_backward_keeps_its_hand_shakes(bits):
     finally:
         e.set_attn_bwd_ablation(0)
     assert ops.check_status() == 0
+
+
+_BAD_OFFSETS = """
+import torch
+from nmtgminor_b200 import ops
+e, heads, W = ops.ext(), 2, 128
+cu = torch.tensor([0, 20, 149, 140, 200], dtype=torch.int32, device="cuda")       # 20, 129, -9 and 60 tokens
+qkv, dout = torch.randn(200, 3 * W, device="cuda").bfloat16(), torch.randn(200, W, device="cuda").bfloat16()
+out, lse = torch.zeros(200, W, dtype=torch.bfloat16, device="cuda"), torch.zeros(heads, 200, device="cuda")
+q, k, v = qkv[:, :W], qkv[:, W:2 * W], qkv[:, 2 * W:]
+counts = [e.bounds_violations()]
+for p in (0.0, 0.1):
+    e.attn_fwd(q, k, v, out, lse, cu, cu, heads, 128, 128, False, 0.125, p, 1, 1)
+    counts.append(e.bounds_violations())
+    grads = torch.zeros_like(qkv)
+    e.attn_bwd(q, k, v, out, lse, dout, grads[:, :W], grads[:, W:2 * W], grads[:, 2 * W:], None, cu, cu, heads, 128, 128, False, 0.125, p, 1, 1)
+    counts.append(e.bounds_violations())
+assert counts in ([-1] * 5, [2 * heads * i for i in range(5)]), counts
+assert out[:20].any() and out[140:].any() and not out[20:140].any()
+assert ops.check_status() == 0
+"""
+
+
+def test_bad_offsets_are_counted_in_the_debug_build():
+    """A build with NMTG_DEBUG_BOUNDS=1 counts sequences that do not fit a tile, or run backwards, once per head in each direction; every build
+    skips them.  In a process of its own: other tests assert that this one has counted none."""
+    import subprocess
+    import sys
+    ran = subprocess.run([sys.executable, "-c", _BAD_OFFSETS], capture_output=True, text=True, timeout=300)
+    assert ran.returncode == 0, ran.stderr[-2000:]
