@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t round2(Pair x) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-constexpr int kFrontWarps = 8, kFrames = 4, kTaps = 16;      // taps: at most
+constexpr int kFrontWarps = 8, kFrames = 4, kTaps = 16, kStride = 64;      // taps and stride: at most
 
 // A warp takes four neighbouring frames of an utterance, a lane the channel pairs 2 lane + 64 j: the weights of a tap are read from shared
 // memory once for the four.
@@ -160,11 +160,8 @@ int front_grid(long warps_of_work) {
 template <int kPairs>
 const char* launch_conv(const float* wav, long wav_stride, const float* w, const float* bias, const float* gamma, const float* beta, float eps,
                         __nv_bfloat16* out, int B, int samples, int T, int out_rows, int taps, int stride, cudaStream_t stream) {
+  static_assert(sizeof(float) * ((kTaps + 3) * 64 * kPairs + kFrontWarps * ((kFrames - 1) * kStride + kTaps)) <= 48 * 1024, "shared memory");
   const size_t smem = sizeof(float) * ((taps + 3) * 64 * kPairs + kFrontWarps * ((kFrames - 1) * stride + taps));
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(conv_norm_gelu_kernel<kPairs>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return cudaGetErrorString(e);
-  }
   conv_norm_gelu_kernel<kPairs><<<front_grid(static_cast<long>(B) * ((T + kFrames - 1) / kFrames)), 32 * kFrontWarps, smem, stream>>>(
       wav, wav_stride, w, bias, gamma, beta, eps, out, B, samples, T, out_rows, taps, stride);
   cudaError_t e = cudaGetLastError();
@@ -182,7 +179,7 @@ const char* nmtg_conv_norm_gelu(const float* wav, long wav_stride, const float* 
                                 float eps, void* out, int B, int samples, int T, int out_rows, int channels, int taps, int stride,
                                 cudaStream_t stream) {
   if (B <= 0 || T <= 0) return nullptr;
-  if (taps < 1 || taps > kTaps || stride < 1 || stride > 64 || out_rows < T || static_cast<long>(T - 1) * stride + taps > samples)
+  if (taps < 1 || taps > kTaps || stride < 1 || stride > kStride || out_rows < T || static_cast<long>(T - 1) * stride + taps > samples)
     return "conv_norm_gelu: sizes out of range";
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   switch (channels) {

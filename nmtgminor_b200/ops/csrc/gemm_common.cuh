@@ -90,11 +90,6 @@ __device__ __forceinline__ float gelu_f(float x) {
   float bell;
   return x * normal_cdf(x, bell);
 }
-__device__ __forceinline__ float gelu_grad(float x) {
-  float bell;
-  const float cdf = normal_cdf(x, bell);
-  return cdf + x * (0.3989422804014327f * bell);
-}
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 
 // Two elements at a time: the 32-bit pairs of sm_100 (one instruction, both halves rounded as the single one rounds).

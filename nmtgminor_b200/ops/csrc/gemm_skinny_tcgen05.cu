@@ -303,12 +303,13 @@ static int skinny_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 // with programmatic launch / the tiled kernel): 1024 x 1024, 4 rows
 // 3.6 / 8.4, 256 rows 7.2 / 9.3, 512 rows 7.5 / 9.3; 4096 x 1024, 64 rows 6.0 / 8.6; 1024 x 4096, 4 rows 5.4 / 22.8; 32000 x
 // 1024, 33 rows 13.9 / 20.3.  Beyond one wave (32000 x 1024 with 128 rows: 25 us against 19) the tiled kernel is the better one; up to 32 rows
-// two waves are no slower (51865 x 1280, 4 rows 30.4 / 36.1, 20 rows 32.5 / 35.0, 32 rows 32.9 / 32.6, 48 rows 36.6 / 30.6).
+// two waves are no slower (51865 x 1280, six matrices in turn, 4 rows 28.8 / 31.9, 17 rows 30.7 / 30.2, 20 rows 30.7 / 32.0, 28 rows 30.9 / 31.4,
+// 32 rows 31.3 / 31.8; 48 rows 31.2 / 31.3).
 bool skinny_takes(const GemmDesc* d, int sms) {
   const long tiles = static_cast<long>((d->N + kSkinnyFeat - 1) / kSkinnyFeat) * ((d->M + skinny_rows(d->M) - 1) / skinny_rows(d->M));
   return d->allow_split_k && d->M <= 512 && tiles <= (d->M <= 32 ? 4L : 2L) * sms && !d->out_fp32 && !d->a_mn_major && !d->b_mn_major && !d->gather && !d->preact && !d->mask &&
          !d->colsum && !d->aux && d->act >= 0 && d->act <= kActSilu && d->dropout_p <= 0.f && d->split_k <= 1 && d->force_bn == 0 &&
-         d->ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(d->out) & 7) == 0 && (!d->residual || d->N % 4 == 0) && (!d->residual || (d->ld_res % 4 == 0 && (reinterpret_cast<uintptr_t>(d->residual) & 7) == 0)) &&
+         (!d->residual || (d->N % 4 == 0 && d->ld_res % 4 == 0 && (reinterpret_cast<uintptr_t>(d->residual) & 7) == 0)) &&
          (reinterpret_cast<uintptr_t>(d->bias) & 7) == 0;
 }
 
