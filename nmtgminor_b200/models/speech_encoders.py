@@ -50,6 +50,11 @@ def compute_mask_spans(B: int, T: int, lengths, mask_prob: float, mask_length: i
     return mask
 
 
+def _sent(mask, device):
+    """A mask made on the host, on ``device``; the host does not wait for what the device has still to do before."""
+    return mask.pin_memory().to(device, non_blocking=True) if device.type == "cuda" else mask.to(device)
+
+
 class ConvFeatureExtractor(nn.Module):
     """7-layer strided Conv1d stack over the raw waveform (total stride 320).  ``mode='layer_norm'`` normalises every
     layer's channels; ``mode='default'`` applies GroupNorm on the first layer only."""
@@ -246,9 +251,9 @@ class Wav2Vec2Encoder(nn.Module):
             raise ValueError("this encoder has language adapters: the batch must carry its source language id")
         feats, lengths = split_audio_batch(source)
         wav = feats[:, :, 0].float()
-        # the number of frames is asked for before the front end runs: the host then launches ahead of the device all the way
+        # the numbers of frames are asked for once, before the front end runs: the host then launches ahead of the device all the way
         frames = int(self.extractor.output_lengths(torch.tensor(wav.shape[1])))
-        total = int(self.extractor.output_lengths(lengths).clamp(max=frames).sum()) if wav.is_cuda else None
+        known = self.extractor.output_lengths(lengths).clamp(max=frames).cpu() if wav.is_cuda else None
         if self.freeze_extractor:
             with torch.no_grad():
                 x = self.extractor(wav)
@@ -259,17 +264,19 @@ class Wav2Vec2Encoder(nn.Module):
         if self.dropout_input > 0:
             x = F.dropout(x, self.dropout_input, self.training)
         B, T, _ = x.shape
+        if T != frames:
+            known = None
         valid = torch.arange(T, device=x.device)[None, :] < out_len[:, None]
         if self.training and self.mask_prob > 0:
-            m = compute_mask_spans(B, T, out_len.cpu(), self.mask_prob, self.mask_length).to(x.device)
+            m = _sent(compute_mask_spans(B, T, out_len.cpu() if known is None else known, self.mask_prob, self.mask_length), x.device)
             x = torch.where(m.unsqueeze(-1), self.mask_emb.to(x.dtype).expand_as(x), x)
         if self.training and self.mask_channel_prob > 0:
             full = torch.full((B,), x.shape[2], dtype=torch.long)
-            cm = compute_mask_spans(B, x.shape[2], full, self.mask_channel_prob, self.mask_channel_length).to(x.device)
+            cm = _sent(compute_mask_spans(B, x.shape[2], full, self.mask_channel_prob, self.mask_channel_length), x.device)
             x = x.masked_fill(cm.unsqueeze(1), 0.0)
         x = x * valid.unsqueeze(-1)
         x = x + self.pos_conv(x)
-        packed, seqs = pack_padded(x, out_len, total=total if T == frames else None)
+        packed, seqs = pack_padded(x, out_len, total=None if known is None else int(known.sum()))
         packed = packed.to(torch.bfloat16) if (packed.is_cuda and ops.fused_param(self.input_norm.weight)) else packed
         if not self.layer_norm_first:
             packed = self.input_norm(packed)

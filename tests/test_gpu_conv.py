@@ -179,3 +179,28 @@ def test_modes_see_the_operations_that_kernels_replace():
     with Dispatched():
         torch.autograd.grad(loss, list(pos.parameters()))
     assert any("sum" in name for name in seen)
+
+
+@pytest.mark.parametrize("masked", [False, True])
+def test_a_speech_encoder_waits_for_the_device_once(masked):
+    """Lengths reach the host before the front end runs; masks that are drawn from them go the other way without a wait."""
+    import warnings
+
+    from nmtgminor_b200.models.speech_encoders import Wav2Vec2Encoder
+    p = 0.5 if masked else 0.0
+    enc = Wav2Vec2Encoder(dim=128, layers=2, heads=2, ffn=256, conv_layers=[(256, 10, 5), (256, 3, 2)], pos_kernel=16, pos_groups=2, mask_prob=p,
+                          mask_length=3, mask_channel_prob=p, mask_channel_length=8).cuda().train()
+    FlatParameterStore(enc, "cuda")
+    source = torch.randn(3000, 3, 2, device="cuda")
+    source[:, :, 0] = torch.arange(3000, device="cuda")[:, None] < torch.tensor([3000, 1234, 700], device="cuda")
+    x, seqs = enc(source)
+    assert x.shape[0] == int(seqs.cu[-1]) == sum(((n - 10) // 5 + 1 - 3) // 2 + 1 for n in (3000, 1234, 700)) and torch.isfinite(x).all()
+    with warnings.catch_warnings(record=True) as seen:
+        warnings.simplefilter("always")
+        torch.cuda.set_sync_debug_mode("warn")
+        try:
+            enc(source)
+        finally:
+            torch.cuda.set_sync_debug_mode("default")
+    waits = ["%s:%d" % (w.filename, w.lineno) for w in seen if "called a synchronizing" in str(w.message)]
+    assert len(waits) == 1, waits
