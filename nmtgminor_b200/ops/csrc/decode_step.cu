@@ -900,9 +900,12 @@ const char* launch_self(const void* qkv, long ld, void* kc, void* vc, const int*
                         int cap, float scale, int sms, cudaStream_t stream) {
   const Groups of(K);
   const long ctas = static_cast<long>(heads) * B * of.count;
-  // many small CTAs where they fill the GPU: 64 sentences x 4 hypotheses x 16 heads, 80 words of past of their own: two warps 24.6 us,
-  // four 30.2, one 33.5 (memory: 13.4); 8 sentences x 20 heads, 50 words: eight warps 6.7
-  const int warps = ctas > 4L * sms ? 2 : ctas > 2L * sms ? 4 : 8;
+  // as many warps to a CTA as the GPU holds at once, 16 to an SM with several hypotheses (128 registers): 64 sentences x 4 hypotheses x 16
+  // heads, 80 words of past of their own: two warps 24.6 us, four 30.2, one 33.5 (memory: 13.4); 8 sentences x 20 heads, 50 words:
+  // eight warps 6.7.  24 to an SM with one hypothesis, and a block of keys for every warp (us, with the product before it, two warps / by
+  // this rule: 32 sentences x 20 heads, 186 words 23.1 / 18.1; 61 x 12, 106 words 18.1 / 14.5; four warps: 20 x 16, 80 words 10.8 / 10.1)
+  int warps = kStepWarps;
+  while (warps > 2 && (ctas * warps > (K == 1 ? 24L : 16L) * sms || (K == 1 && 16 * warps > cap))) warps >>= 1;
   return by_rows(B * of.count, [&](int first, int n) {
     return launch(K == 1 ? decode_self_kernel<1> : decode_self_kernel<4>, dim3(heads, n), dim3(32 * warps), warps * kQueries * kRowLd * sizeof(float), 1, stream,
                   static_cast<const __nv_bfloat16*>(qkv), ld, static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), anc, pos_rows,

@@ -611,3 +611,9 @@ def test_infinite_values_of_a_step(K):
     vc[0, 20, 7], vc[R - 1, 35, 100], qkv[K - 1, 2 * hid + 9] = inf, inf, -inf
     want[:K, 7], want[R - 1, 100], want[K - 1, 9] = inf, inf, -inf
     assert torch.equal(step(), want)
+
+
+@pytest.mark.parametrize("B,heads,cap,pos", [(30, 16, 64, 50), (30, 16, 192, 131), (28, 16, 128, 127), (56, 16, 320, 300), (3, 2, 64, 40)])
+def test_step_self_attention_of_one_hypothesis(B, heads, cap, pos):
+    """Greedy searches on either side of every line between two, four and eight warps to a CTA."""
+    test_step_self_attention(B, 1, heads, cap, pos)
