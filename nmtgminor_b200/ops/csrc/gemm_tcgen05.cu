@@ -125,7 +125,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------- UMMA issuer ---------------------------------------------
-    {                       // all lanes: see elect_one
+    // All lanes, see elect_one; one lane for tiles of 256 columns, whose MMAs take as long as their issue and where the other lanes' polling
+    // only costs (us, one lane / all: 384 x 32000 x 1024 31 / 33, 384 x 51865 x 768 42 / 45; but 64 x 4096 x 4096, 64 columns, 19.7 / 17.4)
+    constexpr bool kWarp = BN < 256;
+    if (kWarp || lane == 0) {
       const uint32_t idesc = make_idesc_bf16(BM, BN, p.a_mn_major, p.b_mn_major);
       const uint32_t a_lbo = p.a_mn_major ? BK * 128 : 16, b_lbo = p.b_mn_major ? BK * 128 : 16;
       const uint32_t a_kstep = p.a_mn_major ? (16 * 128) >> 4 : 32 >> 4;  // descriptor units of 16 B
@@ -141,20 +144,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (kb_begin >= kb_end) continue;  // empty split range: no accumulator is produced
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!all_lanes(mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_word, p.status, kTimeoutTmemEmpty))) break;
+        if (!all_lanes<kWarp>(mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_word, p.status, kTimeoutTmemEmpty))) break;
         tc_fence_after_sync();
-        const uint32_t d_tmem = uniform(tmem_base) + acc * BN;
+        const uint32_t d_tmem = (kWarp ? uniform(tmem_base) : tmem_base) + acc * BN;
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!all_lanes(mbar_wait(&full_bar[stage], phase, abort_word, p.status, kTimeoutTmaFull))) {
+          if (!all_lanes<kWarp>(mbar_wait(&full_bar[stage], phase, abort_word, p.status, kTimeoutTmaFull))) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          const uint32_t sa = uniform(smem_u32(smem)) + stage * S::kStageBytes;
+          const uint32_t sa = (kWarp ? uniform(smem_u32(smem)) : smem_u32(smem)) + stage * S::kStageBytes;
           const uint32_t sb = sa + S::kABytes;
           const uint64_t adesc = make_smem_desc_sw128(sa, a_lbo, 1024);
           const uint64_t bdesc = make_smem_desc_sw128(sb, b_lbo, 1024);
-          if (elect_one()) {
+          if (!kWarp || elect_one()) {
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k)
               umma_bf16(d_tmem, adesc + static_cast<uint64_t>(k * a_kstep), bdesc + static_cast<uint64_t>(k * b_kstep),
@@ -166,7 +169,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             phase ^= 1;
           }
         }
-        if (ok && elect_one()) umma_commit(&tmem_full[acc]);
+        if (ok && (!kWarp || elect_one())) umma_commit(&tmem_full[acc]);
         ++it;
       }
     }
