@@ -625,10 +625,14 @@ const char* nmtg_gemm_bf16(const GemmDesc* d, cudaStream_t stream) {
     // Where 128 columns are more than one wave, the 256-row tiles of the CTA-pair kernel read every weight once instead of once per 128 rows
     // (us, here / pairs: 256 x 32000 x 1024 25.6 / 20.5, 256 x 250056 x 1024 157 / 129, 512 x 32000 x 512 29.6 / 21.5, 400 x 6144 x 2048
     // 25.9 / 17.2).  Not with an odd number of 128-row halves beyond one wave of pairs (320 x 250056 x 1024 199 / 208), nor with a second
-    // wave of a few tiles (400 x 10000 x 512 15.3 / 16.7); in one wave the narrow tiles are sooner done (256 x 4096 x 1024 8.9 / 11.8).
+    // wave that is less than half full (400 x 10000 x 512 15.3 / 16.7, 512 x 12000 x 256 14.7 / 16.4, x 1280 25.3 / 25.0); in one wave the narrow tiles are
+    // sooner done (256 x 4096 x 1024 8.9 / 11.8).  Widths that need the general epilogue pay more for it in pairs, which only a long sum or
+    // many waves make good (160 x 32001 x 256 14.1 / 17.3, x 1024 22.4 / 23.3, x 1280 28.4 / 27.2; 51865 columns, x 256 20.8 / 21.0, x 1024 36 / 33).
     if (d->M > BM && tiles_of(128) > sms) {
       const long pairs = static_cast<long>((num_m + 1) / 2) * ((d->N + 255) / 256), clusters = sms / 2;
-      if (pairs <= clusters || (num_m % 2 == 0 && (pairs > 2 * clusters || 4 * pairs >= 5 * clusters))) return launch_gemm_pair(d, a, 256, stream);
+      const bool general = (gemm_epilogue_features(a) & kEpiRagged) != 0, many = pairs > 2 * clusters, enough = 2 * pairs >= 3 * clusters;
+      if (general ? num_m % 2 == 0 && ((many && d->K > 512) || (enough && d->K > 1024)) : pairs <= clusters || (num_m % 2 == 0 && (many || enough)))
+        return launch_gemm_pair(d, a, 256, stream);
     }
     CUtensorMap ta, tb;
     bool ok;

@@ -545,3 +545,11 @@ def test_wide_outputs_of_few_rows(M, N, K, epilogue):
     assert ((outs[0].double() - want).abs() <= 2 ** -8 * want.abs() + K ** 0.5 * 2 ** -22 * size).all()
     assert torch.equal(*outs)
     assert ops.check_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 38150, 520), (256, 38150, 512), (130, 28500, 1032), (130, 28500, 1024), (130, 28300, 1032), (512, 14336, 64), (512, 13824, 64),
+                                   (400, 14273, 64)])
+@pytest.mark.parametrize("epilogue", ["plain", "residual"])
+def test_wide_outputs_beyond_one_wave_of_pairs(M, N, K, epilogue):
+    """Either side of the lines between 256 columns of one CTA and CTA pairs: widths of whole tiles and others, one and a half waves and two."""
+    test_wide_outputs_of_few_rows(M, N, K, epilogue)
