@@ -184,11 +184,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         mbar_expect_tx(&full_bar[i], S::kStageBytes);
         tma_load_2d(smem + i * S::kStageBytes, &tmap_w, &full_bar[i], (kb0 + i) * BK, n0);
       }
-      if (p.early) {
-        // what the ring does not hold yet waits in L2
-        for (int i = first; i < n_kb; ++i) tma_prefetch_2d(&tmap_w, (kb0 + i) * BK, n0);
-        pdl_wait();
-      }
+      // (Fetching the rest of the weights into L2 meanwhile gained nothing between the kernels of a step, and took traffic from the product that
+      // was still running: 32000 x 2048, 8 rows, back to back 22.4 us without, 26.9 with it; 6944 x 5120, 256 rows 30.2, 42.3.)
+      if (p.early) pdl_wait();
       for (int i = 0; i < first; ++i)
         tma_load_2d(smem + i * S::kStageBytes + S::kWBytes, &tmap_x, &full_bar[i], (kb0 + i) * BK, m0);
       int stage = 0;
@@ -303,8 +301,7 @@ static int skinny_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 // with programmatic launch / the tiled kernel): 1024 x 1024, 4 rows
 // 3.6 / 8.4, 256 rows 7.2 / 9.3, 512 rows 7.5 / 9.3; 4096 x 1024, 64 rows 6.0 / 8.6; 1024 x 4096, 4 rows 5.4 / 22.8; 32000 x
 // 1024, 33 rows 13.9 / 20.3.  Beyond one wave (32000 x 1024 with 128 rows: 25 us against 19) the tiled kernel is the better one; up to 32 rows
-// two waves are no slower (51865 x 1280, six matrices in turn, 4 rows 28.8 / 31.9, 17 rows 30.7 / 30.2, 20 rows 30.7 / 32.0, 28 rows 30.9 / 31.4,
-// 32 rows 31.3 / 31.8; 48 rows 31.2 / 31.3).
+// two waves are no slower (51865 x 1280, four matrices in turn, 1 row 24.0 / 32.2, 8 rows 26.6 / 31.8, 32 rows 27.5 / 31.8).
 bool skinny_takes(const GemmDesc* d, int sms) {
   const long tiles = static_cast<long>((d->N + kSkinnyFeat - 1) / kSkinnyFeat) * ((d->M + skinny_rows(d->M) - 1) / skinny_rows(d->M));
   return d->allow_split_k && d->M <= 512 && tiles <= (d->M <= 32 ? 4L : 2L) * sms && !d->out_fp32 && !d->a_mn_major && !d->b_mn_major && !d->gather && !d->preact && !d->mask &&
