@@ -57,7 +57,7 @@ __device__ __forceinline__ Item get_item(const AttnArgs& p, int item, bool repor
 // 100 words x 16 heads, two groups (157 KB of code) / four (39): without dropout 40.3 / 26.2 us, with it 50.9 / 32.3.
 constexpr int kFwdSlotBytes = 3 * kTileBytes;
 constexpr int fwd_short_threads(int groups) { return groups * 128 + 64; }   // softmax groups, TMA producer warp, MMA warp
-constexpr int fwd_short_smem(int groups) { return groups * kFwdSlotBytes + 512 + 1024; }
+constexpr int fwd_short_smem(int groups) { return groups * kFwdSlotBytes + 512 + 1024 > kOwnSm ? groups * kFwdSlotBytes + 512 + 1024 : kOwnSm; }
 
 // Up to 64 queries leave two of a group's four warps without work, and a warp's number decides both its rows (TMEM lanes) and its
 // scheduler: odd groups take such items in rows 64 .. 127 (the tile starts 64 rows early; a load may start before the matrix).

@@ -579,7 +579,7 @@ const char* nmtg_layernorm_fwd(const void* x, const void* gamma, const void* bet
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = step_overlap() || launch_overlap() ? 1 : 0;
+    cfg.numAttrs = step_overlap() || overlaps(grid / 4, 0) ? 1 : 0;      // blocks of four rows: four crowd an SM as little as one of sixteen warps
     auto kern = step_overlap() ? ln_fwd_kernel<decltype(vpl)::value, true> : ln_fwd_kernel<decltype(vpl)::value>;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, reinterpret_cast<const __nv_bfloat16*>(x),
                                        reinterpret_cast<const __nv_bfloat16*>(gamma), reinterpret_cast<const __nv_bfloat16*>(beta),
@@ -609,7 +609,7 @@ template <int VPL, int kWarps, int kStages>
 static const char* launch_ln_bwd_stream(const void* dy, const void* x, const float* mean, const float* rstd, const void* gamma, const void* dres,
                                         void* dx, float* dgamma, float* dbeta, int rows, int hidden, cudaStream_t stream) {
   static_assert(kStages >= 2, "the warps' sums take the place of two stages");
-  const size_t smem = static_cast<size_t>(kWarps) * kStages * 3 * hidden * sizeof(__nv_bfloat16);
+  const size_t ring = static_cast<size_t>(kWarps) * kStages * 3 * hidden * sizeof(__nv_bfloat16), smem = ring > kOwnSm ? ring : kOwnSm;
   auto kern = ln_bwd_stream_kernel<VPL, kWarps, kStages>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return cudaGetErrorString(e);
