@@ -370,7 +370,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (tracing) { e_last = clock64(); e_wait += e_last - e0; }
       tc_fence_after_sync();
       const bool row_ok = m0 + q * 32 + lane < p.M;
-      const int row = m0 + q * 32 + lane + (kSumsInParts<kFeat> && p.part_rows ? kb_begin / kb_per_split * p.part_rows : 0);
+      const int row = m0 + q * 32 + lane + ((kFeat & kEpiParts) ? kb_begin / kb_per_split * p.part_rows : 0);
       if ((kFeat & kEpiBf16) && p.tma_store) {
         // 64-column groups: both 32-column halves go to this warp's staging tile, one TMA store per group writes
         // full 128-byte lines (rows / columns outside the matrix are clipped by the copy engine)
@@ -603,8 +603,8 @@ const char* launch_gemm_pair(const GemmDesc* d, const GemmArgs& a, int bn, cudaS
   // (GELU / SiLU feed-forward blocks, in speech and pretrained-decoder models, keep the pre-activation instead of sign bits)
   const int grid = clusters * 2;
   if ((need & ~kPlain) == 0) return launch_pair<256, false, kPlain>(ta, tb, tc, tc, args, grid, stream, g);
+  if (args.part_rows) return launch_pair<256, false, kAccum | kEpiRagged | kEpiParts>(ta, tb, tc, tc, args, grid, stream, g);
   if ((need & ~kAccum) == 0) return launch_pair<256, false, kAccum>(ta, tb, tc, tc, args, grid, stream, g);
-  if (args.part_rows) return launch_pair<256, false, kAccum | kEpiRagged>(ta, tb, tc, tc, args, grid, stream, g);
   if ((need & ~kDgradMask) == 0) return launch_pair<256, false, kDgradMask>(ta, tb, tc, tc, args, grid, stream, g);
   if ((need & ~kOutRes) == 0) return launch_pair<256, false, kOutRes>(ta, tb, tc, tc, args, grid, stream, g);
   if ((need & ~kFc1) == 0) return launch_pair<256, false, kFc1>(ta, tb, tc, tc, args, grid, stream, g);

@@ -39,7 +39,7 @@ struct GemmArgs {
   int tma_second;          // so does the pre-activation, and the aux operand comes in that way (see two_stagings)
   int ablate;              // profiling aid: 1 = read the accumulator but skip arithmetic and stores, 2 = skip the epilogue body,
                            // 3 (traced kernel only) = also skip the MMAs: operand streaming alone
-  int part_rows;           // > 0: part s of the sum over K is stored at row s * part_rows of the output, by itself (kernels with kSumsInParts)
+  int part_rows;           // > 0: part s of the sum over K is stored at row s * part_rows of the output, by itself (kernels with kEpiParts)
   long long* trace;        // profiling aid: when set, the CTA-pair kernel writes up to 16 cycle counters per cluster (see gemm2cta_tcgen05.cu)
 };
 
@@ -154,11 +154,8 @@ __device__ __forceinline__ Pair normal_cdf2(Pair x, Pair& bell) {
 constexpr uint32_t kEpiBias = 1u, kEpiPreact = 2u, kEpiActFwd = 4u, kEpiActBwd = 8u, kEpiMaskBwd = 16u, kEpiDrop = 32u,
                    kEpiMaskOut = 64u, kEpiRes = 128u, kEpiF32 = 256u, kEpiBf16 = 512u,
                    kEpiRagged = 1024u /* N not a multiple of 64, or unaligned operands: column chunks element by element */,
-                   kEpiColsum = 2048u /* column sums of the output */, kEpiAll = 4095u;
-
-// The plain fp32 kernels store the parts of a sum apart (GemmArgs::part_rows).  Not the general one, which would spill more registers.
-template <uint32_t kFeat>
-constexpr bool kSumsInParts = (kFeat & ~kEpiRagged) == kEpiF32;
+                   kEpiColsum = 2048u /* column sums of the output */, kEpiAll = 4095u,
+                   kEpiParts = 4096u /* GemmArgs::part_rows; in kernels of its own */;
 
 // Features a problem needs (host side).
 inline uint32_t gemm_epilogue_features(const GemmArgs& a) {
@@ -358,7 +355,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmArgs& p, const Dro
     if ((kFeat & kEpiF32) && (p.out_fp32 || !(kFeat & kEpiBf16))) {
       float* op = reinterpret_cast<float*>(p.out) + static_cast<size_t>(row) * p.ld_out + col0;
       // accumulation into an existing fp32 buffer goes through the L2 reduction unit as well: no read round trip
-      if ((p.split_k > 1 && !(kSumsInParts<kFeat> && p.part_rows)) || p.accumulate || p.stream_k) {
+      if ((p.split_k > 1 && !(kFeat & kEpiParts)) || p.accumulate || p.stream_k) {
         if (full_cols) {
 #pragma unroll
           for (int g = 0; g < 8; ++g)

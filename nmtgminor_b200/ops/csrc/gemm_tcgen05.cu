@@ -193,7 +193,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_word, p.status, kTimeoutTmemFull)) break;
       tc_fence_after_sync();
       const bool row_ok = m0 + q * 32 + lane < p.M;
-      const int row = m0 + q * 32 + lane + (kSumsInParts<kFeat> && p.part_rows ? tile / (num_m * num_n) * p.part_rows : 0);
+      const int row = m0 + q * 32 + lane + ((kFeat & kEpiParts) ? tile / (num_m * num_n) * p.part_rows : 0);
 #pragma unroll 1
       for (int c = chunk_par; c < BN / 32; c += kEpilogueWarps / 4) {
         const int col0 = n0 + c * 32;
@@ -552,10 +552,8 @@ static const char* launch_gemm_single(const GemmDesc* d, const GemmArgs& a, int 
   const long tiles = static_cast<long>((d->M + BM - 1) / BM) * ((d->N + bn - 1) / bn) * a.split_k;
   const int grid = static_cast<int>(tiles < sms ? tiles : sms);
   if (a.part_rows) {
-    const bool ragged = d->N % 64 != 0;
-    if (bn == 256) return ragged ? launch_gemm<256, kEpiF32 | kEpiRagged>(ta, tb, a, grid, stream) : launch_gemm<256, kEpiF32>(ta, tb, a, grid, stream);
-    if (bn == 128) return ragged ? launch_gemm<128, kEpiF32 | kEpiRagged>(ta, tb, a, grid, stream) : launch_gemm<128, kEpiF32>(ta, tb, a, grid, stream);
-    return ragged ? launch_gemm<64, kEpiF32 | kEpiRagged>(ta, tb, a, grid, stream) : launch_gemm<64, kEpiF32>(ta, tb, a, grid, stream);
+    constexpr uint32_t kParts = kEpiF32 | kEpiRagged | kEpiParts;
+    return bn == 256 ? launch_gemm<256, kParts>(ta, tb, a, grid, stream) : bn == 128 ? launch_gemm<128, kParts>(ta, tb, a, grid, stream) : launch_gemm<64, kParts>(ta, tb, a, grid, stream);
   }
   if (bn == 256) return launch_gemm<256>(ta, tb, a, grid, stream);
   if (bn == 64) return launch_gemm_special<64>(ta, tb, a, grid, b200::g_pair_generic_epilogue != 0, stream);
