@@ -17,7 +17,6 @@ namespace b200 {
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-
 // ---------------------------------------------------------------------------------------------
 // status word written by kernels (0 = ok)
 // ---------------------------------------------------------------------------------------------
@@ -185,6 +184,13 @@ __device__ __forceinline__ T uniform(T v) { return __shfl_sync(0xffffffffu, v, 0
 // the same answer for all lanes
 template <bool kWarp = true>
 __device__ __forceinline__ bool all_lanes(bool v) { return kWarp ? __all_sync(0xffffffffu, v) != 0 : v; }
+
+// m16n8k16 of a warp, operands in registers: for the few rows of a decoding step (a tcgen05 tile has 128)
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 
 // D[tmem] (+)= A[smem] * B[smem]; one thread issues.  accumulate = 0 overwrites D.
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,

@@ -58,7 +58,6 @@ const unsigned long long* seed_ptr(const Tensor& like) {
 }
 Tensor get_seed_tensor(int64_t device) { return seed_tensor(static_cast<int>(device)); }
 
-// C[M,N] = epilogue(alpha * A B^T) ; see GemmDesc
 // [residual +] act([LayerNorm](x) W^T + bias) of a decoding step, or nothing where the kernel does not take these operands.
 std::optional<Tensor> step_linear(const Tensor& x, const OptTensor& gamma, const OptTensor& beta, double eps, const Tensor& w, const OptTensor& bias,
                                   const OptTensor& residual, int64_t act) {
@@ -86,6 +85,7 @@ std::optional<Tensor> step_linear(const Tensor& x, const OptTensor& gamma, const
   return out;
 }
 
+// C[M,N] = epilogue(alpha * A B^T) ; see GemmDesc
 void gemm(const Tensor& a, bool a_mn_major, const Tensor& b, bool b_mn_major, Tensor& out, const OptTensor& bias,
           const OptTensor& residual, const OptTensor& aux, const OptTensor& preact, int64_t act, double dropout_p,
           int64_t seed, int64_t stream_id, double alpha, bool accumulate, bool allow_split_k, int64_t split_k,

@@ -25,8 +25,6 @@ bool step_overlap();
 
 namespace {
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... A, typename... P>
 const char* launch(void (*kernel)(A...), dim3 grid, dim3 block, size_t smem, int cluster_z, cudaStream_t stream, P... args) {
@@ -82,11 +80,6 @@ constexpr int kStepWarps = 8;        // at most
 constexpr int kQueries = 8;          // to a CTA
 constexpr int kRowLd = 68;           // 64 dimensions, maximum, sum, padding
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ uint32_t transpose8(uint32_t x) {
   uint32_t y;
   asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
@@ -265,8 +258,8 @@ decode_self_kernel(const __nv_bfloat16* __restrict__ qkv, long ld, __nv_bfloat16
   const int queries = min(per, K - k0);
   const int hid = heads * 64;
   const int g = lane >> 2, t = lane & 3;
-  pdl_trigger();
-  if (!early) pdl_wait();
+  let_next_start();
+  if (!early) wait_for_previous();
   const long pos_l = pos_rows[r0];                     // the same for all hypotheses of a sentence
   const int pos = pos_l < 0 ? 0 : (pos_l >= cap ? cap - 1 : static_cast<int>(pos_l));
   WarpTile tile;
@@ -299,7 +292,7 @@ decode_self_kernel(const __nv_bfloat16* __restrict__ qkv, long ld, __nv_bfloat16
             prefetch_l2(vc + e);
           }
     if (c0 == 0) {
-      if (early) pdl_wait();
+      if (early) wait_for_previous();
       tile.init(qkv + r0 * ld + h * 64, ld, queries, lane);
     }
     for (int blk = warp; blk < kPast / 16 && c0 + blk * 16 <= pos; blk += warps) {
@@ -402,8 +395,8 @@ decode_cross_kernel(const __nv_bfloat16* __restrict__ q, long ld, const __nv_bfl
   const int share = blockIdx.z;
   const int hid = heads * 64;
   const int g = lane >> 2, t = lane & 3;
-  pdl_trigger();
-  if (!early) pdl_wait();
+  let_next_start();
+  if (!early) wait_for_previous();
   int len = lengths[b];
   len = len < 0 ? 0 : (len > cap ? cap : len);
   const int chunk = ((len + splits - 1) / splits + 15) & ~15;
@@ -439,7 +432,7 @@ decode_cross_kernel(const __nv_bfloat16* __restrict__ q, long ld, const __nv_bfl
       prefetch_l2(ck + at);
       prefetch_l2(cv + at);
     }
-    pdl_wait();
+    wait_for_previous();
   }
   WarpTile tile;
   tile.init(q + (static_cast<long>(b) * K + k0) * ld + h * 64, ld, queries, lane);
@@ -562,14 +555,14 @@ beam_part_kernel(const T* __restrict__ logits, long ld, const uint8_t* __restric
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kPartThreads / 32;
   const int r = first + blockIdx.y, piece = blockIdx.x;
   const int c0 = piece * kPartCols;
-  pdl_trigger();
+  let_next_start();
   const T* x = logits + static_cast<long>(r) * ld + c0;
   constexpr int kPer = 16 / sizeof(T);
   // kWarm: once over no columns, storing nothing, before the wait; a step runs these instructions once, and fetching them took longer than
   // running them (4 rows of 32000 in a search 6.6 us, 4.3 so; not where the blocks are several waves: 256 rows 13.5 and 16.5)
 #pragma unroll 1
   for (int pass = kWarm ? 0 : 1; pass < 2; ++pass) {
-    if (pass == 1) pdl_wait();
+    if (pass == 1) wait_for_previous();
     const int cols = pass == 1 ? min(kPartCols, V - c0) : 0;
     float f[kPartEach];
     int col[kPartEach / kPer];
@@ -701,8 +694,8 @@ beam_advance_kernel(const NmtgBeam s, const void* logits, int bf16, long ld, con
   int* plain = f_row + K;                                    // [K] the hypothesis is searched (not dead, not bound to end)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int b = blockIdx.x;
-  pdl_trigger();
-  pdl_wait();
+  let_next_start();
+  wait_for_previous();
   const int step = static_cast<int>(s.pos_rows[b * K]);
   const int T = s.ctl[0], min_len = s.ctl[1], normalize = s.ctl[2];
   const int count0 = s.fin_count[b], done0 = s.done[b], limit = s.max_rows[b];

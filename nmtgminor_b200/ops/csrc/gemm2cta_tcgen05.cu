@@ -7,10 +7,10 @@
 //   rank 1         : TMA producer for its operand halves       + epilogue of rows [m0 + 128, m0 + 256)
 //
 // Synchronisation (all mbarriers live in shared memory; remote ones are addressed through the cluster
-// window, no broadcast forms are used anywhere):
+// window; loads are never broadcast, only the leader's commits arrive at both CTAs):
 //   full[s]       on the leader, count 1 + 2 x stage bytes: both CTAs' TMA loads complete_tx on it
-//   empty[s]      on each CTA, signalled by two tcgen05.commit of the leader (local + peer address)
-//   tmem_full[a]  on each CTA, same two-commit scheme after the last k-block of a tile
+//   empty[s]      on each CTA, signalled by one tcgen05.commit of the leader that arrives at both
+//   tmem_full[a]  on each CTA, the same after the last k-block of a tile
 //   tmem_empty[a] on the leader, count 2 x 256: every epilogue thread of both CTAs arrives (peer: remote arrive)
 // Every wait is bounded; all exits go through the final cluster barrier so a CTA never leaves while its peer
 // may still touch its shared memory.
@@ -226,7 +226,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   } else if (warp == 1) {
     // ------------------------------- UMMA issuer (leader only) -------------------------------
     // All lanes, see elect_one; one lane for weight gradients, whose partial tiles then meet in the output less often at the same time
-    // (5120 x 1280 over 1800 rows: 32 us so, 35.5 with all lanes; 8192 rows 59 both ways)
+    // (us, one lane / all: 5120 x 1280 over 1800 rows 31 / 34, 5120 x 2048 over 2304 45 / 53, 4096 x 4096 over 1934 66 / 80; 8192 rows the same)
     constexpr bool kWarp = kFeat != kEpiF32;
     if (leader && (kWarp || lane == 0)) {
       const uint32_t idesc = make_idesc_bf16(2 * BM, BN, p.a_mn_major, p.b_mn_major);

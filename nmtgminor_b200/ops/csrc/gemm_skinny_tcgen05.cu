@@ -49,8 +49,6 @@ struct SkinnyArgs {
   int* status;
 };
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
   uint32_t remote;
@@ -173,20 +171,20 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
+  let_next_start();
 
   if (warp == 4) {
     if (lane == 0) {
       const int n_kb = kb1 - kb0;
       const int first = n_kb < S::kStages ? n_kb : S::kStages;
-      if (!p.early) pdl_wait();
+      if (!p.early) wait_for_previous();
       for (int i = 0; i < first; ++i) {
         mbar_expect_tx(&full_bar[i], S::kStageBytes);
         tma_load_2d(smem + i * S::kStageBytes, &tmap_w, &full_bar[i], (kb0 + i) * BK, n0);
       }
       // (Fetching the rest of the weights into L2 meanwhile gained nothing between the kernels of a step, and took traffic from the product that
       // was still running: 32000 x 2048, 8 rows, back to back 22.4 us without, 26.9 with it; 6944 x 5120, 256 rows 30.2, 42.3.)
-      if (p.early) pdl_wait();
+      if (p.early) wait_for_previous();
       for (int i = 0; i < first; ++i)
         tma_load_2d(smem + i * S::kStageBytes + S::kWBytes, &tmap_x, &full_bar[i], (kb0 + i) * BK, m0);
       int stage = 0;
@@ -222,7 +220,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
     if (ok && elect_one()) umma_commit(done_bar);
   } else {
-    pdl_wait();        // the residual is an earlier kernel's output, and so may be the buffer that is written
+    wait_for_previous();        // the residual is an earlier kernel's output, and so may be the buffer that is written
     const bool ok = mbar_wait(done_bar, 0, abort_word, p.status, kTimeoutTmemFull);
     if (ok) {
       tc_fence_after_sync();

@@ -24,15 +24,8 @@ int num_sms();
 
 namespace {
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ float row_sum(float v) {
 #pragma unroll
@@ -130,7 +123,7 @@ step_linear_kernel(const StepArgs p) {
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem);                          // [8 kRows8][ld], staged rows
   __nv_bfloat16* affine = xs + (kDirect ? 0 : kRows8 * 8 * ld);                          // [2][ld] gamma, beta
   float* red = reinterpret_cast<float*>(smem);                                           // [kWarps][8 kRows8][kF], over the rows
-  pdl_trigger();
+  let_next_start();
   uint4 w[kChunks][kTiles];
 #pragma unroll
   for (int i = 0; i < kChunks; ++i)
@@ -154,7 +147,7 @@ step_linear_kernel(const StepArgs p) {
       }
     __syncthreads();
   }
-  pdl_wait();
+  wait_for_previous();
   // ---- from here on: what the kernel before wrote
   uint4 xd[kDirect ? kChunks : 1];
   if constexpr (kDirect) {
