@@ -13,10 +13,12 @@
 //           two Q/K/V/dO slots; P and dS are staged once in shared memory and consumed K-major (dQ = dS K) and MN-major
 //           (dV = P^T dO, dK = dS^T Q).
 // MMA reduction lengths are trimmed to the real sequence lengths (multiples of 16).
-// What bounds these kernels is the fetching of instructions: all roles run at once, each in code of its own, and the SMs of a GPC share
-// what their own caches cannot hold (CTAs on a GPC with fewer of them ran 1.4 times as fast).  So a loop body is there once: one 32-column
-// chunk a turn, dropout a template argument, MMA steps and gradient matrices in loops that are not unrolled.  The backward pass went from
-// 157 KB and 83.6 us (136 sentences of 20 to 100 words x 16 heads, dropout) to 70 KB and 67.1; unrolling its MMA steps alone cost 12 us.
+// The fetching of instructions bound these kernels when each had 157 KB of code: all roles run at once, each in code of its own, and the SMs
+// of a GPC share what their own caches cannot hold (CTAs on a GPC with fewer of them ran 1.4 times as fast).  So a loop body is there once: one
+// 32-column chunk a turn, dropout a template argument, MMA steps and gradient matrices in loops that are not unrolled (unrolling the
+// backward pass's MMA steps alone cost 12 us).  With 39 and 70 KB a scheduler waits 0.5 cycles an instruction for the next one and 5 to 9 for
+// tensor memory, barriers and loads: the chain of an item.  135 sentences of 20 to 100 words x 16 heads, us back to back, 157 KB / now:
+// forward 38.8 / 22.6, with dropout 49.9 / 29.7, backward 74.4 / 61.0, with dropout 83.8 / 66.7.
 // Same numerics, dropout counters and interfaces as the general kernels in attention_tcgen05.cu.
 #include "attention_common.cuh"
 #include "bounds_check.cuh"
@@ -53,8 +55,8 @@ __device__ __forceinline__ Item get_item(const AttnArgs& p, int item, bool repor
 // Four items are in flight, each in a slot and with a softmax group of its own: an item is a chain of waits (S, two passes over it, P,
 // O, about 5500 cycles for 60 keys with dropout) that one or two warps of a scheduler cannot fill.  To fit, P overwrites the Q and K
 // tiles (S = Q K^T is complete when a group starts) and O the columns of S.  Only the producer looks items up: the look-up is a
-// round trip to memory, and in the MMA warp it took 1300 of the 3260 cycles that an item took with two groups.  136 sentences of 20 to
-// 100 words x 16 heads, two groups (157 KB of code) / four (39): without dropout 40.3 / 26.2 us, with it 50.9 / 32.3.
+// round trip to memory, and in the MMA warp it took 1300 of the 3260 cycles that an item took with two groups.  Two groups took
+// 38.8 us where four take 22.6, with dropout 49.9 and 29.7 (figures above).
 constexpr int kFwdSlotBytes = 3 * kTileBytes;
 constexpr int fwd_short_threads(int groups) { return groups * 128 + 64; }   // softmax groups, TMA producer warp, MMA warp
 constexpr int fwd_short_smem(int groups) { return groups * kFwdSlotBytes + 512 + 1024 > kOwnSm ? groups * kFwdSlotBytes + 512 + 1024 : kOwnSm; }

@@ -67,7 +67,7 @@ __device__ __forceinline__ float exp_diff(float a, float b) { return a == -INFIN
 // ---------------------------------------------------------------------------------------------------------------------
 // Attention of one new position.  Both kernels serve the hypotheses of a sentence, up to eight, from one CTA (head, sentence), whose
 // warps take blocks of 16 keys.  The products run on the tensor cores (m16n8k16): with dot products, folds and weights in ordinary
-// instructions a block cost 560 of them, about 150 this way, and attention over 1500 frames was bound by that.  tcgen05 would want
+// instructions a block cost 560 of them, about 180 this way, and attention over 1500 frames was bound by that.  tcgen05 would want
 // 128 rows; here the keys are the 16 rows of the first product, the dimensions those of the second, and the queries the 8 columns.
 //   * The weights of the softmax are 32-bit numbers, and the product with the values takes 16-bit ones: it runs three times, with
 //     the weights' rounding to bf16, the rounding of the rest, and the rest of that, which add up to all 24 bits.
@@ -239,8 +239,9 @@ __device__ __forceinline__ void merge_rows(const float* rows, int n, int query, 
 // of the tile keeps those of its own query, and the softmax is again one for all.  The loads of four hypotheses are in flight together;
 // one after the other they had a warp wait for memory four times a block.  Within a search step (`early`) the ancestors, and what
 // the caches hold of earlier positions, come from earlier steps, and a step begins with a launch that waits for all before it: they
-// are staged, and the keys and values fetched into L2, while the projection before this kernel still runs.  In a search (us a layer,
-// before / after): one sentence 10.9 / 6.4, 64 sentences x 4 hypotheses 28.5 / 24.8, 8 x 4 with 20 heads 10.4 / 7.1.
+// are staged, and the keys and values fetched into L2, while the projection before this kernel still runs.  Back to back (us, dot
+// products in ordinary instructions / this): 64 sentences x 4 hypotheses x 16 heads, 80 words 23.4 / 20.3; with the projection before it, one
+// sentence 10.3 / 8.6, 8 x 4 with 20 heads, 50 words 14.7 / 11.8.
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int kPast = 256;           // positions whose ancestors are staged at a time
 
@@ -378,8 +379,8 @@ decode_self_kernel(const __nv_bfloat16* __restrict__ qkv, long ld, __nv_bfloat16
 // encoder-decoder attention.  CTA = (head, sentence and group of hypotheses, share of the keys); the shares of a sentence are one
 // cluster and meet in distributed shared memory.  Within a search step (`early`) nothing that may still run writes the encoder's
 // keys, values and lengths: each warp loads its first block, and has the rest of its share fetched into L2, while the previous
-// kernels of the step run.  In a search (us a layer, before / after): 8 sentences x 1500 frames x 20 heads 31.0 / 15.2 (62 MB: 9.9 at the
-// copy rate), 64 sentences of 60 words 11.5 / 8.1, one sentence 5.3 / 2.4.
+// kernels of the step run.  Back to back (us, dot products in ordinary instructions / this): 8 sentences x 1500 frames x 20 heads 22.9 / 13.9
+// (62 MB: 9.4 at the copy rate), 64 sentences of 60 words 7.5 / 5.9, one sentence 4.3 / 3.5.
 // ---------------------------------------------------------------------------------------------------------------------
 // (320 x 2 threads: 96 registers, so that five CTAs of four warps fit an SM; with 102 the 640 CTAs of 8 sentences are two waves, 19.3 us for 13.4)
 __global__ void __launch_bounds__(320, 2)
