@@ -553,3 +553,9 @@ def test_wide_outputs_of_few_rows(M, N, K, epilogue):
 def test_wide_outputs_beyond_one_wave_of_pairs(M, N, K, epilogue):
     """Either side of the lines between 256 columns of one CTA and CTA pairs: widths of whole tiles and others, one and a half waves and two."""
     test_wide_outputs_of_few_rows(M, N, K, epilogue)
+
+
+@pytest.mark.parametrize("M,N,K", [(30, 1024, 9000), (128, 4104, 5000), (400, 1000, 30011), (2304, 1024, 4160), (1, 8, 4096)])
+def test_long_sums_in_wide_tiles_and_pairs(M, N, K):
+    """Parts of 256 columns from one CTA and from pairs, ragged widths, and two parts as well as many."""
+    test_long_sums_of_small_outputs(M, N, K)
